@@ -217,19 +217,18 @@ typedef struct psim_day_stats {
     double expected_new_infections;    /* sum of infection probabilities since the last midnight */
 } psim_day_stats;
 
-/* Launch and algorithm choices of the per-step kernels, picked per device
+/* Launch and algorithm choices of the day and phase kernels, picked per device
  * and workload by the autotuner (pansim_gb300/autotune.py).  A new context
  * starts with agg_slot 0, blocks_per_sm 4, scan_items 4, scan_mode 3. */
 typedef struct psim_tuning {
     uint32_t agg_count;      /* no effect (the histogram is updated by movers only) */
     uint32_t agg_slot;       /* warp-aggregated agent-list slot atomics */
-    uint32_t blocks_per_sm;  /* 256-thread blocks per SM of the step kernel; 0 = occupancy */
-    uint32_t variant;        /* the day graph's step kernel (agent list rebuilt at the steps
-                                where agents took new locations, draws over the agents at
-                                locations with an infectious agent, decisions of the agents
-                                whose decision step it is): 3 = one launch per timestep,
-                                4 = one launch for the whole day with a grid barrier between
-                                timesteps (slower on GB300 at 2M and 20M agents) */
+    uint32_t blocks_per_sm;  /* the day kernel's blocks per SM in units of 256 threads; 0 = occupancy */
+    uint32_t variant;        /* 3 or 4, without a difference: the day graph runs one launch of
+                                the day kernel (agent list rebuilt at the steps where agents
+                                took new locations, draws over the agents at locations with an
+                                infectious agent, decisions of the agents whose decision step
+                                it is) */
     uint32_t scan_items;     /* locations per thread of the scan: 2, 4 or 8 (0 = 8) */
     uint32_t scan_mode;      /* 0 = single pass with decoupled look-back, 1 = tile sums + scan,
                                 2 = tile sums + scan with each thread owning consecutive
@@ -412,7 +411,7 @@ int psim_run_steps(psim_ctx* ctx, uint32_t day);
 /* One day: psim_midnight at t = day*steps_per_day, then psim_run_steps. */
 int psim_run_day(psim_ctx* ctx, uint32_t day, psim_day_stats* out /* [replicas] */);
 
-/* Sets the tuning of the per-step kernels (recaptures the day graph). */
+/* Sets the tuning of the day and phase kernels (recaptures the day graph). */
 int psim_set_tuning(psim_ctx* ctx, const psim_tuning* tuning);
 int psim_get_tuning(psim_ctx* ctx, psim_tuning* tuning);
 
@@ -446,14 +445,14 @@ int psim_set_tracking(psim_ctx* ctx, int expected);
 /* Location CSR (LocationsList::locationListOffsets / locationAgentList) of
  * the current positions.  With canonical != 0 each location's agents are
  * sorted by id, which equals thrust::stable_sort_by_key's output
- * (util.cpp:69).  After day graphs (whose step kernel keeps agent lists only
+ * (util.cpp:69).  After day graphs (whose day kernel keeps agent lists only
  * for the locations its draws visit) the full list is built first. */
 int psim_get_csr(psim_ctx* ctx, int canonical, uint32_t* offsets /*[L+1]*/, uint32_t* agents /*[N]*/);
 /* Per-location hazard r_l of the last psim_infect call (infectionRatios). */
 int psim_get_hazard(psim_ctx* ctx, float* out /*[L]*/, int64_t* fixed_sum /*[L] or NULL*/);
 
 /* Step t as the day graph runs it, after movement(t) with the sums afresh and
- * a rebuild of the agent list pending, with CUDA events around the step
+ * a rebuild of the agent list pending, with CUDA events around the day
  * kernel's three phases launched apart: the rebuild, the draws of t and the
  * queue + decisions of t + 1; ms[3] receives those three durations.  t and
  * t + 1 must lie in the same day. */
@@ -461,16 +460,16 @@ int psim_time_step_kernels(psim_ctx* ctx, uint32_t t, float* ms /* [3] */);
 /* Timing of the last psim_run_steps graph launch, milliseconds. */
 int psim_last_day_ms(psim_ctx* ctx, float* ms);
 /* With on != 0 the day graph is captured with timeline stamps in its kernels
- * (the global nanosecond timer at every block's entry, at the end of each
- * phase of the step kernel and at its exit; one atomic per block and stamp)
- * and counters.  For the last psim_run_steps: psim_day_kernel_ms gives ms[5]
- * = {the day's first movement kernel, the step kernel's rebuilds (listing +
- * agent-list slots), its draws, its queues + decisions, and the time between
- * the kernels}, summed over the day; psim_day_timeline gives per step
- * s, at us[7*s .. 7*s+6], {the kernel's span from its first block's entry to
- * its last block's exit, the rebuild's listing, its slots, the draws, the
- * queue, the decisions (0 when the phase did not run), the time since the
- * previous kernel's last exit}, microseconds;
+ * (the global nanosecond timer at every block's start of a segment of
+ * timesteps, at the end of each phase and of the segment; one atomic per
+ * block and stamp) and counters.  For the last psim_run_steps:
+ * psim_day_kernel_ms gives ms[5] = {the day's first movement kernel, the day
+ * kernel's rebuilds (listing + agent-list slots), its draws, its queues +
+ * decisions, and the time between its segments}, summed over the day;
+ * psim_day_timeline gives per step s, at us[7*s .. 7*s+6], {the step's span,
+ * the rebuild's listing, its slots, the draws (a segment's, divided among its
+ * steps), the queue, the decisions (0 when the phase did not run), the time
+ * since the previous segment's end}, microseconds;
  * psim_day_counts gives out[7] = {agent-list entries the draws expanded,
  * those at a location with a nonzero ratio, agents queued for a decision,
  * steps at which agents were queued, steps that rebuilt the agent list,

@@ -1,7 +1,7 @@
-"""Autotuner of the step kernel.
+"""Autotuner of the day kernel.
 
 Times each candidate tuning (warp aggregation of the agent-list slot
-atomics, resident blocks per SM of the persistent step kernel) on the live
+atomics, resident blocks per SM of the persistent day kernel) on the live
 workload: every candidate runs the same whole day (the day graph, all its
 steps) from the same checkpoint taken after that day's midnight phases,
 timed with CUDA events, and the fastest is kept.  Steps at different times
@@ -16,7 +16,7 @@ LARGE_AGENTS = 8_000_000
 
 
 def candidates(grid=None):
-    """blocks_per_sm 0 = as many as the step kernel's occupancy allows (the
+    """blocks_per_sm 0 = as many as the day kernel's occupancy allows (the
     library caps every value there: its grid barriers need every block
     resident)."""
     for agg_slot, bps in itertools.product([1, 0], grid or DEFAULT_GRID):

@@ -28,7 +28,7 @@ int check_device_err(psim_ctx* c) {
         if (e & ERR_TEST_WAIT) m += " bounded wait expired;";
         if (e & ERR_SCAN_WAIT) m += " scan tile wait expired;";
         if (e & ERR_AGENT_LIST) m += " agent list inconsistent;";
-        if (e & ERR_BARRIER) m += " step kernel grid barrier expired;";
+        if (e & ERR_BARRIER) m += " day kernel grid barrier expired;";
         return fail(c, PSIM_ERR_DEVICE, m);
     }
     return 0;
@@ -279,7 +279,6 @@ int upload_mutable(psim_ctx* c, const psim_agents* a, const psim_locations* l) {
 // (k_movement, k_count): the first step of each day and the regroups.
 int reset_sums(psim_ctx* c) {
     CK(cudaMemsetAsync(c->k.l.sfix, 0, sizeof(unsigned long long) * c->L * c->V, c->stream));
-    CK(cudaMemsetAsync(c->k.l.sfix_b, 0, sizeof(unsigned long long) * c->L * c->V, c->stream));
     CK(cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream));
     return 0;
 }
@@ -313,7 +312,7 @@ int do_step(psim_ctx* c, uint32_t step, bool draw, bool movement) {
     if (movement) {
         int rc = reset_sums(c);
         if (rc) return rc;
-        launch_movement(c->k, step, c->stream);
+        launch_movement(c->k, step, false, c->stream);
     }
     launch_scan(c->k, step, 1, merge_q, c->stream);
     launch_scatter_draw(c->k, step, 1, draw ? 1 : 0, c->stream);
@@ -328,7 +327,7 @@ int capture_day_graph(psim_ctx* c) {
         c->day_graph = nullptr;
     }
     cudaGraph_t g = nullptr;
-    // profiled: the step kernel's counters and timeline stamps (KArgs::prof)
+    // profiled: the day kernel's counters and timeline stamps (KArgs::prof)
     c->k.prof = c->profile ? c->d_prof : nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     // (the capture stays open until EndCapture: errors are checked after it)
@@ -336,29 +335,16 @@ int capture_day_graph(psim_ctx* c) {
     // agent list rebuilt (its slots take the susceptibilities the midnight
     // phases left), the mask of decision steps recomputed from every agent.
     cudaError_t me = cudaMemsetAsync(c->k.l.sfix, 0, sizeof(unsigned long long) * c->L * c->V, c->stream);
-    if (me == cudaSuccess) me = cudaMemsetAsync(c->k.l.sfix_b, 0, sizeof(unsigned long long) * c->L * c->V, c->stream);
     if (me == cudaSuccess)
         me = cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream);
     if (me == cudaSuccess) me = cudaMemsetAsync(c->k.a.move_mask, 0, sizeof(uint32_t) * MOVE_MASK_WORDS, c->stream);
     if (me == cudaSuccess) me = cudaMemsetAsync(c->k.l.build + 1, 0xFF, sizeof(uint32_t), c->stream);
     if (me == cudaSuccess) me = cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t) * BAR_WORDS, c->stream);
     if (me == cudaSuccess && c->profile) me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
-    launch_movement(c->k, 0, c->stream);
-    // Per timestep one launch of the step kernel (rebuild, draws, decisions
-    // for the next timestep, grid barriers between its phases), or with
-    // tuning variant 4 one launch for the whole day with a grid barrier
-    // between timesteps (measured slower on GB300: a barrier takes longer than
-    // the gap between two kernel nodes of the graph); the profiled graph is
-    // the same launches with the kernel's timeline stamps.
-    if (c->k.tune.variant == 4)
-        launch_steps(c->k, 0, c->spd, PH_ALL, c->stream);
-    else
-        for (uint32_t s = 0; s < c->spd; ++s) launch_step(c->k, s, PH_ALL, c->stream);
-    // the day's final sums are in the copy its next step would read: with an
-    // odd number of steps that is the second one
-    if (me == cudaSuccess && (c->spd & 1u))
-        me = cudaMemcpyAsync(c->k.l.sfix, c->k.l.sfix_b, sizeof(unsigned long long) * c->L * c->V,
-                             cudaMemcpyDeviceToDevice, c->stream);
+    launch_movement(c->k, 0, true, c->stream);
+    // one launch of the day kernel for all timesteps; the profiled graph is
+    // the same launch with the kernel's timeline stamps
+    launch_day(c->k, 0, c->spd, PH_ALL, c->stream);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e == cudaSuccess && me != cudaSuccess) {
         cudaGraphDestroy(g);
@@ -368,8 +354,7 @@ int capture_day_graph(psim_ctx* c) {
     e = cudaGraphInstantiate(&c->day_graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(c, PSIM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    // movement(0) and the step kernel launches
-    c->graph_kernels = 1 + (c->k.tune.variant == 4 ? 1ull : (uint64_t)c->spd);
+    c->graph_kernels = 2;  // movement(0) and the day kernel
     c->graph_dirty = false;
     c->prof_valid = false;
     return 0;
@@ -640,8 +625,8 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     }
 #define AL(field, cnt) \
     if ((rc = dalloc(c, &da.field, cnt))) return bail(rc);
-    AL(hcw, N) AL(rank, N) AL(home, N)
-    AL(worklist, (size_t)N + (size_t)WORK_MAX_BLOCKS * 1024 + 4)
+    AL(hcw, N) AL(rank, N) AL(home, N) AL(dinfo, N)
+    AL(worklist, (size_t)N + (size_t)WORK_MAX_THREADS * 4 + 4)
     AL(move_mask, MOVE_MASK_WORDS)
 #undef AL
     // locations
@@ -660,11 +645,11 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     if ((rc = dalloc(c, &dl.cursor, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.csr_agents, N))) return bail(rc);
     if ((rc = dalloc(c, &dl.slot_loc, N))) return bail(rc);
-    if ((rc = dalloc(c, &dl.inf_pending, 3 * N))) return bail(rc);
+    if ((rc = dalloc(c, &dl.replay_stamp, L))) return bail(rc);
+    if ((rc = dalloc(c, &dl.replay_list, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.slot_su, N * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.qu_pending, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.sfix, L * V))) return bail(rc);
-    if ((rc = dalloc(c, &dl.sfix_b, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hazard, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hazard_x, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hmask, ((size_t)L + 2047) / 2048 * 64 + 64))) return bail(rc);
@@ -894,7 +879,7 @@ int psim_set_tuning(psim_ctx* c, const psim_tuning* t) {
     c->k.tune.agg_slot = t->agg_slot ? 1u : 0u;
     c->k.tune.blocks_per_sm = t->blocks_per_sm;
     if (t->variant != 3 && t->variant != 4)
-        return fail(c, PSIM_ERR_ARG, "variant must be 3 (a launch per timestep) or 4 (a launch per day)");
+        return fail(c, PSIM_ERR_ARG, "variant must be 3 or 4");
     c->k.tune.variant = t->variant;
     if (t->scan_items != 0 && t->scan_items != 2 && t->scan_items != 4 && t->scan_items != 8)
         return fail(c, PSIM_ERR_ARG, "scan_items must be 2, 4 or 8");
@@ -1038,7 +1023,7 @@ int psim_movement(psim_ctx* c, uint32_t t) {
     int rc = set_clock(c, t);
     if (rc) return rc;
     if ((rc = reset_sums(c))) return rc;
-    launch_movement(c->k, t % c->spd, c->stream);
+    launch_movement(c->k, t % c->spd, false, c->stream);
     c->launches += 1;
     c->csr_fresh = true;
     c->t_next = t + 1;
@@ -1247,10 +1232,10 @@ int psim_run_day(psim_ctx* c, uint32_t day, psim_day_stats* out) {
 int psim_get_csr(psim_ctx* c, int canonical, uint32_t* offsets, uint32_t* agents) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     if (c->list_sparse) {
-        // the step kernel lists only the locations its draws visit: the full
+        // the day kernel lists only the locations its draws visit: the full
         // agent list of the current positions (prefix of the histogram,
-        // slots), which no later step reads (the day graph's and the step
-        // kernel's first step rebuild)
+        // slots), which no later step reads (the day graph's first
+        // step rebuilds)
         int rc = force_rebuild(c);
         if (rc) return rc;
         launch_scan(c->k, 0, 0, 0, c->stream);
@@ -1314,23 +1299,44 @@ static int read_timeline(psim_ctx* c, std::vector<unsigned long long>& h) {
 }
 
 // Per step of the profiled day, in microseconds (TL_COLS values): the
-// kernel's span (first block entry to last block exit), the rebuild's
-// listing, its slots, the draws, the queue, the decisions (0 where the phase
-// did not run), and the time from the previous kernel's last exit to this
-// kernel's first entry.
+// step's span, the rebuild's listing, its slots, the draws, the queue, the
+// decisions (0 where the phase did not run), and the time since the previous
+// segment's last exit.  The day kernel draws a segment's timesteps together:
+// their time (with the replay's) is divided among them; the rebuild and the
+// gap belong to the segment's first step, the queue and the decisions to its
+// last one, the step before the one they decide for.
 constexpr int TL_COLS = 7;
-static void step_times(psim_ctx* c, const std::vector<unsigned long long>& h, uint32_t s, float* o) {
-    const unsigned long long* T = &h[PROF_T + PROF_TW * (size_t)s];
-    const unsigned long long t0 = ~T[0], r1 = T[1], r2 = T[2], drw = T[3], que = T[4], end = T[5];
-    const unsigned long long prev = s == 0 ? h[PROF_N + 1] : h[PROF_T + PROF_TW * (size_t)(s - 1) + 5];
-    auto us = [](unsigned long long a, unsigned long long b) { return b > a ? (float)((double)(b - a) * 1e-3) : 0.0f; };
-    o[0] = us(t0, end);
-    o[1] = r1 ? us(t0, r1) : 0.0f;
-    o[2] = r2 ? us(r1, r2) : 0.0f;
-    o[3] = us(r2 ? r2 : t0, drw);
-    o[4] = que ? us(drw, que) : 0.0f;
-    o[5] = que ? us(que, end) : 0.0f;
-    o[6] = us(prev, t0);
+static void step_times(psim_ctx* c, const std::vector<unsigned long long>& h, float* us) {
+    auto dur = [](unsigned long long a, unsigned long long b) { return b > a ? (float)((double)(b - a) * 1e-3) : 0.0f; };
+    unsigned long long prev = h[PROF_N + 1];
+    uint32_t s = 0;
+    while (s < c->spd) {
+        const unsigned long long* T = &h[PROF_T + PROF_TW * (size_t)s];
+        uint32_t e = s + 1;
+        while (e < c->spd && h[PROF_T + PROF_TW * (size_t)e] == 0ull) ++e;
+        const unsigned long long t0 = ~T[0], lst = T[1], slt = T[2], drw = T[3], que = T[4], rep = T[5], end = T[6];
+        const unsigned long long qd = que ? que : drw;
+        float draw = dur(slt ? slt : t0, drw);
+        if (rep) draw += dur(qd, rep);
+        if (!que) draw += dur(rep ? rep : drw, end);
+        for (uint32_t q = s; q < e; ++q) {
+            float* o = us + TL_COLS * (size_t)q;
+            for (int j = 0; j < TL_COLS; ++j) o[j] = 0.0f;
+            o[3] = draw / (float)(e - s);
+            if (q == s) {
+                o[1] = lst ? dur(t0, lst) : 0.0f;
+                o[2] = slt ? dur(lst, slt) : 0.0f;
+                o[6] = dur(prev, t0);
+            }
+            if (q + 1 == e && que) {
+                o[4] = dur(drw, que);
+                o[5] = dur(rep ? rep : que, end);
+            }
+            o[0] = o[1] + o[2] + o[3] + o[4] + o[5];
+        }
+        prev = end;
+        s = e;
+    }
 }
 
 int psim_day_kernel_ms(psim_ctx* c, float* ms) {
@@ -1340,9 +1346,10 @@ int psim_day_kernel_ms(psim_ctx* c, float* ms) {
     if (rc) return rc;
     ms[0] = h[PROF_N + 1] > ~h[PROF_N] ? (float)((double)(h[PROF_N + 1] - ~h[PROF_N]) * 1e-6) : 0.0f;
     ms[1] = ms[2] = ms[3] = ms[4] = 0.f;
+    std::vector<float> us((size_t)TL_COLS * c->spd);
+    step_times(c, h, us.data());
     for (uint32_t s = 0; s < c->spd; ++s) {
-        float o[TL_COLS];
-        step_times(c, h, s, o);
+        const float* o = &us[TL_COLS * (size_t)s];
         ms[1] += (o[1] + o[2]) * 1e-3f;
         ms[2] += o[3] * 1e-3f;
         ms[3] += (o[4] + o[5]) * 1e-3f;
@@ -1356,7 +1363,7 @@ int psim_day_timeline(psim_ctx* c, float* us) {
     std::vector<unsigned long long> h;
     int rc = read_timeline(c, h);
     if (rc) return rc;
-    for (uint32_t s = 0; s < c->spd; ++s) step_times(c, h, s, us + TL_COLS * (size_t)s);
+    step_times(c, h, us);
     return 0;
 }
 
@@ -1398,26 +1405,22 @@ int psim_time_step_kernels(psim_ctx* c, uint32_t t, float* ms) {
     const uint32_t step = t % c->spd;
     // step t as the day graph runs it, from movement(t) with the sums afresh
     // and the agent list rebuilt: the rebuild, the draws, the queue +
-    // decisions of t + 1 (the step kernel's phases as separate launches);
+    // decisions of t + 1 (the day kernel's phases as separate launches);
     // then step t + 1 untimed
     if ((rc = reset_sums(c))) return rc;
     CK(cudaMemsetAsync(c->k.a.move_mask, 0, sizeof(uint32_t) * MOVE_MASK_WORDS, c->stream));
     CK(cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t) * BAR_WORDS, c->stream));
     if ((rc = force_rebuild(c))) return rc;
-    launch_movement(c->k, step, c->stream);
+    launch_movement(c->k, step, true, c->stream);
     CK(cudaEventRecord(ev[0], c->stream));
-    launch_step(c->k, step, PH_REBUILD, c->stream);
+    launch_day(c->k, step, step + 1, PH_REBUILD, c->stream);
     CK(cudaEventRecord(ev[1], c->stream));
-    launch_step(c->k, step, PH_DRAW, c->stream);
+    launch_day(c->k, step, step + 1, PH_DRAW, c->stream);
     CK(cudaEventRecord(ev[2], c->stream));
-    launch_step(c->k, step, PH_DECIDE, c->stream);
+    launch_day(c->k, step, step + 1, PH_DECIDE, c->stream);
     CK(cudaEventRecord(ev[3], c->stream));
-    launch_step(c->k, step + 1, PH_REBUILD | PH_DRAW, c->stream);
+    launch_day(c->k, step + 1, step + 2, PH_REBUILD | PH_DRAW, c->stream);
     c->launches += 5;
-    // the sums as the step after them reads them, in the first copy
-    if ((step + 2) & 1u)
-        CK(cudaMemcpyAsync(c->k.l.sfix, c->k.l.sfix_b, sizeof(unsigned long long) * c->L * c->V,
-                           cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     for (int j = 0; j < 3; ++j) CK(cudaEventElapsedTime(&ms[j], ev[j], ev[j + 1]));
     for (int j = 0; j < 4; ++j) cudaEventDestroy(ev[j]);

@@ -62,7 +62,7 @@ struct psim_ctx {
     uint64_t launches = 0;
     bool uploaded = false;
     bool csr_fresh = false;      // counts of the current positions are built
-    bool list_sparse = false;    // the agent list holds only the locations the step kernel's
+    bool list_sparse = false;    // the agent list holds only the locations the day kernel's
                                  // last rebuild listed (psim_get_csr builds the full one)
     // pinned host memory (one block): the statistics accumulators and the
     // expected-infection sums copied back, the clock copied in, the error

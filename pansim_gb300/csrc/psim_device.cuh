@@ -17,7 +17,7 @@ constexpr uint32_t ERR_LOCATION = 2u;      // an agent ended on an invalid locat
 constexpr uint32_t ERR_TEST_WAIT = 4u;     // bounded-wait self test expired (expected in tests)
 constexpr uint32_t ERR_SCAN_WAIT = 1u;     // a scan tile gave up waiting for its predecessors
 constexpr uint32_t ERR_AGENT_LIST = 8u;    // the agent list disagrees with the histogram or work list
-constexpr uint32_t ERR_BARRIER = 16u;      // a grid barrier of the step kernel gave up waiting
+constexpr uint32_t ERR_BARRIER = 16u;      // a grid barrier of the day kernel gave up waiting
 
 struct DevModel {
     uint32_t n_states, n_variants, n_prog, n_agent_types;
@@ -110,9 +110,25 @@ struct DevAgents {
     uint32_t* home;               // [N] the agent's home: the first home-type entry of its location
                                   // list (findActualLocationForType's first match, no draw),
                                   // computed when the context is made or the home type changes
+    uint32_t* dinfo;              // [N] the decision word of the running day (DW_*)
     uint32_t* move_mask;          // [MOVE_MASK_WORDS] bit s: some agent decides at step s of the
                                   // running day (a superset; rebuilt by the day's first step)
 };
+
+// The decision word: what a movement decision needs to know of its agent, in
+// one load.  Computed from the agent's fields for the day's first step and
+// kept by whoever changes them during the day's timesteps (the decisions
+// themselves and the draw that infects the agent).  The fields behind a flag
+// are read only where the flag is set.
+constexpr uint32_t DW_TYPE = 0xFFu;          // agent type
+constexpr uint32_t DW_WB_SHIFT = 8;          // 3 bits: state_wb of the agent's state
+constexpr uint32_t DW_QUARANTINED = 1u << 11;  // its quarantined flag
+constexpr uint32_t DW_HOSPITAL = 1u << 12;   // hospitalized beyond the day's first step
+constexpr uint32_t DW_DIAGNOSED = 1u << 13;  // its diagnosed flag
+constexpr uint32_t DW_DIAG_TS = 1u << 14;    // st_diagnosed_ts > 0
+constexpr uint32_t DW_INFECTIOUS = 1u << 15;  // infectious != 0
+constexpr uint32_t DW_NO_WORK = 1u << 16;    // its no_work flag
+constexpr uint32_t DW_TOO_OLD = 1u << 17;    // at or above the school age restriction
 
 struct DevLocs {
     uint32_t n;
@@ -135,8 +151,6 @@ struct DevLocs {
                                   // to the variant times its age band's factor
     uint32_t* qu_pending;         // quarantine writes of the running step
     unsigned long long* sfix;     // [V][n] fixed-point infectiousness sums
-    unsigned long long* sfix_b;   // [V][n] the step kernel's second copy: even steps of the day
-                                  // read sfix, odd steps sfix_b (see k_step)
     float* hazard;                // [V][n] infection ratio of the last step
     uint32_t* hmask;              // bit l: some variant's hazard at location l is > 0
     uint32_t* smask;              // bit l: some variant's fixed-point sum at l received a term this step
@@ -144,11 +158,11 @@ struct DevLocs {
     uint32_t* no_work_loc;
     uint8_t* flags;               // testing flags
     uint32_t* tile_sums;          // per-tile sums of the histogram (two-pass scan)
-    uint32_t* bar;                // the step kernel's grid barrier ([0] arrivals, [1] generation),
-                                  // the counts of the three infection lists, the listing counter
-    uint32_t* slot_loc;           // [N] the location of each agent-list slot the step kernel listed
-    uint4* inf_pending;           // [3][N] the infections of a step (location, infectiousness
-                                  // before and after, variants), in list step % 3
+    uint32_t* bar;                // the day kernel's grid barrier ([0] arrivals), the count of the
+                                  // replay list, the listing counter
+    uint32_t* slot_loc;           // [N] the location of each agent-list slot the day kernel listed
+    uint32_t* replay_stamp;       // [n] the last segment of draws that flagged the location
+    uint32_t* replay_list;        // [n] the locations the running segment flagged
     uint64_t* scan_status;        // per-tile status words of the single-pass scan (epoch | flag | value)
     uint32_t* scan_state;         // [0] epoch of the next single-pass scan, [1] its tile ticket
     uint32_t* build;              // [0] timestamp at which agents last took new locations,
@@ -158,8 +172,11 @@ struct DevLocs {
                                   //     the step's first scan kernel, read by its later kernels),
                                   // [3] the timestamp of the last step whose decisions wrote a
                                   //     location quarantine (merged by that step's scan),
-                                  // [5] the agent-list entries the step kernel's last rebuild
+                                  // [5] the agent-list entries the day kernel's last rebuild
                                   //     listed
+                                  // [6] the stamp of the last segment of draws (counts segments
+                                  //     over the context's lifetime, so a replayed day never meets
+                                  //     its own stamps)
 };
 
 // Incremental CSR: at most steps of a day no agent moves, and then the
@@ -199,7 +216,7 @@ struct DevTune {
     uint32_t agg_count;      // no effect: the histogram is updated by movers only
     uint32_t agg_slot;       // warp-aggregate the CSR slot atomics
     uint32_t blocks_per_sm;  // grid of the per-agent kernels (0 = one occupancy wave)
-    uint32_t variant;        // 3: the location-ordered step (the only form)
+    uint32_t variant;        // 3 or 4: the day kernel (the only form)
     uint32_t scan_items;     // locations per scan thread: 2, 4 or 8 (tile = 256 x items)
     uint32_t scan_mode;      // 0 = single pass with decoupled look-back, 1 = tile sums + scan,
                              // 2 = tile sums + scan with thread-contiguous locations (items 4, 8)
@@ -233,12 +250,13 @@ enum {
     // Then the day's timeline (globaltimer, ns; a first entry is kept as the
     // maximum of complements, so one zero fill starts every slot):
     // [PROF_N] ~first block entry of the day's first movement, [PROF_N + 1]
-    // its last block exit; per step s at PROF_T + PROF_TW * s: ~first block
-    // entry, the last block past the rebuild's listing, past its slots, past
-    // the draws, past the queue, last block exit (the rebuild and queue
-    // slots stay 0 at steps without that phase).
+    // its last block exit; per segment of the day, at PROF_T + PROF_TW * (its
+    // first step): ~first block entry, the last block past the rebuild's
+    // listing, past its slots, past the draws, past the queue, past the
+    // replay, last block exit (slots of phases the segment did not run and of
+    // steps that start no segment stay 0).
     PROF_T = PROF_N + 2,
-    PROF_TW = 6,
+    PROF_TW = 7,
     PROF_WORDS = PROF_T + PROF_TW * 1440
 };
 
@@ -313,7 +331,8 @@ __device__ __forceinline__ void update_meta(const KArgs& k, uint32_t i) {
 #endif
 
 // launchers (psim_kernels.cu)
-void launch_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
+// day: the day kernel runs the steps after it
+void launch_movement(const KArgs& k, uint32_t step_in_day, bool day, cudaStream_t s);
 void launch_count(const KArgs& k, cudaStream_t s);
 // merge_quarantine: 0 no, 1 at the steps whose decisions wrote location
 // quarantines, 2 always
@@ -321,20 +340,19 @@ void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merg
 void launch_scatter_draw(const KArgs& k, uint32_t step_in_day, int scatter, int draw, cudaStream_t s);
 void launch_offsets(const KArgs& k, cudaStream_t s);
 int scan_kernels(const KArgs& k);
-// the step kernel (psim_kernels.cu, k_step): the phases a launch runs, and
-// launches of one timestep or of a range of timesteps (grid barriers between)
+// the day kernel (psim_kernels.cu, k_day): the phases a launch runs, for the
+// timesteps step0 .. step_end - 1 of the day
 constexpr uint32_t PH_REBUILD = 1u, PH_DRAW = 2u, PH_DECIDE = 4u, PH_ALL = 7u;
-void launch_step(const KArgs& k, uint32_t step_in_day, uint32_t phases, cudaStream_t s);
-void launch_steps(const KArgs& k, uint32_t step0, uint32_t nsteps, uint32_t phases, cudaStream_t s);
+void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s);
 void launch_time_shift(uint32_t* a, uint32_t n, uint32_t delta, cudaStream_t s);
-// words of the barrier array: two for the barrier, then the counts of the
-// infections of the steps in lists 0-2 (step % 3), then the rebuild's listing
-// counter (slots reserved so far)
-constexpr uint32_t BAR_INFECTIONS = 2;
-constexpr uint32_t BAR_LISTED = BAR_INFECTIONS + 3;
-constexpr uint32_t BAR_WORDS = BAR_LISTED + 1;
-// work-list segments of the decisions (blocks of the queue kernel at most)
-constexpr uint32_t WORK_MAX_BLOCKS = 152u * 64u;
+// words of the barrier array: the barrier's arrivals, the count of the replay
+// list, the rebuild's listing counter (slots reserved so far); the arrivals
+// in a line of their own
+constexpr uint32_t BAR_REPLAY = 32;
+constexpr uint32_t BAR_LISTED = 33;
+constexpr uint32_t BAR_WORDS = 64;
+// threads of the day kernel at most (work-list segments)
+constexpr uint32_t WORK_MAX_THREADS = 160u * 2048u;
 // words of the per-day mask of decision steps (1440 steps of one minute at most)
 constexpr uint32_t MOVE_MASK_WORDS = 48;
 

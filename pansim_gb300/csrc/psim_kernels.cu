@@ -4,10 +4,10 @@
 // movementPolicies.h:263-1041, for every agent at the day's first step, with
 // the per-location histogram and the per-location infectiousness sums of
 // Util::reduce_by_location, util.h:48-101, as exact 2^-40 fixed-point int64
-// sums), then one k_step per timestep: the agent list rebuilt where agents
-// took new locations (replaces thrust::stable_sort_by_key, util.cpp:69), the
-// infection ratio and draws over the locations with an infectious agent
-// (infectionPolicies.h:520-546, LocationsList::infectAgents,
+// sums), then one k_day for all timesteps of the day: the agent list rebuilt
+// where agents took new locations (replaces thrust::stable_sort_by_key,
+// util.cpp:69), the infection ratio and draws over the locations with an
+// infectious agent (infectionPolicies.h:520-546, LocationsList::infectAgents,
 // locationList.h:233-310), and the decisions of the agents whose decision
 // step comes next.
 // The per-phase entry points (psim_movement, psim_regroup, psim_infect) use
@@ -149,12 +149,14 @@ __device__ bool quarantine_agent(const KArgs& k, uint32_t i, uint32_t t, uint32_
 // an unsigned char, so a difference that went negative folds modulo 256 hours
 __device__ __forceinline__ uint32_t td_minutes(uint32_t mins) { return (uint32_t)(uint8_t)(mins / 60u) * 60u + mins % 60u; }
 
-__device__ void diagnose_and_quarantine(const KArgs& k, uint32_t i, uint32_t t, uint32_t sum, psim_stream* rng) {
+// returns the decision word's flags of what it set
+__device__ uint32_t diagnose_and_quarantine(const KArgs& k, uint32_t i, uint32_t t, uint32_t sum, psim_stream* rng) {
     const uint32_t dt = k.p.time_step;
     k.a.diagnosed[i] = 1;
-    k.a.st_diagnosed_ts[i] = t;
-    if (sum == 24u * 60u / dt) k.a.st_diagnosed_ts[i]++;
-    (void)quarantine_agent(k, i, t, t + k.p.quarantine_length * 24u * 60u / dt, rng);
+    const uint32_t ts = sum == 24u * 60u / dt ? t + 1u : t;
+    k.a.st_diagnosed_ts[i] = ts;
+    return DW_DIAGNOSED | (ts > 0 ? DW_DIAG_TS : 0u) |
+           (quarantine_agent(k, i, t, t + k.p.quarantine_length * 24u * 60u / dt, rng) ? DW_QUARANTINED : 0u);
 }
 
 // S: the agent's countdown (stepsUntilMove) as the decision just set it;
@@ -164,31 +166,29 @@ __device__ __forceinline__ void stayed_home_check(const KArgs& k, uint32_t i, ui
     if (agent_home != NONE && cur != agent_home && S > 60u / k.p.time_step) k.a.stayed_home[i] = 0;
 }
 
-// The agent's fields that a decision reads, loaded together before it
-// starts: read where they are needed, behind branches and stores, each would
-// cost a round trip of its own.  The decision keeps its own copies of the two
-// it writes (location, quarantined flag).
+// The agent's decision word (DW_*) from its fields; t = the first timestep it
+// is used at.
+__device__ __forceinline__ uint32_t decision_word(const KArgs& k, uint32_t i, uint32_t t) {
+    const uint32_t type = k.a.type[i], st = (uint8_t)k.a.state[i], age = k.a.age[i];
+    const bool quar = k.a.quarantined[i] != 0, diag = k.a.diagnosed[i] != 0, no_work = k.a.no_work[i] != 0;
+    const bool hosp = k.a.st_hospitalized_until[i] > t, diag_ts = k.a.st_diagnosed_ts[i] > 0;
+    const bool inf = k.a.infectious[i] != 0.0f;
+    return type | (uint32_t)k.m.state_wb[st] << DW_WB_SHIFT | (quar ? DW_QUARANTINED : 0u) | (hosp ? DW_HOSPITAL : 0u) |
+           (diag ? DW_DIAGNOSED : 0u) | (diag_ts ? DW_DIAG_TS : 0u) | (inf ? DW_INFECTIOUS : 0u) |
+           (no_work ? DW_NO_WORK : 0u) | (age >= k.p.school_age_restriction ? DW_TOO_OLD : 0u);
+}
+
+// What a decision reads of its agent, loaded together before it starts: the
+// decision word, the current location, the agent's entries in the per-agent
+// location list, the replica.
 struct DecisionIn {
-    uint32_t loc, q_until, h_ts, h_until, lb, le, diag_ts, rep;
-    float inf;
-    uint8_t state, type, diag, no_work, age, quarantined;
+    uint32_t w, loc, lb, le, rep;
 };
 __device__ __forceinline__ void decision_in(const KArgs& k, uint32_t i, DecisionIn& d) {
     d.loc = k.a.location[i];
-    d.q_until = k.a.st_quarantined_until[i];
-    d.h_ts = k.a.st_hospitalized_ts[i];
-    d.h_until = k.a.st_hospitalized_until[i];
     d.lb = k.a.loc_offset[i];
     d.le = k.a.loc_offset[i + 1];
-    d.diag_ts = k.a.st_diagnosed_ts[i];
-    d.rep = k.a.rep[i];
-    d.inf = k.a.infectious[i];
-    d.state = (uint8_t)k.a.state[i];
-    d.type = k.a.type[i];
-    d.diag = k.a.diagnosed[i];
-    d.no_work = k.a.no_work[i];
-    d.age = k.a.age[i];
-    d.quarantined = k.a.quarantined[i];
+    d.rep = k.r.n == 1 ? 0u : k.a.rep[i];
 }
 
 // Quarantine end and type of a location (the quarantine rule's inputs);
@@ -213,9 +213,10 @@ __device__ __forceinline__ bool quarantine_type(const KArgs& k, uint32_t ty) {
 // decision, cur the agent's location after it (d.loc before).  The
 // location-dependent inputs (the quarantine rule's at the current and at the
 // chosen location, the chosen location's flags) load together as soon as the
-// location is known.
-__device__ void move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t minutes, uint32_t day, uint32_t sum,
-                            psim_stream* rng, uint32_t& S, const DecisionIn& d, uint32_t& cur) {
+// location is known.  Returns the agent's decision word after it.
+__device__ __forceinline__ uint32_t move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t minutes, uint32_t day,
+                                                uint32_t sum, psim_stream* rng, uint32_t& S, const DecisionIn& d,
+                                                uint32_t& cur) {
     const psim_params& p = k.p;
     const uint32_t dt = p.time_step;
     const bool qrule = p.quarantine_policy > 1;
@@ -228,61 +229,73 @@ __device__ void move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t min
         cur = l;
         k.a.location[i] = l;
     };
-    bool quar = d.quarantined != 0;
-    if (d.q_until <= t) {
-        quar = false;
+    uint32_t w = d.w;
+    if ((w & DW_QUARANTINED) && k.a.st_quarantined_until[i] <= t) {
+        w &= ~DW_QUARANTINED;
         k.a.quarantined[i] = 0;
     }
+    // quarantine_agent and the word's flag
+    auto quarantine = [&](uint32_t until) {
+        if (quarantine_agent(k, i, t, until, rng)) w |= DW_QUARANTINED;
+    };
+    // an infectious agent not diagnosed yet: diagnosed at the hospital or doctor
+    auto diagnose = [&]() {
+        if ((w & (DW_DIAGNOSED | DW_INFECTIOUS)) == DW_INFECTIOUS) w |= diagnose_and_quarantine(k, i, t, sum, rng);
+    };
 
-    const uint32_t wb = k.m.state_wb[d.state];
+    const uint32_t wb = (w >> DW_WB_SHIFT) & 7u;
     if (wb == WB_D) {
         S = NONE;
         set_loc(k.r.cemetery[d.rep]);
-        return;
+        return w;
     }
     const uint32_t agent_home = fl(p.home_type, 0);
 
-    if (d.h_ts <= t && d.h_until > t && wb != WB_S && wb != WB_D) {
-        uint32_t x = d.h_until - t - 1;
-        S = x < sum ? x : sum;
-        set_loc(fl(p.hospital_type, 0));
-        if (!d.diag && d.inf != 0.0f) diagnose_and_quarantine(k, i, t, sum, rng);
-        return;
+    if ((w & DW_HOSPITAL) && wb != WB_S) {
+        const uint32_t h_until = k.a.st_hospitalized_until[i];
+        if (k.a.st_hospitalized_ts[i] <= t && h_until > t) {
+            uint32_t x = h_until - t - 1;
+            S = x < sum ? x : sum;
+            set_loc(fl(p.hospital_type, 0));
+            diagnose();
+            return w;
+        }
     }
     if (wb == WB_S) {
         S = sum;
         set_loc(fl(p.hospital_type, 0));
-        if (!d.diag && d.inf != 0.0f) diagnose_and_quarantine(k, i, t, sum, rng);
-        return;
+        diagnose();
+        return w;
     }
     if (qrule && t < q_now.qu && quarantine_type(k, q_now.ty)) {
-        if (!quar) quar = quarantine_agent(k, i, t, q_now.qu, rng);
-        if (quar) {
+        if (!(w & DW_QUARANTINED)) quarantine(q_now.qu);
+        if (w & DW_QUARANTINED) {
             // the location is still the current one
             uint32_t x = q_now.qu - t - 1;
             S = x < sum ? x : sum;
             uint32_t home_location = fl(p.home_type, 0);
             if (home_location != cur) set_loc(home_location);
             stayed_home_check(k, i, agent_home, cur, S);
-            return;
+            return w;
         }
     }
-    if ((p.quarantine_policy > 0 &&
-         (d.diag || (d.diag_ts > 0 && (t - d.diag_ts) < p.quarantine_length * 24u * 60u / dt))) ||
-        (p.quarantine_policy > 0 && quar)) {
-        if (p.quarantine_policy > 0 && !quar) quar = quarantine_agent(k, i, t, t + p.quarantine_length * 24u * 60u / dt, rng);
-        if (quar) {
-            set_loc(fl(p.home_type, 0));
-            S = sum;
-            stayed_home_check(k, i, agent_home, cur, S);
-            return;
+    if (p.quarantine_policy > 0 && (w & (DW_DIAGNOSED | DW_DIAG_TS | DW_QUARANTINED))) {
+        const uint32_t ql = p.quarantine_length * 24u * 60u / dt;
+        if ((w & (DW_DIAGNOSED | DW_QUARANTINED)) || t - k.a.st_diagnosed_ts[i] < ql) {
+            if (!(w & DW_QUARANTINED)) quarantine(t + ql);
+            if (w & DW_QUARANTINED) {
+                set_loc(fl(p.home_type, 0));
+                S = sum;
+                stayed_home_check(k, i, agent_home, cur, S);
+                return w;
+            }
         }
     }
 
     // schedule window (AgentTypeList::getOffsetIndex, agentType.cpp:13-15;
     // the window of the slot at this step, movementPolicies.h:585-603, from
     // the table the host computed)
-    const uint32_t agent_type = d.type;
+    const uint32_t agent_type = w & DW_TYPE;
     const uint32_t off_idx = 7u * wb + day + agent_type * 28u;
     const int2 win = k.m.window[(size_t)off_idx * k.spd + minutes / dt];
     const int act_b = win.x, act_e = win.y;
@@ -303,25 +316,32 @@ __device__ void move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t min
             new_type = k.m.ev_loc_type[act_b];
             dur = k.m.ev_duration[act_b];
         } else {
-            double rnd = psim_u01(rng) * 1.0;
-            double thr = k.m.ev_chance[act_b];
+            // U > chance of the first event, in integers: U = K 2^-53 and
+            // chance 2^53 (exact in float), so K > floor(chance 2^53); the
+            // few that go on compare in double as the reference does
+            const uint64_t K = psim_u53(rng);
+            const float c0 = k.m.ev_chance[act_b];
             uint32_t idx = 0;
-            while (rnd > thr && idx < num_pot) {
-                idx++;
-                thr += k.m.ev_chance[act_b + idx];
+            if (c0 < 0.0f || (c0 < 1.0f && K > __float2ull_rd(c0 * 9007199254740992.0f))) {
+                const double rnd = (double)K * (1.0 / 9007199254740992.0);
+                double thr = c0;
+                while (rnd > thr && idx < num_pot) {
+                    idx++;
+                    thr += k.m.ev_chance[act_b + idx];
+                }
             }
             if (idx == num_pot) idx--;
             picked = idx;
             new_type = k.m.ev_loc_type[act_b + idx];
             dur = k.m.ev_duration[act_b + idx];
         }
-        if (d.no_work != 0 && new_type == p.work_type) {
+        if ((w & DW_NO_WORK) && new_type == p.work_type) {
             new_type = p.home_type;
             num_pot = 1;
-            if (!quar) k.a.st_days_in_quarantine[i]++;
+            if (!(w & DW_QUARANTINED)) k.a.st_days_in_quarantine[i]++;
         }
         uint32_t new_loc = fl(new_type, num_pot == 1);
-        bool too_old = (new_type == p.school_type || new_type == p.classroom_type) && d.age >= p.school_age_restriction;
+        bool too_old = (new_type == p.school_type || new_type == p.classroom_type) && (w & DW_TOO_OLD);
         // the new location's flags and quarantine inputs load together
         const uint8_t nl_open = loc_open(k, new_loc);
         const uint32_t nl_closed = loc_closed_until(k, new_loc);
@@ -396,22 +416,21 @@ __device__ void move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t min
     if (qrule) {
         const LocQ q = cur == spec_loc ? spec_q : cur == d.loc ? q_now : loc_q(k, cur);
         if (t < q.qu && quarantine_type(k, q.ty)) {
-            if (!quar) quar = quarantine_agent(k, i, t, q.qu, rng);
-            if (quar) {
+            if (!(w & DW_QUARANTINED)) quarantine(q.qu);
+            if (w & DW_QUARANTINED) {
                 uint32_t x = q.qu - t - 1;
                 S = x < sum ? x : sum;
                 uint32_t home_location = fl(p.home_type, 0);
                 if (home_location != cur) set_loc(home_location);
                 stayed_home_check(k, i, agent_home, cur, S);
-                return;
+                return w;
             }
         }
     }
-    if (new_type == p.hospital_type || (new_type == p.doctor_type && psim_u01(rng) * 1.0 < 0.7)) {
-        if (!d.diag && d.inf != 0.0f) diagnose_and_quarantine(k, i, t, sum, rng);
-    }
+    if (new_type == p.hospital_type || (new_type == p.doctor_type && psim_u01(rng) * 1.0 < 0.7)) diagnose();
     stayed_home_check(k, i, agent_home, cur, S);
     S = S - 1u;
+    return w;
 }
 
 // curfew prologue of doMovement (movementPolicies.h:267-326); returns true if
@@ -507,17 +526,10 @@ __device__ __forceinline__ void mask_flush(const KArgs& k, uint32_t* s_mm) {
 
 // doMovement for agent i at step c.t; s = its countdown before the step
 // (move_at - c.t).  Writes move_at when the agent decides or the curfew
-// prologue resets its countdown.  pre: the decision's inputs when the caller
-// loaded them (its agents all decide), else null (loaded here if needed).
-// Returns the agent's location after the step (loc0: before it).
+// prologue resets its countdown.  d: the decision's inputs.  Returns the
+// agent's location after the step; w receives its decision word after it.
 __device__ __forceinline__ uint32_t move_agent(const KArgs& k, uint32_t i, const StepClock& c, uint32_t s,
-                                               uint32_t* s_mm, const DecisionIn* pre, uint32_t loc0) {
-    if (!(c.curfew_now || s == 0)) return loc0;  // counts down: move_at stays
-    DecisionIn d;
-    if (pre)
-        d = *pre;
-    else
-        decision_in(k, i, d);
+                                               uint32_t* s_mm, DecisionIn d, uint32_t* w) {
     psim_stream rng;
     psim_stream_init(&rng, k.r.seed[d.rep], i - k.r.agent_off[d.rep], c.t, PSIM_PHASE_MOVE);
     bool done = false;
@@ -527,11 +539,12 @@ __device__ __forceinline__ uint32_t move_agent(const KArgs& k, uint32_t i, const
         d.loc = k.a.location[i];  // the prologue may have sent the agent home
     }
     uint32_t cur = d.loc;
+    *w = d.w;
     if (!done) {
         if (S > 0)
             S = S - 1u;
         else
-            move_decide(k, i, c.t, c.minutes, c.day, c.sum, &rng, S, d, cur);
+            *w = move_decide(k, i, c.t, c.minutes, c.day, c.sum, &rng, S, d, cur);
     }
     const uint32_t m = c.t + 1u + S;
     k.a.move_at[i] = m;
@@ -545,7 +558,7 @@ constexpr int SCAN_THREADS = 256;
 
 // A location that receives an infectious term sets its hazard-mask bit at
 // once, so the mask is always a superset of the locations with a nonzero sum
-// (the step kernel's rebuild lists from it and clears the bits of zero sums;
+// (the day kernel's rebuild lists from it and clears the bits of zero sums;
 // the per-phase scans recompute the bits of their dirty locations).
 __device__ __forceinline__ void mark_hazardous(const KArgs& k, uint32_t loc) {
     atomicOr(&k.l.hmask[loc >> 5], 1u << (loc & 31u));
@@ -571,7 +584,6 @@ __device__ __forceinline__ bool count_agent(const KArgs& k, bool act, uint32_t l
     if (act && loc != NONE && inf > 0.0f) {
         const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
         atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicAdd(&k.l.sfix_b[(size_t)variant * L + loc], (unsigned long long)q);
         atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
         mark_hazardous(k, loc);
     }
@@ -582,9 +594,9 @@ __device__ __forceinline__ bool count_agent(const KArgs& k, bool act, uint32_t l
 // when it moves or its infectiousness changes (a draw that infects).  The
 // first step of a day (k_movement after a reset of the sums) adds every
 // agent's term afresh.
-// The agent went from (loc0, inf0, var0) to (loc, inf, var) in a step
+// The agent went from (loc0, inf0, var0) to (loc, inf, var) in a day
 // kernel's decision: its count moves, its fixed-point term leaves (loc0,
-// var0) and joins (loc, var).  The step kernel computes every ratio from the
+// var0) and joins (loc, var).  The day kernel computes every ratio from the
 // sums, so it keeps no dirty marks (the day graph marks every location dirty
 // at its start: a scan after it recomputes every ratio).  Returns whether the
 // agent took a new location.
@@ -604,15 +616,9 @@ __device__ __forceinline__ bool count_agent_delta(const KArgs& k, bool act, uint
         const long long q0 = (loc0 < L && inf0 > 0.0f) ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
         const long long q1 = (loc != NONE && inf > 0.0f) ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
         if (mv || q0 != q1 || var0 != var) {
-            // both copies of the step kernel's sums (the next step reads
-            // the other one)
-            if (q0) {
-                atomicAdd(&k.l.sfix[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
-                atomicAdd(&k.l.sfix_b[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
-            }
+            if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
             if (q1) {
                 atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
-                atomicAdd(&k.l.sfix_b[(size_t)var * L + loc], (unsigned long long)q1);
                 mark_hazardous(k, loc);
             }
         }
@@ -632,7 +638,6 @@ __device__ __forceinline__ void count_full(const KArgs& k, bool act, uint32_t lo
     if (inf > 0.0f) {
         const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
         atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicAdd(&k.l.sfix_b[(size_t)variant * L + loc], (unsigned long long)q);
         atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
         mark_hazardous(k, loc);
     }
@@ -673,10 +678,11 @@ __device__ __forceinline__ void store_slot(const KArgs& k, uint32_t pos, uint32_
 // d p / d theta of one draw (p = r * s * sigma_band, r = 1 - exp(-x),
 // x = k * S/n * w * season * dt), weighted by the replica's dL/dE, added to the
 // block's FP64 accumulators
-// x: the location's hazard argument k*S/n*w*season*dt for variant v
+// x: the location's hazard argument k*S/n*w*season*dt for variant v; times:
+// how many timesteps made this draw with the same p
 __device__ __noinline__ void adjoint_terms(const KArgs& k, uint32_t i, uint32_t loc, uint32_t v, uint32_t rep, float r,
-                                           float su, float s_eff, double* s_grad, float x_f) {
-    const double g = k.adj.weight[rep];
+                                           float su, float s_eff, double* s_grad, float x_f, uint32_t times) {
+    const double g = k.adj.weight[rep] * (double)times;
     if (g == 0.0) return;
     const double x = (double)x_f;
     const double dpdx = (double)s_eff * (1.0 - (double)r);
@@ -709,7 +715,7 @@ __device__ __forceinline__ double draw_agent(const KArgs& k, uint32_t i, uint32_
         const float pf = h * s_eff;
         term_sum += pf < 1.0f ? (double)pf : 1.0;
         if (k.adj.on && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, su, s_eff, s_grad, k.l.hazard_x[(size_t)v * L + loc]);
+            adjoint_terms(k, i, loc, v, rep, h, su, s_eff, s_grad, k.l.hazard_x[(size_t)v * L + loc], 1u);
         const double U = psim_u01_once(seed, li, t, PSIM_PHASE_INFECT + v);
         if (U < (double)pf) {
             k.a.state[i] = (int8_t)k.m.first_infected;
@@ -778,9 +784,11 @@ __device__ __forceinline__ void prof_mark(const KArgs& k, uint32_t slot) {
 // Movement of every agent + histogram + fixed-point infectiousness sums (the
 // day's first step, after a reset of the sums, and the per-phase entry
 // points).  Records the steps of the day at which agents decide next.
-__global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
+// day: the day kernel follows (the agents' decision words of the day are
+// written).
+__global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step, int day) {
     __shared__ uint32_t s_mm[MOVE_MASK_WORDS];
-    if (step == 0) prof_enter(k, PROF_N);
+    if (day) prof_enter(k, PROF_N);
     mask_clear_shared(s_mm);
     const uint32_t N = k.a.n;
     const StepClock c = step_clock(k, step);
@@ -794,17 +802,26 @@ __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
         if (act) {
             const uint32_t m0 = k.a.move_at[i];
             const uint32_t s = m0 - c.t;
-            loc0 = k.a.location[i];
+            DecisionIn d;
+            loc0 = loc = k.a.location[i];
             inf = k.a.infectious[i];
-            loc = move_agent(k, i, c, s, s_mm, nullptr, loc0);
-            if (!(c.curfew_now || s == 0)) mask_note(k, s_mm, m0);  // an agent counting down decides later today
+            const bool decides = c.curfew_now || s == 0;
+            uint32_t w = day || decides ? decision_word(k, i, c.t) : 0u;
+            if (decides) {
+                decision_in(k, i, d);
+                d.w = w;
+                loc = move_agent(k, i, c, s, s_mm, d, &w);
+            } else {
+                mask_note(k, s_mm, m0);  // an agent counting down decides later today
+            }
+            if (day) k.a.dinfo[i] = w;
             if (inf > 0.0f) var = k.a.variant[i];
         }
         moved |= count_agent(k, act, loc0, loc, inf, var);
     }
     publish_moved(k, moved, c.t);
     mask_flush(k, s_mm);
-    if (step == 0) prof_mark(k, PROF_N + 1);
+    if (day) prof_mark(k, PROF_N + 1);
 }
 
 // Histogram + fixed-point sums without movement (regroup after an upload).
@@ -1277,78 +1294,90 @@ __global__ void __launch_bounds__(256) k_scatter_draw(KArgs k, uint32_t step, in
 }
 
 // ---------------------------------------------------------------------------
-// The day graph's step kernel.  One launch per timestep t (step s of the day),
-// a persistent grid (every block resident; see launch_step) whose phases are
-// separated by grid barriers only where one phase needs another's results:
-//   rebuild   only when agents took new locations for t (or a rebuild is
-//             pending): the locations with a nonzero sum listed and their
-//             segments reserved | every agent at a listed location takes a
-//             slot, which keeps its id, its susceptibility x age-band factor
-//             of every variant and its location.  The step's location
-//             quarantine writes are merged here too (or alone when there were
-//             some but no rebuild).
-//   draw      every listed entry, one per thread: the location's infection
-//             ratio from its sum and the agent's draws (LocationsList::
-//             infectAgents, locationList.h:233-310); the infections' sum
-//             changes are applied once every draw of t is done
-//   decide    only when some agent decides at s + 1 (or everyone at the
-//             curfew step): the block queues its own agents that decide |
-//             doMovement of the queued agents for s + 1 (work segments taken
-//             in turn) and the histogram and sum deltas of their moves
-// A step at which nobody takes a new location and nobody decides next runs
-// the draw alone, without a barrier: its cost is the listed entries, not the
-// whole population.
+// The day graph's day kernel: one launch for all timesteps of a day, a
+// persistent grid (every block resident, a cooperative launch) whose phases
+// are separated by grid barriers only where one phase needs another's results.
+// Most timesteps of a day move nobody (at 2M agents 22 of 144 have deciders),
+// so the day is cut into segments: the timesteps from one whose agents took
+// new locations to the next that somebody decides at.  Per segment:
+//   rebuild   when agents took new locations (or a rebuild is pending): the
+//             locations with a nonzero sum listed and their segments reserved |
+//             every agent at a listed location takes a slot, which keeps its
+//             id, its susceptibility x age-band factor of every variant and
+//             its location.  The location quarantine writes of the decisions
+//             before are merged here too (or alone when nobody moved).
+//   draw      every listed entry, one per thread, for all the timesteps of the
+//             segment at once: nobody moves, so a location's infection ratio
+//             stays what it is until somebody there is infected.  An entry
+//             that would be infected commits nothing: it flags its location |
+//             the flagged locations (a few) replayed exactly, a warp each,
+//             timestep by timestep with the ratio of the location's sum as the
+//             timestep started (LocationsList::infectAgents,
+//             locationList.h:233-310)
+//   decide    the block queues its own agents that decide at the segment's end
+//             | doMovement of the queued agents and the histogram and sum
+//             deltas of their moves
+// What it replaces drew every timestep in a launch of its own (2.9-5.8 us and
+// a launch gap of 0.9-1.3 us each at 10k-2M agents, ~100 timesteps of a day).
 
-// Grid barrier of the persistent step kernel: the last block to arrive
-// resets the count and advances the generation the others wait on (a
-// two-level arrival, 8 groups then the grid, measured slower: the second
-// atomic round trip costs more than the serialized arrivals it saves).
-// Every wait is bounded: on expiry the block records ERR_BARRIER and returns
-// false, and every later barrier and step kernel returns at once, so a
-// failure ends in an error report, never a hang.  The block's writes reach
-// the other blocks through the arrival (release: the block's threads' writes
-// are ordered before it by the __syncthreads before) and the generation read
-// (acquire).
+constexpr uint32_t DAY_THREADS = 512;  // two blocks per SM at 64 registers
+
+// Grid barrier of the day kernel: every block adds one to a count that only
+// grows (zeroed when the day graph starts) and waits until it reaches the
+// barrier's target.  On GB300 1.4 us with 304 blocks of 512 threads, against
+// 2.5 us for a returning arrival, a reset and a generation word with 608
+// blocks of 256 (arrivals on one address are serialized, so fewer blocks and
+// no returned value).  Every wait is bounded: on expiry the block records
+// ERR_BARRIER and returns false, the others follow (they look at the error
+// flags while they wait), and every later barrier and day kernel returns at
+// once, so a failure ends in an error report, never a hang.  The block's
+// writes reach the other blocks through the arrival (release: the block's
+// threads' writes are ordered before it by the __syncthreads before) and the
+// count's read (acquire).
 constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(uint32_t* p, uint32_t x) {
-    uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
-    return old;
+__device__ __forceinline__ void red_add_release_gpu(uint32_t* p, uint32_t x) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
 }
-__device__ __forceinline__ void st_relaxed_gpu(uint32_t* p, uint32_t x) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
-__device__ __forceinline__ bool grid_barrier(const KArgs& k, bool* s_ok) {
+
+// Block-shared scratch of the day kernel.
+struct DayShared {
+    double grad[GRAD_N];
+    float h[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // per warp: a replayed location's ratios
+    float x[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // and their arguments
+    uint32_t mm[MOVE_MASK_WORDS];
+    uint32_t red[32];
+    uint32_t target;  // the barrier count the next barrier waits for
+    uint32_t cnt, base;
+    bool ok;
+};
+
+__device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        bool ok = (ld_acquire_gpu(k.err) & ERR_BARRIER) == 0;
-        if (ok) {
-            const uint32_t gen = ld_acquire_gpu(&k.l.bar[1]);
-            const uint32_t arrived = atom_add_acq_rel_gpu(&k.l.bar[0], 1u) + 1u;
-            if (arrived == gridDim.x) {
-                st_relaxed_gpu(&k.l.bar[0], 0u);
-                atom_add_acq_rel_gpu(&k.l.bar[1], 1u);
-            } else {
-                uint32_t spins = 0;
-                while (ld_acquire_gpu(&k.l.bar[1]) == gen) {
-                    if (++spins > BARRIER_SPIN_LIMIT) {
-                        atomicOr(k.err, ERR_BARRIER);
-                        ok = false;
-                        break;
-                    }
-                    __nanosleep(32);
+        const uint32_t target = sh.target;
+        bool ok = true;
+        red_add_release_gpu(&k.l.bar[0], 1u);
+        uint32_t spins = 0;
+        while ((int32_t)(ld_acquire_gpu(&k.l.bar[0]) - target) < 0) {
+            if ((++spins & 1023u) == 0u) {
+                if (spins >= BARRIER_SPIN_LIMIT) atomicOr(k.err, ERR_BARRIER);
+                if (ld_acquire_gpu(k.err) & ERR_BARRIER) {
+                    ok = false;
+                    break;
                 }
             }
+            __nanosleep(20);
         }
-        *s_ok = ok;
+        sh.target = target + gridDim.x;
+        sh.ok = ok;
     }
     __syncthreads();
-    return *s_ok;
+    return sh.ok;
 }
 
 // Slot data of the agent list: csr_agents[pos] = agent, slot_su[v][pos] =
@@ -1367,10 +1396,10 @@ __device__ __forceinline__ void slot_fill(const KArgs& k, uint32_t pos, uint32_t
         k.l.slot_su[(size_t)v * N + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
 }
 
+// the sum of v over the block's threads; every thread calls it
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    v = __reduce_add_sync(0xffffffffu, v);
     if (lane == 0) s_red[warp] = v;
     __syncthreads();
     uint32_t tot = 0;
@@ -1379,7 +1408,8 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_red) {
     return tot;
 }
 
-// the step's location quarantine writes into quarantine_until (grid-stride)
+// the location quarantine writes of the last decisions into quarantine_until
+// (grid-stride)
 __device__ __forceinline__ void merge_quarantine(const KArgs& k) {
     const uint32_t L = k.l.n;
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < L; l += gridDim.x * blockDim.x) {
@@ -1391,64 +1421,6 @@ __device__ __forceinline__ void merge_quarantine(const KArgs& k) {
     }
 }
 
-// Exclusive prefix of v over the block's threads in thread order; *total
-// receives the block's sum.  Every thread calls it.
-__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* s_red, uint32_t* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) s_red[warp] = x;
-    __syncthreads();
-    uint32_t woff = 0, tot = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-        const uint32_t wq = s_red[q];
-        if (q < warp) woff += wq;
-        tot += wq;
-    }
-    __syncthreads();
-    *total = tot;
-    return woff + x - v;
-}
-
-// the set bits of mask word w whose location has a nonzero sum of some
-// variant (returned) and the agents at those locations (*agents); the loads of
-// four set bits at a time are issued together
-__device__ __forceinline__ uint32_t nonzero_sum_bits(const KArgs& k, const unsigned long long* sums, uint32_t hm,
-                                                     uint32_t w, uint32_t* agents) {
-    const uint32_t L = k.l.n, V = k.m.n_variants;
-    uint32_t keep = 0, rest = hm, cnt = 0;
-    while (rest) {
-        uint32_t b[4], l[4];
-        unsigned long long f[4];
-        uint32_t c[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            b[u] = rest ? (uint32_t)(__ffs(rest) - 1) : 32u;
-            if (rest) rest &= rest - 1u;
-            l[u] = b[u] < 32u ? w * 32u + b[u] : NONE;
-            const bool in = l[u] < L;
-            f[u] = in ? sums[l[u]] : 0ull;
-            c[u] = in ? k.l.counts[l[u]] : 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if (l[u] >= L) continue;
-            bool nz = f[u] != 0ull;
-            for (uint32_t v = 1; v < V && !nz; ++v) nz = sums[(size_t)v * L + l[u]] != 0ull;
-            if (nz) {
-                keep |= 1u << b[u];
-                cnt += c[u];
-            }
-        }
-    }
-    *agents = cnt;
-    return keep;
-}
-
 // Rebuild of the agent list.  Only the locations with a nonzero sum are
 // listed, because the draws of every step until the next rebuild need no
 // other location: until then no other location gains a nonzero sum (nobody
@@ -1458,60 +1430,123 @@ __device__ __forceinline__ uint32_t nonzero_sum_bits(const KArgs& k, const unsig
 // once); the listing clears the bits of the locations whose sums are zero
 // again.  The listed locations' agents fill the first *n_listed slots, each
 // slot with its agent, susceptibility products and location; the order of
-// the locations' segments is the order in which their chunks reserved them
+// the locations' segments is the order in which their blocks reserved them
 // (the draws do not depend on it).  In two parts between grid barriers:
-// 1 (listing): per chunk of 256 mask words of the block's range, the listed
-// locations, one atomic on the listing counter reserving the chunk's slots,
-// each location's first slot (cursor); 2 (slots): every agent at a listed
-// location takes a slot (one returning atomic on the location's cursor, or
-// one per location and warp with agg_slot).  Returns false when a barrier
-// expired.
-__device__ bool phase_rebuild(const KArgs& k, const unsigned long long* sums, uint32_t* s_red, bool* s_ok,
-                              uint32_t tl, uint32_t* s_base, uint32_t* n_listed) {
+// 1 (listing): each warp takes groups of mask words, a lane per location of
+// a nonzero word and LIST_BATCH words at a time in flight: once to clear the
+// bits of zero sums and add up the listed agents (one atomic on the listing
+// counter reserves the block's slots), once more for each listed location's
+// first slot (cursor).  A thread per word, the set bits of a word one after
+// another, took 9.5 us at 2M agents and 22 us with 3% infected; 2 (slots):
+// every agent at a listed location takes a slot (one returning atomic on the
+// location's cursor, or one per location and warp with agg_slot).  Returns
+// false when a barrier expired.
+constexpr int LIST_BATCH = 4;
+__device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
+    bool nz = k.l.sfix[l] != 0ull;
+    for (uint32_t v = 1; v < k.m.n_variants && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
+    return nz;
+}
+__device__ bool phase_rebuild(const KArgs& k, DayShared& sh, uint32_t tl, uint32_t* n_listed) {
     const uint32_t L = k.l.n, N = k.a.n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t n_words = (L + 31u) >> 5;
-    const uint32_t per = (n_words + gridDim.x - 1) / gridDim.x;
-    const uint32_t wb = min(n_words, blockIdx.x * per), we = min(n_words, wb + per);
-    // 1
+    // the warps take the words in groups of up to 8 (a sector), dealt in turn:
+    // the words of a busy type of location, which lie together, are many warps'
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5), wg = (uint32_t)warp * gridDim.x + blockIdx.x;
+    uint32_t lg = 0;
+    while (lg < 3u && (n_words >> (lg + 1u)) >= warps) ++lg;
+    const uint32_t per = 32u >> lg;                           // groups of a warp's trip
+    const uint32_t groups = (n_words + (1u << lg) - 1u) >> lg;  // of the whole mask
+    const auto word_of = [&](uint32_t trip, int src) {
+        return ((((trip * per + ((uint32_t)src >> lg)) * warps + wg) << lg) | ((uint32_t)src & ((1u << lg) - 1u)));
+    };
+    const uint32_t trips = groups > wg ? ((groups - wg + warps - 1u) / warps + per - 1u) / per : 0u;
+    // 1: the agents at the locations that stay listed
     uint32_t locs = 0, agents = 0;
-    for (uint32_t c0 = wb; c0 < we; c0 += blockDim.x) {  // block-uniform trips
-        const uint32_t w = c0 + threadIdx.x;
-        uint32_t hm = w < we ? k.l.hmask[w] : 0u;
-        uint32_t wc = 0;
-        if (hm) {
-            const uint32_t keep = nonzero_sum_bits(k, sums, hm, w, &wc);
-            if (keep != hm) k.l.hmask[w] = keep;
-            hm = keep;
+    for (uint32_t trip = 0; trip < trips; ++trip) {
+        const uint32_t w = word_of(trip, lane);
+        const uint32_t hm = w < n_words ? k.l.hmask[w] : 0u;
+        unsigned rest = __ballot_sync(0xffffffffu, hm != 0u);
+        while (rest) {
+            uint32_t m[LIST_BATCH], c[LIST_BATCH], at[LIST_BATCH];
+            bool nz[LIST_BATCH];
+#pragma unroll
+            for (int u = 0; u < LIST_BATCH; ++u) {
+                const int src = rest ? __ffs(rest) - 1 : 0;
+                const uint32_t word = __shfl_sync(0xffffffffu, hm, src);
+                at[u] = word_of(trip, src);
+                m[u] = rest ? word : 0u;
+                if (rest) rest &= rest - 1u;
+                const uint32_t l = at[u] * 32u + (uint32_t)lane;
+                const bool in = ((m[u] >> lane) & 1u) && l < L;
+                nz[u] = in && nonzero_sum(k, l);
+                c[u] = in ? k.l.counts[l] : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < LIST_BATCH; ++u) {
+                const unsigned keep = __ballot_sync(0xffffffffu, nz[u]);
+                if (lane == 0 && keep != m[u]) k.l.hmask[at[u]] = keep;
+                if (nz[u]) agents += c[u];
+                locs += nz[u] ? 1u : 0u;
+            }
         }
-        uint32_t chunk = 0;
-        const uint32_t ex = block_scan_excl(wc, s_red, &chunk);
-        if (chunk == 0) continue;  // block-uniform
-        if (threadIdx.x == 0) *s_base = atomicAdd(&k.l.bar[BAR_LISTED], chunk);
-        __syncthreads();
-        uint32_t run = *s_base + ex;
-        __syncthreads();
-        locs += __popc(hm);
-        agents += chunk;
-        while (hm) {
-            const uint32_t l = w * 32u + (uint32_t)(__ffs(hm) - 1);
-            hm &= hm - 1u;
-            if (l < L) {
-                k.l.cursor[l] = run;
-                run += k.l.counts[l];
+    }
+    // the warp's and the block's agents, the block's slots
+    uint32_t inc = agents;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) sh.red[warp] = inc;
+    __syncthreads();
+    uint32_t woff = 0, tot = 0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
+        const uint32_t wq = sh.red[q];
+        if (q < warp) woff += wq;
+        tot += wq;
+    }
+    if (threadIdx.x == 0 && tot) sh.base = atomicAdd(&k.l.bar[BAR_LISTED], tot);
+    __syncthreads();
+    if (tot) {
+        // each lane's locations in its own order: the words' bits are exact now
+        uint32_t run = sh.base + woff + inc - agents;
+        for (uint32_t trip = 0; trip < trips; ++trip) {
+            const uint32_t w = word_of(trip, lane);
+            const uint32_t hm = w < n_words ? k.l.hmask[w] : 0u;
+            unsigned rest = __ballot_sync(0xffffffffu, hm != 0u);
+            while (rest) {
+                uint32_t l[LIST_BATCH], c[LIST_BATCH];
+#pragma unroll
+                for (int u = 0; u < LIST_BATCH; ++u) {
+                    const int src = rest ? __ffs(rest) - 1 : 0;
+                    const uint32_t word = __shfl_sync(0xffffffffu, hm, src);
+                    const bool in = rest && ((word >> lane) & 1u);
+                    if (rest) rest &= rest - 1u;
+                    l[u] = in ? word_of(trip, src) * 32u + (uint32_t)lane : NONE;
+                    c[u] = in ? k.l.counts[l[u]] : 0u;
+                }
+#pragma unroll
+                for (int u = 0; u < LIST_BATCH; ++u)
+                    if (l[u] != NONE) {
+                        k.l.cursor[l[u]] = run;
+                        run += c[u];
+                    }
             }
         }
     }
     if (k.prof) {
-        const uint32_t nl = block_sum(locs, s_red);
-        if (threadIdx.x == 0 && (nl | agents)) {
+        const uint32_t nl = block_sum(locs, sh.red);
+        if (threadIdx.x == 0 && (nl | tot)) {
             atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)nl);
-            atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)agents);
+            atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)tot);
         }
     }
-    if (!grid_barrier(k, s_ok)) return false;
+    if (!grid_barrier(k, sh)) return false;
     prof_mark(k, tl + 1);
     *n_listed = k.l.bar[BAR_LISTED];  // every block's reservation is in
-    // 3: four consecutive agents per thread (one 16-byte load of their
+    // 2: four consecutive agents per thread (one 16-byte load of their
     // locations), two quads in flight
     const bool one = k.m.n_variants == 1;
     const uint32_t quads = (N + 3u) >> 2;
@@ -1522,7 +1557,7 @@ __device__ bool phase_rebuild(const KArgs& k, const unsigned long long* sums, ui
         for (int h = 0; h < 2; ++h) {
             const uint32_t q = q0 + (uint32_t)h * stride + threadIdx.x;
             const uint32_t i0 = q * 4u;
-            if (i0 + 3u < N) {
+            if (q < quads && i0 + 3u < N) {
                 const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
                 loc[4 * h + 0] = v.x;
                 loc[4 * h + 1] = v.y;
@@ -1530,7 +1565,7 @@ __device__ bool phase_rebuild(const KArgs& k, const unsigned long long* sums, ui
                 loc[4 * h + 3] = v.w;
             } else {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) loc[4 * h + u] = i0 + u < N ? k.a.location[i0 + u] : NONE;
+                for (int u = 0; u < 4; ++u) loc[4 * h + u] = q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
             }
         }
         uint32_t lw[8];
@@ -1555,7 +1590,7 @@ __device__ bool phase_rebuild(const KArgs& k, const unsigned long long* sums, ui
             if (pos < N) k.l.slot_loc[pos] = loc[u];
         }
     }
-    if (!grid_barrier(k, s_ok)) return false;
+    if (!grid_barrier(k, sh)) return false;
     // every block has read the listing counter: block 0 keeps the count for
     // the steps until the next rebuild and starts the counter at 0 for it
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1595,63 +1630,42 @@ __device__ __forceinline__ void infect_agent(const KArgs& k, uint32_t i, uint32_
     k.a.st_worst_state[i] = (int8_t)k.m.first_infected;
     k.a.st_worst_ts[i] = t;
     k.a.st_variant_mask[i] |= 1u << v;
+    const uint32_t w = k.a.dinfo[i] & ~(7u << DW_WB_SHIFT | DW_INFECTIOUS);
+    k.a.dinfo[i] = w | (uint32_t)k.m.state_wb[k.m.first_infected] << DW_WB_SHIFT |
+                   (k.a.infectious[i] != 0.0f ? DW_INFECTIOUS : 0u);
 }
 
 // U < p for the 53-bit uniform U = K * 2^-53 of the words (a, b)
 // (psim_u01_from) and a float probability p > 0, in integers: p * 2^53 is
 // exact in float (a power-of-two scaling of a normal or subnormal p), and
-// K < p * 2^53 holds exactly when K < ceil(p * 2^53).
-__device__ __forceinline__ bool u01_below(uint32_t a, uint32_t b, float p) {
-    if (p >= 1.0f) return true;
-    const unsigned long long K = ((unsigned long long)(a >> 5) << 26) | (unsigned long long)(b >> 6);
-    return K < __float2ull_ru(p * 9007199254740992.0f);
+// K < p * 2^53 holds exactly when K < ceil(p * 2^53).  u01_limit is that
+// bound (above every K for p >= 1).
+__device__ __forceinline__ unsigned long long u01_limit(float p) {
+    return p >= 1.0f ? ~0ull : __float2ull_ru(p * 9007199254740992.0f);
+}
+__device__ __forceinline__ bool u01_below(uint32_t a, uint32_t b, unsigned long long limit) {
+    return (((unsigned long long)(a >> 5) << 26) | (unsigned long long)(b >> 6)) < limit;
+}
+// the first two words of the stream (seed, agent, t, infection + v), as
+// psim_u01_once draws them
+__device__ __forceinline__ psim_ctr4 infect_words(unsigned long long seed, uint32_t li, uint32_t t, uint32_t v) {
+    psim_ctr4 c;
+    c.v[0] = li;
+    c.v[1] = t;
+    c.v[2] = PSIM_PHASE_INFECT + v;
+    c.v[3] = 0u;
+    return psim_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
 }
 
 // Infection ratio of variant v at location loc (count cnt, weight wl,
-// replica coefficient kf) from the location's fixed-point sum as the step
-// started: the formula the scans evaluate (psim_hazard_x), so every entry of
-// a location computes the same value.  x receives its argument.
-__device__ __forceinline__ float entry_hazard(const KArgs& k, const unsigned long long* sums, uint32_t loc, uint32_t v,
-                                              uint32_t cnt, float wl, float kf, float season, uint32_t dt, float* x) {
-    const long long fix = (long long)sums[(size_t)v * k.l.n + loc];
+// replica coefficient kf) from the location's fixed-point sum: the formula
+// the scans evaluate (psim_hazard_x), so every entry of a location computes
+// the same value.  x receives its argument.
+__device__ __forceinline__ float entry_hazard(const KArgs& k, uint32_t loc, uint32_t v, uint32_t cnt, float wl,
+                                              float kf, float season, uint32_t dt, float* x) {
+    const long long fix = (long long)k.l.sfix[(size_t)v * k.l.n + loc];
     *x = 0.0f;
     return fix != 0 ? psim_hazard_x(fix, cnt, kf, wl, season, dt, x) : 0.0f;
-}
-
-// The sums of the step kernel are kept twice: step s of the day reads copy
-// s & 1 (sfix, sfix_b) as the step started, and every change of step s goes
-// to the other copy, which step s + 1 reads.  The decisions change both
-// copies (they come after the step's draws); an infection changes the other
-// copy at once and is listed (list s % 3), and step s + 1 applies the list to
-// the copy it does not read, so that copy is complete when step s + 2 reads it
-// (apply_previous_infections).
-__device__ __forceinline__ unsigned long long* sums_read(const KArgs& k, uint32_t step) {
-    return (step & 1u) ? k.l.sfix_b : k.l.sfix;
-}
-__device__ __forceinline__ unsigned long long* sums_next(const KArgs& k, uint32_t step) {
-    return (step & 1u) ? k.l.sfix : k.l.sfix_b;
-}
-__device__ __forceinline__ void add_infection_change(const KArgs& k, unsigned long long* sums, uint32_t loc,
-                                                     float inf0, uint32_t var0, float inf, uint32_t var) {
-    const uint32_t L = k.l.n;
-    const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
-    const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
-    if (q0) atomicAdd(&sums[(size_t)var0 * L + loc], (unsigned long long)(-q0));
-    if (q1) {
-        atomicAdd(&sums[(size_t)var * L + loc], (unsigned long long)q1);
-        mark_hazardous(k, loc);
-    }
-}
-__device__ __forceinline__ void record_infection(const KArgs& k, uint32_t step, uint32_t loc, float inf0,
-                                                 uint32_t var0, float inf, uint32_t var) {
-    add_infection_change(k, sums_next(k, step), loc, inf0, var0, inf, var);
-    const uint32_t list = step % 3u;
-    const uint32_t j = atomicAdd(&k.l.bar[BAR_INFECTIONS + list], 1u);
-    if (j < k.a.n)
-        k.l.inf_pending[(size_t)list * k.a.n + j] =
-            make_uint4(loc, __float_as_uint(inf0), __float_as_uint(inf), var0 | (var << 8));
-    else
-        atomicOr(k.err, ERR_AGENT_LIST);
 }
 
 // A replica's infection coefficient, seed and first agent.
@@ -1668,50 +1682,148 @@ __device__ __forceinline__ RepConst rep_const(const KArgs& k, uint32_t rep) {
     return c;
 }
 
-// The draws of one agent-list entry: the agent in slot pos at location loc
-// of replica rep (count cnt, weight wl).  Returns the sum of min(1, p) over
-// its draws when expected infections are tracked (else 0).  An agent that is
-// infected updates its slot's susceptibility products (read by no other
-// entry) and records its location's sum change for the next steps.
-__device__ __forceinline__ double draw_entry(const KArgs& k, const unsigned long long* sums, uint32_t step,
-                                             uint32_t pos, uint32_t i, uint32_t loc, uint32_t rep, uint32_t cnt,
-                                             float wl, float su0, const RepConst& rc, float season, uint32_t t,
-                                             double* s_grad, bool* any_h) {
-    const uint32_t N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
-    const float kf = rc.kf;
-    const unsigned long long seed = rc.seed;
-    const uint32_t li = i - rc.off;
-    double term = 0.0;
+// The timesteps of one segment's draws: its first one (timestamp t), how many
+// there are, the day's season, the replay stamp of its flagged locations.
+struct DrawRun {
+    uint32_t t, n, epoch;
+    float season;
+};
+
+// The draws of every entry of the agent list (the agents at the locations
+// the last rebuild listed) for all the timesteps of the segment, one entry per
+// thread, slots in order (coalesced loads of the slot's location, agent and
+// susceptibility products).  Each entry evaluates its location's ratio from
+// the location's sum, count and weight (the same inputs give the same value at
+// every entry) and compares the agent's Philox draw of every timestep with it.
+// Nothing is committed here: an entry that would be infected flags its
+// location (a stamp per location keeps it in the list once), and
+// phase_replay repeats that location's draws with the ratio changing as its
+// agents are infected.  At a location without such an entry the ratio
+// cannot change, so the draws compared with it were the right ones.
+__device__ void phase_draw(const KArgs& k, const DrawRun& dr, uint32_t n_listed, uint32_t* n_entries,
+                           uint32_t* n_hazard) {
+    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    const bool one_rep = k.r.n == 1;
+    const RepConst rc0 = rep_const(k, 0);
+    uint32_t entries = 0, hazard = 0;
+    for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n_listed && pos < N; pos += stride) {
+        const uint32_t loc = k.l.slot_loc[pos];
+        const uint32_t i = k.l.csr_agents[pos];
+        const float su0 = k.l.slot_su[pos];
+        if (loc >= L || i >= N) {
+            atomicOr(k.err, ERR_AGENT_LIST);
+            continue;
+        }
+        const uint32_t cnt = k.l.counts[loc];
+        const float wl = k.l.infectiousness[loc];
+        const uint32_t rep = one_rep ? 0u : k.l.rep[loc];
+        const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
+        bool any_h = false, hit = false;
+        for (uint32_t v = 0; v < V && !hit; ++v) {
+            float x;
+            const float h = entry_hazard(k, loc, v, cnt, wl, rc.kf, dr.season, dt, &x);
+            if (!(h > 0.0f)) continue;
+            any_h = true;
+            if (!k.r.variant_active[rep * V + v]) continue;
+            const float s_eff = v == 0 ? su0 : k.l.slot_su[(size_t)v * N + pos];
+            if (!(s_eff > 0.0f)) continue;
+            const unsigned long long limit = u01_limit(h * s_eff);
+            const uint32_t li = i - rc.off;
+#pragma unroll 2
+            for (uint32_t j = 0; j < dr.n; ++j) {
+                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + j, v);
+                hit |= u01_below(o.v[0], o.v[1], limit);
+            }
+        }
+        if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
+            const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
+            if (at < L)
+                k.l.replay_list[at] = loc;
+            else
+                atomicOr(k.err, ERR_AGENT_LIST);
+        }
+        entries += dr.n;
+        hazard += any_h ? dr.n : 0u;
+    }
+    *n_entries += entries;
+    *n_hazard += hazard;
+}
+
+// The expected infections (and the adjoint's terms) of the segment's draws at
+// the locations that are not replayed: every timestep's are the same.
+__device__ void phase_expected(const KArgs& k, const DrawRun& dr, uint32_t n_listed, double* s_grad) {
+    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n_listed; base += stride) {  // block-uniform trips
+        const uint32_t pos = base + threadIdx.x;
+        const uint32_t loc = pos < n_listed && pos < N ? k.l.slot_loc[pos] : NONE;
+        const uint32_t i = loc < L ? k.l.csr_agents[pos] : NONE;
+        const bool act = loc < L && i < N && k.l.replay_stamp[loc] != dr.epoch;
+        uint32_t rep = 0;
+        double term = 0.0;
+        if (act) {
+            const uint32_t cnt = k.l.counts[loc];
+            const float wl = k.l.infectiousness[loc];
+            rep = k.l.rep[loc];
+            const float kf = k.r.k_f[rep];
+            for (uint32_t v = 0; v < V; ++v) {
+                float x;
+                const float h = entry_hazard(k, loc, v, cnt, wl, kf, dr.season, dt, &x);
+                if (!(h > 0.0f) || !k.r.variant_active[rep * V + v]) continue;
+                const float s_eff = k.l.slot_su[(size_t)v * N + pos];
+                if (!(s_eff > 0.0f)) continue;
+                const float pf = h * s_eff;
+                term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
+                if (k.adj.on && pf < 1.0f)
+                    adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x, dr.n);
+            }
+        }
+        if (k.track_expected) add_expected_rep(k, act, rep, term);
+    }
+}
+
+// The sum change of an agent at location loc infected there.
+__device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t loc, float inf0, uint32_t var0,
+                                                     float inf, uint32_t var) {
+    const uint32_t L = k.l.n;
+    const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
+    const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
+    if (q0 == q1 && var0 == var) return;
+    if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc], (unsigned long long)(-q0));
+    if (q1) {
+        atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
+        mark_hazardous(k, loc);
+    }
+}
+
+// One entry's draws of timestep t with its location's ratios s_h (arguments
+// s_x): the agent in slot pos.  An agent that is infected updates its slot's
+// susceptibility products (read by no other entry) and its location's sums,
+// which the ratios of the next timestep are computed from.  Adds the sum of
+// min(1, p) over its draws to *term when expected infections are tracked;
+// returns whether the agent was infected.
+__device__ __forceinline__ bool draw_entry(const KArgs& k, uint32_t pos, uint32_t i, uint32_t loc, uint32_t rep,
+                                           const RepConst& rc, uint32_t t, const float* s_h, const float* s_x,
+                                           double* s_grad, double* term) {
+    const uint32_t N = k.a.n, V = k.m.n_variants;
     bool infected = false;
     float inf0 = 0.0f, sigma = 0.0f;
     uint32_t var0 = 0;
     for (uint32_t v = 0; v < V; ++v) {
-        float x;
-        const float h = entry_hazard(k, sums, loc, v, cnt, wl, kf, season, dt, &x);
+        const float h = s_h[v];
         if (!(h > 0.0f)) continue;
-        *any_h = true;
         if (!k.r.variant_active[rep * V + v]) continue;
         // after an infection the later variants read the agent's new
         // susceptibility (what the slot then gets)
-        float s_eff;
-        if (!infected)
-            s_eff = v == 0 ? su0 : k.l.slot_su[(size_t)v * N + pos];
-        else
-            s_eff = k.a.susceptible[(size_t)v * N + i] * sigma;
+        const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.slot_su[(size_t)v * N + pos];
         if (!(s_eff > 0.0f)) continue;
         const float pf = h * s_eff;
-        if (k.track_expected) term += pf < 1.0f ? (double)pf : 1.0;
+        if (k.track_expected) *term += pf < 1.0f ? (double)pf : 1.0;
         if (k.adj.on && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x);
-        // the uniform of the stream (seed, agent, t, infection + v), as
-        // psim_u01_once draws it
-        psim_ctr4 c;
-        c.v[0] = li;
-        c.v[1] = t;
-        c.v[2] = PSIM_PHASE_INFECT + v;
-        c.v[3] = 0u;
-        const psim_ctr4 o = psim_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-        if (u01_below(o.v[0], o.v[1], pf)) {
+            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1u);
+        const psim_ctr4 o = infect_words(rc.seed, i - rc.off, t, v);
+        if (u01_below(o.v[0], o.v[1], u01_limit(pf))) {
             if (!infected) {
                 inf0 = k.a.infectious[i];
                 var0 = inf0 > 0.0f ? k.a.variant[i] : 0u;
@@ -1724,97 +1836,63 @@ __device__ __forceinline__ double draw_entry(const KArgs& k, const unsigned long
     if (infected) {
         for (uint32_t v = 0; v < V; ++v) k.l.slot_su[(size_t)v * N + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
         const float inf = k.a.infectious[i];
-        const uint32_t var = inf > 0.0f ? k.a.variant[i] : 0u;
-        const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
-        const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
-        if (q0 != q1 || var0 != var) record_infection(k, step, loc, inf0, var0, inf, var);
+        add_infection_change(k, loc, inf0, var0, inf, inf > 0.0f ? k.a.variant[i] : 0u);
     }
-    return term;
+    return infected;
 }
 
-// The draw phase: every entry of the agent list (the agents at the locations
-// the last rebuild listed, build[5] of them), one per thread, slots in order
-// (coalesced loads of the slot's location, agent and susceptibility
-// products).  Each entry evaluates its location's ratio from the location's
-// sum, count and weight (the same inputs give the same value at every entry)
-// and draws from the agent's Philox stream (seed, agent, t).  The work is the
-// listed entries, spread evenly over the grid, whatever the number of
-// locations.
-// First-trip slot of a thread (its slot, agent and variant-0 product),
-// loaded by the step's prologue with the step's words when the step does not
-// rebuild (its slots are then the last rebuild's).
-struct SlotPre {
-    uint32_t loc, i;
-    float su0;
-    bool ok;
-};
-__device__ __forceinline__ SlotPre slot_pre(const KArgs& k, bool draws) {
-    SlotPre p{NONE, NONE, 0.0f, false};
-    const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (draws && pos < k.a.n) {  // issued before the step's words arrive
-        p.loc = k.l.slot_loc[pos];
-        p.i = k.l.csr_agents[pos];
-        p.su0 = k.l.slot_su[pos];
-        p.ok = true;
-    }
-    return p;
-}
-
-__device__ void phase_draw(const KArgs& k, uint32_t step, uint32_t t, uint32_t n_listed, float season,
-                           const SlotPre& pre, double* s_grad, uint32_t* n_entries, uint32_t* n_hazard) {
-    const unsigned long long* sums = sums_read(k, step);
-    const uint32_t L = k.l.n, N = k.a.n;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const bool one_rep = k.r.n == 1;
-    const RepConst rc0 = rep_const(k, 0);
-    uint32_t entries = 0, hazard = 0;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n_listed; base += stride) {  // block-uniform trips
-        const uint32_t pos = base + threadIdx.x;
-        bool act = pos < n_listed && pos < N;
-        uint32_t loc = NONE, i = NONE, rep = 0, cnt = 0;
-        float wl = 0.0f, su0 = 0.0f;
-        if (act) {
-            const bool first = base == blockIdx.x * blockDim.x && pre.ok;
-            loc = first ? pre.loc : k.l.slot_loc[pos];
-            i = first ? pre.i : k.l.csr_agents[pos];
-            su0 = first ? pre.su0 : k.l.slot_su[pos];
-            if (loc >= L || i >= N) {
-                atomicOr(k.err, ERR_AGENT_LIST);
-                act = false;
-            } else {
-                cnt = k.l.counts[loc];
-                wl = k.l.infectiousness[loc];
-                rep = one_rep ? 0u : k.l.rep[loc];
-            }
+// The flagged locations' draws, a warp per location: its slots 32 at a time,
+// timestep after timestep.  The ratios are kept in shared memory and computed
+// again after a timestep that infected somebody there (all its draws first:
+// a timestep's ratios come from the sums as it started).
+__device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_replay, DayShared& sh) {
+    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a block's warps take locations far apart in the list: few locations
+    // spread over all SMs
+    for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
+        const uint32_t loc = k.l.replay_list[f];
+        if (loc >= L) {
+            if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
+            continue;
         }
-        bool any_h = false;
-        const double term =
-            act ? draw_entry(k, sums, step, pos, i, loc, rep, cnt, wl, su0, one_rep ? rc0 : rep_const(k, rep), season, t,
-                             s_grad, &any_h)
-                : 0.0;
-        entries += act ? 1u : 0u;
-        hazard += any_h ? 1u : 0u;
-        if (k.track_expected) add_expected_rep(k, act, rep, term);
-    }
-    *n_entries += entries;
-    *n_hazard += hazard;
-}
-
-// The infections of step s - 1 into the copy of the sums that step s does not
-// read (every thread of the grid takes a share; list (s - 1) % 3, complete
-// since the kernel of step s - 1 ended).  Block 0 also empties list
-// (s + 1) % 3, applied by step s - 1 and next written by step s + 1.
-__device__ __forceinline__ void apply_previous_infections(const KArgs& k, uint32_t step) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_INFECTIONS + (step + 1u) % 3u] = 0u;
-    if (step == 0) return;  // the day's first step: the sums are afresh
-    const uint32_t list = (step + 2u) % 3u;
-    const uint32_t n = min(k.l.bar[BAR_INFECTIONS + list], k.a.n);
-    unsigned long long* sums = sums_next(k, step);
-    // from the grid's last block down: the draws fill the first blocks
-    const uint32_t g = (gridDim.x - 1u - blockIdx.x) * blockDim.x + threadIdx.x;
-    for (uint32_t j = g; j < n; j += gridDim.x * blockDim.x) {
-        const uint4 e = k.l.inf_pending[(size_t)list * k.a.n + j];
-        add_infection_change(k, sums, e.x, __uint_as_float(e.y), e.w & 0xFFu, __uint_as_float(e.z), (e.w >> 8) & 0xFFu);
+        const uint32_t cnt = k.l.counts[loc], e = k.l.cursor[loc], b = e - cnt;  // the segment the rebuild filled
+        if (e > N || cnt > e) {
+            if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
+            continue;
+        }
+        const float wl = k.l.infectiousness[loc];
+        const uint32_t rep = k.l.rep[loc];
+        const RepConst rc = rep_const(k, rep);
+        double term = 0.0;
+        bool stale = true;  // the ratios: at the start and after an infection
+        for (uint32_t j = 0; j < dr.n; ++j) {
+            if (stale) {
+                __syncwarp();
+                if ((uint32_t)lane < V) {
+                    // past L1: other lanes' reductions changed it in L2
+                    const long long fix = (long long)__ldcg(&k.l.sfix[(size_t)lane * L + loc]);
+                    float x = 0.0f;
+                    sh.h[warp][lane] = fix != 0 ? psim_hazard_x(fix, cnt, rc.kf, wl, dr.season, dt, &x) : 0.0f;
+                    sh.x[warp][lane] = x;
+                }
+                __syncwarp();
+            }
+            bool infected = false;
+            for (uint32_t p0 = b; p0 < e; p0 += 32u) {
+                const uint32_t pos = p0 + (uint32_t)lane;
+                if (pos >= e) break;
+                const uint32_t i = k.l.csr_agents[pos];
+                if (i >= N) {
+                    atomicOr(k.err, ERR_AGENT_LIST);
+                    break;
+                }
+                infected |= draw_entry(k, pos, i, loc, rep, rc, dr.t + j, sh.h[warp], sh.x[warp], sh.grad, &term);
+            }
+            __threadfence();
+            stale = __any_sync(0xffffffffu, infected);
+        }
+        if (k.track_expected) add_expected_rep(k, true, rep, term);
     }
 }
 
@@ -1884,8 +1962,7 @@ __device__ __forceinline__ uint32_t phase_queue(const KArgs& k, uint32_t s1, uin
 // count the queue left in shared memory: every block starts its decisions at
 // the same barrier, so handing segments out by ticket balanced nothing), then
 // the histogram and sum deltas of the agents that took a new location.
-__device__ void phase_decide(const KArgs& k, uint32_t step, uint32_t cap, uint32_t* s_mm, const uint32_t* s_cnt) {
-    const uint32_t s1 = step + 1;
+__device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t* s_mm, const uint32_t* s_cnt) {
     const StepClock c = step_clock(k, s1);
     bool moved = false;
     {
@@ -1910,12 +1987,17 @@ __device__ void phase_decide(const KArgs& k, uint32_t step, uint32_t cap, uint32
                 // every queued agent decides: its inputs load at once
                 DecisionIn d;
                 decision_in(k, i, d);
-                const uint32_t m0 = k.a.move_at[i];
-                const uint32_t vr = k.a.variant[i];
+                d.w = k.a.dinfo[i];
                 loc0 = d.loc;
-                inf = d.inf;
-                if (inf > 0.0f) var = vr;
-                loc = move_agent(k, i, c, m0 - c.t, s_mm, &d, loc0);
+                // (queued for its timestamp, unless everybody is at the curfew)
+                const uint32_t s = c.curfew_now ? k.a.move_at[i] - c.t : 0u;
+                uint32_t w;
+                loc = move_agent(k, i, c, s, s_mm, d, &w);
+                if (w != d.w) k.a.dinfo[i] = w;
+                if (w & DW_INFECTIOUS) {
+                    inf = k.a.infectious[i];
+                    var = k.a.variant[i];
+                }
             }
             moved |= count_agent_delta(k, act, loc0, loc, inf, var, inf, var);
         }
@@ -1923,55 +2005,56 @@ __device__ void phase_decide(const KArgs& k, uint32_t step, uint32_t cap, uint32
     publish_moved(k, moved, c.t);
 }
 
-// Block-shared scratch of the step kernel.
-struct StepShared {
-    double grad[GRAD_N];
-    uint32_t mm[MOVE_MASK_WORDS];
-    uint32_t red[32];
-    uint32_t cnt, base;
-    bool ok;
-};
-
-// One timestep of the step kernel (see the section comment); false when a
-// grid barrier expired (the kernel then ends).  cap = the work-list segment
-// size of a block.
-__device__ __forceinline__ bool step_body(const KArgs& k, uint32_t step, uint32_t phases, uint32_t cap,
-                                          StepShared& sh) {
-    const uint32_t tl = PROF_T + PROF_TW * step;  // the step's timeline slots (profiled graph)
+// One segment of the day (see the section comment), starting at timestep
+// `step`; *next receives the timestep the next one starts at (step_end after
+// the last).  False when a grid barrier expired (the kernel then ends).  cap =
+// the work-list segment size of a block.
+__device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint32_t step_end, uint32_t phases,
+                                            uint32_t cap, DayShared& sh, uint32_t* next) {
+    const uint32_t tl = PROF_T + PROF_TW * step;  // the segment's timeline slots (profiled graph)
     prof_enter(k, tl);
-    // the words the step's phases start from, loaded together: the error
-    // flags, the clock, the rebuild words (a block that starts after block 0
-    // turned BUILD_PENDING into t decides the same), the step of the last
-    // quarantine writes, the decision-mask word of the next step (the
-    // decisions of this step mark later steps only)
-    const uint32_t err0 = *((volatile uint32_t*)k.err);
-    const uint32_t t0 = k.clock->t0;
-    const float season = k.clock->season;
+    const uint32_t t = k.clock->t0 + step;
     const uint32_t moved = k.l.build[0], force = k.l.build[1], q_step = k.l.build[3];
-    uint32_t n_listed = k.l.build[5];  // the last rebuild's entries (this step's if it rebuilds)
-    const uint32_t s1 = step + 1;
-    const uint32_t mm_word = s1 < k.spd ? k.a.move_mask[s1 >> 5] : 0u;
-    // the first-trip slots of the draws, loaded with the words above; used
-    // only when this launch does not rebuild them (moved / force as read)
-    SlotPre pre = slot_pre(k, (phases & PH_DRAW) != 0);
-    const uint32_t t = t0 + step;
-    if ((phases & PH_REBUILD) && (moved == t || force == t || force == BUILD_PENDING)) pre.ok = false;
-    if (err0 & ERR_BARRIER) return false;  // an earlier barrier expired
+    uint32_t n_listed = k.l.build[5];  // the last rebuild's entries (this segment's if it rebuilds)
+    DrawRun dr;
+    dr.t = t;
+    dr.epoch = k.l.build[6] + 1u;  // (0 is the stamp of a location never flagged)
+    dr.season = k.clock->season;
+    // the segment's end: the first later timestep that somebody decides at
+    // (everyone at the curfew)
+    uint32_t e = step + 1;
+    bool decides = false;
+    while (e < k.spd) {
+        uint32_t w = k.a.move_mask[e >> 5] >> (e & 31u);
+        if (k.p.enable_curfew && k.p.curfew_begin >= e && k.p.curfew_begin >> 5 == e >> 5)
+            w |= 1u << (k.p.curfew_begin - e);
+        if (w) {
+            e += (uint32_t)(__ffs(w) - 1);
+            decides = e < k.spd;
+            break;
+        }
+        e = (e & ~31u) + 32u;
+    }
+    if (!decides) e = k.spd;
+    // (a caller's shorter range ends the draws, not the decisions after them)
+    dr.n = min(e, step_end) - step;
+    decides = decides && e <= step_end && (phases & PH_DECIDE);
+    *next = min(e, step_end);
+    bool merged = false;
     if (phases & PH_REBUILD) {
-        const bool rebuild = csr_decide_from(k, t, moved, force);
-        if (rebuild) {
+        if (csr_decide_from(k, t, moved, force)) {
             if (k.prof && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
-            if (!phase_rebuild(k, sums_read(k, step), sh.red, &sh.ok, tl, &sh.base, &n_listed)) return false;
+            if (!phase_rebuild(k, sh, tl, &n_listed)) return false;
             prof_mark(k, tl + 2);
         }
-        // the step's location quarantine writes (decisions of step t)
-        if (k.p.quarantine_policy > 1 && q_step == t) merge_quarantine(k);
+        // the location quarantine writes of the decisions for t
+        merged = k.p.quarantine_policy > 1 && q_step == t;
+        if (merged) merge_quarantine(k);
     }
-    if (phases & PH_DRAW) {
-        apply_previous_infections(k, step);
-        grad_begin(k, sh.grad);
+    const bool draws = (phases & PH_DRAW) && n_listed > 0;
+    if (draws) {
         uint32_t entries = 0, hazard = 0;
-        phase_draw(k, step, t, n_listed, season, pre, sh.grad, &entries, &hazard);
+        phase_draw(k, dr, n_listed, &entries, &hazard);
         if (k.prof) {
             entries = __reduce_add_sync(0xffffffffu, entries);
             hazard = __reduce_add_sync(0xffffffffu, hazard);
@@ -1980,36 +2063,57 @@ __device__ __forceinline__ bool step_body(const KArgs& k, uint32_t step, uint32_
                 atomicAdd(&k.prof[PROF_DRAW_HAZARD], (unsigned long long)hazard);
             }
         }
-        grad_end(k, sh.grad);
-        prof_mark(k, tl + 3);
     }
-    const bool decides = (k.p.enable_curfew && k.p.curfew_begin == s1) || ((mm_word >> (s1 & 31u)) & 1u) != 0;
-    if ((phases & PH_DECIDE) && s1 < k.spd && decides) {
+    prof_mark(k, tl + 3);
+    if (decides) {
         mask_clear_shared(sh.mm);
-        const uint32_t n = phase_queue(k, step + 1, cap, &sh.cnt);
+        const uint32_t n = phase_queue(k, e, cap, &sh.cnt);
         if (k.prof && threadIdx.x == 0) {
             if (n) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)n);
             if (blockIdx.x == 0) atomicAdd(&k.prof[PROF_QUEUE_STEPS], 1ull);
         }
         prof_mark(k, tl + 4);
-        // every draw and every block's queue before any decision
-        if (!grid_barrier(k, &sh.ok)) return false;
-        phase_decide(k, step, cap, sh.mm, &sh.cnt);
+    }
+    // every draw before any replay, every draw and merge before any decision
+    if ((draws || (merged && decides)) && !grid_barrier(k, sh)) return false;
+    if (draws) {
+        const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
+        const bool expected = k.track_expected || k.adj.on;
+        if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
+        if (n_replay || expected) {
+            grad_begin(k, sh.grad);
+            phase_replay(k, dr, n_replay, sh);
+            if (expected) phase_expected(k, dr, n_listed, sh.grad);
+            grad_end(k, sh.grad);
+            if (decides || n_replay) {
+                // every replay before any decision and before the list is emptied
+                if (!grid_barrier(k, sh)) return false;
+                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = 0u;
+            }
+        }
+        prof_mark(k, tl + 5);
+    }
+    if (decides) {
+        phase_decide(k, e, cap, sh.mm, &sh.cnt);
         mask_flush(k, sh.mm);
     }
-    prof_mark(k, tl + 5);
+    prof_mark(k, tl + 6);
     return true;
 }
 
-// The step kernel: timesteps step0 .. step0 + nsteps - 1, a grid barrier
-// between two (the day graph launches it per timestep, or for the whole day
-// with tuning variant 4).
-__global__ void __launch_bounds__(256, 4) k_step(KArgs k, uint32_t step0, uint32_t nsteps, uint32_t phases,
-                                                 uint32_t cap) {
-    __shared__ StepShared sh;
-    for (uint32_t j = 0; j < nsteps; ++j) {
-        if (!step_body(k, step0 + j, phases, cap, sh)) return;
-        if (j + 1 < nsteps && !grid_barrier(k, &sh.ok)) return;
+// The day kernel: timesteps step0 .. step_end - 1.
+__global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0, uint32_t step_end, uint32_t phases,
+                                                        uint32_t cap) {
+    __shared__ DayShared sh;
+    if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
+    if (threadIdx.x == 0) sh.target = gridDim.x;
+    uint32_t step = step0;
+    for (;;) {
+        uint32_t next = step_end;
+        if (!day_segment(k, step, step_end, phases, cap, sh, &next)) return;
+        if (next >= step_end) return;
+        step = next;
+        if (!grid_barrier(k, sh)) return;
     }
 }
 
@@ -2694,40 +2798,53 @@ static unsigned agent_grid(const KArgs& k, unsigned wave) {
     return std::min(g, grid_for(k.a.n, 1 << 20));
 }
 
-void launch_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
+void launch_movement(const KArgs& k, uint32_t step, bool day, cudaStream_t s) {
     static unsigned g = 0;
     if (!g) g = wave_grid(k_movement, 1u << 30);
-    k_movement<<<agent_grid(k, g), 256, 0, s>>>(k, step);
+    k_movement<<<agent_grid(k, g), 256, 0, s>>>(k, step, day ? 1 : 0);
 }
-// The step kernel's grid: every block resident at once (its grid barriers
-// need that), tune.blocks_per_sm capped at the kernel's occupancy, and no
-// more blocks than the population and locations give work to.  Each block's
-// work-list segment holds the agents its queue pass visits.
-static unsigned step_blocks_per_sm() {
+// The day kernel's grid: every block resident at once (its grid barriers
+// need that, and the cooperative launch checks it), tune.blocks_per_sm (in
+// blocks of 256 threads) capped at the kernel's occupancy, and no more blocks
+// than the population and locations give work to.  Each block's work-list
+// segment holds the agents its queue pass visits.
+static unsigned day_blocks_per_sm() {
     static int occ = 0;
     if (!occ) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step, 256, 0) != cudaSuccess || occ < 1) occ = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_day, DAY_THREADS, 0) != cudaSuccess || occ < 1) occ = 1;
     }
     return (unsigned)occ;
 }
-static void step_geometry(const KArgs& k, unsigned* grid, uint32_t* cap) {
-    const unsigned occ = step_blocks_per_sm();
-    const unsigned bps = k.tune.blocks_per_sm ? std::min<unsigned>(k.tune.blocks_per_sm, occ) : occ;
-    const size_t want = std::max<size_t>(((size_t)k.a.n + 255) / 256, (((size_t)k.l.n + 31) / 32 + 7) / 8);
+static void day_geometry(const KArgs& k, unsigned* grid, uint32_t* cap) {
+    const unsigned occ = day_blocks_per_sm();
+    const unsigned bps = k.tune.blocks_per_sm
+                             ? std::min<unsigned>((k.tune.blocks_per_sm * 256u + DAY_THREADS - 1) / DAY_THREADS, occ)
+                             : occ;
+    const size_t want = std::max<size_t>(((size_t)k.a.n + DAY_THREADS - 1) / DAY_THREADS,
+                                         (((size_t)k.l.n + 31) / 32 + DAY_THREADS / 32 - 1) / (DAY_THREADS / 32));
     unsigned g = (unsigned)std::min<size_t>((size_t)sm_count() * bps, std::max<size_t>(want, 1));
-    g = std::min(g, (unsigned)WORK_MAX_BLOCKS);
+    g = std::min(g, (unsigned)(WORK_MAX_THREADS / DAY_THREADS));
     *grid = g;
-    // the queue's quads: ceil(quads / (g * 256)) per thread, 4 agents each
-    const size_t quads = ((size_t)k.a.n + 3) / 4;
-    *cap = (uint32_t)(((quads + (size_t)g * 256 - 1) / ((size_t)g * 256)) * 1024);
+    // the queue's quads: ceil(quads / (g * threads)) per thread, 4 agents each
+    const size_t quads = ((size_t)k.a.n + 3) / 4, threads = (size_t)g * DAY_THREADS;
+    *cap = (uint32_t)(((quads + threads - 1) / threads) * DAY_THREADS * 4);
 }
-void launch_steps(const KArgs& k, uint32_t step0, uint32_t nsteps, uint32_t phases, cudaStream_t s) {
+void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s) {
     unsigned g;
     uint32_t cap;
-    step_geometry(k, &g, &cap);
-    k_step<<<g, 256, 0, s>>>(k, step0, nsteps, phases, cap);
+    day_geometry(k, &g, &cap);
+    cudaMemsetAsync(k.l.bar, 0, sizeof(uint32_t), s);  // the barrier's arrivals
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g);
+    cfg.blockDim = dim3(DAY_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_day, k, step0, step_end, phases, cap);
 }
-void launch_step(const KArgs& k, uint32_t step, uint32_t phases, cudaStream_t s) { launch_steps(k, step, 1, phases, s); }
 void launch_count(const KArgs& k, cudaStream_t s) { k_count<<<grid_for(k.a.n, 8), 256, 0, s>>>(k); }
 // the scan of the histogram with 256 x tune.scan_items locations per tile:
 // single pass with decoupled look-back (tune.scan_mode 0) or tile sums, then

@@ -121,12 +121,23 @@ PSIM_HD uint32_t psim_next_u32(psim_stream* s) {
         s->blk += 1;
         s->idx = 0;
     }
-    return s->buf[s->idx++];
+    // selected, not indexed: a run-time index would keep the stream in
+    // (local) memory
+    const uint32_t q = s->idx;
+    s->idx = q + 1;
+    return q == 0 ? s->buf[0] : q == 1 ? s->buf[1] : q == 2 ? s->buf[2] : s->buf[3];
 }
 
 // 53-bit uniform double in [0, 1).
 PSIM_HD double psim_u01_from(uint32_t a, uint32_t b) {
     return ((double)(a >> 5) * 67108864.0 + (double)(b >> 6)) * (1.0 / 9007199254740992.0);
+}
+
+// The same uniform as the integer K = U * 2^53.
+PSIM_HD uint64_t psim_u53(psim_stream* s) {
+    const uint32_t a = psim_next_u32(s);
+    const uint32_t b = psim_next_u32(s);
+    return ((uint64_t)(a >> 5) << 26) | (uint64_t)(b >> 6);
 }
 
 PSIM_HD double psim_u01(psim_stream* s) {

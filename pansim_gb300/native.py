@@ -302,17 +302,17 @@ class GpuSim:
 
     def day_kernel_ms(self):
         """Of the last profiled day, from the kernels' timeline stamps: the
-        first movement kernel, the step kernel's rebuilds, draws, queues +
-        decisions, and the time between the kernels (ms, summed)."""
+        first movement kernel, the day kernel's rebuilds, draws, queues +
+        decisions, and the time between its segments (ms, summed)."""
         ms = np.zeros(5, np.float32)
         self._ck(lib().psim_day_kernel_ms(self.h, _p(ms)), "day_kernel_ms")
         return ms
 
     def day_timeline(self):
-        """Per step of the last profiled day (rows), microseconds: the step
-        kernel's span, its rebuild's listing and slots, the draws, the queue,
-        the decisions (0 where the phase did not run), the time since the
-        previous kernel ended."""
+        """Per step of the last profiled day (rows), microseconds: the step's
+        span, its rebuild's listing and slots, the draws (a segment's, divided
+        among its steps), the queue, the decisions (0 where the phase did not
+        run), the time since the previous segment ended."""
         us = np.zeros((self.snap.steps_per_day, 7), np.float32)
         self._ck(lib().psim_day_timeline(self.h, _p(us)), "day_timeline")
         return us

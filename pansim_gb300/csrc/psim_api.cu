@@ -644,10 +644,15 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     if ((rc = dalloc(c, &dl.csr_off, L + 1))) return bail(rc);
     if ((rc = dalloc(c, &dl.cursor, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.csr_agents, N))) return bail(rc);
-    if ((rc = dalloc(c, &dl.slot_loc, N))) return bail(rc);
     if ((rc = dalloc(c, &dl.replay_stamp, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.replay_list, L))) return bail(rc);
-    if ((rc = dalloc(c, &dl.slot_su, N * V))) return bail(rc);
+    if ((rc = dalloc(c, &dl.replay_cursor, L))) return bail(rc);
+    if ((rc = dalloc(c, &dl.replay_slot, N))) return bail(rc);
+    dl.list_cap = N + (size_t)WORK_MAX_THREADS * 4 + 4;
+    if ((rc = dalloc(c, &dl.list_agent, dl.list_cap))) return bail(rc);
+    if ((rc = dalloc(c, &dl.list_loc, dl.list_cap))) return bail(rc);
+    if ((rc = dalloc(c, &dl.list_su, dl.list_cap * V))) return bail(rc);
+    if ((rc = dalloc(c, &dl.list_count, WORK_MAX_BLOCKS))) return bail(rc);
     if ((rc = dalloc(c, &dl.qu_pending, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.sfix, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hazard, L * V))) return bail(rc);
@@ -1299,12 +1304,13 @@ static int read_timeline(psim_ctx* c, std::vector<unsigned long long>& h) {
 }
 
 // Per step of the profiled day, in microseconds (TL_COLS values): the
-// step's span, the rebuild's listing, its slots, the draws, the queue, the
+// step's span, 0 (the rebuild has no listing of its own), the lists of a
+// rebuild, the draws, the work list of a segment without a rebuild, the
 // decisions (0 where the phase did not run), and the time since the previous
 // segment's last exit.  The day kernel draws a segment's timesteps together:
-// their time (with the replay's) is divided among them; the rebuild and the
-// gap belong to the segment's first step, the queue and the decisions to its
-// last one, the step before the one they decide for.
+// their time (with the replay's) is divided among them; the lists and the
+// gap belong to the segment's first step, the decisions to its last one, the
+// step before the one they decide for.
 constexpr int TL_COLS = 7;
 static void step_times(psim_ctx* c, const std::vector<unsigned long long>& h, float* us) {
     auto dur = [](unsigned long long a, unsigned long long b) { return b > a ? (float)((double)(b - a) * 1e-3) : 0.0f; };
@@ -1314,24 +1320,19 @@ static void step_times(psim_ctx* c, const std::vector<unsigned long long>& h, fl
         const unsigned long long* T = &h[PROF_T + PROF_TW * (size_t)s];
         uint32_t e = s + 1;
         while (e < c->spd && h[PROF_T + PROF_TW * (size_t)e] == 0ull) ++e;
-        const unsigned long long t0 = ~T[0], lst = T[1], slt = T[2], drw = T[3], que = T[4], rep = T[5], end = T[6];
-        const unsigned long long qd = que ? que : drw;
-        float draw = dur(slt ? slt : t0, drw);
-        if (rep) draw += dur(qd, rep);
-        if (!que) draw += dur(rep ? rep : drw, end);
+        const unsigned long long t0 = ~T[0], listed = T[1], queued = T[2], rep = T[4], end = T[5];
+        // (a block stamps a phase that it leaves at once before others enter it)
+        const unsigned long long t1 = listed ? listed : queued ? queued : t0;
         for (uint32_t q = s; q < e; ++q) {
             float* o = us + TL_COLS * (size_t)q;
             for (int j = 0; j < TL_COLS; ++j) o[j] = 0.0f;
-            o[3] = draw / (float)(e - s);
+            o[3] = dur(t1, rep) / (float)(e - s);
             if (q == s) {
-                o[1] = lst ? dur(t0, lst) : 0.0f;
-                o[2] = slt ? dur(lst, slt) : 0.0f;
+                o[2] = listed ? dur(t0, listed) : 0.0f;
+                o[4] = queued ? dur(t0, queued) : 0.0f;
                 o[6] = dur(prev, t0);
             }
-            if (q + 1 == e && que) {
-                o[4] = dur(drw, que);
-                o[5] = dur(rep ? rep : que, end);
-            }
+            if (q + 1 == e && e < c->spd) o[5] = dur(rep, end);
             o[0] = o[1] + o[2] + o[3] + o[4] + o[5];
         }
         prev = end;

@@ -147,8 +147,6 @@ struct DevLocs {
     uint32_t* cursor;             // [n] next free CSR slot of each location (scan: first slot)
     uint32_t* csr_off;            // [n+1] CSR offsets, derived from the cursors on demand
     uint32_t* csr_agents;         // [N]
-    float* slot_su;               // [V][N] beside each agent-list slot: the agent's susceptibility
-                                  // to the variant times its age band's factor
     uint32_t* qu_pending;         // quarantine writes of the running step
     unsigned long long* sfix;     // [V][n] fixed-point infectiousness sums
     float* hazard;                // [V][n] infection ratio of the last step
@@ -160,9 +158,17 @@ struct DevLocs {
     uint32_t* tile_sums;          // per-tile sums of the histogram (two-pass scan)
     uint32_t* bar;                // the day kernel's grid barrier ([0] arrivals), the count of the
                                   // replay list, the listing counter
-    uint32_t* slot_loc;           // [N] the location of each agent-list slot the day kernel listed
+    // the day kernel's agent list, a segment per block: agent, location,
+    // susceptibility to the variant times its age band's factor
+    uint32_t* list_agent;         // [list_cap]
+    uint32_t* list_loc;           // [list_cap]
+    float* list_su;               // [V][list_cap]
+    size_t list_cap;
+    uint32_t* list_count;         // [WORK_MAX_BLOCKS] entries of each block's segment
     uint32_t* replay_stamp;       // [n] the last segment of draws that flagged the location
     uint32_t* replay_list;        // [n] the locations the running segment flagged
+    uint32_t* replay_cursor;      // [n] next free place of a flagged location in replay_slot
+    uint32_t* replay_slot;        // [N] the flagged locations' list entries, by location
     uint64_t* scan_status;        // per-tile status words of the single-pass scan (epoch | flag | value)
     uint32_t* scan_state;         // [0] epoch of the next single-pass scan, [1] its tile ticket
     uint32_t* build;              // [0] timestamp at which agents last took new locations,
@@ -172,8 +178,6 @@ struct DevLocs {
                                   //     the step's first scan kernel, read by its later kernels),
                                   // [3] the timestamp of the last step whose decisions wrote a
                                   //     location quarantine (merged by that step's scan),
-                                  // [5] the agent-list entries the day kernel's last rebuild
-                                  //     listed
                                   // [6] the stamp of the last segment of draws (counts segments
                                   //     over the context's lifetime, so a replayed day never meets
                                   //     its own stamps)
@@ -251,12 +255,12 @@ enum {
     // maximum of complements, so one zero fill starts every slot):
     // [PROF_N] ~first block entry of the day's first movement, [PROF_N + 1]
     // its last block exit; per segment of the day, at PROF_T + PROF_TW * (its
-    // first step): ~first block entry, the last block past the rebuild's
-    // listing, past its slots, past the draws, past the queue, past the
-    // replay, last block exit (slots of phases the segment did not run and of
-    // steps that start no segment stay 0).
+    // first step): ~first block entry, the last block past the lists of a
+    // rebuild, past those of a segment without one (the work list alone), past
+    // the draws, past the replay, last block exit (slots of phases the segment
+    // did not run and of steps that start no segment stay 0).
     PROF_T = PROF_N + 2,
-    PROF_TW = 7,
+    PROF_TW = 6,
     PROF_WORDS = PROF_T + PROF_TW * 1440
 };
 
@@ -346,13 +350,13 @@ constexpr uint32_t PH_REBUILD = 1u, PH_DRAW = 2u, PH_DECIDE = 4u, PH_ALL = 7u;
 void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s);
 void launch_time_shift(uint32_t* a, uint32_t n, uint32_t delta, cudaStream_t s);
 // words of the barrier array: the barrier's arrivals, the count of the replay
-// list, the rebuild's listing counter (slots reserved so far); the arrivals
-// in a line of their own
+// list and the entries of its locations; the arrivals in a line of their own
 constexpr uint32_t BAR_REPLAY = 32;
-constexpr uint32_t BAR_LISTED = 33;
+constexpr uint32_t BAR_REPLAY_SLOTS = 33;
 constexpr uint32_t BAR_WORDS = 64;
-// threads of the day kernel at most (work-list segments)
+// threads and blocks of the day kernel at most (segments of the lists)
 constexpr uint32_t WORK_MAX_THREADS = 160u * 2048u;
+constexpr uint32_t WORK_MAX_BLOCKS = WORK_MAX_THREADS / 128u;
 // words of the per-day mask of decision steps (1440 steps of one minute at most)
 constexpr uint32_t MOVE_MASK_WORDS = 48;
 

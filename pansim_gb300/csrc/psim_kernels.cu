@@ -1300,23 +1300,26 @@ __global__ void __launch_bounds__(256) k_scatter_draw(KArgs k, uint32_t step, in
 // Most timesteps of a day move nobody (at 2M agents 22 of 144 have deciders),
 // so the day is cut into segments: the timesteps from one whose agents took
 // new locations to the next that somebody decides at.  Per segment:
-//   rebuild   when agents took new locations (or a rebuild is pending): the
-//             locations with a nonzero sum listed and their segments reserved |
-//             every agent at a listed location takes a slot, which keeps its
-//             id, its susceptibility x age-band factor of every variant and
-//             its location.  The location quarantine writes of the decisions
-//             before are merged here too (or alone when nobody moved).
+//   list      one pass over the block's agents: when agents took new locations
+//             (or a rebuild is pending) those at a location with a nonzero sum
+//             enter the block's agent list (their id, location and
+//             susceptibility x age-band factor of every variant); those that
+//             decide at the segment's end enter the block's work list.  The
+//             location quarantine writes of the decisions before are merged
+//             here too.
 //   draw      every listed entry, one per thread, for all the timesteps of the
 //             segment at once: nobody moves, so a location's infection ratio
 //             stays what it is until somebody there is infected.  An entry
 //             that would be infected commits nothing: it flags its location |
+//             if any was flagged, their entries gathered by location |
 //             the flagged locations (a few) replayed exactly, a warp each,
 //             timestep by timestep with the ratio of the location's sum as the
 //             timestep started (LocationsList::infectAgents,
 //             locationList.h:233-310)
-//   decide    the block queues its own agents that decide at the segment's end
-//             | doMovement of the queued agents and the histogram and sum
-//             deltas of their moves
+//   decide  | doMovement of the queued agents and the histogram and sum deltas
+//             of their moves |
+// (| a grid barrier).  A block lists, draws and decides its own agents, so
+// nothing but the flagged locations and the moves passes between blocks.
 // What it replaces drew every timestep in a launch of its own (2.9-5.8 us and
 // a launch gap of 0.9-1.3 us each at 10k-2M agents, ~100 timesteps of a day).
 
@@ -1352,7 +1355,8 @@ struct DayShared {
     uint32_t mm[MOVE_MASK_WORDS];
     uint32_t red[32];
     uint32_t target;  // the barrier count the next barrier waits for
-    uint32_t cnt, base;
+    uint32_t cnt;     // agents in the block's work list
+    uint32_t listed;  // entries of the block's agent list
     bool ok;
 };
 
@@ -1380,34 +1384,6 @@ __device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
     return sh.ok;
 }
 
-// Slot data of the agent list: csr_agents[pos] = agent, slot_su[v][pos] =
-// its susceptibility to variant v times its age band's factor (the product
-// the draw compares with), written when the list is rebuilt and by the draw
-// that infects the agent.
-__device__ __forceinline__ void slot_fill(const KArgs& k, uint32_t pos, uint32_t i) {
-    const uint32_t N = k.a.n;
-    if (pos >= N) {
-        atomicOr(k.err, ERR_LOCATION);
-        return;
-    }
-    k.l.csr_agents[pos] = i;
-    const float sigma = k.p.sigma_band[k.a.band[i]];
-    for (uint32_t v = 0; v < k.m.n_variants; ++v)
-        k.l.slot_su[(size_t)v * N + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
-}
-
-// the sum of v over the block's threads; every thread calls it
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = __reduce_add_sync(0xffffffffu, v);
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    uint32_t tot = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) tot += s_red[q];
-    __syncthreads();
-    return tot;
-}
-
 // the location quarantine writes of the last decisions into quarantine_until
 // (grid-stride)
 __device__ __forceinline__ void merge_quarantine(const KArgs& k) {
@@ -1421,143 +1397,65 @@ __device__ __forceinline__ void merge_quarantine(const KArgs& k) {
     }
 }
 
-// Rebuild of the agent list.  Only the locations with a nonzero sum are
-// listed, because the draws of every step until the next rebuild need no
-// other location: until then no other location gains a nonzero sum (nobody
-// moves, since a move makes the next step rebuild, and a draw infects only
-// agents at a location with a nonzero sum).  The hazard mask is a superset of
-// those locations (every kernel that adds an infectious term sets the bit at
-// once); the listing clears the bits of the locations whose sums are zero
-// again.  The listed locations' agents fill the first *n_listed slots, each
-// slot with its agent, susceptibility products and location; the order of
-// the locations' segments is the order in which their blocks reserved them
-// (the draws do not depend on it).  In two parts between grid barriers:
-// 1 (listing): each warp takes groups of mask words, a lane per location of
-// a nonzero word and LIST_BATCH words at a time in flight: once to clear the
-// bits of zero sums and add up the listed agents (one atomic on the listing
-// counter reserves the block's slots), once more for each listed location's
-// first slot (cursor).  A thread per word, the set bits of a word one after
-// another, took 9.5 us at 2M agents and 22 us with 3% infected; 2 (slots):
-// every agent at a listed location takes a slot (one returning atomic on the
-// location's cursor, or one per location and warp with agg_slot).  Returns
-// false when a barrier expired.
-constexpr int LIST_BATCH = 4;
 __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
     bool nz = k.l.sfix[l] != 0ull;
     for (uint32_t v = 1; v < k.m.n_variants && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
     return nz;
 }
-__device__ bool phase_rebuild(const KArgs& k, DayShared& sh, uint32_t tl, uint32_t* n_listed) {
-    const uint32_t L = k.l.n, N = k.a.n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t n_words = (L + 31u) >> 5;
-    // the warps take the words in groups of up to 8 (a sector), dealt in turn:
-    // the words of a busy type of location, which lie together, are many warps'
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5), wg = (uint32_t)warp * gridDim.x + blockIdx.x;
-    uint32_t lg = 0;
-    while (lg < 3u && (n_words >> (lg + 1u)) >= warps) ++lg;
-    const uint32_t per = 32u >> lg;                           // groups of a warp's trip
-    const uint32_t groups = (n_words + (1u << lg) - 1u) >> lg;  // of the whole mask
-    const auto word_of = [&](uint32_t trip, int src) {
-        return ((((trip * per + ((uint32_t)src >> lg)) * warps + wg) << lg) | ((uint32_t)src & ((1u << lg) - 1u)));
-    };
-    const uint32_t trips = groups > wg ? ((groups - wg + warps - 1u) / warps + per - 1u) / per : 0u;
-    // 1: the agents at the locations that stay listed
-    uint32_t locs = 0, agents = 0;
-    for (uint32_t trip = 0; trip < trips; ++trip) {
-        const uint32_t w = word_of(trip, lane);
-        const uint32_t hm = w < n_words ? k.l.hmask[w] : 0u;
-        unsigned rest = __ballot_sync(0xffffffffu, hm != 0u);
-        while (rest) {
-            uint32_t m[LIST_BATCH], c[LIST_BATCH], at[LIST_BATCH];
-            bool nz[LIST_BATCH];
-#pragma unroll
-            for (int u = 0; u < LIST_BATCH; ++u) {
-                const int src = rest ? __ffs(rest) - 1 : 0;
-                const uint32_t word = __shfl_sync(0xffffffffu, hm, src);
-                at[u] = word_of(trip, src);
-                m[u] = rest ? word : 0u;
-                if (rest) rest &= rest - 1u;
-                const uint32_t l = at[u] * 32u + (uint32_t)lane;
-                const bool in = ((m[u] >> lane) & 1u) && l < L;
-                nz[u] = in && nonzero_sum(k, l);
-                c[u] = in ? k.l.counts[l] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < LIST_BATCH; ++u) {
-                const unsigned keep = __ballot_sync(0xffffffffu, nz[u]);
-                if (lane == 0 && keep != m[u]) k.l.hmask[at[u]] = keep;
-                if (nz[u]) agents += c[u];
-                locs += nz[u] ? 1u : 0u;
-            }
-        }
-    }
-    // the warp's and the block's agents, the block's slots
-    uint32_t inc = agents;
+
+// Where a warp's lanes put the entries they flagged (bits of `flags`, one
+// per agent of the lane) in a block's list: the first one's place (one
+// shared-memory atomic per warp).
+__device__ __forceinline__ uint32_t list_place(uint32_t flags, uint32_t* s_cnt) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t mine = __popc(flags);
+    uint32_t inc = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
     }
-    if (lane == 31) sh.red[warp] = inc;
+    uint32_t base = 0;
+    if (lane == 31 && inc) base = atomicAdd(s_cnt, inc);
+    return __shfl_sync(0xffffffffu, base, 31) + inc - mine;
+}
+
+// The block's lists of its own agents (four consecutive agents per thread,
+// one 16-byte load of a field, two quads in flight; the blocks' quads are
+// dealt in turn).  list: the agent list afresh.  Only the agents at locations
+// with a nonzero sum are listed, because the draws of every step until the
+// next listing need no other location: until then no other location gains a
+// nonzero sum (nobody moves, since a move makes the next segment list again,
+// and a draw infects only agents at a location with a nonzero sum).  The
+// hazard mask is a superset of those locations (every kernel that adds an
+// infectious term sets the bit at once); an agent that finds a zero sum behind
+// its location's bit clears it.  Agents of one location lie in many blocks'
+// lists: the replay gathers those it needs, so no location needs a segment of
+// its own (reserving segments first, a pass over the mask, a barrier and a
+// returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
+// 20M).  queue: the work list of those that decide at s1.
+__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, uint32_t s1, uint32_t cap,
+                                            DayShared& sh) {
+    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants;
     __syncthreads();
-    uint32_t woff = 0, tot = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-        const uint32_t wq = sh.red[q];
-        if (q < warp) woff += wq;
-        tot += wq;
+    if (threadIdx.x == 0) {
+        if (list) sh.listed = 0u;
+        if (queue) sh.cnt = 0u;
     }
-    if (threadIdx.x == 0 && tot) sh.base = atomicAdd(&k.l.bar[BAR_LISTED], tot);
     __syncthreads();
-    if (tot) {
-        // each lane's locations in its own order: the words' bits are exact now
-        uint32_t run = sh.base + woff + inc - agents;
-        for (uint32_t trip = 0; trip < trips; ++trip) {
-            const uint32_t w = word_of(trip, lane);
-            const uint32_t hm = w < n_words ? k.l.hmask[w] : 0u;
-            unsigned rest = __ballot_sync(0xffffffffu, hm != 0u);
-            while (rest) {
-                uint32_t l[LIST_BATCH], c[LIST_BATCH];
-#pragma unroll
-                for (int u = 0; u < LIST_BATCH; ++u) {
-                    const int src = rest ? __ffs(rest) - 1 : 0;
-                    const uint32_t word = __shfl_sync(0xffffffffu, hm, src);
-                    const bool in = rest && ((word >> lane) & 1u);
-                    if (rest) rest &= rest - 1u;
-                    l[u] = in ? word_of(trip, src) * 32u + (uint32_t)lane : NONE;
-                    c[u] = in ? k.l.counts[l[u]] : 0u;
-                }
-#pragma unroll
-                for (int u = 0; u < LIST_BATCH; ++u)
-                    if (l[u] != NONE) {
-                        k.l.cursor[l[u]] = run;
-                        run += c[u];
-                    }
-            }
-        }
-    }
-    if (k.prof) {
-        const uint32_t nl = block_sum(locs, sh.red);
-        if (threadIdx.x == 0 && (nl | tot)) {
-            atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)nl);
-            atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)tot);
-        }
-    }
-    if (!grid_barrier(k, sh)) return false;
-    prof_mark(k, tl + 1);
-    *n_listed = k.l.bar[BAR_LISTED];  // every block's reservation is in
-    // 2: four consecutive agents per thread (one 16-byte load of their
-    // locations), two quads in flight
-    const bool one = k.m.n_variants == 1;
+    const bool everybody = k.p.enable_curfew && k.p.curfew_begin == s1;
+    const uint32_t t1 = k.clock->t0 + s1;
     const uint32_t quads = (N + 3u) >> 2;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // warp-uniform trips
-        uint32_t loc[8];
+    const size_t seg = (size_t)blockIdx.x * cap;
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // block-uniform trips
+        uint32_t loc[8], m[8];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t q = q0 + (uint32_t)h * stride + threadIdx.x;
             const uint32_t i0 = q * 4u;
-            if (q < quads && i0 + 3u < N) {
+            const bool whole = q < quads && i0 + 3u < N;
+            if (list && whole) {
                 const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
                 loc[4 * h + 0] = v.x;
                 loc[4 * h + 1] = v.y;
@@ -1565,39 +1463,76 @@ __device__ bool phase_rebuild(const KArgs& k, DayShared& sh, uint32_t tl, uint32
                 loc[4 * h + 3] = v.w;
             } else {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) loc[4 * h + u] = q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
+                for (int u = 0; u < 4; ++u)
+                    loc[4 * h + u] = list && q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
             }
-        }
-        uint32_t lw[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const uint32_t i = (q0 + (uint32_t)(u >> 2) * stride + threadIdx.x) * 4u + (uint32_t)(u & 3);
-            const bool ok = loc[u] < L && ((lw[u] >> (loc[u] & 31u)) & 1u);
-            float su = 0.0f;
-            if (ok && one) su = k.a.susceptible[i] * k.p.sigma_band[k.a.band[i]];
-            const uint32_t pos = take_slot(k, ok, loc[u], true);
-            if (!ok) continue;
-            if (!one) {
-                slot_fill(k, pos, i);
-            } else if (pos < N) {
-                k.l.csr_agents[pos] = i;
-                k.l.slot_su[pos] = su;
+            if (queue && whole) {
+                const uint4 v = *reinterpret_cast<const uint4*>(k.a.move_at + i0);
+                m[4 * h + 0] = v.x;
+                m[4 * h + 1] = v.y;
+                m[4 * h + 2] = v.z;
+                m[4 * h + 3] = v.w;
             } else {
-                atomicOr(k.err, ERR_LOCATION);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    m[4 * h + u] = queue && q < quads && i0 + u < N ? k.a.move_at[i0 + u] : t1 + 1u;
             }
-            if (pos < N) k.l.slot_loc[pos] = loc[u];
+        }
+        const auto agent_of = [&](int u) {
+            return (q0 + (uint32_t)(u >> 2) * stride + threadIdx.x) * 4u + (uint32_t)(u & 3);
+        };
+        if (list) {
+            uint32_t lw[8], flags = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if ((lw[u] >> (loc[u] & 31u)) & 1u) {
+                    if (nonzero_sum(k, loc[u]))
+                        flags |= 1u << u;
+                    else
+                        atomicAnd(&k.l.hmask[loc[u] >> 5], ~(1u << (loc[u] & 31u)));
+                }
+            if (__any_sync(0xffffffffu, flags != 0u)) {
+                uint32_t at = list_place(flags, &sh.listed);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if ((flags >> u) & 1u) {
+                        const uint32_t i = agent_of(u);
+                        const size_t pos = seg + at++;
+                        k.l.list_agent[pos] = i;
+                        k.l.list_loc[pos] = loc[u];
+                        const float sigma = k.p.sigma_band[k.a.band[i]];
+                        for (uint32_t v = 0; v < V; ++v)
+                            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
+                    }
+            }
+        }
+        if (queue) {
+            uint32_t flags = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (agent_of(u) < N && (everybody || m[u] == t1)) flags |= 1u << u;
+            if (__any_sync(0xffffffffu, flags != 0u)) {
+                uint32_t at = list_place(flags, &sh.cnt);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if ((flags >> u) & 1u) k.a.worklist[seg + at++] = agent_of(u);
+            }
         }
     }
-    if (!grid_barrier(k, sh)) return false;
-    // every block has read the listing counter: block 0 keeps the count for
-    // the steps until the next rebuild and starts the counter at 0 for it
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        k.l.build[5] = *n_listed;
-        k.l.bar[BAR_LISTED] = 0u;
-    }
-    return true;
+    __syncthreads();
+    if (list && threadIdx.x == 0) k.l.list_count[blockIdx.x] = sh.listed;  // for a later launch
+}
+
+// the locations with a nonzero sum and the agents listed (profiled graph only)
+__device__ void count_listed(const KArgs& k, const DayShared& sh) {
+    uint32_t locs = 0;
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < k.l.n; l += gridDim.x * blockDim.x)
+        locs += nonzero_sum(k, l) ? 1u : 0u;
+    locs = __reduce_add_sync(__activemask(), locs);
+    if ((threadIdx.x & 31) == 0 && locs) atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)locs);
+    if (threadIdx.x == 0 && sh.listed) atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)sh.listed);
 }
 
 // expected-infection accumulation of the draws: one atomic per replica
@@ -1689,28 +1624,27 @@ struct DrawRun {
     float season;
 };
 
-// The draws of every entry of the agent list (the agents at the locations
-// the last rebuild listed) for all the timesteps of the segment, one entry per
-// thread, slots in order (coalesced loads of the slot's location, agent and
-// susceptibility products).  Each entry evaluates its location's ratio from
-// the location's sum, count and weight (the same inputs give the same value at
-// every entry) and compares the agent's Philox draw of every timestep with it.
-// Nothing is committed here: an entry that would be infected flags its
-// location (a stamp per location keeps it in the list once), and
+// The draws of every entry of the block's agent list for all the timesteps
+// of the segment, one entry per thread.  Each entry evaluates its location's
+// ratio from the location's sum, count and weight (the same inputs give the
+// same value at every entry) and compares the agent's Philox draw of every
+// timestep with it.  Nothing is committed here: an entry that would be
+// infected flags its location (a stamp per location keeps it in the list
+// once; the first to flag it reserves room for the location's agents), and
 // phase_replay repeats that location's draws with the ratio changing as its
 // agents are infected.  At a location without such an entry the ratio
 // cannot change, so the draws compared with it were the right ones.
-__device__ void phase_draw(const KArgs& k, const DrawRun& dr, uint32_t n_listed, uint32_t* n_entries,
+__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, uint32_t* n_entries,
                            uint32_t* n_hazard) {
     const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
-    const uint32_t stride = gridDim.x * blockDim.x;
     const bool one_rep = k.r.n == 1;
     const RepConst rc0 = rep_const(k, 0);
     uint32_t entries = 0, hazard = 0;
-    for (uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x; pos < n_listed && pos < N; pos += stride) {
-        const uint32_t loc = k.l.slot_loc[pos];
-        const uint32_t i = k.l.csr_agents[pos];
-        const float su0 = k.l.slot_su[pos];
+    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
+        const size_t pos = seg + j;
+        const uint32_t loc = k.l.list_loc[pos];
+        const uint32_t i = k.l.list_agent[pos];
+        const float su0 = k.l.list_su[pos];
         if (loc >= L || i >= N) {
             atomicOr(k.err, ERR_AGENT_LIST);
             continue;
@@ -1726,18 +1660,19 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, uint32_t n_listed,
             if (!(h > 0.0f)) continue;
             any_h = true;
             if (!k.r.variant_active[rep * V + v]) continue;
-            const float s_eff = v == 0 ? su0 : k.l.slot_su[(size_t)v * N + pos];
+            const float s_eff = v == 0 ? su0 : k.l.list_su[v * k.l.list_cap + pos];
             if (!(s_eff > 0.0f)) continue;
             const unsigned long long limit = u01_limit(h * s_eff);
             const uint32_t li = i - rc.off;
 #pragma unroll 2
-            for (uint32_t j = 0; j < dr.n; ++j) {
-                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + j, v);
+            for (uint32_t q = 0; q < dr.n; ++q) {
+                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + q, v);
                 hit |= u01_below(o.v[0], o.v[1], limit);
             }
         }
         if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
             const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
+            k.l.replay_cursor[loc] = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
             if (at < L)
                 k.l.replay_list[at] = loc;
             else
@@ -1750,15 +1685,29 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, uint32_t n_listed,
     *n_hazard += hazard;
 }
 
+// The entries of the flagged locations, gathered by location.
+__device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed) {
+    const uint32_t L = k.l.n, N = k.a.n;
+    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
+        const uint32_t loc = k.l.list_loc[seg + j];
+        if (loc >= L || k.l.replay_stamp[loc] != dr.epoch) continue;
+        const uint32_t p = atomicAdd(&k.l.replay_cursor[loc], 1u);
+        if (p < N)
+            k.l.replay_slot[p] = (uint32_t)(seg + j);
+        else
+            atomicOr(k.err, ERR_AGENT_LIST);
+    }
+}
+
 // The expected infections (and the adjoint's terms) of the segment's draws at
 // the locations that are not replayed: every timestep's are the same.
-__device__ void phase_expected(const KArgs& k, const DrawRun& dr, uint32_t n_listed, double* s_grad) {
+__device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad) {
     const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n_listed; base += stride) {  // block-uniform trips
-        const uint32_t pos = base + threadIdx.x;
-        const uint32_t loc = pos < n_listed && pos < N ? k.l.slot_loc[pos] : NONE;
-        const uint32_t i = loc < L ? k.l.csr_agents[pos] : NONE;
+    for (uint32_t base = 0; base < listed; base += blockDim.x) {  // block-uniform trips
+        const uint32_t j = base + threadIdx.x;
+        const size_t pos = seg + j;
+        const uint32_t loc = j < listed ? k.l.list_loc[pos] : NONE;
+        const uint32_t i = loc < L ? k.l.list_agent[pos] : NONE;
         const bool act = loc < L && i < N && k.l.replay_stamp[loc] != dr.epoch;
         uint32_t rep = 0;
         double term = 0.0;
@@ -1771,7 +1720,7 @@ __device__ void phase_expected(const KArgs& k, const DrawRun& dr, uint32_t n_lis
                 float x;
                 const float h = entry_hazard(k, loc, v, cnt, wl, kf, dr.season, dt, &x);
                 if (!(h > 0.0f) || !k.r.variant_active[rep * V + v]) continue;
-                const float s_eff = k.l.slot_su[(size_t)v * N + pos];
+                const float s_eff = k.l.list_su[v * k.l.list_cap + pos];
                 if (!(s_eff > 0.0f)) continue;
                 const float pf = h * s_eff;
                 term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
@@ -1798,12 +1747,12 @@ __device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t lo
 }
 
 // One entry's draws of timestep t with its location's ratios s_h (arguments
-// s_x): the agent in slot pos.  An agent that is infected updates its slot's
-// susceptibility products (read by no other entry) and its location's sums,
+// s_x): the agent i of list entry pos.  An agent that is infected updates its
+// entry's susceptibility products (read by no other entry) and its location's sums,
 // which the ratios of the next timestep are computed from.  Adds the sum of
 // min(1, p) over its draws to *term when expected infections are tracked;
 // returns whether the agent was infected.
-__device__ __forceinline__ bool draw_entry(const KArgs& k, uint32_t pos, uint32_t i, uint32_t loc, uint32_t rep,
+__device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t i, uint32_t loc, uint32_t rep,
                                            const RepConst& rc, uint32_t t, const float* s_h, const float* s_x,
                                            double* s_grad, double* term) {
     const uint32_t N = k.a.n, V = k.m.n_variants;
@@ -1815,8 +1764,8 @@ __device__ __forceinline__ bool draw_entry(const KArgs& k, uint32_t pos, uint32_
         if (!(h > 0.0f)) continue;
         if (!k.r.variant_active[rep * V + v]) continue;
         // after an infection the later variants read the agent's new
-        // susceptibility (what the slot then gets)
-        const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.slot_su[(size_t)v * N + pos];
+        // susceptibility (what the entry then gets)
+        const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.list_su[v * k.l.list_cap + pos];
         if (!(s_eff > 0.0f)) continue;
         const float pf = h * s_eff;
         if (k.track_expected) *term += pf < 1.0f ? (double)pf : 1.0;
@@ -1834,20 +1783,25 @@ __device__ __forceinline__ bool draw_entry(const KArgs& k, uint32_t pos, uint32_
         }
     }
     if (infected) {
-        for (uint32_t v = 0; v < V; ++v) k.l.slot_su[(size_t)v * N + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
+        for (uint32_t v = 0; v < V; ++v)
+            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
         const float inf = k.a.infectious[i];
         add_infection_change(k, loc, inf0, var0, inf, inf > 0.0f ? k.a.variant[i] : 0u);
     }
     return infected;
 }
 
-// The flagged locations' draws, a warp per location: its slots 32 at a time,
-// timestep after timestep.  The ratios are kept in shared memory and computed
-// again after a timestep that infected somebody there (all its draws first:
-// a timestep's ratios come from the sums as it started).
+// The flagged locations' draws, a warp per location, timestep after timestep.
+// A location of up to 32 agents and one variant (almost all) keeps its sum and
+// a lane per agent in registers: a timestep is a Philox block and a ballot,
+// and an infection adds its change of the sum for the next timestep.  Others
+// go over their entries 32 at a time; the ratios are kept in shared memory
+// and computed again after a timestep that infected somebody there (all its
+// draws first: a timestep's ratios come from the sums as it started).
 __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_replay, DayShared& sh) {
     const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool plain = V == 1 && !k.track_expected && !k.adj.on;
     // a block's warps take locations far apart in the list: few locations
     // spread over all SMs
     for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
@@ -1856,17 +1810,61 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
             if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
             continue;
         }
-        const uint32_t cnt = k.l.counts[loc], e = k.l.cursor[loc], b = e - cnt;  // the segment the rebuild filled
+        const uint32_t cnt = k.l.counts[loc], e = k.l.replay_cursor[loc], b = e - cnt;  // its gathered entries
+        const uint32_t rep = k.l.rep[loc];
+        const float wl = k.l.infectiousness[loc];
         if (e > N || cnt > e) {
             if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
             continue;
         }
-        const float wl = k.l.infectiousness[loc];
-        const uint32_t rep = k.l.rep[loc];
         const RepConst rc = rep_const(k, rep);
+        if (plain && cnt <= 32u) {
+            const bool act = (uint32_t)lane < cnt;
+            const uint32_t pos = act ? k.l.replay_slot[b + lane] : 0u;
+            const uint32_t i = act ? k.l.list_agent[pos] : NONE;
+            float su = i < N ? k.l.list_su[pos] : 0.0f;
+            long long fix = (long long)k.l.sfix[loc];
+            const long long fix0 = fix;
+            unsigned long long limit = 0ull;
+            bool fresh = false;
+            for (uint32_t q = 0; q < dr.n; ++q) {
+                if (!fresh) {
+                    float x;
+                    const float p = psim_hazard_x(fix, cnt, rc.kf, wl, dr.season, dt, &x) * su;
+                    limit = p > 0.0f && k.r.variant_active[rep] ? u01_limit(p) : 0ull;
+                    fresh = true;
+                }
+                bool hit = false;
+                if (limit) {
+                    const psim_ctr4 o = infect_words(rc.seed, i - rc.off, dr.t + q, 0u);
+                    hit = u01_below(o.v[0], o.v[1], limit);
+                }
+                if (__any_sync(0xffffffffu, hit)) {
+                    long long change = 0;
+                    if (hit) {
+                        const float inf0 = k.a.infectious[i];
+                        infect_agent(k, i, 0u, loc, dr.t + q);
+                        const float inf = k.a.infectious[i];
+                        su = k.a.susceptible[i] * k.p.sigma_band[k.a.band[i]];
+                        k.l.list_su[pos] = su;
+                        change = (inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll) -
+                                 (inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) change += __shfl_xor_sync(0xffffffffu, change, o);
+                    fix += change;
+                    fresh = false;
+                }
+            }
+            if (lane == 0 && fix != fix0) {
+                k.l.sfix[loc] = (unsigned long long)fix;
+                if (fix != 0) mark_hazardous(k, loc);
+            }
+            continue;
+        }
         double term = 0.0;
         bool stale = true;  // the ratios: at the start and after an infection
-        for (uint32_t j = 0; j < dr.n; ++j) {
+        for (uint32_t q = 0; q < dr.n; ++q) {
             if (stale) {
                 __syncwarp();
                 if ((uint32_t)lane < V) {
@@ -1879,83 +1877,20 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
                 __syncwarp();
             }
             bool infected = false;
-            for (uint32_t p0 = b; p0 < e; p0 += 32u) {
-                const uint32_t pos = p0 + (uint32_t)lane;
-                if (pos >= e) break;
-                const uint32_t i = k.l.csr_agents[pos];
+            for (uint32_t p = b + (uint32_t)lane; p < e; p += 32u) {
+                const uint32_t pos = k.l.replay_slot[p];
+                const uint32_t i = k.l.list_agent[pos];
                 if (i >= N) {
                     atomicOr(k.err, ERR_AGENT_LIST);
                     break;
                 }
-                infected |= draw_entry(k, pos, i, loc, rep, rc, dr.t + j, sh.h[warp], sh.x[warp], sh.grad, &term);
+                infected |= draw_entry(k, pos, i, loc, rep, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
             }
-            __threadfence();
             stale = __any_sync(0xffffffffu, infected);
+            if (stale) __threadfence();  // the reductions before the sums are read again
         }
         if (k.track_expected) add_expected_rep(k, true, rep, term);
     }
-}
-
-// The block's agents that decide at s1, in its own segment of the work list
-// (shared-memory counter: no global contention).  Reads one word per agent:
-// four consecutive agents per thread (one 16-byte load), two quads in flight.
-__device__ __forceinline__ uint32_t phase_queue(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t* s_cnt) {
-    if (threadIdx.x == 0) *s_cnt = 0u;
-    __syncthreads();
-    const uint32_t N = k.a.n;
-    const bool curfew_now = k.p.enable_curfew && k.p.curfew_begin == s1;
-    const uint32_t t1 = k.clock->t0 + s1;
-    const uint32_t quads = (N + 3u) >> 2;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t* seg = k.a.worklist + (size_t)blockIdx.x * cap;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // warp-uniform trips
-        uint32_t m[8];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t i0 = (q0 + (uint32_t)h * stride + threadIdx.x) * 4u;
-            if (i0 + 3u < N) {
-                const uint4 v = *reinterpret_cast<const uint4*>(k.a.move_at + i0);
-                m[4 * h + 0] = v.x;
-                m[4 * h + 1] = v.y;
-                m[4 * h + 2] = v.z;
-                m[4 * h + 3] = v.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) m[4 * h + u] = i0 + u < N ? k.a.move_at[i0 + u] : t1 + 1u;
-            }
-        }
-        // each quad's deciders in agent order: the warp's 128 agents of the
-        // first quad, then those of the second
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t i0 = (q0 + (uint32_t)h * stride + threadIdx.x) * 4u;
-            uint32_t flags = 0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (i0 + u < N && (curfew_now || m[4 * h + u] == t1)) flags |= 1u << u;
-            const uint32_t mine = __popc(flags);
-            uint32_t inc = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            const uint32_t wtot = __shfl_sync(0xffffffffu, inc, 31);
-            if (wtot) {
-                uint32_t basew = 0;
-                if (lane == 31) basew = atomicAdd(s_cnt, wtot);
-                uint32_t pos = __shfl_sync(0xffffffffu, basew, 31) + inc - mine;
-                while (flags) {
-                    const int u = __ffs(flags) - 1;
-                    flags &= flags - 1u;
-                    seg[pos++] = i0 + (uint32_t)u;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    return *s_cnt;
 }
 
 // doMovement of the agents the block queued for s1 (its own segment, whose
@@ -2015,7 +1950,6 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     prof_enter(k, tl);
     const uint32_t t = k.clock->t0 + step;
     const uint32_t moved = k.l.build[0], force = k.l.build[1], q_step = k.l.build[3];
-    uint32_t n_listed = k.l.build[5];  // the last rebuild's entries (this segment's if it rebuilds)
     DrawRun dr;
     dr.t = t;
     dr.epoch = k.l.build[6] + 1u;  // (0 is the stamp of a location never flagged)
@@ -2040,22 +1974,30 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     dr.n = min(e, step_end) - step;
     decides = decides && e <= step_end && (phases & PH_DECIDE);
     *next = min(e, step_end);
-    bool merged = false;
-    if (phases & PH_REBUILD) {
-        if (csr_decide_from(k, t, moved, force)) {
-            if (k.prof && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
-            if (!phase_rebuild(k, sh, tl, &n_listed)) return false;
-            prof_mark(k, tl + 2);
+    const bool list = (phases & PH_REBUILD) && csr_decide_from(k, t, moved, force);
+    // the location quarantine writes of the decisions for t
+    const bool merge = (phases & PH_REBUILD) && k.p.quarantine_policy > 1 && q_step == t;
+    if (merge) merge_quarantine(k);
+    const size_t seg = (size_t)blockIdx.x * cap;
+    if (list || decides) {
+        phase_lists(k, list, decides, e, cap, sh);
+        if (decides) mask_clear_shared(sh.mm);
+        if (k.prof) {
+            if (list) count_listed(k, sh);
+            if (threadIdx.x == 0) {
+                if (list && blockIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
+                if (decides && sh.cnt) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)sh.cnt);
+                if (decides && blockIdx.x == 0) atomicAdd(&k.prof[PROF_QUEUE_STEPS], 1ull);
+            }
         }
-        // the location quarantine writes of the decisions for t
-        merged = k.p.quarantine_policy > 1 && q_step == t;
-        if (merged) merge_quarantine(k);
+        prof_mark(k, tl + (list ? 1 : 2));
     }
-    const bool draws = (phases & PH_DRAW) && n_listed > 0;
+    const bool draws = (phases & PH_DRAW) != 0;
     if (draws) {
         uint32_t entries = 0, hazard = 0;
-        phase_draw(k, dr, n_listed, &entries, &hazard);
+        phase_draw(k, dr, seg, sh.listed, &entries, &hazard);
         if (k.prof) {
+            __syncwarp();
             entries = __reduce_add_sync(0xffffffffu, entries);
             hazard = __reduce_add_sync(0xffffffffu, hazard);
             if ((threadIdx.x & 31) == 0 && (entries | hazard)) {
@@ -2065,39 +2007,34 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
         }
     }
     prof_mark(k, tl + 3);
-    if (decides) {
-        mask_clear_shared(sh.mm);
-        const uint32_t n = phase_queue(k, e, cap, &sh.cnt);
-        if (k.prof && threadIdx.x == 0) {
-            if (n) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)n);
-            if (blockIdx.x == 0) atomicAdd(&k.prof[PROF_QUEUE_STEPS], 1ull);
-        }
-        prof_mark(k, tl + 4);
-    }
     // every draw before any replay, every draw and merge before any decision
-    if ((draws || (merged && decides)) && !grid_barrier(k, sh)) return false;
+    if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
     if (draws) {
         const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
         const bool expected = k.track_expected || k.adj.on;
         if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
         if (n_replay || expected) {
             grad_begin(k, sh.grad);
-            phase_replay(k, dr, n_replay, sh);
-            if (expected) phase_expected(k, dr, n_listed, sh.grad);
+            if (n_replay) {
+                phase_gather(k, dr, seg, sh.listed);
+                if (!grid_barrier(k, sh)) return false;
+                phase_replay(k, dr, n_replay, sh);
+            }
+            if (expected) phase_expected(k, dr, seg, sh.listed, sh.grad);
             grad_end(k, sh.grad);
             if (decides || n_replay) {
                 // every replay before any decision and before the list is emptied
                 if (!grid_barrier(k, sh)) return false;
-                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = 0u;
+                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
             }
         }
-        prof_mark(k, tl + 5);
     }
+    prof_mark(k, tl + 4);
     if (decides) {
         phase_decide(k, e, cap, sh.mm, &sh.cnt);
         mask_flush(k, sh.mm);
     }
-    prof_mark(k, tl + 6);
+    prof_mark(k, tl + 5);
     return true;
 }
 
@@ -2106,7 +2043,12 @@ __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0,
                                                         uint32_t cap) {
     __shared__ DayShared sh;
     if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
-    if (threadIdx.x == 0) sh.target = gridDim.x;
+    if (threadIdx.x == 0) {
+        sh.target = gridDim.x;
+        sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
+        sh.cnt = 0u;
+    }
+    __syncthreads();
     uint32_t step = step0;
     for (;;) {
         uint32_t next = step_end;
@@ -2806,8 +2748,8 @@ void launch_movement(const KArgs& k, uint32_t step, bool day, cudaStream_t s) {
 // The day kernel's grid: every block resident at once (its grid barriers
 // need that, and the cooperative launch checks it), tune.blocks_per_sm (in
 // blocks of 256 threads) capped at the kernel's occupancy, and no more blocks
-// than the population and locations give work to.  Each block's work-list
-// segment holds the agents its queue pass visits.
+// than the population gives work to.  Each block's segment of the lists holds
+// the agents its pass visits.
 static unsigned day_blocks_per_sm() {
     static int occ = 0;
     if (!occ) {
@@ -2820,8 +2762,7 @@ static void day_geometry(const KArgs& k, unsigned* grid, uint32_t* cap) {
     const unsigned bps = k.tune.blocks_per_sm
                              ? std::min<unsigned>((k.tune.blocks_per_sm * 256u + DAY_THREADS - 1) / DAY_THREADS, occ)
                              : occ;
-    const size_t want = std::max<size_t>(((size_t)k.a.n + DAY_THREADS - 1) / DAY_THREADS,
-                                         (((size_t)k.l.n + 31) / 32 + DAY_THREADS / 32 - 1) / (DAY_THREADS / 32));
+    const size_t want = ((size_t)k.a.n + DAY_THREADS - 1) / DAY_THREADS;
     unsigned g = (unsigned)std::min<size_t>((size_t)sm_count() * bps, std::max<size_t>(want, 1));
     g = std::min(g, (unsigned)(WORK_MAX_THREADS / DAY_THREADS));
     *grid = g;

@@ -331,16 +331,9 @@ int capture_day_graph(psim_ctx* c) {
     c->k.prof = c->profile ? c->d_prof : nullptr;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     // (the capture stays open until EndCapture: errors are checked after it)
-    // The day's first step: the sums afresh (every location dirty), the
-    // agent list rebuilt (its slots take the susceptibilities the midnight
-    // phases left), the mask of decision steps recomputed from every agent.
-    cudaError_t me = cudaMemsetAsync(c->k.l.sfix, 0, sizeof(unsigned long long) * c->L * c->V, c->stream);
-    if (me == cudaSuccess)
-        me = cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream);
-    if (me == cudaSuccess) me = cudaMemsetAsync(c->k.a.move_mask, 0, sizeof(uint32_t) * MOVE_MASK_WORDS, c->stream);
-    if (me == cudaSuccess) me = cudaMemsetAsync(c->k.l.build + 1, 0xFF, sizeof(uint32_t), c->stream);
-    if (me == cudaSuccess) me = cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t) * BAR_WORDS, c->stream);
-    if (me == cudaSuccess && c->profile) me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
+    cudaError_t me = cudaSuccess;
+    if (c->profile) me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
+    launch_day_begin(c->k, c->stream);
     launch_movement(c->k, 0, true, c->stream);
     // one launch of the day kernel for all timesteps; the profiled graph is
     // the same launch with the kernel's timeline stamps
@@ -354,7 +347,7 @@ int capture_day_graph(psim_ctx* c) {
     e = cudaGraphInstantiate(&c->day_graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(c, PSIM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    c->graph_kernels = 2;  // movement(0) and the day kernel
+    c->graph_kernels = 3;  // the day's beginning, movement(0), the day kernel
     c->graph_dirty = false;
     c->prof_valid = false;
     return 0;
@@ -404,8 +397,13 @@ void assemble_stats(psim_ctx* c, uint32_t t, psim_day_stats* out) {
 
 }  // namespace
 
+// minutes of TimeDayDuration(unsigned mins) (timeDay.cpp:64): the hours are
+// an unsigned char, so a difference that went negative folds modulo 256 hours
+static uint32_t td_minutes(uint32_t mins) { return (uint32_t)(uint8_t)(mins / 60u) * 60u + mins % 60u; }
+
 // The schedule window of doMovement (movementPolicies.h:585-603) for every
-// schedule slot and step of the day: act_b = the first event of the slot
+// schedule slot and step of the day, and what a decision then does with each
+// of its events (:737-811, :842-860): act_b = the first event of the slot
 // active at the step's minute, act_e = the first event starting after it (or
 // the slot's end when its last event is the active one), -1 where none.
 int upload_window_table(psim_ctx* c) {
@@ -413,11 +411,13 @@ int upload_window_table(psim_ctx* c) {
     const std::vector<uint16_t>&st = c->h_ev_start, &en = c->h_ev_end;
     const size_t n_slots = off.empty() ? 0 : off.size() - 1;
     const uint32_t spd = c->spd, dt = 1440u / spd;
-    std::vector<int2> win(n_slots * spd);
+    const size_t ne = c->h_ev_loc_type.size();
+    std::vector<DecWindow> win(n_slots * spd);
+    std::vector<DecChoice> choice;
     for (size_t q = 0; q < n_slots; ++q) {
         const uint32_t ev_b = off[q], ev_e = off[q + 1];
         for (uint32_t s = 0; s < spd; ++s) {
-            const uint32_t minutes = s * dt;
+            const uint32_t minutes = s * dt, sum = spd - s;
             int act_b = -1, act_e = -1;
             for (uint32_t j = ev_b; j < ev_e; ++j) {
                 const uint32_t a = st[j], b = en[j];
@@ -428,20 +428,57 @@ int upload_window_table(psim_ctx* c) {
                 }
                 if (j == ev_e - 1 && minutes >= a && minutes < b) act_e = (int)ev_e;
             }
-            win[q * spd + s] = make_int2(act_b, act_e);
+            // a read past the last event yields a 24:00 window
+            const bool in = act_e >= 0 && (size_t)act_e < ne;
+            const uint32_t nstart = in ? st[act_e] : 1440u, nend = in ? en[act_e] : 1440u;
+            DecWindow& w = win[q * spd + s];
+            w = DecWindow{0u, 0u, 0u, act_e != -1 ? 1u : 0u, DecChoice{0u, 0u, 0u, 0.0f}};
+            if (act_b == -1) {
+                w.choice.steps = td_minutes(nstart - minutes) / dt;
+                w.choice.draw = td_minutes(nend - nstart) / dt;
+                continue;
+            }
+            w.num = (uint32_t)((act_e == -1 ? act_b + 1 : act_e) - act_b);
+            w.event = (uint32_t)act_b;
+            w.choice_at = (uint32_t)choice.size();
+            for (uint32_t j = 0; j < w.num; ++j) {
+                const uint32_t dur = c->h_ev_duration[act_b + j];
+                DecChoice x{c->h_ev_loc_type[act_b + j], 0u, 0u, c->h_ev_chance[act_b + j]};
+                if (dur / 60u > 24u) {
+                    x.steps = sum;
+                } else if (act_e == -1) {
+                    x.steps = minutes + dur >= 1440u ? sum : dur / dt;
+                } else if (minutes + dur < nstart) {
+                    x.steps = dur / dt;
+                } else if (minutes + dur > nend) {
+                    x.steps = td_minutes(nend - minutes) / dt - 1u;
+                } else {
+                    x.steps = dur / dt;
+                    x.draw = td_minutes(nend - (minutes + dur)) / dt;
+                }
+                choice.push_back(x);
+            }
+            w.choice = choice[w.choice_at];
         }
     }
-    int2* d = nullptr;
-    const size_t bytes = std::max<size_t>(win.size() * sizeof(int2), 16);
-    cudaError_t e = psim_device_malloc((void**)&d, bytes);
-    if (e != cudaSuccess) return fail(c, PSIM_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
-    c->allocs.push_back(d);
-    if (!win.empty()) CK(cudaMemcpyAsync(d, win.data(), win.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
+    auto put = [&](const void* host, size_t bytes, const void** dst) -> int {
+        void* d = nullptr;
+        cudaError_t e = psim_device_malloc(&d, std::max<size_t>(bytes, 32));
+        if (e != cudaSuccess) return fail(c, PSIM_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
+        c->allocs.push_back(d);
+        if (bytes) CK(cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, c->stream));
+        *dst = d;
+        return 0;
+    };
+    int rc;
+    const void *dw = nullptr, *dc = nullptr;
+    if ((rc = put(win.data(), win.size() * sizeof(DecWindow), &dw))) return rc;
+    if ((rc = put(choice.data(), choice.size() * sizeof(DecChoice), &dc))) return rc;
     CK(cudaStreamSynchronize(c->stream));
-    c->k.m.window = d;
+    c->k.m.window = (const DecWindow*)dw;
+    c->k.m.choice = (const DecChoice*)dc;
     return 0;
 }
-
 
 extern "C" {
 
@@ -485,6 +522,8 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     c->n_poss = a->n_poss;
     c->params = *p;
     c->spd = 1440 / p->time_step;
+    c->k.hour_steps = 60u / p->time_step;
+    c->k.half_hour_steps = 30u / p->time_step;
     // replicas
     if (reps && reps->n > 0) {
         c->R = reps->n;
@@ -654,6 +693,7 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     if ((rc = dalloc(c, &dl.list_su, dl.list_cap * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.list_count, WORK_MAX_BLOCKS))) return bail(rc);
     if ((rc = dalloc(c, &dl.qu_pending, L))) return bail(rc);
+    if ((rc = dalloc(c, &dl.lflags, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.sfix, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hazard, L * V))) return bail(rc);
     if ((rc = dalloc(c, &dl.hazard_x, L * V))) return bail(rc);
@@ -1408,20 +1448,21 @@ int psim_time_step_kernels(psim_ctx* c, uint32_t t, float* ms) {
     // and the agent list rebuilt: the rebuild, the draws, the queue +
     // decisions of t + 1 (the day kernel's phases as separate launches);
     // then step t + 1 untimed
-    if ((rc = reset_sums(c))) return rc;
-    CK(cudaMemsetAsync(c->k.a.move_mask, 0, sizeof(uint32_t) * MOVE_MASK_WORDS, c->stream));
-    CK(cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t) * BAR_WORDS, c->stream));
-    if ((rc = force_rebuild(c))) return rc;
+    launch_day_begin(c->k, c->stream);
     launch_movement(c->k, step, true, c->stream);
     CK(cudaEventRecord(ev[0], c->stream));
+    // (a launch counts its barrier's arrivals from 0)
     launch_day(c->k, step, step + 1, PH_REBUILD, c->stream);
     CK(cudaEventRecord(ev[1], c->stream));
+    CK(cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t), c->stream));
     launch_day(c->k, step, step + 1, PH_DRAW, c->stream);
     CK(cudaEventRecord(ev[2], c->stream));
+    CK(cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t), c->stream));
     launch_day(c->k, step, step + 1, PH_DECIDE, c->stream);
     CK(cudaEventRecord(ev[3], c->stream));
+    CK(cudaMemsetAsync(c->k.l.bar, 0, sizeof(uint32_t), c->stream));
     launch_day(c->k, step + 1, step + 2, PH_REBUILD | PH_DRAW, c->stream);
-    c->launches += 5;
+    c->launches += 6;
     CK(cudaStreamSynchronize(c->stream));
     for (int j = 0; j < 3; ++j) CK(cudaEventElapsedTime(&ms[j], ev[j], ev[j + 1]));
     for (int j = 0; j < 4; ++j) cudaEventDestroy(ev[j]);

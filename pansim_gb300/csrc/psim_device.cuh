@@ -19,6 +19,22 @@ constexpr uint32_t ERR_SCAN_WAIT = 1u;     // a scan tile gave up waiting for it
 constexpr uint32_t ERR_AGENT_LIST = 8u;    // the agent list disagrees with the histogram or work list
 constexpr uint32_t ERR_BARRIER = 16u;      // a grid barrier of the day kernel gave up waiting
 
+// What a decision does with one event of its window: the location type and
+// the new countdown, steps + (a draw below `draw`), for the window's step.
+struct __align__(16) DecChoice {
+    uint32_t type, steps, draw;
+    float chance;
+};
+// The event window of a schedule slot at a step of the day: the number of
+// events that compete (0: none is active), the first of them in the events'
+// own arrays and in DevModel::choice, and the first choice itself.  With no
+// active event `next` says whether one follows later in the day: the choice
+// then holds the wait for it.
+struct __align__(16) DecWindow {
+    uint32_t num, event, choice_at, next;
+    DecChoice choice;
+};
+
 struct DevModel {
     uint32_t n_states, n_variants, n_prog, n_agent_types;
     uint32_t first_infected, noncovid_dead, dead_state, n_trans;
@@ -48,9 +64,9 @@ struct DevModel {
     const uint16_t* ev_end;
     const uint16_t* ev_duration;
     // per schedule slot and step of the day, the decision's active event
-    // window (first event active at the step, first event starting after it;
-    // -1 for none), computed on the host from the schedule table
-    const int2* window;        // [n_agent_types * 28 * steps_per_day]
+    // window, computed on the host from the schedule table
+    const DecWindow* window;   // [n_agent_types * 28 * steps_per_day]
+    const DecChoice* choice;   // the windows' choices, window after window
 };
 
 struct DevAgents {
@@ -130,6 +146,15 @@ constexpr uint32_t DW_INFECTIOUS = 1u << 15;  // infectious != 0
 constexpr uint32_t DW_NO_WORK = 1u << 16;    // its no_work flag
 constexpr uint32_t DW_TOO_OLD = 1u << 17;    // at or above the school age restriction
 
+// The flag word of a location: what a decision needs to know of it, in one
+// 2-byte load.  Computed for the day's timesteps before its first one; during
+// them only the merge of location quarantines sets LF_QUARANTINE.  The
+// timestamps behind a flag are read only where it is set.
+constexpr uint32_t LF_TYPE = 0xFFu;           // location type
+constexpr uint32_t LF_OPEN = 1u << 8;         // its open flag
+constexpr uint32_t LF_CLOSED = 1u << 9;       // closed_until lies beyond the day's first timestep
+constexpr uint32_t LF_QUARANTINE = 1u << 10;  // so does quarantine_until
+
 struct DevLocs {
     uint32_t n;
     uint32_t n_schools;
@@ -147,6 +172,7 @@ struct DevLocs {
     uint32_t* cursor;             // [n] next free CSR slot of each location (scan: first slot)
     uint32_t* csr_off;            // [n+1] CSR offsets, derived from the cursors on demand
     uint32_t* csr_agents;         // [N]
+    uint16_t* lflags;             // [n] the flag words of the running day (LF_*)
     uint32_t* qu_pending;         // quarantine writes of the running step
     unsigned long long* sfix;     // [V][n] fixed-point infectiousness sums
     float* hazard;                // [V][n] infection ratio of the last step
@@ -274,6 +300,7 @@ struct KArgs {
     uint32_t* err;
     DevStatsAcc* stats;   // [R]
     uint32_t spd;         // steps per day
+    uint32_t hour_steps, half_hour_steps;  // 60 and 30 minutes in steps (rounded down)
     uint32_t track_expected;
     DevTune tune;
     DevAdjoint adj;
@@ -335,6 +362,8 @@ __device__ __forceinline__ void update_meta(const KArgs& k, uint32_t i) {
 #endif
 
 // launchers (psim_kernels.cu)
+// what a day's first step starts from: the sums, the flag words, the masks
+void launch_day_begin(const KArgs& k, cudaStream_t s);
 // day: the day kernel runs the steps after it
 void launch_movement(const KArgs& k, uint32_t step_in_day, bool day, cudaStream_t s);
 void launch_count(const KArgs& k, cudaStream_t s);

@@ -16,11 +16,15 @@
 
 using namespace psim;
 
-// the kernels' error flags: reads and clears them
+// the kernels' error flags: reads and clears them.  A kernel that raises one
+// also sets the host's word, so that a call without an error copies nothing.
 int check_device_err(psim_ctx* c) {
+    CK(cudaStreamSynchronize(c->stream));
+    if (!*(volatile uint32_t*)c->k.err_host) return 0;
     uint32_t e = 0;
     CK(cudaMemcpyAsync(&e, c->k.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    *c->k.err_host = 0u;
     if (e) {
         CK(cudaMemsetAsync(c->k.err, 0, sizeof(uint32_t), c->stream));
         std::string m = "device error flags 0x" + std::to_string(e) + ":";
@@ -298,6 +302,7 @@ int initial_regroup(psim_ctx* c) {
     launch_scan(c->k, 0, 1, 0, c->stream);
     launch_scatter_draw(c->k, 0, 1, 0, c->stream);
     c->list_sparse = false;
+    c->csr_full = true;
     // the variant gating of the first steps (the statistics come at midnight)
     launch_variant_flags(c->k, c->stream);
     c->launches += 3 + (uint64_t)scan_kernels(c->k);
@@ -307,17 +312,18 @@ int initial_regroup(psim_ctx* c) {
     return check_device_err(c);
 }
 
-int do_step(psim_ctx* c, uint32_t step, bool draw, bool movement) {
-    const int merge_q = c->params.quarantine_policy > 1 ? 2 : 0;
-    if (movement) {
-        int rc = reset_sums(c);
+int do_step(psim_ctx* c, uint32_t step) {
+    if (!c->csr_full) {
+        int rc = force_rebuild(c);
         if (rc) return rc;
-        launch_movement(c->k, step, false, c->stream);
     }
-    launch_scan(c->k, step, 1, merge_q, c->stream);
-    launch_scatter_draw(c->k, step, 1, draw ? 1 : 0, c->stream);
-    c->launches += (movement ? 2 : 1) + (uint64_t)scan_kernels(c->k);
+    launch_phase_movement(c->k, step, c->stream);
+    const bool merge = c->params.quarantine_policy > 1;
+    launch_scan(c->k, step, 1, merge, c->stream);
+    launch_scatter_draw(c->k, step, merge ? 2 : 1, 1, c->stream);
+    c->launches += 3 + (uint64_t)scan_kernels(c->k);
     c->list_sparse = false;
+    c->csr_full = true;
     return launch_check(c);
 }
 
@@ -334,7 +340,7 @@ int capture_day_graph(psim_ctx* c) {
     cudaError_t me = cudaSuccess;
     if (c->profile) me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
     launch_day_begin(c->k, c->stream);
-    launch_movement(c->k, 0, true, c->stream);
+    launch_movement(c->k, 0, c->stream);
     // one launch of the day kernel for all timesteps; the profiled graph is
     // the same launch with the kernel's timeline stamps
     launch_day(c->k, 0, c->spd, PH_ALL, c->stream);
@@ -776,7 +782,7 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
         c->h_stats = (DevStatsAcc*)p;
         c->h_expected = (double*)(p + b_stats);
         c->h_clock_pin = (DevClock*)(p + b_stats + b_exp);
-        c->h_err_pin = (uint32_t*)(p + b_stats + b_exp + sizeof(DevClock) + 32);
+        c->k.err_host = (uint32_t*)(p + b_stats + b_exp + sizeof(DevClock) + 32);
     }
     // healthcare workers per replica (Simulation::flagHealthcareWorkers, simulation.h:670-693)
     c->hcw_count.assign(R, 0u);
@@ -1023,9 +1029,12 @@ int psim_checkpoint_restore(psim_ctx* c, uint32_t slot) {
         src += r.second;
     }
     c->t_next = c->checkpoint_t_next[slot];
-    // the restored locations need not match the agent list of the last step
+    // the restored locations need not match the agent list of the last step,
+    // nor the restored sums the hazard mask
     int rc = force_rebuild(c);
     if (rc) return rc;
+    CK(cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream));
+    c->csr_full = false;
     CK(cudaStreamSynchronize(c->stream));
     c->csr_fresh = false;
     return 0;
@@ -1067,9 +1076,8 @@ int psim_movement(psim_ctx* c, uint32_t t) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     int rc = set_clock(c, t);
     if (rc) return rc;
-    if ((rc = reset_sums(c))) return rc;
-    launch_movement(c->k, t % c->spd, false, c->stream);
-    c->launches += 1;
+    launch_phase_movement(c->k, t % c->spd, c->stream);
+    c->launches += 2;
     c->csr_fresh = true;
     c->t_next = t + 1;
     rc = launch_check(c);
@@ -1079,19 +1087,25 @@ int psim_movement(psim_ctx* c, uint32_t t) {
 
 int psim_regroup(psim_ctx* c) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
-    int rc0 = force_rebuild(c);
-    if (rc0) return rc0;
+    // the list of the last regroup serves when nobody has moved since
+    int rc0 = 0;
+    if (!(c->csr_full && c->csr_fresh) && (rc0 = force_rebuild(c))) return rc0;
     if (!c->csr_fresh) {
         CK(cudaMemsetAsync(c->k.l.counts, 0, sizeof(uint32_t) * c->L, c->stream));
         if ((rc0 = reset_sums(c))) return rc0;
         launch_count(c->k, c->stream);
         c->launches += 1;
     }
-    launch_scan(c->k, 0, 1, c->params.quarantine_policy > 1 ? 2 : 0, c->stream);
-    launch_scatter_draw(c->k, 0, 1, 0, c->stream);
+    // the step that was moved last, where it is one of the running day
+    const uint32_t since = c->t_next - 1u - c->h_clock.t0;
+    const uint32_t step = c->csr_fresh && since < c->spd ? since : 0u;
+    const bool merge = c->params.quarantine_policy > 1;
+    launch_scan(c->k, step, 1, merge, c->stream);
+    launch_scatter_draw(c->k, step, merge ? 2 : 1, 0, c->stream);
     c->launches += 1 + (uint64_t)scan_kernels(c->k);
     c->csr_fresh = false;
     c->list_sparse = false;
+    c->csr_full = true;
     int rc = launch_check(c);
     if (rc) return rc;
     return check_device_err(c);
@@ -1117,7 +1131,7 @@ int psim_step(psim_ctx* c, uint32_t t) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     int rc = set_clock(c, t);
     if (rc) return rc;
-    rc = do_step(c, t % c->spd, true, true);
+    rc = do_step(c, t % c->spd);
     if (rc) return rc;
     c->csr_fresh = false;
     c->t_next = t + 1;
@@ -1218,6 +1232,7 @@ int psim_run_steps(psim_ctx* c, uint32_t day) {
     c->prof_valid = c->profile;
     c->csr_fresh = false;
     c->list_sparse = true;
+    c->csr_full = false;
     c->t_next = (day + 1) * c->spd;
     return check_device_err(c);
 }
@@ -1261,15 +1276,15 @@ int psim_run_day(psim_ctx* c, uint32_t day, psim_day_stats* out) {
     CK(cudaEventRecord(c->ev0, c->stream));
     CK(cudaGraphLaunch(c->day_graph, c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaMemcpyAsync(c->h_err_pin, c->k.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
     c->launches += c->graph_kernels;
     c->prof_valid = c->profile;
     c->csr_fresh = false;
     c->list_sparse = true;
+    c->csr_full = false;
     c->t_next = (day + 1) * c->spd;
-    if (*c->h_err_pin) return check_device_err(c);
+    if (*(volatile uint32_t*)c->k.err_host) return check_device_err(c);
     if (out) assemble_stats(c, t, out);
     return 0;
 }
@@ -1287,6 +1302,7 @@ int psim_get_csr(psim_ctx* c, int canonical, uint32_t* offsets, uint32_t* agents
         launch_scatter_draw(c->k, 0, 1, 0, c->stream);
         c->launches += 1 + (uint64_t)scan_kernels(c->k);
         c->list_sparse = false;
+        c->csr_full = true;
     }
     launch_offsets(c->k, c->stream);
     c->launches += 1;
@@ -1449,7 +1465,7 @@ int psim_time_step_kernels(psim_ctx* c, uint32_t t, float* ms) {
     // decisions of t + 1 (the day kernel's phases as separate launches);
     // then step t + 1 untimed
     launch_day_begin(c->k, c->stream);
-    launch_movement(c->k, step, true, c->stream);
+    launch_movement(c->k, step, c->stream);
     CK(cudaEventRecord(ev[0], c->stream));
     // (a launch counts its barrier's arrivals from 0)
     launch_day(c->k, step, step + 1, PH_REBUILD, c->stream);
@@ -1468,6 +1484,7 @@ int psim_time_step_kernels(psim_ctx* c, uint32_t t, float* ms) {
     for (int j = 0; j < 4; ++j) cudaEventDestroy(ev[j]);
     c->csr_fresh = false;
     c->list_sparse = true;
+    c->csr_full = false;
     c->t_next = t + 2;
     rc = launch_check(c);
     if (rc) return rc;

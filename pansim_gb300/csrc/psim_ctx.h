@@ -62,16 +62,17 @@ struct psim_ctx {
     uint64_t launches = 0;
     bool uploaded = false;
     bool csr_fresh = false;      // counts of the current positions are built
+    bool csr_full = false;       // the agent list is that of the last regroup; movements since then
+                                 // that moved somebody have marked it (build[1])
     bool list_sparse = false;    // the agent list holds only the locations the day kernel's
                                  // last rebuild listed (psim_get_csr builds the full one)
     // pinned host memory (one block): the statistics accumulators and the
-    // expected-infection sums copied back, the clock copied in, the error
-    // flags copied back, so that a day needs no synchronisation in between
+    // expected-infection sums copied back, the clock copied in, the kernels'
+    // error word, so that a day needs no synchronisation in between
     void* pinned = nullptr;
     DevStatsAcc* h_stats = nullptr;   // [R]
     double* h_expected = nullptr;     // [R]
     DevClock* h_clock_pin = nullptr;
-    uint32_t* h_err_pin = nullptr;
     // adjoint
     double* d_adj_weight = nullptr;
     double* d_grad = nullptr;

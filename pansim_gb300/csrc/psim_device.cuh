@@ -204,6 +204,8 @@ struct DevLocs {
                                   //     the step's first scan kernel, read by its later kernels),
                                   // [3] the timestamp of the last step whose decisions wrote a
                                   //     location quarantine (merged by that step's scan),
+                                  // [4] nonzero: decisions wrote location quarantines since the
+                                  //     last merge of a scan
                                   // [6] the stamp of the last segment of draws (counts segments
                                   //     over the context's lifetime, so a replayed day never meets
                                   //     its own stamps)
@@ -298,6 +300,7 @@ struct KArgs {
     psim_params p;
     DevClock* clock;
     uint32_t* err;
+    uint32_t* err_host;   // nonzero after an error (host memory, read after a wait for the stream)
     DevStatsAcc* stats;   // [R]
     uint32_t spd;         // steps per day
     uint32_t hour_steps, half_hour_steps;  // 60 and 30 minutes in steps (rounded down)
@@ -364,11 +367,12 @@ __device__ __forceinline__ void update_meta(const KArgs& k, uint32_t i) {
 // launchers (psim_kernels.cu)
 // what a day's first step starts from: the sums, the flag words, the masks
 void launch_day_begin(const KArgs& k, cudaStream_t s);
-// day: the day kernel runs the steps after it
-void launch_movement(const KArgs& k, uint32_t step_in_day, bool day, cudaStream_t s);
+// the day's first step, before the day kernel
+void launch_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
+// a step of the per-phase entry points, the sums afresh
+void launch_phase_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
 void launch_count(const KArgs& k, cudaStream_t s);
-// merge_quarantine: 0 no, 1 at the steps whose decisions wrote location
-// quarantines, 2 always
+// merge_quarantine: the location quarantines that decisions wrote since the last merge
 void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merge_quarantine, cudaStream_t s);
 void launch_scatter_draw(const KArgs& k, uint32_t step_in_day, int scatter, int draw, cudaStream_t s);
 void launch_offsets(const KArgs& k, cudaStream_t s);

@@ -24,6 +24,12 @@
 
 namespace psim {
 
+// An error flag: in device memory for the kernels, and the host's word, which
+// the host looks at after it has waited for the stream (no copy per call).
+__device__ __forceinline__ void raise_error(const KArgs& k, uint32_t bits) {
+    atomicOr(k.err, bits);
+    *(volatile uint32_t*)k.err_host = 1u;
+}
 __device__ __forceinline__ uint32_t wb_of(const KArgs& k, uint32_t i) {
     return k.m.state_wb[(uint8_t)k.a.state[i]];
 }
@@ -112,6 +118,7 @@ __device__ __forceinline__ void qu_write(const KArgs& k, uint32_t loc, uint32_t 
     if (loc < k.l.n) {
         atomicMax(&k.l.qu_pending[loc], until);
         k.l.build[3] = t;
+        k.l.build[4] = 1u;
     }
 }
 
@@ -439,16 +446,6 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
-// Hazard of variant 0 at `loc` and whether an infectious agent is there, for
-// the agent-ordered draws of the per-phase entry points (the scan computed
-// the location's hazards this step; elsewhere every hazard is 0): the hazard
-// itself is gathered only at infectious locations.
-__device__ __forceinline__ float hazard_at(const KArgs& k, uint32_t loc, bool* any) {
-    const uint32_t w = k.l.hmask[loc >> 5];
-    *any = ((w >> (loc & 31u)) & 1u) != 0;
-    return *any ? k.l.hazard[loc] : 0.0f;
-}
-
 // ---------------------------------------------------------------------------
 // Per-agent pieces of a step.
 
@@ -549,7 +546,7 @@ __device__ __forceinline__ bool count_agent(const KArgs& k, bool act, uint32_t l
                                             uint32_t variant) {
     const uint32_t L = k.l.n;
     if (act && loc >= L) {
-        atomicOr(k.err, ERR_LOCATION);
+        raise_error(k, ERR_LOCATION);
         loc = NONE;
     }
     const bool mv = act && loc != loc0;
@@ -580,7 +577,7 @@ __device__ __forceinline__ bool count_agent_delta(const KArgs& k, bool act, uint
                                                   uint32_t var0, float inf, uint32_t var) {
     const uint32_t L = k.l.n;
     if (act && loc >= L) {
-        atomicOr(k.err, ERR_LOCATION);
+        raise_error(k, ERR_LOCATION);
         loc = NONE;
     }
     const bool mv = act && loc != loc0;
@@ -607,7 +604,7 @@ __device__ __forceinline__ void count_full(const KArgs& k, bool act, uint32_t lo
     const uint32_t L = k.l.n;
     if (!act) return;
     if (loc >= L) {
-        atomicOr(k.err, ERR_LOCATION);
+        raise_error(k, ERR_LOCATION);
         return;
     }
     atomicAdd(&k.l.counts[loc], 1u);
@@ -621,11 +618,7 @@ __device__ __forceinline__ void count_full(const KArgs& k, bool act, uint32_t lo
 
 // CSR slot of an agent: a warp-aggregated returning atomic on the location's
 // cursor, which the scan set to the location's first slot.  Warp-collective.
-// the slot of an agent whose step keeps the agent list of the step before
-constexpr uint32_t SLOT_KEEP = 0xFFFFFFFEu;
-
-__device__ __forceinline__ uint32_t take_slot(const KArgs& k, bool ok, uint32_t loc, bool rebuild) {
-    if (!rebuild) return SLOT_KEEP;
+__device__ __forceinline__ uint32_t take_slot(const KArgs& k, bool ok, uint32_t loc) {
     if (!k.tune.agg_slot) return ok ? atomicAdd(&k.l.cursor[loc], 1u) : NONE;
     const unsigned valid = __ballot_sync(0xffffffffu, ok);
     uint32_t pos = NONE;
@@ -641,11 +634,10 @@ __device__ __forceinline__ uint32_t take_slot(const KArgs& k, bool ok, uint32_t 
 }
 
 __device__ __forceinline__ void store_slot(const KArgs& k, uint32_t pos, uint32_t i) {
-    if (pos == SLOT_KEEP) return;
     if (pos < k.a.n)
         k.l.csr_agents[pos] = i;
     else
-        atomicOr(k.err, ERR_LOCATION);
+        raise_error(k, ERR_LOCATION);
 }
 
 // Infection draws of agent i at location loc with hazard h0 of variant 0
@@ -757,15 +749,30 @@ __device__ __forceinline__ void prof_mark(const KArgs& k, uint32_t slot) {
     if (threadIdx.x == 0) atomicMax(&k.prof[slot], global_ns());
 }
 
+// Where a warp's lanes put the entries they flagged (bits of `flags`, one
+// per agent of the lane) in a block's list: the first one's place (one
+// shared-memory atomic per warp).
+__device__ __forceinline__ uint32_t list_place(uint32_t flags, uint32_t* s_cnt) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t mine = __popc(flags);
+    uint32_t inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    uint32_t base = 0;
+    if (lane == 31 && inc) base = atomicAdd(s_cnt, inc);
+    return __shfl_sync(0xffffffffu, base, 31) + inc - mine;
+}
+
 // Movement of every agent + histogram + fixed-point infectiousness sums (the
-// day's first step, after a reset of the sums, and the per-phase entry
-// points).  Records the steps of the day at which agents decide next.
-// DAY: the day kernel follows (the locations' flag words of the day are
-// there, the agents' decision words are written).
-template <bool DAY>
+// day's first step, after a reset of the sums).  Records the steps of the day
+// at which agents decide next.  The day kernel follows: the locations' flag
+// words of the day are there, the agents' decision words are written.
 __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
     __shared__ uint32_t s_mm[MOVE_MASK_WORDS];
-    if (DAY) prof_enter(k, PROF_N);
+    prof_enter(k, PROF_N);
     mask_clear_shared(s_mm);
     const uint32_t N = k.a.n;
     const StepClock c = step_clock(k, step);
@@ -782,23 +789,110 @@ __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
             DecisionIn d;
             loc0 = loc = k.a.location[i];
             inf = k.a.infectious[i];
-            const bool decides = c.curfew_now || s == 0;
-            uint32_t w = DAY || decides ? decision_word(k, i, c.t) : 0u;
-            if (decides) {
+            uint32_t w = decision_word(k, i, c.t);
+            if (c.curfew_now || s == 0) {
                 decision_in(k, i, d);
                 d.w = w;
-                loc = move_agent<DAY>(k, i, c, s, s_mm, d, &w);
+                loc = move_agent<true>(k, i, c, s, s_mm, d, &w);
             } else {
                 mask_note(k, s_mm, m0);  // an agent counting down decides later today
             }
-            if (DAY) k.a.dinfo[i] = w;
+            k.a.dinfo[i] = w;
             if (inf > 0.0f) var = k.a.variant[i];
         }
         moved |= count_agent(k, act, loc0, loc, inf, var);
     }
     publish_moved(k, moved, c.t);
     mask_flush(k, s_mm);
-    if (DAY) prof_mark(k, PROF_N + 1);
+    prof_mark(k, PROF_N + 1);
+}
+
+// The same for a step of the per-phase entry points (psim_movement): most
+// agents count down and are not infectious, so a thread reads three words of
+// four agents each (16-byte loads); the block's deciders are collected and
+// decide together, full warps of them.
+constexpr uint32_t PHASE_THREADS = 256;
+__global__ void __launch_bounds__(PHASE_THREADS) k_phase_movement(KArgs k, uint32_t step) {
+    __shared__ uint32_t s_mm[MOVE_MASK_WORDS];
+    __shared__ uint32_t s_list[PHASE_THREADS * 4];
+    __shared__ uint32_t s_cnt;
+    const uint32_t N = k.a.n, L = k.l.n;
+    const StepClock c = step_clock(k, step);
+    const uint32_t quads = (N + 3u) >> 2;
+    bool moved = false;
+    mask_clear_shared(s_mm);
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += gridDim.x * blockDim.x) {  // block-uniform trips
+        if (threadIdx.x == 0) s_cnt = 0u;
+        __syncthreads();
+        const uint32_t i0 = (q0 + threadIdx.x) * 4u;
+        uint32_t m[4], loc[4];
+        float inf[4];
+        if (q0 + threadIdx.x < quads && i0 + 3u < N) {
+            const uint4 v = *reinterpret_cast<const uint4*>(k.a.move_at + i0);
+            const float4 f = *reinterpret_cast<const float4*>(k.a.infectious + i0);
+            const uint4 w = *reinterpret_cast<const uint4*>(k.a.location + i0);
+            loc[0] = w.x, loc[1] = w.y, loc[2] = w.z, loc[3] = w.w;
+            m[0] = v.x, m[1] = v.y, m[2] = v.z, m[3] = v.w;
+            inf[0] = f.x, inf[1] = f.y, inf[2] = f.z, inf[3] = f.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool in = q0 + threadIdx.x < quads && i0 + u < N;
+                m[u] = in ? k.a.move_at[i0 + u] : c.t + 1u;
+                loc[u] = in ? k.a.location[i0 + u] : 0u;
+                inf[u] = in ? k.a.infectious[i0 + u] : 0.0f;
+            }
+        }
+        uint32_t flags = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool in = q0 + threadIdx.x < quads && i0 + u < N;
+            if (in && (c.curfew_now || m[u] == c.t)) {
+                flags |= 1u << u;
+            } else if (in && (inf[u] > 0.0f || loc[u] >= L)) {
+                count_agent(k, true, loc[u], loc[u], inf[u], k.a.variant[i0 + u]);
+            }
+        }
+        if (__any_sync(0xffffffffu, flags != 0u)) {
+            uint32_t at = list_place(flags, &s_cnt);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if ((flags >> u) & 1u) s_list[at++] = i0 + (uint32_t)u;
+        }
+        __syncthreads();
+        const uint32_t n = s_cnt;
+        for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+            const uint32_t i = s_list[j];
+            DecisionIn d;
+            decision_in(k, i, d);
+            uint32_t w = d.w = decision_word(k, i, c.t);
+            const float f = k.a.infectious[i];
+            const uint32_t loc = move_agent<false>(k, i, c, k.a.move_at[i] - c.t, s_mm, d, &w);
+            moved |= count_agent(k, true, d.loc, loc, f, f > 0.0f ? k.a.variant[i] : 0u);
+        }
+        __syncthreads();
+    }
+    // the agent list of the last regroup is not this step's any more
+    if (__syncthreads_or(moved) && threadIdx.x == 0) {
+        k.l.build[0] = c.t;
+        k.l.build[1] = BUILD_PENDING;
+    }
+}
+
+// The sums afresh before a step of the per-phase entry points: zeroed where
+// the masks say that one may be nonzero (every kernel that adds a term marks
+// its location), and those locations dirty for the scan.
+__global__ void __launch_bounds__(256) k_reset_sums(KArgs k) {
+    const uint32_t L = k.l.n, V = k.m.n_variants;
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < (L + 31u) >> 5; w += gridDim.x * blockDim.x) {
+        const uint32_t sm = k.l.smask[w], m = sm | k.l.hmask[w];
+        if (m != sm) k.l.smask[w] = m;
+        for (uint32_t rest = m; rest; rest &= rest - 1u) {
+            const uint32_t l = w * 32u + (uint32_t)(__ffs(rest) - 1);
+            if (l < L)
+                for (uint32_t v = 0; v < V; ++v) k.l.sfix[(size_t)v * L + l] = 0ull;
+        }
+    }
 }
 
 // What a day's first step starts from, in one pass over the locations (a
@@ -926,7 +1020,7 @@ __device__ __forceinline__ uint32_t scan_lookback(const KArgs& k, uint32_t tile,
                     }
                     if (__all_sync(0xffffffffu, fl != 0u)) break;
                     if (spin >= SCAN_SPIN_LIMIT) {
-                        if (lane == 0) atomicOr(k.err, ERR_SCAN_WAIT);
+                        if (lane == 0) raise_error(k, ERR_SCAN_WAIT);
                         if (fl == 0u) {
                             fl = 2u;
                             w = 0;
@@ -971,9 +1065,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
     // before (no prefix, no cursor writes).
     const uint32_t t_step = k.clock->t0 + step;
     const bool rebuild = LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step);
-    // merge_q 1: the location quarantines are merged at the steps whose
-    // decisions wrote some (the day graph); 2: at every call
-    merge_q = merge_q == 2 || (merge_q == 1 && k.l.build[3] == t_step);
+    // merge_q: the location quarantines are merged if decisions wrote some
+    merge_q = merge_q && k.l.build[4] != 0u;
     if (!rebuild && !with_hazard && !merge_q) return;
     uint32_t tile = blockIdx.x;
     if (LOOKBACK && rebuild) {
@@ -1145,7 +1238,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
     // the counts are read at the flagged locations only
     const uint32_t t_step = k.clock->t0 + step;
     const bool rebuild = LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step);
-    merge_q = merge_q == 2 || (merge_q == 1 && k.l.build[3] == t_step);
+    merge_q = merge_q && k.l.build[4] != 0u;
     if (!rebuild && !with_hazard && !merge_q) return;
     uint32_t tile = blockIdx.x;
     if (LOOKBACK && rebuild) {
@@ -1262,28 +1355,53 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
     }
 }
 
-// CSR scatter and/or infection draw of one step.
+// CSR scatter and/or infection draw of one step, four consecutive agents per
+// thread (one 16-byte load of their locations, their slots' returning atomics
+// and their locations' mask words in flight together).  A scatter of a step
+// without a rebuild has nothing to do.  scatter 2: the scan before merged the
+// location quarantines.
 __global__ void __launch_bounds__(256) k_scatter_draw(KArgs k, uint32_t step, int scatter, int draw) {
     __shared__ double s_grad[GRAD_N];
-    grad_begin(k, s_grad);
     const uint32_t N = k.a.n, L = k.l.n;
     const uint32_t t = k.clock->t0 + step;
-    const bool rebuild = csr_rebuild(k, t);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < N; base += stride) {
-        const uint32_t i = base + threadIdx.x;
-        const bool act = i < N;
-        double term = 0.0;
-        const uint32_t loc = act ? k.a.location[i] : NONE;
-        const bool ok = act && loc < L;
-        bool hz = false;
-        const float h0 = (draw && ok) ? hazard_at(k, loc, &hz) : 0.0f;
-        if (scatter) {
-            const uint32_t pos = take_slot(k, ok, loc, rebuild);
-            if (ok) store_slot(k, pos, i);
+    const bool rebuild = scatter && csr_rebuild(k, t);
+    if (scatter == 2 && blockIdx.x == 0 && threadIdx.x == 0) k.l.build[4] = 0u;
+    if (!rebuild && !draw) return;
+    grad_begin(k, s_grad);
+    const uint32_t quads = (N + 3u) >> 2;
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += gridDim.x * blockDim.x) {  // warp-uniform trips
+        const uint32_t q = q0 + threadIdx.x, i0 = q * 4u;
+        uint32_t loc[4];
+        if (q < quads && i0 + 3u < N) {
+            const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
+            loc[0] = v.x, loc[1] = v.y, loc[2] = v.z, loc[3] = v.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) loc[u] = q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
         }
-        if (ok && draw && hz) term = draw_agent(k, i, loc, t, h0, s_grad);
-        if (k.track_expected) add_expected(k, act, i, term);
+        if (rebuild) {
+            uint32_t pos[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) pos[u] = take_slot(k, loc[u] < L, loc[u]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (loc[u] < L) store_slot(k, pos[u], i0 + (uint32_t)u);
+        }
+        if (draw) {
+            uint32_t hz = 0;  // the agents at a location with a ratio
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (loc[u] < L) hz |= (k.l.hmask[loc[u] >> 5] >> (loc[u] & 31u) & 1u) << u;
+#pragma unroll 1
+            for (int u = 0; u < 4; ++u) {  // (one copy of the draw; few warps have any)
+                const bool mine = (hz >> u) & 1u;
+                if (!__any_sync(0xffffffffu, mine)) continue;
+                const uint32_t l = u == 0 ? loc[0] : u == 1 ? loc[1] : u == 2 ? loc[2] : loc[3];
+                double term = 0.0;
+                if (mine) term = draw_agent(k, i0 + (uint32_t)u, l, t, k.l.hazard[l], s_grad);
+                if (k.track_expected) add_expected(k, mine, i0 + (uint32_t)u, term);
+            }
+        }
     }
     grad_end(k, s_grad);
 }
@@ -1364,7 +1482,7 @@ __device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
         uint32_t spins = 0;
         while ((int32_t)(ld_acquire_gpu(&k.l.bar[0]) - target) < 0) {
             if ((++spins & 1023u) == 0u) {
-                if (spins >= BARRIER_SPIN_LIMIT) atomicOr(k.err, ERR_BARRIER);
+                if (spins >= BARRIER_SPIN_LIMIT) raise_error(k, ERR_BARRIER);
                 if (ld_acquire_gpu(k.err) & ERR_BARRIER) {
                     ok = false;
                     break;
@@ -1397,23 +1515,6 @@ __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
     bool nz = k.l.sfix[l] != 0ull;
     for (uint32_t v = 1; v < k.m.n_variants && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
     return nz;
-}
-
-// Where a warp's lanes put the entries they flagged (bits of `flags`, one
-// per agent of the lane) in a block's list: the first one's place (one
-// shared-memory atomic per warp).
-__device__ __forceinline__ uint32_t list_place(uint32_t flags, uint32_t* s_cnt) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t mine = __popc(flags);
-    uint32_t inc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    uint32_t base = 0;
-    if (lane == 31 && inc) base = atomicAdd(s_cnt, inc);
-    return __shfl_sync(0xffffffffu, base, 31) + inc - mine;
 }
 
 // The block's lists of its own agents (four consecutive agents per thread,
@@ -1642,7 +1743,7 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32
         const uint32_t i = k.l.list_agent[pos];
         const float su0 = k.l.list_su[pos];
         if (loc >= L || i >= N) {
-            atomicOr(k.err, ERR_AGENT_LIST);
+            raise_error(k, ERR_AGENT_LIST);
             continue;
         }
         const uint32_t cnt = k.l.counts[loc];
@@ -1672,7 +1773,7 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32
             if (at < L)
                 k.l.replay_list[at] = loc;
             else
-                atomicOr(k.err, ERR_AGENT_LIST);
+                raise_error(k, ERR_AGENT_LIST);
         }
         entries += dr.n;
         hazard += any_h ? dr.n : 0u;
@@ -1691,7 +1792,7 @@ __device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, 
         if (p < N)
             k.l.replay_slot[p] = (uint32_t)(seg + j);
         else
-            atomicOr(k.err, ERR_AGENT_LIST);
+            raise_error(k, ERR_AGENT_LIST);
     }
 }
 
@@ -1803,14 +1904,14 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
     for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
         const uint32_t loc = k.l.replay_list[f];
         if (loc >= L) {
-            if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
+            if (lane == 0) raise_error(k, ERR_AGENT_LIST);
             continue;
         }
         const uint32_t cnt = k.l.counts[loc], e = k.l.replay_cursor[loc], b = e - cnt;  // its gathered entries
         const uint32_t rep = k.l.rep[loc];
         const float wl = k.l.infectiousness[loc];
         if (e > N || cnt > e) {
-            if (lane == 0) atomicOr(k.err, ERR_AGENT_LIST);
+            if (lane == 0) raise_error(k, ERR_AGENT_LIST);
             continue;
         }
         const RepConst rc = rep_const(k, rep);
@@ -1877,7 +1978,7 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
                 const uint32_t pos = k.l.replay_slot[p];
                 const uint32_t i = k.l.list_agent[pos];
                 if (i >= N) {
-                    atomicOr(k.err, ERR_AGENT_LIST);
+                    raise_error(k, ERR_AGENT_LIST);
                     break;
                 }
                 infected |= draw_entry(k, pos, i, loc, rep, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
@@ -1899,7 +2000,7 @@ __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t
     {
         uint32_t n = *s_cnt;
         if (n > cap) {
-            if (threadIdx.x == 0) atomicOr(k.err, ERR_AGENT_LIST);
+            if (threadIdx.x == 0) raise_error(k, ERR_AGENT_LIST);
             n = 0;
         }
         const uint32_t* seg = k.a.worklist + (size_t)blockIdx.x * cap;
@@ -1923,7 +2024,7 @@ __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t
             inputs(ni, nd);
             n2 = j + 2u * T < n ? seg[j + 2u * T] : NONE;
             if (i >= k.a.n) {
-                atomicOr(k.err, ERR_AGENT_LIST);
+                raise_error(k, ERR_AGENT_LIST);
                 continue;
             }
             // (queued for its timestamp, unless everybody is at the curfew)
@@ -2703,7 +2804,7 @@ __global__ void k_bounded_wait_probe(KArgs k, uint32_t iters) {
     uint32_t n = 0;
     while (*flag == 0u) {
         if (++n >= iters) {
-            atomicOr(k.err, ERR_TEST_WAIT);
+            raise_error(k, ERR_TEST_WAIT);
             return;
         }
     }
@@ -2742,13 +2843,17 @@ static unsigned agent_grid(const KArgs& k, unsigned wave) {
     return std::min(g, grid_for(k.a.n, 1 << 20));
 }
 
-void launch_movement(const KArgs& k, uint32_t step, bool day, cudaStream_t s) {
+void launch_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
     static unsigned g = 0;
-    if (!g) g = wave_grid(k_movement<false>, 1u << 30);
-    if (day)
-        k_movement<true><<<agent_grid(k, g), 256, 0, s>>>(k, step);
-    else
-        k_movement<false><<<agent_grid(k, g), 256, 0, s>>>(k, step);
+    if (!g) g = wave_grid(k_movement, 1u << 30);
+    k_movement<<<agent_grid(k, g), 256, 0, s>>>(k, step);
+}
+static unsigned quad_grid(uint32_t n, unsigned wave) { return std::min(wave, grid_for((n + 3u) / 4u, 1 << 20)); }
+void launch_phase_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
+    static unsigned g = 0;
+    if (!g) g = wave_grid(k_phase_movement, 1u << 30);
+    k_reset_sums<<<grid_for((k.l.n + 31u) / 32u, 8), 256, 0, s>>>(k);
+    k_phase_movement<<<quad_grid(k.a.n, g), PHASE_THREADS, 0, s>>>(k, step);
 }
 void launch_day_begin(const KArgs& k, cudaStream_t s) { k_day_begin<<<grid_for(k.l.n, 8), 256, 0, s>>>(k); }
 // The day kernel's grid: every block resident at once (its grid barriers
@@ -2832,7 +2937,7 @@ int scan_kernels(const KArgs& k) { return k.tune.scan_mode == 0 || k.tune.scan_m
 void launch_scatter_draw(const KArgs& k, uint32_t step, int scatter, int draw, cudaStream_t s) {
     static unsigned g = 0;
     if (!g) g = wave_grid(k_scatter_draw, 1u << 30);
-    k_scatter_draw<<<agent_grid(k, g), 256, 0, s>>>(k, step, scatter, draw);
+    k_scatter_draw<<<quad_grid(k.a.n, g), 256, 0, s>>>(k, step, scatter, draw);
 }
 void launch_offsets(const KArgs& k, cudaStream_t s) {
     k_offsets_from_cursor<<<grid_for(k.l.n + 1, 8), 256, 0, s>>>(k, k.l.csr_off);

@@ -192,9 +192,10 @@ struct DevLocs {
     size_t list_cap;
     uint32_t* list_count;         // [WORK_MAX_BLOCKS] entries of each block's segment
     uint32_t* replay_stamp;       // [n] the last segment of draws that flagged the location
-    uint32_t* replay_list;        // [n] the locations the running segment flagged
+    uint4* replay_list;           // [n] the locations the running segment flagged: location, first
+                                  // entry in replay_slot, agents, replica
     uint32_t* replay_cursor;      // [n] next free place of a flagged location in replay_slot
-    uint32_t* replay_slot;        // [N] the flagged locations' list entries, by location
+    uint2* replay_slot;           // [N] the flagged locations' list entries (entry, agent), by location
     uint64_t* scan_status;        // per-tile status words of the single-pass scan (epoch | flag | value)
     uint32_t* scan_state;         // [0] epoch of the next single-pass scan, [1] its tile ticket
     uint32_t* build;              // [0] timestamp at which agents last took new locations,

@@ -1511,9 +1511,19 @@ __device__ __forceinline__ void merge_quarantine(const KArgs& k) {
     }
 }
 
+// The day kernel is compiled for VC variants (0: any number) and with or
+// without the expected infections and the adjoint (SUMS): what a simulation
+// without them does not need costs its decisions registers (one kernel for
+// all spilled 224 bytes a thread and decided 7% slower).
+template <int VC>
+__device__ __forceinline__ uint32_t nvar(const KArgs& k) {
+    return VC ? (uint32_t)VC : k.m.n_variants;
+}
+
+template <int VC, bool SUMS>
 __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
     bool nz = k.l.sfix[l] != 0ull;
-    for (uint32_t v = 1; v < k.m.n_variants && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
+    for (uint32_t v = 1; v < nvar<VC>(k) && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
     return nz;
 }
 
@@ -1531,9 +1541,10 @@ __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
 // its own (reserving segments first, a pass over the mask, a barrier and a
 // returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
 // 20M).  queue: the work list of those that decide at s1.
+template <int VC, bool SUMS>
 __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, uint32_t s1, uint32_t cap,
                                             DayShared& sh) {
-    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants;
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
     __syncthreads();
     if (threadIdx.x == 0) {
         if (list) sh.listed = 0u;
@@ -1585,7 +1596,7 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
 #pragma unroll
             for (int u = 0; u < 8; ++u)
                 if ((lw[u] >> (loc[u] & 31u)) & 1u) {
-                    if (nonzero_sum(k, loc[u]))
+                    if (nonzero_sum<VC, SUMS>(k, loc[u]))
                         flags |= 1u << u;
                     else
                         atomicAnd(&k.l.hmask[loc[u] >> 5], ~(1u << (loc[u] & 31u)));
@@ -1623,10 +1634,11 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
 }
 
 // the locations with a nonzero sum and the agents listed (profiled graph only)
+template <int VC, bool SUMS>
 __device__ void count_listed(const KArgs& k, const DayShared& sh) {
     uint32_t locs = 0;
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < k.l.n; l += gridDim.x * blockDim.x)
-        locs += nonzero_sum(k, l) ? 1u : 0u;
+        locs += nonzero_sum<VC, SUMS>(k, l) ? 1u : 0u;
     locs = __reduce_add_sync(__activemask(), locs);
     if ((threadIdx.x & 31) == 0 && locs) atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)locs);
     if (threadIdx.x == 0 && sh.listed) atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)sh.listed);
@@ -1650,21 +1662,29 @@ __device__ __forceinline__ void add_expected_rep(const KArgs& k, bool act, uint3
 }
 
 // DynamicPPState::gotInfected (dynamicPPState.cpp:235-244) and the agent's
-// statistics (locationList.h:283-304)
-__device__ __forceinline__ void infect_agent(const KArgs& k, uint32_t i, uint32_t v, uint32_t loc, uint32_t t) {
-    k.a.state[i] = (int8_t)k.m.first_infected;
+// statistics (locationList.h:283-304); inf: its new infectiousness
+// (update_meta).  What it reads it reads first, in one round trip.
+template <int VC, bool SUMS>
+__device__ __forceinline__ void infect_agent(const KArgs& k, uint32_t i, uint32_t v, uint32_t loc, uint32_t t,
+                                             float inf) {
+    const uint32_t N = k.a.n, st = k.m.first_infected;
+    const uint8_t count = k.a.st_infected_count[i];
+    const uint32_t mask = k.a.st_variant_mask[i];
+    const uint32_t w = k.a.dinfo[i] & ~(7u << DW_WB_SHIFT | DW_INFECTIOUS);
+    const uint32_t wb = k.m.state_wb[st];
+    const float su = k.m.state_susceptible[st] ? 1.0f : 0.0f;
+    k.a.state[i] = (int8_t)st;
     k.a.variant[i] = (uint8_t)v;
     k.a.days[i] = -2;
-    update_meta(k, i);
+    k.a.infectious[i] = inf;
+    for (uint32_t q = 0; q < nvar<VC>(k); ++q) k.a.susceptible[(size_t)q * N + i] = su;
     k.a.st_infected_ts[i] = t;
-    k.a.st_infected_count[i] = k.a.st_infected_count[i] + 1;
+    k.a.st_infected_count[i] = (uint8_t)(count + 1);
     k.a.st_infected_loc[i] = loc;
-    k.a.st_worst_state[i] = (int8_t)k.m.first_infected;
+    k.a.st_worst_state[i] = (int8_t)st;
     k.a.st_worst_ts[i] = t;
-    k.a.st_variant_mask[i] |= 1u << v;
-    const uint32_t w = k.a.dinfo[i] & ~(7u << DW_WB_SHIFT | DW_INFECTIOUS);
-    k.a.dinfo[i] = w | (uint32_t)k.m.state_wb[k.m.first_infected] << DW_WB_SHIFT |
-                   (k.a.infectious[i] != 0.0f ? DW_INFECTIOUS : 0u);
+    k.a.st_variant_mask[i] = mask | 1u << v;
+    k.a.dinfo[i] = w | wb << DW_WB_SHIFT | (inf != 0.0f ? DW_INFECTIOUS : 0u);
 }
 
 // U < p for the 53-bit uniform U = K * 2^-53 of the words (a, b)
@@ -1731,9 +1751,10 @@ struct DrawRun {
 // phase_replay repeats that location's draws with the ratio changing as its
 // agents are infected.  At a location without such an entry the ratio
 // cannot change, so the draws compared with it were the right ones.
+template <int VC, bool SUMS>
 __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, uint32_t* n_entries,
                            uint32_t* n_hazard) {
-    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
     const bool one_rep = k.r.n == 1;
     const RepConst rc0 = rep_const(k, 0);
     uint32_t entries = 0, hazard = 0;
@@ -1769,9 +1790,10 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32
         }
         if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
             const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
-            k.l.replay_cursor[loc] = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
+            const uint32_t room = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
+            k.l.replay_cursor[loc] = room;
             if (at < L)
-                k.l.replay_list[at] = loc;
+                k.l.replay_list[at] = make_uint4(loc, room, cnt, rep);
             else
                 raise_error(k, ERR_AGENT_LIST);
         }
@@ -1788,9 +1810,10 @@ __device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, 
     for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
         const uint32_t loc = k.l.list_loc[seg + j];
         if (loc >= L || k.l.replay_stamp[loc] != dr.epoch) continue;
+        const uint32_t i = k.l.list_agent[seg + j];
         const uint32_t p = atomicAdd(&k.l.replay_cursor[loc], 1u);
         if (p < N)
-            k.l.replay_slot[p] = (uint32_t)(seg + j);
+            k.l.replay_slot[p] = make_uint2((uint32_t)(seg + j), i);
         else
             raise_error(k, ERR_AGENT_LIST);
     }
@@ -1798,8 +1821,9 @@ __device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, 
 
 // The expected infections (and the adjoint's terms) of the segment's draws at
 // the locations that are not replayed: every timestep's are the same.
+template <int VC, bool SUMS>
 __device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad) {
-    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
     for (uint32_t base = 0; base < listed; base += blockDim.x) {  // block-uniform trips
         const uint32_t j = base + threadIdx.x;
         const size_t pos = seg + j;
@@ -1821,15 +1845,16 @@ __device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, ui
                 if (!(s_eff > 0.0f)) continue;
                 const float pf = h * s_eff;
                 term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
-                if (k.adj.on && pf < 1.0f)
+                if ((SUMS && k.adj.on) && pf < 1.0f)
                     adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x, dr.n);
             }
         }
-        if (k.track_expected) add_expected_rep(k, act, rep, term);
+        if ((SUMS && k.track_expected)) add_expected_rep(k, act, rep, term);
     }
 }
 
 // The sum change of an agent at location loc infected there.
+template <int VC, bool SUMS>
 __device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t loc, float inf0, uint32_t var0,
                                                      float inf, uint32_t var) {
     const uint32_t L = k.l.n;
@@ -1849,13 +1874,14 @@ __device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t lo
 // which the ratios of the next timestep are computed from.  Adds the sum of
 // min(1, p) over its draws to *term when expected infections are tracked;
 // returns whether the agent was infected.
+template <int VC, bool SUMS>
 __device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t i, uint32_t loc, uint32_t rep,
                                            const RepConst& rc, uint32_t t, const float* s_h, const float* s_x,
                                            double* s_grad, double* term) {
-    const uint32_t N = k.a.n, V = k.m.n_variants;
+    const uint32_t N = k.a.n, V = nvar<VC>(k);
     bool infected = false;
-    float inf0 = 0.0f, sigma = 0.0f;
-    uint32_t var0 = 0;
+    float inf0 = 0.0f, inf = 0.0f, sigma = 0.0f;
+    uint32_t var0 = 0, var = 0;
     for (uint32_t v = 0; v < V; ++v) {
         const float h = s_h[v];
         if (!(h > 0.0f)) continue;
@@ -1865,8 +1891,8 @@ __device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t 
         const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.list_su[v * k.l.list_cap + pos];
         if (!(s_eff > 0.0f)) continue;
         const float pf = h * s_eff;
-        if (k.track_expected) *term += pf < 1.0f ? (double)pf : 1.0;
-        if (k.adj.on && pf < 1.0f)
+        if ((SUMS && k.track_expected)) *term += pf < 1.0f ? (double)pf : 1.0;
+        if ((SUMS && k.adj.on) && pf < 1.0f)
             adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1u);
         const psim_ctr4 o = infect_words(rc.seed, i - rc.off, t, v);
         if (u01_below(o.v[0], o.v[1], u01_limit(pf))) {
@@ -1876,117 +1902,159 @@ __device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t 
                 sigma = k.p.sigma_band[k.a.band[i]];
                 infected = true;
             }
-            infect_agent(k, i, v, loc, t);
+            inf = k.m.state_infectious[k.m.first_infected] * k.m.variant_multiplier[v];
+            var = v;
+            infect_agent<VC, SUMS>(k, i, v, loc, t, inf);
         }
     }
     if (infected) {
-        for (uint32_t v = 0; v < V; ++v)
-            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
-        const float inf = k.a.infectious[i];
-        add_infection_change(k, loc, inf0, var0, inf, inf > 0.0f ? k.a.variant[i] : 0u);
+        const float su = (k.m.state_susceptible[k.m.first_infected] ? 1.0f : 0.0f) * sigma;
+        for (uint32_t v = 0; v < V; ++v) k.l.list_su[v * k.l.list_cap + pos] = su;
+        add_infection_change<VC, SUMS>(k, loc, inf0, var0, inf, inf > 0.0f ? var : 0u);
     }
     return infected;
 }
 
-// The flagged locations' draws, a warp per location, timestep after timestep.
-// A location of up to 32 agents and one variant (almost all) keeps its sum and
-// a lane per agent in registers: a timestep is a Philox block and a ballot,
-// and an infection adds its change of the sum for the next timestep.  Others
-// go over their entries 32 at a time; the ratios are kept in shared memory
-// and computed again after a timestep that infected somebody there (all its
+// The ratios of a replayed location (and their arguments) from its sums, in
+// the warp's shared memory.  Past L1: the sums change in L2 (reductions).
+template <int VC, bool SUMS>
+__device__ __forceinline__ void replay_ratios(const KArgs& k, const DrawRun& dr, const uint4& r, float wl, float kf,
+                                              float* s_h, float* s_x) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    if (lane < nvar<VC>(k)) {
+        const long long fix = (long long)__ldcg(&k.l.sfix[(size_t)lane * k.l.n + r.x]);
+        float x = 0.0f;
+        s_h[lane] = fix != 0 ? psim_hazard_x(fix, r.z, kf, wl, dr.season, k.p.time_step, &x) : 0.0f;
+        s_x[lane] = x;
+    }
+    __syncwarp();
+}
+
+// A replayed location of up to 64 agents and VM variants at most (almost all
+// of them): two entries per lane in registers, with the draws' bounds.  A
+// timestep without an infection is a Philox block per entry and variant and a
+// vote; one with an infection goes through draw_entry for the agents it hit
+// and computes the bounds again.  Expected infections and adjoint terms are
+// added for all timesteps since the bounds last changed.
+template <int VC, bool SUMS, int VM>
+__device__ __forceinline__ void replay_registers(const KArgs& k, const DrawRun& dr, const uint4& r, float wl,
+                                                 const RepConst& rc, float* s_h, float* s_x, double* s_grad,
+                                                 double* term) {
+    constexpr int Q = 2;
+    const uint32_t N = k.a.n, lane = threadIdx.x & 31u;
+    const bool sums = (SUMS && k.track_expected) || (SUMS && k.adj.on);
+    uint32_t pos[Q], id[Q];
+    float su[Q][VM];
+    unsigned long long limit[Q][VM];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+        const uint32_t p = lane + 32u * (uint32_t)e;
+        const uint2 s = p < r.z ? k.l.replay_slot[r.y + p] : make_uint2(0u, NONE);
+        pos[e] = s.x;
+        id[e] = s.y;
+    }
+    uint32_t active = 0;
+#pragma unroll
+    for (int v = 0; v < VM; ++v)
+        if ((uint32_t)v < nvar<VC>(k) && k.r.variant_active[r.w * nvar<VC>(k) + v]) active |= 1u << v;
+    const auto bounds = [&]() {
+        replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, s_h, s_x);
+#pragma unroll
+        for (int e = 0; e < Q; ++e)
+#pragma unroll
+            for (int v = 0; v < VM; ++v) {
+                const bool on = id[e] < N && ((active >> v) & 1u);
+                su[e][v] = on ? k.l.list_su[v * k.l.list_cap + pos[e]] : 0.0f;
+                const float p = on ? s_h[v] * su[e][v] : 0.0f;
+                limit[e][v] = p > 0.0f ? u01_limit(p) : 0ull;
+            }
+    };
+    // (one copy each of what is rare)
+    const auto add = [&](uint32_t hit, uint32_t times) {
+#pragma unroll 1
+        for (int e = 0; e < Q; ++e) {
+            const uint32_t i = e ? id[1] : id[0], n = times - ((hit >> e) & 1u);
+#pragma unroll
+            for (int v = 0; v < VM; ++v) {
+                const float s = e ? su[1][v] : su[0][v], h = s_h[v], pf = h * s;
+                if (!((active >> v) & 1u) || !(pf > 0.0f) || !n) continue;
+                if ((SUMS && k.track_expected)) *term += (double)n * (pf < 1.0f ? (double)pf : 1.0);
+                if ((SUMS && k.adj.on) && pf < 1.0f)
+                    adjoint_terms(k, i, r.x, v, r.w, h, k.a.susceptible[(size_t)v * N + i], s, s_grad, s_x[v], n);
+            }
+        }
+    };
+    bounds();
+    uint32_t since = 0;  // timesteps since the bounds changed
+    for (uint32_t q = 0; q < dr.n; ++q) {
+        uint32_t hit = 0;
+#pragma unroll
+        for (int e = 0; e < Q; ++e)
+#pragma unroll
+            for (int v = 0; v < VM; ++v)
+                if (limit[e][v]) {
+                    const psim_ctr4 o = infect_words(rc.seed, id[e] - rc.off, dr.t + q, v);
+                    hit |= u01_below(o.v[0], o.v[1], limit[e][v]) ? 1u << e : 0u;
+                }
+        if (!__any_sync(0xffffffffu, hit)) {
+            ++since;
+            continue;
+        }
+        if (sums) add(hit, since + 1u);  // (draw_entry adds this timestep's of those it hit)
+#pragma unroll 1
+        for (int e = 0; e < Q; ++e)
+            if ((hit >> e) & 1u)
+                draw_entry<VC, SUMS>(k, e ? pos[1] : pos[0], e ? id[1] : id[0], r.x, r.w, rc, dr.t + q, s_h, s_x, s_grad, term);
+        since = 0;
+        if (q + 1u == dr.n) break;
+        __threadfence();  // the reductions before the sums are read again
+        bounds();
+    }
+    if (sums && since) add(0u, since);
+}
+
+// The flagged locations' draws, a warp per location, timestep after timestep:
+// in registers where they fit, else over the entries 32 at a time with the
+// ratios computed again after a timestep that infected somebody (all its
 // draws first: a timestep's ratios come from the sums as it started).
+template <int VC, bool SUMS>
 __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_replay, DayShared& sh) {
-    const uint32_t L = k.l.n, N = k.a.n, V = k.m.n_variants, dt = k.p.time_step;
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool plain = V == 1 && !k.track_expected && !k.adj.on;
     // a block's warps take locations far apart in the list: few locations
     // spread over all SMs
     for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
-        const uint32_t loc = k.l.replay_list[f];
-        if (loc >= L) {
+        const uint4 r = k.l.replay_list[f];  // location, first entry, agents, replica
+        if (r.x >= L || r.y > N || r.z > N - r.y) {
             if (lane == 0) raise_error(k, ERR_AGENT_LIST);
             continue;
         }
-        const uint32_t cnt = k.l.counts[loc], e = k.l.replay_cursor[loc], b = e - cnt;  // its gathered entries
-        const uint32_t rep = k.l.rep[loc];
-        const float wl = k.l.infectiousness[loc];
-        if (e > N || cnt > e) {
-            if (lane == 0) raise_error(k, ERR_AGENT_LIST);
-            continue;
-        }
-        const RepConst rc = rep_const(k, rep);
-        if (plain && cnt <= 32u) {
-            const bool act = (uint32_t)lane < cnt;
-            const uint32_t pos = act ? k.l.replay_slot[b + lane] : 0u;
-            const uint32_t i = act ? k.l.list_agent[pos] : NONE;
-            float su = i < N ? k.l.list_su[pos] : 0.0f;
-            long long fix = (long long)k.l.sfix[loc];
-            const long long fix0 = fix;
-            unsigned long long limit = 0ull;
-            bool fresh = false;
-            for (uint32_t q = 0; q < dr.n; ++q) {
-                if (!fresh) {
-                    float x;
-                    const float p = psim_hazard_x(fix, cnt, rc.kf, wl, dr.season, dt, &x) * su;
-                    limit = p > 0.0f && k.r.variant_active[rep] ? u01_limit(p) : 0ull;
-                    fresh = true;
-                }
-                bool hit = false;
-                if (limit) {
-                    const psim_ctr4 o = infect_words(rc.seed, i - rc.off, dr.t + q, 0u);
-                    hit = u01_below(o.v[0], o.v[1], limit);
-                }
-                if (__any_sync(0xffffffffu, hit)) {
-                    long long change = 0;
-                    if (hit) {
-                        const float inf0 = k.a.infectious[i];
-                        infect_agent(k, i, 0u, loc, dr.t + q);
-                        const float inf = k.a.infectious[i];
-                        su = k.a.susceptible[i] * k.p.sigma_band[k.a.band[i]];
-                        k.l.list_su[pos] = su;
-                        change = (inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll) -
-                                 (inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll);
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) change += __shfl_xor_sync(0xffffffffu, change, o);
-                    fix += change;
-                    fresh = false;
-                }
-            }
-            if (lane == 0 && fix != fix0) {
-                k.l.sfix[loc] = (unsigned long long)fix;
-                if (fix != 0) mark_hazardous(k, loc);
-            }
-            continue;
-        }
+        const float wl = k.l.infectiousness[r.x];
+        const RepConst rc = rep_const(k, r.w);
         double term = 0.0;
-        bool stale = true;  // the ratios: at the start and after an infection
-        for (uint32_t q = 0; q < dr.n; ++q) {
-            if (stale) {
-                __syncwarp();
-                if ((uint32_t)lane < V) {
-                    // past L1: other lanes' reductions changed it in L2
-                    const long long fix = (long long)__ldcg(&k.l.sfix[(size_t)lane * L + loc]);
-                    float x = 0.0f;
-                    sh.h[warp][lane] = fix != 0 ? psim_hazard_x(fix, cnt, rc.kf, wl, dr.season, dt, &x) : 0.0f;
-                    sh.x[warp][lane] = x;
+        if (VC != 2 && V == 1 && r.z <= 64u) {
+            replay_registers<VC, SUMS, 1>(k, dr, r, wl, rc, sh.h[warp], sh.x[warp], sh.grad, &term);
+        } else if (VC != 1 && V == 2 && r.z <= 64u) {
+            replay_registers<VC, SUMS, 2>(k, dr, r, wl, rc, sh.h[warp], sh.x[warp], sh.grad, &term);
+        } else {
+            bool stale = true;  // the ratios: at the start and after an infection
+            for (uint32_t q = 0; q < dr.n; ++q) {
+                if (stale) replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, sh.h[warp], sh.x[warp]);
+                bool infected = false;
+                for (uint32_t p = (uint32_t)lane; p < r.z; p += 32u) {
+                    const uint2 s = k.l.replay_slot[r.y + p];
+                    if (s.y >= N) {
+                        raise_error(k, ERR_AGENT_LIST);
+                        break;
+                    }
+                    infected |= draw_entry<VC, SUMS>(k, s.x, s.y, r.x, r.w, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
                 }
-                __syncwarp();
+                stale = __any_sync(0xffffffffu, infected);
+                if (stale) __threadfence();  // the reductions before the sums are read again
             }
-            bool infected = false;
-            for (uint32_t p = b + (uint32_t)lane; p < e; p += 32u) {
-                const uint32_t pos = k.l.replay_slot[p];
-                const uint32_t i = k.l.list_agent[pos];
-                if (i >= N) {
-                    raise_error(k, ERR_AGENT_LIST);
-                    break;
-                }
-                infected |= draw_entry(k, pos, i, loc, rep, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
-            }
-            stale = __any_sync(0xffffffffu, infected);
-            if (stale) __threadfence();  // the reductions before the sums are read again
         }
-        if (k.track_expected) add_expected_rep(k, true, rep, term);
+        if ((SUMS && k.track_expected)) add_expected_rep(k, true, r.w, term);
     }
 }
 
@@ -1994,6 +2062,7 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
 // count the queue left in shared memory: every block starts its decisions at
 // the same barrier, so handing segments out by ticket balanced nothing), then
 // the histogram and sum deltas of the agents that took a new location.
+template <int VC, bool SUMS>
 __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t* s_mm, const uint32_t* s_cnt) {
     const StepClock c = step_clock(k, s1);
     bool moved = false;
@@ -2035,7 +2104,7 @@ __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t
             if (w != d.w) k.a.dinfo[i] = w;
             if (w & DW_INFECTIOUS) {
                 inf = k.a.infectious[i];
-                var = k.a.variant[i];
+                var = VC == 1 ? 0u : k.a.variant[i];
             }
             moved |= count_agent_delta(k, true, d.loc, loc, inf, var, inf, var);
         }
@@ -2047,6 +2116,7 @@ __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t
 // `step`; *next receives the timestep the next one starts at (step_end after
 // the last).  False when a grid barrier expired (the kernel then ends).  cap =
 // the work-list segment size of a block.
+template <int VC, bool SUMS>
 __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint32_t step_end, uint32_t phases,
                                             uint32_t cap, DayShared& sh, uint32_t* next) {
     const uint32_t tl = PROF_T + PROF_TW * step;  // the segment's timeline slots (profiled graph)
@@ -2083,10 +2153,10 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     if (merge) merge_quarantine(k);
     const size_t seg = (size_t)blockIdx.x * cap;
     if (list || decides) {
-        phase_lists(k, list, decides, e, cap, sh);
+        phase_lists<VC, SUMS>(k, list, decides, e, cap, sh);
         if (decides) mask_clear_shared(sh.mm);
         if (k.prof) {
-            if (list) count_listed(k, sh);
+            if (list) count_listed<VC, SUMS>(k, sh);
             if (threadIdx.x == 0) {
                 if (list && blockIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
                 if (decides && sh.cnt) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)sh.cnt);
@@ -2098,7 +2168,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     const bool draws = (phases & PH_DRAW) != 0;
     if (draws) {
         uint32_t entries = 0, hazard = 0;
-        phase_draw(k, dr, seg, sh.listed, &entries, &hazard);
+        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, &entries, &hazard);
         if (k.prof) {
             __syncwarp();
             entries = __reduce_add_sync(0xffffffffu, entries);
@@ -2114,16 +2184,16 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
     if (draws) {
         const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
-        const bool expected = k.track_expected || k.adj.on;
+        const bool expected = (SUMS && k.track_expected) || (SUMS && k.adj.on);
         if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
         if (n_replay || expected) {
             grad_begin(k, sh.grad);
             if (n_replay) {
                 phase_gather(k, dr, seg, sh.listed);
                 if (!grid_barrier(k, sh)) return false;
-                phase_replay(k, dr, n_replay, sh);
+                phase_replay<VC, SUMS>(k, dr, n_replay, sh);
             }
-            if (expected) phase_expected(k, dr, seg, sh.listed, sh.grad);
+            if (expected) phase_expected<VC, SUMS>(k, dr, seg, sh.listed, sh.grad);
             grad_end(k, sh.grad);
             if (decides || n_replay) {
                 // every replay before any decision and before the list is emptied
@@ -2134,7 +2204,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     }
     prof_mark(k, tl + 4);
     if (decides) {
-        phase_decide(k, e, cap, sh.mm, &sh.cnt);
+        phase_decide<VC, SUMS>(k, e, cap, sh.mm, &sh.cnt);
         mask_flush(k, sh.mm);
     }
     prof_mark(k, tl + 5);
@@ -2142,6 +2212,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
 }
 
 // The day kernel: timesteps step0 .. step_end - 1.
+template <int VC, bool SUMS>
 __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0, uint32_t step_end, uint32_t phases,
                                                         uint32_t cap) {
     __shared__ DayShared sh;
@@ -2155,7 +2226,7 @@ __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0,
     uint32_t step = step0;
     for (;;) {
         uint32_t next = step_end;
-        if (!day_segment(k, step, step_end, phases, cap, sh, &next)) return;
+        if (!day_segment<VC, SUMS>(k, step, step_end, phases, cap, sh, &next)) return;
         if (next >= step_end) return;
         step = next;
         if (!grid_barrier(k, sh)) return;
@@ -2861,15 +2932,22 @@ void launch_day_begin(const KArgs& k, cudaStream_t s) { k_day_begin<<<grid_for(k
 // blocks of 256 threads) capped at the kernel's occupancy, and no more blocks
 // than the population gives work to.  Each block's segment of the lists holds
 // the agents its pass visits.
-static unsigned day_blocks_per_sm() {
-    static int occ = 0;
-    if (!occ) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_day, DAY_THREADS, 0) != cudaSuccess || occ < 1) occ = 1;
+typedef void (*DayKernel)(KArgs, uint32_t, uint32_t, uint32_t, uint32_t);
+// the instance for a context, and its resident blocks per SM
+static DayKernel day_kernel(const KArgs& k, unsigned* per_sm) {
+    static const DayKernel kernels[4] = {k_day<1, false>, k_day<2, false>, k_day<1, true>, k_day<0, true>};
+    static int occ[4] = {0, 0, 0, 0};
+    const bool sums = k.track_expected || k.adj.on;
+    const int q = k.m.n_variants == 1 ? (sums ? 2 : 0) : k.m.n_variants == 2 && !sums ? 1 : 3;
+    if (!occ[q]) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernels[q], DAY_THREADS, 0) != cudaSuccess || n < 1) n = 1;
+        occ[q] = n;
     }
-    return (unsigned)occ;
+    *per_sm = (unsigned)occ[q];
+    return kernels[q];
 }
-static void day_geometry(const KArgs& k, unsigned* grid, uint32_t* cap) {
-    const unsigned occ = day_blocks_per_sm();
+static void day_geometry(const KArgs& k, unsigned occ, unsigned* grid, uint32_t* cap) {
     const unsigned bps = k.tune.blocks_per_sm
                              ? std::min<unsigned>((k.tune.blocks_per_sm * 256u + DAY_THREADS - 1) / DAY_THREADS, occ)
                              : occ;
@@ -2884,7 +2962,9 @@ static void day_geometry(const KArgs& k, unsigned* grid, uint32_t* cap) {
 void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s) {
     unsigned g;
     uint32_t cap;
-    day_geometry(k, &g, &cap);
+    unsigned occ;
+    const DayKernel kernel = day_kernel(k, &occ);
+    day_geometry(k, occ, &g, &cap);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g);
     cfg.blockDim = dim3(DAY_THREADS);
@@ -2894,7 +2974,7 @@ void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phas
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_day, k, step0, step_end, phases, cap);
+    cudaLaunchKernelEx(&cfg, kernel, k, step0, step_end, phases, cap);
 }
 void launch_count(const KArgs& k, cudaStream_t s) { k_count<<<grid_for(k.a.n, 8), 256, 0, s>>>(k); }
 // the scan of the histogram with 256 x tune.scan_items locations per tile:

@@ -112,6 +112,10 @@ size_t state_layout(size_t N, size_t L, size_t V, uint64_t* off) {
     return o;
 }
 
+// entries of the day kernel's lists: the agents, and each thread's last quad
+// past them (a grid of at most N + one block's threads)
+size_t list_capacity(size_t N) { return N + 4 * std::min<size_t>(WORK_MAX_THREADS, N + 1024) + 4; }
+
 template <typename T>
 int dcopy_in(psim_ctx* c, const T* dptr, const T* host, size_t count) {
     if (count == 0) return 0;
@@ -300,7 +304,7 @@ int initial_regroup(psim_ctx* c) {
     if ((rc0 = reset_sums(c))) return rc0;
     launch_count(c->k, c->stream);
     launch_scan(c->k, 0, 1, 0, c->stream);
-    launch_scatter_draw(c->k, 0, 1, 0, c->stream);
+    launch_scatter(c->k, 0, false, c->stream);
     c->list_sparse = false;
     c->csr_full = true;
     // the variant gating of the first steps (the statistics come at midnight)
@@ -320,8 +324,9 @@ int do_step(psim_ctx* c, uint32_t step) {
     launch_phase_movement(c->k, step, c->stream);
     const bool merge = c->params.quarantine_policy > 1;
     launch_scan(c->k, step, 1, merge, c->stream);
-    launch_scatter_draw(c->k, step, merge ? 2 : 1, 1, c->stream);
-    c->launches += 3 + (uint64_t)scan_kernels(c->k);
+    launch_scatter(c->k, step, merge, c->stream);
+    launch_phase_draw(c->k, step, c->stream);
+    c->launches += 4 + (uint64_t)scan_kernels(c->k);
     c->list_sparse = false;
     c->csr_full = true;
     return launch_check(c);
@@ -671,7 +676,7 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
 #define AL(field, cnt) \
     if ((rc = dalloc(c, &da.field, cnt))) return bail(rc);
     AL(hcw, N) AL(rank, N) AL(home, N) AL(dinfo, N)
-    AL(worklist, (size_t)N + (size_t)WORK_MAX_THREADS * 4 + 4)
+    AL(worklist, list_capacity(N))
     AL(move_mask, MOVE_MASK_WORDS)
 #undef AL
     // locations
@@ -693,7 +698,7 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     if ((rc = dalloc(c, &dl.replay_list, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.replay_cursor, L))) return bail(rc);
     if ((rc = dalloc(c, &dl.replay_slot, N))) return bail(rc);
-    dl.list_cap = N + (size_t)WORK_MAX_THREADS * 4 + 4;
+    dl.list_cap = list_capacity(N);
     if ((rc = dalloc(c, &dl.list_agent, dl.list_cap))) return bail(rc);
     if ((rc = dalloc(c, &dl.list_loc, dl.list_cap))) return bail(rc);
     if ((rc = dalloc(c, &dl.list_su, dl.list_cap * V))) return bail(rc);
@@ -744,19 +749,10 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
     // the mutable state saved by a checkpoint
     {
         auto add = [&](void* ptr, size_t bytes) { c->regions.push_back({ptr, bytes}); c->checkpoint_bytes += bytes; };
-        DevAgents& a2 = k.a;
-        add(a2.location, 4 * N); add(a2.move_at, 4 * N); add(a2.state, N); add(a2.days, 2 * N);
-        add(a2.variant, N); add(a2.infectious, 4 * N); add(a2.susceptible, 4 * N * V); add(a2.diagnosed, N);
-        add(a2.quarantined, N); add(a2.stayed_home, N); add(a2.no_work, N); add(a2.last_test, 4 * N);
-        add(a2.st_infected_ts, 4 * N); add(a2.st_infected_loc, 4 * N); add(a2.st_worst_ts, 4 * N);
-        add(a2.st_worst_end_ts, 4 * N); add(a2.st_diagnosed_ts, 4 * N); add(a2.st_quarantined_ts, 4 * N);
-        add(a2.st_quarantined_until, 4 * N); add(a2.st_days_in_quarantine, 4 * N); add(a2.st_hospitalized_ts, 4 * N);
-        add(a2.st_hospitalized_until, 4 * N); add(a2.st_immunization_ts, 4 * N); add(a2.st_recovered_ts, 4 * N);
-        add(a2.st_variant_mask, 4 * N); add(a2.st_immunization_count, N); add(a2.st_infected_count, N);
-        add(a2.st_worst_state, N); add(a2.imm_round, N); add(a2.scaling_v, 4 * N * V);
-        add(dl.infectiousness, 4 * L); add(dl.open, L); add(dl.closed_until, 4 * L); add(dl.quarantine_until, 4 * L);
-        // the histogram is kept incrementally across steps and days
-        add(dl.counts, 4 * L); add(dl.sfix, 8 * L * V); add(dl.smask, 4 * ((L + 2047) / 2048 * 64 + 64));
+        add(c->state_slab, c->state_bytes);
+        // the histogram is kept incrementally across steps and days (the sums
+        // start afresh after a restore)
+        add(dl.counts, 4 * L);
         add(dr.variant_active, R * V); add(dr.expected, 8 * R);
     }
     k.p = c->params;
@@ -1035,6 +1031,7 @@ int psim_checkpoint_restore(psim_ctx* c, uint32_t slot) {
     if (rc) return rc;
     CK(cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream));
     c->csr_full = false;
+    c->list_sparse = true;
     CK(cudaStreamSynchronize(c->stream));
     c->csr_fresh = false;
     return 0;
@@ -1101,7 +1098,7 @@ int psim_regroup(psim_ctx* c) {
     const uint32_t step = c->csr_fresh && since < c->spd ? since : 0u;
     const bool merge = c->params.quarantine_policy > 1;
     launch_scan(c->k, step, 1, merge, c->stream);
-    launch_scatter_draw(c->k, step, merge ? 2 : 1, 0, c->stream);
+    launch_scatter(c->k, step, merge, c->stream);
     c->launches += 1 + (uint64_t)scan_kernels(c->k);
     c->csr_fresh = false;
     c->list_sparse = false;
@@ -1120,7 +1117,7 @@ int psim_infect(psim_ctx* c, uint32_t t, uint32_t variant) {
     int rc = set_clock(c, t);
     if (rc) return rc;
     // the draw only (the CSR was scattered by psim_regroup)
-    launch_scatter_draw(c->k, t % c->spd, 0, 1, c->stream);
+    launch_phase_draw(c->k, t % c->spd, c->stream);
     c->launches += 1;
     rc = launch_check(c);
     if (rc) return rc;
@@ -1299,7 +1296,7 @@ int psim_get_csr(psim_ctx* c, int canonical, uint32_t* offsets, uint32_t* agents
         int rc = force_rebuild(c);
         if (rc) return rc;
         launch_scan(c->k, 0, 0, 0, c->stream);
-        launch_scatter_draw(c->k, 0, 1, 0, c->stream);
+        launch_scatter(c->k, 0, false, c->stream);
         c->launches += 1 + (uint64_t)scan_kernels(c->k);
         c->list_sparse = false;
         c->csr_full = true;
@@ -1323,13 +1320,10 @@ int psim_get_hazard(psim_ctx* c, float* out, int64_t* fixed_sum) {
     (void)fixed_sum;
     if (!out) return 0;
     // hazards are kept only where the mask says some variant's is > 0
-    std::vector<uint32_t> mask((c->L + 31) / 32);
+    launch_clean_hazard(c->k, c->stream);
+    c->launches += 1;
     CK(cudaMemcpyAsync(out, c->k.l.hazard, sizeof(float) * c->L * c->V, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(mask.data(), c->k.l.hmask, sizeof(uint32_t) * mask.size(), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    for (uint32_t l = 0; l < c->L; ++l)
-        if (!((mask[l >> 5] >> (l & 31)) & 1u))
-            for (uint32_t v = 0; v < c->V; ++v) out[(size_t)v * c->L + l] = 0.0f;
     return 0;
 }
 

@@ -375,7 +375,10 @@ void launch_phase_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s)
 void launch_count(const KArgs& k, cudaStream_t s);
 // merge_quarantine: the location quarantines that decisions wrote since the last merge
 void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merge_quarantine, cudaStream_t s);
-void launch_scatter_draw(const KArgs& k, uint32_t step_in_day, int scatter, int draw, cudaStream_t s);
+// merged: the scan before merged the location quarantines
+void launch_scatter(const KArgs& k, uint32_t step_in_day, bool merged, cudaStream_t s);
+void launch_phase_draw(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
+void launch_clean_hazard(const KArgs& k, cudaStream_t s);
 void launch_offsets(const KArgs& k, cudaStream_t s);
 int scan_kernels(const KArgs& k);
 // the day kernel (psim_kernels.cu, k_day): the phases a launch runs, for the
@@ -389,7 +392,7 @@ constexpr uint32_t BAR_REPLAY = 32;
 constexpr uint32_t BAR_REPLAY_SLOTS = 33;
 constexpr uint32_t BAR_WORDS = 64;
 // threads and blocks of the day kernel at most (segments of the lists)
-constexpr uint32_t WORK_MAX_THREADS = 160u * 2048u;
+constexpr uint32_t WORK_MAX_THREADS = 160u * 1024u;
 constexpr uint32_t WORK_MAX_BLOCKS = WORK_MAX_THREADS / 128u;
 // words of the per-day mask of decision steps (1440 steps of one minute at most)
 constexpr uint32_t MOVE_MASK_WORDS = 48;

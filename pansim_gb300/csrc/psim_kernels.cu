@@ -11,8 +11,9 @@
 // locationList.h:233-310), and the decisions of the agents whose decision
 // step comes next.
 // The per-phase entry points (psim_movement, psim_regroup, psim_infect) use
-// k_movement, the scans (k_scan / k_scan_v: prefix of the histogram, ratio
-// of every dirty location) and k_scatter_draw (slots and agent-ordered draws).
+// k_phase_movement, the scans (k_scan / k_scan_v: prefix of the histogram, ratio
+// of every dirty location), k_scatter (slots) and k_phase_draw (agent-ordered
+// draws).
 // Per day: k_progress (DynamicPPState::update), k_test_flag/k_test (DetailedTesting),
 // k_stats (refreshAndPrintStatistics), k_plan_* (RealMovement::planLocations).
 //
@@ -1355,53 +1356,80 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
     }
 }
 
-// CSR scatter and/or infection draw of one step, four consecutive agents per
-// thread (one 16-byte load of their locations, their slots' returning atomics
-// and their locations' mask words in flight together).  A scatter of a step
-// without a rebuild has nothing to do.  scatter 2: the scan before merged the
-// location quarantines.
-__global__ void __launch_bounds__(256) k_scatter_draw(KArgs k, uint32_t step, int scatter, int draw) {
-    __shared__ double s_grad[GRAD_N];
+// A thread's four consecutive locations (one 16-byte load where they are
+// whole), NONE past the last agent.
+__device__ __forceinline__ void load_locations4(const KArgs& k, uint32_t q, uint32_t quads, uint32_t* loc) {
+    const uint32_t N = k.a.n, i0 = q * 4u;
+    if (q < quads && i0 + 3u < N) {
+        const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
+        loc[0] = v.x, loc[1] = v.y, loc[2] = v.z, loc[3] = v.w;
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) loc[u] = q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
+    }
+}
+
+// CSR scatter of one step, four consecutive agents per thread (their slots'
+// returning atomics in flight together).  A step without a rebuild has
+// nothing to do.  merged: the scan before merged the location quarantines.
+__global__ void __launch_bounds__(256) k_scatter(KArgs k, uint32_t step, int merged) {
     const uint32_t N = k.a.n, L = k.l.n;
-    const uint32_t t = k.clock->t0 + step;
-    const bool rebuild = scatter && csr_rebuild(k, t);
-    if (scatter == 2 && blockIdx.x == 0 && threadIdx.x == 0) k.l.build[4] = 0u;
-    if (!rebuild && !draw) return;
-    grad_begin(k, s_grad);
+    if (merged && blockIdx.x == 0 && threadIdx.x == 0) k.l.build[4] = 0u;
+    if (!csr_rebuild(k, k.clock->t0 + step)) return;
     const uint32_t quads = (N + 3u) >> 2;
     for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += gridDim.x * blockDim.x) {  // warp-uniform trips
-        const uint32_t q = q0 + threadIdx.x, i0 = q * 4u;
-        uint32_t loc[4];
-        if (q < quads && i0 + 3u < N) {
-            const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
-            loc[0] = v.x, loc[1] = v.y, loc[2] = v.z, loc[3] = v.w;
-        } else {
+        uint32_t loc[4], pos[4];
+        load_locations4(k, q0 + threadIdx.x, quads, loc);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) loc[u] = q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
+        for (int u = 0; u < 4; ++u) pos[u] = take_slot(k, loc[u] < L, loc[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (loc[u] < L) store_slot(k, pos[u], (q0 + threadIdx.x) * 4u + (uint32_t)u);
+    }
+}
+
+// The infection draws of one step for the per-phase entry points.  A few
+// agents in a thousand are at a location with a ratio: the block collects
+// those of its quads (two in flight per thread) and draws for them in full
+// warps; drawn in place, nearly every warp went through the draw for a lane
+// or two.
+constexpr uint32_t PHASE_DRAW_QUADS = 2;
+__global__ void __launch_bounds__(PHASE_THREADS, 4) k_phase_draw(KArgs k, uint32_t step) {
+    __shared__ double s_grad[GRAD_N];
+    __shared__ uint2 s_list[PHASE_THREADS * 4 * PHASE_DRAW_QUADS];  // agent, location
+    __shared__ uint32_t s_cnt;
+    grad_begin(k, s_grad);
+    const uint32_t N = k.a.n, L = k.l.n;
+    const uint32_t t = k.clock->t0 + step;
+    const uint32_t quads = (N + 3u) >> 2, stride = gridDim.x * blockDim.x;
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += PHASE_DRAW_QUADS * stride) {  // block-uniform trips
+        if (threadIdx.x == 0) s_cnt = 0u;
+        __syncthreads();
+        uint32_t loc[4 * PHASE_DRAW_QUADS], flags = 0;
+#pragma unroll
+        for (uint32_t h = 0; h < PHASE_DRAW_QUADS; ++h)
+            load_locations4(k, q0 + h * stride + threadIdx.x, quads, loc + 4 * h);
+#pragma unroll
+        for (uint32_t u = 0; u < 4 * PHASE_DRAW_QUADS; ++u)
+            if (loc[u] < L) flags |= (k.l.hmask[loc[u] >> 5] >> (loc[u] & 31u) & 1u) << u;
+        if (__any_sync(0xffffffffu, flags != 0u)) {
+            uint32_t at = list_place(flags, &s_cnt);
+#pragma unroll
+            for (uint32_t u = 0; u < 4 * PHASE_DRAW_QUADS; ++u)
+                if ((flags >> u) & 1u)
+                    s_list[at++] = make_uint2((q0 + (u >> 2) * stride + threadIdx.x) * 4u + (u & 3u), loc[u]);
         }
-        if (rebuild) {
-            uint32_t pos[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) pos[u] = take_slot(k, loc[u] < L, loc[u]);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (loc[u] < L) store_slot(k, pos[u], i0 + (uint32_t)u);
+        __syncthreads();
+        const uint32_t n = s_cnt;
+        for (uint32_t b = 0; b < n; b += blockDim.x) {  // block-uniform trips
+            const uint32_t j = b + threadIdx.x;
+            const bool act = j < n;
+            const uint2 e = act ? s_list[j] : make_uint2(0u, 0u);
+            double term = 0.0;
+            if (act) term = draw_agent(k, e.x, e.y, t, k.l.hazard[e.y], s_grad);
+            if (k.track_expected) add_expected(k, act, e.x, term);
         }
-        if (draw) {
-            uint32_t hz = 0;  // the agents at a location with a ratio
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (loc[u] < L) hz |= (k.l.hmask[loc[u] >> 5] >> (loc[u] & 31u) & 1u) << u;
-#pragma unroll 1
-            for (int u = 0; u < 4; ++u) {  // (one copy of the draw; few warps have any)
-                const bool mine = (hz >> u) & 1u;
-                if (!__any_sync(0xffffffffu, mine)) continue;
-                const uint32_t l = u == 0 ? loc[0] : u == 1 ? loc[1] : u == 2 ? loc[2] : loc[3];
-                double term = 0.0;
-                if (mine) term = draw_agent(k, i0 + (uint32_t)u, l, t, k.l.hazard[l], s_grad);
-                if (k.track_expected) add_expected(k, mine, i0 + (uint32_t)u, term);
-            }
-        }
+        __syncthreads();
     }
     grad_end(k, s_grad);
 }
@@ -3014,11 +3042,24 @@ void launch_scan(const KArgs& k, uint32_t step, int with_hazard, int merge_q, cu
         launch_scan_items<8>(k, step, with_hazard, merge_q, s);
 }
 int scan_kernels(const KArgs& k) { return k.tune.scan_mode == 0 || k.tune.scan_mode == 3 ? 1 : 2; }
-void launch_scatter_draw(const KArgs& k, uint32_t step, int scatter, int draw, cudaStream_t s) {
+void launch_scatter(const KArgs& k, uint32_t step, bool merged, cudaStream_t s) {
     static unsigned g = 0;
-    if (!g) g = wave_grid(k_scatter_draw, 1u << 30);
-    k_scatter_draw<<<quad_grid(k.a.n, g), 256, 0, s>>>(k, step, scatter, draw);
+    if (!g) g = wave_grid(k_scatter, 1u << 30);
+    k_scatter<<<quad_grid(k.a.n, g), 256, 0, s>>>(k, step, merged ? 1 : 0);
 }
+void launch_phase_draw(const KArgs& k, uint32_t step, cudaStream_t s) {
+    static unsigned g = 0;
+    if (!g) g = wave_grid(k_phase_draw, 1u << 30);
+    k_phase_draw<<<quad_grid(k.a.n, g), PHASE_THREADS, 0, s>>>(k, step);
+}
+// the ratios of the locations without an infectious agent are zeros
+__global__ void k_clean_hazard(KArgs k) {
+    const uint32_t L = k.l.n, V = k.m.n_variants;
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < L; l += gridDim.x * blockDim.x)
+        if (!((k.l.hmask[l >> 5] >> (l & 31u)) & 1u))
+            for (uint32_t v = 0; v < V; ++v) k.l.hazard[(size_t)v * L + l] = 0.0f;
+}
+void launch_clean_hazard(const KArgs& k, cudaStream_t s) { k_clean_hazard<<<grid_for(k.l.n, 8), 256, 0, s>>>(k); }
 void launch_offsets(const KArgs& k, cudaStream_t s) {
     k_offsets_from_cursor<<<grid_for(k.l.n + 1, 8), 256, 0, s>>>(k, k.l.csr_off);
 }

@@ -644,6 +644,15 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
             da.poss4 = nullptr;
         }
     }
+    // the lists' layouts (0 for all where the lists are not packed in 4 bytes)
+    if ((rc = dalloc(c, &da.layout, N))) return bail(rc);
+    if ((rc = dalloc(c, &k.m.layout, (size_t)LAYOUTS * LAYOUT_TYPES))) return bail(rc);
+    if (da.poss4) {
+        uint32_t* owner = nullptr;
+        if ((rc = dalloc(c, &owner, LAYOUTS))) return bail(rc);
+        launch_layouts(k, owner, c->stream);
+        c->launches += 2;
+    }
     if (a->precond) {
         if ((rc = dupload(c, &da.precond, a->precond, N))) return bail(rc);
     } else {

@@ -67,6 +67,7 @@ struct DevModel {
     // window, computed on the host from the schedule table
     const DecWindow* window;   // [n_agent_types * 28 * steps_per_day]
     const DecChoice* choice;   // the windows' choices, window after window
+    uint16_t* layout;          // [LAYOUTS][LAYOUT_TYPES] rows of the location list layouts
 };
 
 struct DevAgents {
@@ -84,6 +85,8 @@ struct DevAgents {
                                   // holds them
     const uint32_t* poss4;        // the same entries in 4 bytes when they fit (locations below
                                   // 2^26, types below 64): location | type << 26; else null
+    uint16_t* layout;             // which types stand where in the agent's location list (below;
+                                  // 0: any list)
     const uint16_t* rep;          // replica of each agent
     uint32_t* location;
     uint32_t* move_at;            // absolute timestamp of the agent's next decision: the
@@ -145,6 +148,17 @@ constexpr uint32_t DW_DIAG_TS = 1u << 14;    // st_diagnosed_ts > 0
 constexpr uint32_t DW_INFECTIOUS = 1u << 15;  // infectious != 0
 constexpr uint32_t DW_NO_WORK = 1u << 16;    // its no_work flag
 constexpr uint32_t DW_TOO_OLD = 1u << 17;    // at or above the school age restriction
+constexpr uint32_t DW_LAYOUT_SHIFT = 18;     // 12 bits: the layout of its location list
+
+// The layouts of the per-agent location lists: most agents' lists are one of a
+// few sequences of types (home, work, two shops, a hospital), so an agent
+// keeps the number of its sequence and a lookup reads from the sequence's row
+// where the entries of a type begin and how many they are.  Row entry: first
+// entry | number << 8, per type.  Sequences of packed lists (poss4) with every
+// type in one run and at most 120 entries have rows; others are walked.
+constexpr uint32_t LAYOUTS = 4096;           // row 0 unused
+constexpr uint32_t LAYOUT_TYPES = 64;
+constexpr uint32_t LAYOUT_MAX_ENTRIES = 120;
 
 // The flag word of a location: what a decision needs to know of it, in one
 // 2-byte load.  Computed for the day's timesteps before its first one; during
@@ -411,6 +425,8 @@ void launch_test(const KArgs& k, uint32_t t, cudaStream_t s);
 void launch_stats(const KArgs& k, uint32_t t, cudaStream_t s);
 void launch_variant_flags(const KArgs& k, cudaStream_t s);
 void launch_homes(const KArgs& k, cudaStream_t s);
+// the location lists' layouts; owner [LAYOUTS] zeroed: scratch
+void launch_layouts(const KArgs& k, uint32_t* owner, cudaStream_t s);
 void launch_plan(const KArgs& k, uint32_t t, cudaStream_t s);
 void launch_flag_hcw(const KArgs& k, cudaStream_t s);
 void launch_bounded_wait_probe(const KArgs& k, uint32_t iters, cudaStream_t s);

@@ -103,9 +103,31 @@ __device__ uint32_t find_location_range(const KArgs& k, uint32_t b, uint32_t e, 
     return NONE;
 }
 
+// The same for agent i by its list's layout; lb: the list's first entry.
+__device__ __forceinline__ uint32_t find_location_at(const KArgs& k, uint32_t i, uint32_t layout, uint32_t lb,
+                                                     uint32_t lt, int retry, psim_stream* rng, uint32_t f0,
+                                                     uint32_t f1, uint32_t f2) {
+    if (layout == 0) return find_location_range(k, lb, k.a.loc_offset[i + 1], lt, retry, rng, f0, f1, f2);
+    if (lt >= LAYOUT_TYPES) return NONE;
+    const uint32_t e = k.m.layout[layout * LAYOUT_TYPES + lt];
+    const uint32_t count = e >> 8, first = lb + (e & 0xFFu);
+    if (count == 0) return NONE;
+    uint32_t pick = 0;
+    const bool any = count > 1 && lt != f0 && lt != f1 && lt != f2;
+    if (any) pick = psim_below(rng, count);
+    uint32_t loc = k.a.poss4[first + pick] & 0x3FFFFFFu;
+    if (any && retry && loc_open(k, loc) == 0) {
+        // its one retry: another pick, open or not
+        const uint32_t before = pick;
+        while (pick == before) pick = psim_below(rng, count);
+        loc = k.a.poss4[first + pick] & 0x3FFFFFFu;
+    }
+    return loc;
+}
+
 __device__ __forceinline__ uint32_t find_location3(const KArgs& k, uint32_t i, uint32_t lt, int retry, psim_stream* rng,
                                                    uint32_t f0, uint32_t f1, uint32_t f2) {
-    return find_location_range(k, k.a.loc_offset[i], k.a.loc_offset[i + 1], lt, retry, rng, f0, f1, f2);
+    return find_location_at(k, i, k.a.layout[i], k.a.loc_offset[i], lt, retry, rng, f0, f1, f2);
 }
 
 __device__ __forceinline__ uint32_t find_location(const KArgs& k, uint32_t i, uint32_t lt, int retry, psim_stream* rng) {
@@ -183,19 +205,19 @@ __device__ __forceinline__ uint32_t decision_word(const KArgs& k, uint32_t i, ui
     const bool inf = k.a.infectious[i] != 0.0f;
     return type | (uint32_t)k.m.state_wb[st] << DW_WB_SHIFT | (quar ? DW_QUARANTINED : 0u) | (hosp ? DW_HOSPITAL : 0u) |
            (diag ? DW_DIAGNOSED : 0u) | (diag_ts ? DW_DIAG_TS : 0u) | (inf ? DW_INFECTIOUS : 0u) |
-           (no_work ? DW_NO_WORK : 0u) | (age >= k.p.school_age_restriction ? DW_TOO_OLD : 0u);
+           (no_work ? DW_NO_WORK : 0u) | (age >= k.p.school_age_restriction ? DW_TOO_OLD : 0u) |
+           (uint32_t)k.a.layout[i] << DW_LAYOUT_SHIFT;
 }
 
 // What a decision reads of its agent, loaded together before it starts: the
-// decision word, the current location, the agent's entries in the per-agent
-// location list, the replica.
+// decision word, the current location, the agent's first entry in the
+// per-agent location lists, the replica.
 struct DecisionIn {
-    uint32_t w, loc, lb, le, rep;
+    uint32_t w, loc, lb, rep;
 };
 __device__ __forceinline__ void decision_in(const KArgs& k, uint32_t i, DecisionIn& d) {
     d.loc = k.a.location[i];
     d.lb = k.a.loc_offset[i];
-    d.le = k.a.loc_offset[i + 1];
     d.rep = k.r.n == 1 ? 0u : k.a.rep[i];
 }
 
@@ -228,7 +250,8 @@ __device__ __forceinline__ bool quarantine_type(const KArgs& k, uint32_t ty) {
 // list, window, chosen location's flags) and by instructions, not by bytes:
 // the countdowns of every event at every step come from a table computed on
 // the host (no divisions here), a location's flags are one word, the home is
-// looked up once.  22 us of decisions a step at 2M agents, against 25 without
+// looked up once, and an entry of a location list is found by the list's
+// layout.  22 us of decisions a step at 2M agents, against 25 without
 // those; the rare quarantine out of line (its arguments through memory) took
 // 26, and the location list in registers 23.6.
 template <bool DAY>
@@ -243,7 +266,8 @@ __device__ __forceinline__ uint32_t move_decide(const KArgs& k, uint32_t i, uint
         return (f & LF_QUARANTINE) && quarantine_type(k, f & LF_TYPE) ? k.l.quarantine_until[loc] : 0u;
     };
     auto fl = [&](uint32_t lt, int retry) {
-        return find_location_range(k, d.lb, d.le, lt, retry, rng, p.home_type, p.school_type, p.work_type);
+        return find_location_at(k, i, d.w >> DW_LAYOUT_SHIFT, d.lb, lt, retry, rng, p.home_type, p.school_type,
+                                p.work_type);
     };
     uint32_t w = d.w;
     if ((w & DW_QUARANTINED) && k.a.st_quarantined_until[i] <= t) {
@@ -2823,6 +2847,53 @@ __global__ void k_homes(KArgs k) {
     }
 }
 
+// The layout of every agent's location list.  A list whose sequence of types
+// hashes to a row takes it if the row is free or its owner's list has the same
+// sequence (compared entry by entry), else tries the next rows.
+__global__ void k_layouts(KArgs k, uint32_t* owner) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
+        const uint32_t b = k.a.loc_offset[i], n = k.a.loc_offset[i + 1] - b;
+        uint32_t layout = 0;
+        if (n && n <= LAYOUT_MAX_ENTRIES) {
+            unsigned long long seen = 0ull;
+            uint32_t hash = 2166136261u, last = NONE;
+            bool runs = true;
+            for (uint32_t j = 0; j < n; ++j) {
+                const uint32_t ty = k.a.poss4[b + j] >> 26;
+                if (ty != last) {
+                    runs = runs && !((seen >> ty) & 1ull);
+                    seen |= 1ull << ty;
+                    last = ty;
+                }
+                hash = (hash ^ (ty + 1u)) * 16777619u;
+            }
+            for (uint32_t probe = 0; runs && probe < 16u && !layout; ++probe) {
+                const uint32_t row = 1u + (hash + probe) % (LAYOUTS - 1u);
+                const uint32_t prev = atomicCAS(&owner[row], 0u, i + 1u);
+                bool same = prev == 0u;
+                if (!same) {
+                    const uint32_t ob = k.a.loc_offset[prev - 1u];
+                    same = k.a.loc_offset[prev] - ob == n;
+                    for (uint32_t j = 0; same && j < n; ++j) same = k.a.poss4[ob + j] >> 26 == k.a.poss4[b + j] >> 26;
+                }
+                if (same) layout = row;
+            }
+        }
+        k.a.layout[i] = (uint16_t)layout;
+    }
+}
+// the rows, from their owners' lists
+__global__ void k_layout_rows(KArgs k, const uint32_t* owner) {
+    const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= LAYOUTS || owner[row] == 0u) return;
+    const uint32_t i = owner[row] - 1u, b = k.a.loc_offset[i], n = k.a.loc_offset[i + 1] - b;
+    uint16_t* r = k.m.layout + (size_t)row * LAYOUT_TYPES;
+    for (uint32_t j = 0; j < n; ++j) {
+        const uint32_t ty = k.a.poss4[b + j] >> 26, e = r[ty];
+        r[ty] = (uint16_t)(e ? e + 0x100u : j | 0x100u);
+    }
+}
+
 // Simulation::flagHealthcareWorkers, simulation.h:670-693 (type ids 4 / 12 / 14 as
 // hard-coded in the reference)
 __global__ void k_flag_hcw(KArgs k) {
@@ -3111,6 +3182,10 @@ void launch_plan(const KArgs& k, uint32_t t, cudaStream_t s) {
     k_plan_nowork_set<<<grid_for(k.a.n, 8), 256, 0, s>>>(k, t);
 }
 void launch_flag_hcw(const KArgs& k, cudaStream_t s) { k_flag_hcw<<<grid_for(k.a.n, 8), 256, 0, s>>>(k); }
+void launch_layouts(const KArgs& k, uint32_t* owner, cudaStream_t s) {
+    k_layouts<<<grid_for(k.a.n, 8), 256, 0, s>>>(k, owner);
+    k_layout_rows<<<LAYOUTS / 256, 256, 0, s>>>(k, owner);
+}
 void launch_homes(const KArgs& k, cudaStream_t s) { k_homes<<<grid_for(k.a.n, 8), 256, 0, s>>>(k); }
 void launch_type_weights(const KArgs& k, const float* w_by_type, cudaStream_t s) {
     k_type_weights<<<grid_for(k.l.n, 8), 256, 0, s>>>(k, w_by_type);

@@ -1,0 +1,879 @@
+// The day graph's day kernel (templates; psim_day_*.cu compile its instances
+// in parallel).
+#pragma once
+#include "psim_agent.cuh"
+
+namespace psim {
+
+// ---------------------------------------------------------------------------
+// The day graph's day kernel: one launch for all timesteps of a day, a
+// persistent grid (every block resident, a cooperative launch) whose phases
+// are separated by grid barriers only where one phase needs another's results.
+// Most timesteps of a day move nobody (at 2M agents 22 of 144 have deciders),
+// so the day is cut into segments: the timesteps from one whose agents took
+// new locations to the next that somebody decides at.  Per segment:
+//   list      one pass over the block's agents: when agents took new locations
+//             (or a rebuild is pending) those at a location with a nonzero sum
+//             enter the block's agent list (their id, location and
+//             susceptibility x age-band factor of every variant); those that
+//             decide at the segment's end enter the block's work list.  The
+//             location quarantine writes of the decisions before are merged
+//             here too.
+//   draw      every listed entry, one per thread, for all the timesteps of the
+//             segment at once: nobody moves, so a location's infection ratio
+//             stays what it is until somebody there is infected.  An entry
+//             that would be infected commits nothing: it flags its location |
+//             if any was flagged, their entries gathered by location |
+//             the flagged locations (a few) replayed exactly, a warp each,
+//             timestep by timestep with the ratio of the location's sum as the
+//             timestep started (LocationsList::infectAgents,
+//             locationList.h:233-310)
+//   decide  | doMovement of the queued agents and the histogram and sum deltas
+//             of their moves |
+// (| a grid barrier).  A block lists, draws and decides its own agents, so
+// nothing but the flagged locations and the moves passes between blocks.
+// What it replaces drew every timestep in a launch of its own (2.9-5.8 us and
+// a launch gap of 0.9-1.3 us each at 10k-2M agents, ~100 timesteps of a day).
+
+// Grid barrier of the day kernel: every block adds one to a count that only
+// grows (zeroed when the day graph starts) and waits until it reaches the
+// barrier's target.  On GB300 1.4 us with 304 blocks of 512 threads, against
+// 2.5 us for a returning arrival, a reset and a generation word with 608
+// blocks of 256 (arrivals on one address are serialized, so fewer blocks and
+// no returned value).  Every wait is bounded: on expiry the block records
+// ERR_BARRIER and returns false, the others follow (they look at the error
+// flags while they wait), and every later barrier and day kernel returns at
+// once, so a failure ends in an error report, never a hang.  The block's
+// writes reach the other blocks through the arrival (release: the block's
+// threads' writes are ordered before it by the __syncthreads before) and the
+// count's read (acquire).
+constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_add_release_gpu(uint32_t* p, uint32_t x) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+
+// Block-shared scratch of the day kernel.
+struct DayShared {
+    double grad[GRAD_N];
+    float h[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // per warp: a replayed location's ratios
+    float x[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // and their arguments
+    uint32_t mm[MOVE_MASK_WORDS];
+    uint32_t red[32];
+    uint32_t target;  // the barrier count the next barrier waits for
+    uint32_t cnt;     // agents in the block's work list
+    uint32_t listed;  // entries of the block's agent list
+    bool ok;
+};
+
+__device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t target = sh.target;
+        bool ok = true;
+        red_add_release_gpu(&k.l.bar[0], 1u);
+        uint32_t spins = 0;
+        while ((int32_t)(ld_acquire_gpu(&k.l.bar[0]) - target) < 0) {
+            if ((++spins & 1023u) == 0u) {
+                if (spins >= BARRIER_SPIN_LIMIT) raise_error(k, ERR_BARRIER);
+                if (ld_acquire_gpu(k.err) & ERR_BARRIER) {
+                    ok = false;
+                    break;
+                }
+            }
+            __nanosleep(20);
+        }
+        sh.target = target + gridDim.x;
+        sh.ok = ok;
+    }
+    __syncthreads();
+    return sh.ok;
+}
+
+// the location quarantine writes of the last decisions into quarantine_until
+// (grid-stride)
+__device__ __forceinline__ void merge_quarantine(const KArgs& k) {
+    const uint32_t L = k.l.n;
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < L; l += gridDim.x * blockDim.x) {
+        const uint32_t qq = k.l.qu_pending[l];
+        if (qq) {
+            if (qq > k.l.quarantine_until[l]) k.l.quarantine_until[l] = qq;
+            k.l.lflags[l] |= (uint16_t)LF_QUARANTINE;
+            k.l.qu_pending[l] = 0u;
+        }
+    }
+}
+
+// The day kernel is compiled for VC variants (0: any number), with or without
+// the expected infections and the adjoint (SUMS) and for the policies POL of
+// the decisions (move_decide): what a simulation does not use costs its
+// decisions registers (one kernel for all variants and sums spilled 224 bytes
+// a thread and decided 7% slower).
+template <int VC>
+__device__ __forceinline__ uint32_t nvar(const KArgs& k) {
+    return VC ? (uint32_t)VC : k.m.n_variants;
+}
+
+template <int VC, bool SUMS>
+__device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
+    bool nz = k.l.sfix[l] != 0ull;
+    for (uint32_t v = 1; v < nvar<VC>(k) && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
+    return nz;
+}
+
+// The block's lists of its own agents (four consecutive agents per thread,
+// one 16-byte load of a field, two quads in flight; the blocks' quads are
+// dealt in turn).  list: the agent list afresh.  Only the agents at locations
+// with a nonzero sum are listed, because the draws of every step until the
+// next listing need no other location: until then no other location gains a
+// nonzero sum (nobody moves, since a move makes the next segment list again,
+// and a draw infects only agents at a location with a nonzero sum).  The
+// hazard mask is a superset of those locations (every kernel that adds an
+// infectious term sets the bit at once); an agent that finds a zero sum behind
+// its location's bit clears it.  Agents of one location lie in many blocks'
+// lists: the replay gathers those it needs, so no location needs a segment of
+// its own (reserving segments first, a pass over the mask, a barrier and a
+// returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
+// 20M).  queue: the work list of those that decide at s1.
+template <int VC, bool SUMS, int POL>
+__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, uint32_t s1, uint32_t cap,
+                                            DayShared& sh) {
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (list) sh.listed = 0u;
+        if (queue) sh.cnt = 0u;
+    }
+    __syncthreads();
+    const bool everybody = POL == 2 && k.p.enable_curfew && k.p.curfew_begin == s1;
+    const uint32_t t1 = k.clock->t0 + s1;
+    const uint32_t quads = (N + 3u) >> 2;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    const size_t seg = (size_t)blockIdx.x * cap;
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // block-uniform trips
+        uint32_t loc[8], m[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t q = q0 + (uint32_t)h * stride + threadIdx.x;
+            const uint32_t i0 = q * 4u;
+            const bool whole = q < quads && i0 + 3u < N;
+            if (list && whole) {
+                const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
+                loc[4 * h + 0] = v.x;
+                loc[4 * h + 1] = v.y;
+                loc[4 * h + 2] = v.z;
+                loc[4 * h + 3] = v.w;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    loc[4 * h + u] = list && q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
+            }
+            if (queue && whole) {
+                const uint4 v = *reinterpret_cast<const uint4*>(k.a.move_at + i0);
+                m[4 * h + 0] = v.x;
+                m[4 * h + 1] = v.y;
+                m[4 * h + 2] = v.z;
+                m[4 * h + 3] = v.w;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    m[4 * h + u] = queue && q < quads && i0 + u < N ? k.a.move_at[i0 + u] : t1 + 1u;
+            }
+        }
+        const auto agent_of = [&](int u) {
+            return (q0 + (uint32_t)(u >> 2) * stride + threadIdx.x) * 4u + (uint32_t)(u & 3);
+        };
+        if (list) {
+            uint32_t lw[8], flags = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if ((lw[u] >> (loc[u] & 31u)) & 1u) {
+                    if (nonzero_sum<VC, SUMS>(k, loc[u]))
+                        flags |= 1u << u;
+                    else
+                        atomicAnd(&k.l.hmask[loc[u] >> 5], ~(1u << (loc[u] & 31u)));
+                }
+            if (__any_sync(0xffffffffu, flags != 0u)) {
+                uint32_t at = list_place(flags, &sh.listed);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if ((flags >> u) & 1u) {
+                        const uint32_t i = agent_of(u);
+                        const size_t pos = seg + at++;
+                        k.l.list_agent[pos] = i;
+                        k.l.list_loc[pos] = loc[u];
+                        const float sigma = k.p.sigma_band[k.a.band[i]];
+                        for (uint32_t v = 0; v < V; ++v)
+                            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
+                    }
+            }
+        }
+        if (queue) {
+            uint32_t flags = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (agent_of(u) < N && (everybody || m[u] == t1)) flags |= 1u << u;
+            if (__any_sync(0xffffffffu, flags != 0u)) {
+                uint32_t at = list_place(flags, &sh.cnt);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if ((flags >> u) & 1u) k.a.worklist[seg + at++] = agent_of(u);
+            }
+        }
+    }
+    __syncthreads();
+    if (list && threadIdx.x == 0) k.l.list_count[blockIdx.x] = sh.listed;  // for a later launch
+}
+
+// the locations with a nonzero sum and the agents listed (profiled graph only)
+template <int VC, bool SUMS>
+__device__ void count_listed(const KArgs& k, const DayShared& sh) {
+    uint32_t locs = 0;
+    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < k.l.n; l += gridDim.x * blockDim.x)
+        locs += nonzero_sum<VC, SUMS>(k, l) ? 1u : 0u;
+    locs = __reduce_add_sync(__activemask(), locs);
+    if ((threadIdx.x & 31) == 0 && locs) atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)locs);
+    if (threadIdx.x == 0 && sh.listed) atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)sh.listed);
+}
+
+// expected-infection accumulation of the draws: one atomic per replica
+// present in the warp (warp-collective; rep given, not looked up)
+__device__ __forceinline__ void add_expected_rep(const KArgs& k, bool act, uint32_t rep, double term) {
+    const unsigned am = __ballot_sync(0xffffffffu, act && term != 0.0);
+    if (!(act && term != 0.0)) return;
+    const unsigned peers = __match_any_sync(am, rep);
+    const int leader = __ffs(peers) - 1;
+    unsigned rest = peers;
+    double tot = 0.0;
+    while (rest) {
+        const int src = __ffs(rest) - 1;
+        tot += __shfl_sync(peers, term, src);
+        rest &= rest - 1;
+    }
+    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&k.r.expected[rep], tot);
+}
+
+// DynamicPPState::gotInfected (dynamicPPState.cpp:235-244) and the agent's
+// statistics (locationList.h:283-304); inf: its new infectiousness
+// (update_meta).  What it reads it reads first, in one round trip.
+template <int VC, bool SUMS>
+__device__ __forceinline__ void infect_agent(const KArgs& k, uint32_t i, uint32_t v, uint32_t loc, uint32_t t,
+                                             float inf) {
+    const uint32_t N = k.a.n, st = k.m.first_infected;
+    const uint8_t count = k.a.st_infected_count[i];
+    const uint32_t mask = k.a.st_variant_mask[i];
+    const uint32_t w = k.a.dinfo[i] & ~(7u << DW_WB_SHIFT | DW_INFECTIOUS);
+    const uint32_t wb = k.m.state_wb[st];
+    const float su = k.m.state_susceptible[st] ? 1.0f : 0.0f;
+    k.a.state[i] = (int8_t)st;
+    k.a.variant[i] = (uint8_t)v;
+    k.a.days[i] = -2;
+    k.a.infectious[i] = inf;
+    for (uint32_t q = 0; q < nvar<VC>(k); ++q) k.a.susceptible[(size_t)q * N + i] = su;
+    k.a.st_infected_ts[i] = t;
+    k.a.st_infected_count[i] = (uint8_t)(count + 1);
+    k.a.st_infected_loc[i] = loc;
+    k.a.st_worst_state[i] = (int8_t)st;
+    k.a.st_worst_ts[i] = t;
+    k.a.st_variant_mask[i] = mask | 1u << v;
+    k.a.dinfo[i] = w | wb << DW_WB_SHIFT | (inf != 0.0f ? DW_INFECTIOUS : 0u);
+}
+
+// U < p for the 53-bit uniform U = K * 2^-53 of the words (a, b)
+// (psim_u01_from) and a float probability p > 0, in integers: p * 2^53 is
+// exact in float (a power-of-two scaling of a normal or subnormal p), and
+// K < p * 2^53 holds exactly when K < ceil(p * 2^53).  u01_limit is that
+// bound (above every K for p >= 1).
+__device__ __forceinline__ unsigned long long u01_limit(float p) {
+    return p >= 1.0f ? ~0ull : __float2ull_ru(p * 9007199254740992.0f);
+}
+__device__ __forceinline__ bool u01_below(uint32_t a, uint32_t b, unsigned long long limit) {
+    return (((unsigned long long)(a >> 5) << 26) | (unsigned long long)(b >> 6)) < limit;
+}
+// the first two words of the stream (seed, agent, t, infection + v), as
+// psim_u01_once draws them
+__device__ __forceinline__ psim_ctr4 infect_words(unsigned long long seed, uint32_t li, uint32_t t, uint32_t v) {
+    psim_ctr4 c;
+    c.v[0] = li;
+    c.v[1] = t;
+    c.v[2] = PSIM_PHASE_INFECT + v;
+    c.v[3] = 0u;
+    return psim_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+}
+
+// Infection ratio of variant v at location loc (count cnt, weight wl,
+// replica coefficient kf) from the location's fixed-point sum: the formula
+// the scans evaluate (psim_hazard_x), so every entry of a location computes
+// the same value.  x receives its argument.
+__device__ __forceinline__ float entry_hazard(const KArgs& k, uint32_t loc, uint32_t v, uint32_t cnt, float wl,
+                                              float kf, float season, uint32_t dt, float* x) {
+    const long long fix = (long long)k.l.sfix[(size_t)v * k.l.n + loc];
+    *x = 0.0f;
+    return fix != 0 ? psim_hazard_x(fix, cnt, kf, wl, season, dt, x) : 0.0f;
+}
+
+// A replica's infection coefficient, seed and first agent.
+struct RepConst {
+    float kf;
+    uint32_t off;
+    unsigned long long seed;
+};
+__device__ __forceinline__ RepConst rep_const(const KArgs& k, uint32_t rep) {
+    RepConst c;
+    c.kf = k.r.k_f[rep];
+    c.off = k.r.agent_off[rep];
+    c.seed = k.r.seed[rep];
+    return c;
+}
+
+// The timesteps of one segment's draws: its first one (timestamp t), how many
+// there are, the day's season, the replay stamp of its flagged locations.
+struct DrawRun {
+    uint32_t t, n, epoch;
+    float season;
+};
+
+// The draws of every entry of the block's agent list for all the timesteps
+// of the segment, one entry per thread.  Each entry evaluates its location's
+// ratio from the location's sum, count and weight (the same inputs give the
+// same value at every entry) and compares the agent's Philox draw of every
+// timestep with it.  Nothing is committed here: an entry that would be
+// infected flags its location (a stamp per location keeps it in the list
+// once; the first to flag it reserves room for the location's agents), and
+// phase_replay repeats that location's draws with the ratio changing as its
+// agents are infected.  At a location without such an entry the ratio
+// cannot change, so the draws compared with it were the right ones.
+template <int VC, bool SUMS>
+__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, uint32_t* n_entries,
+                           uint32_t* n_hazard) {
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
+    const bool one_rep = k.r.n == 1;
+    const RepConst rc0 = rep_const(k, 0);
+    uint32_t entries = 0, hazard = 0;
+    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
+        const size_t pos = seg + j;
+        const uint32_t loc = k.l.list_loc[pos];
+        const uint32_t i = k.l.list_agent[pos];
+        const float su0 = k.l.list_su[pos];
+        if (loc >= L || i >= N) {
+            raise_error(k, ERR_AGENT_LIST);
+            continue;
+        }
+        const uint32_t cnt = k.l.counts[loc];
+        const float wl = k.l.infectiousness[loc];
+        const uint32_t rep = one_rep ? 0u : k.l.rep[loc];
+        const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
+        bool any_h = false, hit = false;
+        for (uint32_t v = 0; v < V && !hit; ++v) {
+            float x;
+            const float h = entry_hazard(k, loc, v, cnt, wl, rc.kf, dr.season, dt, &x);
+            if (!(h > 0.0f)) continue;
+            any_h = true;
+            if (!k.r.variant_active[rep * V + v]) continue;
+            const float s_eff = v == 0 ? su0 : k.l.list_su[v * k.l.list_cap + pos];
+            if (!(s_eff > 0.0f)) continue;
+            const unsigned long long limit = u01_limit(h * s_eff);
+            const uint32_t li = i - rc.off;
+#pragma unroll 1
+            for (uint32_t q = 0; q < dr.n; ++q) {
+                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + q, v);
+                hit |= u01_below(o.v[0], o.v[1], limit);
+            }
+        }
+        if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
+            const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
+            const uint32_t room = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
+            k.l.replay_cursor[loc] = room;
+            if (at < L)
+                k.l.replay_list[at] = make_uint4(loc, room, cnt, rep);
+            else
+                raise_error(k, ERR_AGENT_LIST);
+        }
+        entries += dr.n;
+        hazard += any_h ? dr.n : 0u;
+    }
+    *n_entries += entries;
+    *n_hazard += hazard;
+}
+
+// The entries of the flagged locations, gathered by location.
+__device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed) {
+    const uint32_t L = k.l.n, N = k.a.n;
+    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
+        const uint32_t loc = k.l.list_loc[seg + j];
+        if (loc >= L || k.l.replay_stamp[loc] != dr.epoch) continue;
+        const uint32_t i = k.l.list_agent[seg + j];
+        const uint32_t p = atomicAdd(&k.l.replay_cursor[loc], 1u);
+        if (p < N)
+            k.l.replay_slot[p] = make_uint2((uint32_t)(seg + j), i);
+        else
+            raise_error(k, ERR_AGENT_LIST);
+    }
+}
+
+// The expected infections (and the adjoint's terms) of the segment's draws at
+// the locations that are not replayed: every timestep's are the same.
+template <int VC, bool SUMS>
+__device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad) {
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
+    for (uint32_t base = 0; base < listed; base += blockDim.x) {  // block-uniform trips
+        const uint32_t j = base + threadIdx.x;
+        const size_t pos = seg + j;
+        const uint32_t loc = j < listed ? k.l.list_loc[pos] : NONE;
+        const uint32_t i = loc < L ? k.l.list_agent[pos] : NONE;
+        const bool act = loc < L && i < N && k.l.replay_stamp[loc] != dr.epoch;
+        uint32_t rep = 0;
+        double term = 0.0;
+        if (act) {
+            const uint32_t cnt = k.l.counts[loc];
+            const float wl = k.l.infectiousness[loc];
+            rep = k.l.rep[loc];
+            const float kf = k.r.k_f[rep];
+            for (uint32_t v = 0; v < V; ++v) {
+                float x;
+                const float h = entry_hazard(k, loc, v, cnt, wl, kf, dr.season, dt, &x);
+                if (!(h > 0.0f) || !k.r.variant_active[rep * V + v]) continue;
+                const float s_eff = k.l.list_su[v * k.l.list_cap + pos];
+                if (!(s_eff > 0.0f)) continue;
+                const float pf = h * s_eff;
+                term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
+                if ((SUMS && k.adj.on) && pf < 1.0f)
+                    adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x, dr.n);
+            }
+        }
+        if ((SUMS && k.track_expected)) add_expected_rep(k, act, rep, term);
+    }
+}
+
+// The sum change of an agent at location loc infected there.
+template <int VC, bool SUMS>
+__device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t loc, float inf0, uint32_t var0,
+                                                     float inf, uint32_t var) {
+    const uint32_t L = k.l.n;
+    const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
+    const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
+    if (q0 == q1 && var0 == var) return;
+    if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc], (unsigned long long)(-q0));
+    if (q1) {
+        atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
+        mark_hazardous(k, loc);
+    }
+}
+
+// One entry's draws of timestep t with its location's ratios s_h (arguments
+// s_x): the agent i of list entry pos.  An agent that is infected updates its
+// entry's susceptibility products (read by no other entry) and its location's sums,
+// which the ratios of the next timestep are computed from.  Adds the sum of
+// min(1, p) over its draws to *term when expected infections are tracked;
+// returns whether the agent was infected.
+template <int VC, bool SUMS>
+__device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t i, uint32_t loc, uint32_t rep,
+                                           const RepConst& rc, uint32_t t, const float* s_h, const float* s_x,
+                                           double* s_grad, double* term) {
+    const uint32_t N = k.a.n, V = nvar<VC>(k);
+    bool infected = false;
+    float inf0 = 0.0f, inf = 0.0f, sigma = 0.0f;
+    uint32_t var0 = 0, var = 0;
+    for (uint32_t v = 0; v < V; ++v) {
+        const float h = s_h[v];
+        if (!(h > 0.0f)) continue;
+        if (!k.r.variant_active[rep * V + v]) continue;
+        // after an infection the later variants read the agent's new
+        // susceptibility (what the entry then gets)
+        const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.list_su[v * k.l.list_cap + pos];
+        if (!(s_eff > 0.0f)) continue;
+        const float pf = h * s_eff;
+        if ((SUMS && k.track_expected)) *term += pf < 1.0f ? (double)pf : 1.0;
+        if ((SUMS && k.adj.on) && pf < 1.0f)
+            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1u);
+        const psim_ctr4 o = infect_words(rc.seed, i - rc.off, t, v);
+        if (u01_below(o.v[0], o.v[1], u01_limit(pf))) {
+            if (!infected) {
+                inf0 = k.a.infectious[i];
+                var0 = inf0 > 0.0f ? k.a.variant[i] : 0u;
+                sigma = k.p.sigma_band[k.a.band[i]];
+                infected = true;
+            }
+            inf = k.m.state_infectious[k.m.first_infected] * k.m.variant_multiplier[v];
+            var = v;
+            infect_agent<VC, SUMS>(k, i, v, loc, t, inf);
+        }
+    }
+    if (infected) {
+        const float su = (k.m.state_susceptible[k.m.first_infected] ? 1.0f : 0.0f) * sigma;
+        for (uint32_t v = 0; v < V; ++v) k.l.list_su[v * k.l.list_cap + pos] = su;
+        add_infection_change<VC, SUMS>(k, loc, inf0, var0, inf, inf > 0.0f ? var : 0u);
+    }
+    return infected;
+}
+
+// The ratios of a replayed location (and their arguments) from its sums, in
+// the warp's shared memory.  Past L1: the sums change in L2 (reductions).
+template <int VC, bool SUMS>
+__device__ __forceinline__ void replay_ratios(const KArgs& k, const DrawRun& dr, const uint4& r, float wl, float kf,
+                                              float* s_h, float* s_x) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    if (lane < nvar<VC>(k)) {
+        const long long fix = (long long)__ldcg(&k.l.sfix[(size_t)lane * k.l.n + r.x]);
+        float x = 0.0f;
+        s_h[lane] = fix != 0 ? psim_hazard_x(fix, r.z, kf, wl, dr.season, k.p.time_step, &x) : 0.0f;
+        s_x[lane] = x;
+    }
+    __syncwarp();
+}
+
+// A replayed location of up to 64 agents and VM variants at most, in a model
+// whose newly infected are not susceptible (almost all of them): two entries
+// per lane in registers with the draws' bounds, and the location's sums in
+// every lane.  A timestep without an infection is a Philox block per entry
+// and variant and a vote; an infection changes the sums and the bounds where
+// they are, and its agent's fields without anybody waiting for them (going
+// through memory and a fence took 4-5 us an infection).  Expected infections
+// and adjoint terms are added for all timesteps since the bounds last changed.
+template <int VC, bool SUMS, int VM>
+__device__ __forceinline__ void replay_registers(const KArgs& k, const DrawRun& dr, const uint4& r, float wl,
+                                                 const RepConst& rc, double* s_grad, double* term) {
+    constexpr int Q = 2;
+    const uint32_t N = k.a.n, L = k.l.n, V = nvar<VC>(k), lane = threadIdx.x & 31u;
+    const bool sums = SUMS && (k.track_expected || k.adj.on);
+    uint32_t pos[Q], id[Q];
+    float su[Q][VM], h[VM], x[VM];
+    unsigned long long limit[Q][VM];
+    long long fix[VM];
+    uint32_t active = 0, changed = 0;
+#pragma unroll
+    for (int v = 0; v < VM; ++v) {
+        fix[v] = (uint32_t)v < V ? (long long)k.l.sfix[(size_t)v * L + r.x] : 0ll;
+        if ((uint32_t)v < V && k.r.variant_active[r.w * V + v]) active |= 1u << v;
+    }
+#pragma unroll
+    for (int e = 0; e < Q; ++e) {
+        const uint32_t p = lane + 32u * (uint32_t)e;
+        const uint2 s = p < r.z ? k.l.replay_slot[r.y + p] : make_uint2(0u, NONE);
+        pos[e] = s.x;
+        id[e] = s.y;
+#pragma unroll
+        for (int v = 0; v < VM; ++v)
+            su[e][v] = id[e] < N && ((active >> v) & 1u) ? k.l.list_su[v * k.l.list_cap + pos[e]] : 0.0f;
+    }
+    const auto bounds = [&]() {
+#pragma unroll
+        for (int v = 0; v < VM; ++v) {
+            x[v] = h[v] = 0.0f;
+            if (fix[v] != 0) h[v] = psim_hazard_x(fix[v], r.z, rc.kf, wl, dr.season, k.p.time_step, &x[v]);
+#pragma unroll
+            for (int e = 0; e < Q; ++e) {
+                const float p = h[v] * su[e][v];
+                limit[e][v] = p > 0.0f ? u01_limit(p) : 0ull;
+            }
+        }
+    };
+    // the terms of `times` timesteps, of which the last infected the entries of
+    // hit0, hit1 (an agent infected by a variant is not susceptible to the
+    // later ones); one copy of what is rare
+    const auto add = [&](uint32_t times, uint32_t hit0, uint32_t hit1) {
+#pragma unroll 1
+        for (int e = 0; e < Q; ++e) {
+            const uint32_t i = e ? id[1] : id[0], by = e ? hit1 : hit0;
+#pragma unroll
+            for (int v = 0; v < VM; ++v) {
+                const float s = e ? su[1][v] : su[0][v], pf = h[v] * s;
+                const uint32_t n = times - (by && (uint32_t)v >= by ? 1u : 0u);
+                if (!(pf > 0.0f) || !n) continue;
+                if (k.track_expected) *term += (double)n * (pf < 1.0f ? (double)pf : 1.0);
+                if (k.adj.on && pf < 1.0f)
+                    adjoint_terms(k, i, r.x, v, r.w, h[v], k.a.susceptible[(size_t)v * N + i], s, s_grad, x[v], n);
+            }
+        }
+    };
+    bounds();
+    uint32_t since = 0;  // timesteps since the bounds changed
+    for (uint32_t q = 0; q < dr.n; ++q) {
+        uint32_t hit[Q];  // 1 + the variant that infects the entry, in the reference's order
+#pragma unroll
+        for (int e = 0; e < Q; ++e) {
+            hit[e] = 0u;
+#pragma unroll
+            for (int v = VM - 1; v >= 0; --v)
+                if (limit[e][v]) {
+                    const psim_ctr4 o = infect_words(rc.seed, id[e] - rc.off, dr.t + q, v);
+                    if (u01_below(o.v[0], o.v[1], limit[e][v])) hit[e] = v + 1;
+                }
+        }
+        ++since;
+        if (!__any_sync(0xffffffffu, hit[0] | hit[1])) continue;
+        if (sums) add(since, hit[0], hit[1]);
+        since = 0;
+#pragma unroll
+        for (int e = 0; e < Q; ++e) {
+            unsigned who = __ballot_sync(0xffffffffu, hit[e] != 0u);
+            if (!who) continue;
+            long long q0 = 0, q1 = 0;
+            uint32_t var0 = 0;
+            if (hit[e]) {
+                const uint32_t v = hit[e] - 1u, i = id[e];
+                const float inf0 = k.a.infectious[i];
+                const float inf = k.m.state_infectious[k.m.first_infected] * k.m.variant_multiplier[v];
+                if (VM > 1 && inf0 > 0.0f) var0 = k.a.variant[i];
+                q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
+                q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
+                infect_agent<VC, SUMS>(k, i, v, r.x, dr.t + q, inf);
+                for (uint32_t w = 0; w < V; ++w) k.l.list_su[w * k.l.list_cap + pos[e]] = 0.0f;
+#pragma unroll
+                for (int w = 0; w < VM; ++w) su[e][w] = 0.0f;
+            }
+            while (who) {
+                const int src = __ffs(who) - 1;
+                who &= who - 1u;
+                const long long d0 = __shfl_sync(0xffffffffu, q0, src), d1 = __shfl_sync(0xffffffffu, q1, src);
+                const uint32_t v0 = VM > 1 ? __shfl_sync(0xffffffffu, var0, src) : 0u;
+                const uint32_t v1 = VM > 1 ? __shfl_sync(0xffffffffu, hit[e], src) - 1u : 0u;
+#pragma unroll
+                for (int v = 0; v < VM; ++v) {
+                    if (v0 == (uint32_t)v) fix[v] -= d0;
+                    if (v1 == (uint32_t)v) fix[v] += d1;
+                }
+                if (d0 | d1) changed = 1u;
+            }
+        }
+        bounds();
+    }
+    if (sums && since) add(since, 0u, 0u);
+    if (changed) {
+#pragma unroll
+        for (int v = 0; v < VM; ++v)
+            if ((uint32_t)v < V && lane == (uint32_t)v) {
+                k.l.sfix[(size_t)v * L + r.x] = (unsigned long long)fix[v];
+                if (fix[v] != 0) mark_hazardous(k, r.x);
+            }
+    }
+}
+
+// The flagged locations' draws, a warp per location, timestep after timestep:
+// in registers where they fit, else over the entries 32 at a time with the
+// ratios computed again after a timestep that infected somebody (all its
+// draws first: a timestep's ratios come from the sums as it started).
+template <int VC, bool SUMS>
+__device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_replay, DayShared& sh) {
+    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a block's warps take locations far apart in the list: few locations
+    // spread over all SMs
+    for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
+        const uint4 r = k.l.replay_list[f];  // location, first entry, agents, replica
+        if (r.x >= L || r.y > N || r.z > N - r.y) {
+            if (lane == 0) raise_error(k, ERR_AGENT_LIST);
+            continue;
+        }
+        const float wl = k.l.infectiousness[r.x];
+        const RepConst rc = rep_const(k, r.w);
+        double term = 0.0;
+        const bool fits = r.z <= 64u && !k.m.state_susceptible[k.m.first_infected];
+        if (VC != 2 && V == 1 && fits) {
+            replay_registers<VC, SUMS, 1>(k, dr, r, wl, rc, sh.grad, &term);
+        } else if (VC != 1 && V == 2 && fits) {
+            replay_registers<VC, SUMS, 2>(k, dr, r, wl, rc, sh.grad, &term);
+        } else {
+            bool stale = true;  // the ratios: at the start and after an infection
+            for (uint32_t q = 0; q < dr.n; ++q) {
+                if (stale) replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, sh.h[warp], sh.x[warp]);
+                bool infected = false;
+                for (uint32_t p = (uint32_t)lane; p < r.z; p += 32u) {
+                    const uint2 s = k.l.replay_slot[r.y + p];
+                    if (s.y >= N) {
+                        raise_error(k, ERR_AGENT_LIST);
+                        break;
+                    }
+                    infected |= draw_entry<VC, SUMS>(k, s.x, s.y, r.x, r.w, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
+                }
+                stale = __any_sync(0xffffffffu, infected);
+                if (stale) __threadfence();  // the reductions before the sums are read again
+            }
+        }
+        if ((SUMS && k.track_expected)) add_expected_rep(k, true, r.w, term);
+    }
+}
+
+// doMovement of the agents the block queued for s1 (its own segment, whose
+// count the queue left in shared memory: every block starts its decisions at
+// the same barrier, so handing segments out by ticket balanced nothing), then
+// the histogram and sum deltas of the agents that took a new location.
+template <int VC, bool SUMS, int POL>
+__device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t* s_mm, const uint32_t* s_cnt) {
+    const StepClock c = step_clock(k, s1);
+    bool moved = false;
+    {
+        uint32_t n = *s_cnt;
+        if (n > cap) {
+            if (threadIdx.x == 0) raise_error(k, ERR_AGENT_LIST);
+            n = 0;
+        }
+        const uint32_t* seg = k.a.worklist + (size_t)blockIdx.x * cap;
+        // the next trip's inputs are loaded before this trip's decision, its
+        // agent a trip earlier still (22.0 -> 21.1 us a step at 2M agents,
+        // 201 -> 190 at 20M)
+        const uint32_t tid = threadIdx.x, T = blockDim.x;
+        DecisionIn nd;
+        auto inputs = [&](uint32_t i, DecisionIn& d) {
+            if (i >= k.a.n) return;
+            decision_in(k, i, d);
+            d.w = k.a.dinfo[i];
+        };
+        uint32_t ni = tid < n ? seg[tid] : NONE;
+        inputs(ni, nd);
+        uint32_t n2 = tid + T < n ? seg[tid + T] : NONE;
+        for (uint32_t j = tid; j < n; j += T) {
+            const uint32_t i = ni;
+            const DecisionIn d = nd;
+            ni = n2;
+            inputs(ni, nd);
+            n2 = j + 2u * T < n ? seg[j + 2u * T] : NONE;
+            if (i >= k.a.n) {
+                raise_error(k, ERR_AGENT_LIST);
+                continue;
+            }
+            // (queued for its timestamp, unless everybody is at the curfew)
+            const uint32_t s = POL == 2 && c.curfew_now ? k.a.move_at[i] - c.t : 0u;
+            uint32_t w, var = 0;
+            float inf = 0.0f;
+            const uint32_t loc = move_agent<true, POL>(k, i, c, s, s_mm, d, &w);
+            if (w != d.w) k.a.dinfo[i] = w;
+            if (w & DW_INFECTIOUS) {
+                inf = k.a.infectious[i];
+                var = VC == 1 ? 0u : k.a.variant[i];
+            }
+            moved |= count_agent_delta(k, true, d.loc, loc, inf, var, inf, var);
+        }
+    }
+    publish_moved(k, moved, c.t);
+}
+
+// One segment of the day (see the section comment), starting at timestep
+// `step`; *next receives the timestep the next one starts at (step_end after
+// the last).  False when a grid barrier expired (the kernel then ends).  cap =
+// the work-list segment size of a block.
+template <int VC, bool SUMS, int POL>
+__device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint32_t step_end, uint32_t phases,
+                                            uint32_t cap, DayShared& sh, uint32_t* next) {
+    const uint32_t tl = PROF_T + PROF_TW * step;  // the segment's timeline slots (profiled graph)
+    prof_enter(k, tl);
+    const uint32_t t = k.clock->t0 + step;
+    const uint32_t moved = k.l.build[0], force = k.l.build[1], q_step = k.l.build[3];
+    DrawRun dr;
+    dr.t = t;
+    dr.epoch = k.l.build[6] + 1u;  // (0 is the stamp of a location never flagged)
+    dr.season = k.clock->season;
+    // the segment's end: the first later timestep that somebody decides at
+    // (everyone at the curfew)
+    uint32_t e = step + 1;
+    bool decides = false;
+    while (e < k.spd) {
+        uint32_t w = k.a.move_mask[e >> 5] >> (e & 31u);
+        if (POL == 2 && k.p.enable_curfew && k.p.curfew_begin >= e && k.p.curfew_begin >> 5 == e >> 5)
+            w |= 1u << (k.p.curfew_begin - e);
+        if (w) {
+            e += (uint32_t)(__ffs(w) - 1);
+            decides = e < k.spd;
+            break;
+        }
+        e = (e & ~31u) + 32u;
+    }
+    if (!decides) e = k.spd;
+    // (a caller's shorter range ends the draws, not the decisions after them)
+    dr.n = min(e, step_end) - step;
+    decides = decides && e <= step_end && (phases & PH_DECIDE);
+    *next = min(e, step_end);
+    const bool list = (phases & PH_REBUILD) && csr_decide_from(k, t, moved, force);
+    // the location quarantine writes of the decisions for t
+    const bool merge = POL > 0 && (phases & PH_REBUILD) && k.p.quarantine_policy > 1 && q_step == t;
+    if (merge) merge_quarantine(k);
+    const size_t seg = (size_t)blockIdx.x * cap;
+    if (list || decides) {
+        phase_lists<VC, SUMS, POL>(k, list, decides, e, cap, sh);
+        if (decides) mask_clear_shared(sh.mm);
+        if (k.prof) {
+            if (list) count_listed<VC, SUMS>(k, sh);
+            if (threadIdx.x == 0) {
+                if (list && blockIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
+                if (decides && sh.cnt) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)sh.cnt);
+                if (decides && blockIdx.x == 0) atomicAdd(&k.prof[PROF_QUEUE_STEPS], 1ull);
+            }
+        }
+        prof_mark(k, tl + (list ? 1 : 2));
+    }
+    const bool draws = (phases & PH_DRAW) != 0;
+    if (draws) {
+        uint32_t entries = 0, hazard = 0;
+        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, &entries, &hazard);
+        if (k.prof) {
+            __syncwarp();
+            entries = __reduce_add_sync(0xffffffffu, entries);
+            hazard = __reduce_add_sync(0xffffffffu, hazard);
+            if ((threadIdx.x & 31) == 0 && (entries | hazard)) {
+                atomicAdd(&k.prof[PROF_DRAW_ENTRIES], (unsigned long long)entries);
+                atomicAdd(&k.prof[PROF_DRAW_HAZARD], (unsigned long long)hazard);
+            }
+        }
+    }
+    prof_mark(k, tl + 3);
+    // every draw before any replay, every draw and merge before any decision
+    if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
+    if (draws) {
+        const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
+        const bool expected = (SUMS && k.track_expected) || (SUMS && k.adj.on);
+        if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
+        if (n_replay || expected) {
+            grad_begin(k, sh.grad);
+            if (n_replay) {
+                phase_gather(k, dr, seg, sh.listed);
+                if (!grid_barrier(k, sh)) return false;
+                phase_replay<VC, SUMS>(k, dr, n_replay, sh);
+            }
+            if (expected) phase_expected<VC, SUMS>(k, dr, seg, sh.listed, sh.grad);
+            grad_end(k, sh.grad);
+            if (decides || n_replay) {
+                // every replay before any decision and before the list is emptied
+                if (!grid_barrier(k, sh)) return false;
+                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
+            }
+        }
+    }
+    prof_mark(k, tl + 4);
+    if (decides) {
+        phase_decide<VC, SUMS, POL>(k, e, cap, sh.mm, &sh.cnt);
+        mask_flush(k, sh.mm);
+    }
+    prof_mark(k, tl + 5);
+    return true;
+}
+
+// The day kernel: timesteps step0 .. step_end - 1.
+template <int VC, bool SUMS, int POL>
+__global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0, uint32_t step_end, uint32_t phases,
+                                                        uint32_t cap) {
+    __shared__ DayShared sh;
+    if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
+    if (threadIdx.x == 0) {
+        sh.target = gridDim.x;
+        sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
+        sh.cnt = 0u;
+    }
+    __syncthreads();
+    uint32_t step = step0;
+    for (;;) {
+        uint32_t next = step_end;
+        if (!day_segment<VC, SUMS, POL>(k, step, step_end, phases, cap, sh, &next)) return;
+        if (next >= step_end) return;
+        step = next;
+        if (!grid_barrier(k, sh)) return;
+    }
+}
+
+}  // namespace psim

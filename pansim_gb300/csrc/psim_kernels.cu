@@ -21,780 +21,15 @@
 // expression rounds exactly like the host oracle compiled with -ffp-contract=off.
 #include <algorithm>
 
-#include "psim_device.cuh"
+#include "psim_agent.cuh"
 
 namespace psim {
-
-// An error flag: in device memory for the kernels, and the host's word, which
-// the host looks at after it has waited for the stream (no copy per call).
-__device__ __forceinline__ void raise_error(const KArgs& k, uint32_t bits) {
-    atomicOr(k.err, bits);
-    *(volatile uint32_t*)k.err_host = 1u;
-}
-__device__ __forceinline__ uint32_t wb_of(const KArgs& k, uint32_t i) {
-    return k.m.state_wb[(uint8_t)k.a.state[i]];
-}
-__device__ __forceinline__ bool infected_of(const KArgs& k, uint32_t i) {
-    return k.m.state_infected[(uint8_t)k.a.state[i]] != 0;
-}
-__device__ __forceinline__ uint8_t loc_open(const KArgs& k, uint32_t l) { return l < k.l.n ? k.l.open[l] : 0; }
-__device__ __forceinline__ uint32_t loc_closed_until(const KArgs& k, uint32_t l) {
-    return l < k.l.n ? k.l.closed_until[l] : 0u;
-}
-__device__ __forceinline__ uint32_t loc_qu(const KArgs& k, uint32_t l) { return l < k.l.n ? k.l.quarantine_until[l] : 0u; }
-__device__ __forceinline__ uint32_t loc_type(const KArgs& k, uint32_t l) { return l < k.l.n ? k.l.type[l] : NONE; }
-
-// Entry j of the per-agent location lists: x = location, y = its type.
-__device__ __forceinline__ uint2 poss_entry(const KArgs& k, uint32_t j) {
-    if (k.a.poss4) {
-        const uint32_t v = k.a.poss4[j];
-        return make_uint2(v & 0x3FFFFFFu, v >> 26);
-    }
-    return k.a.poss[j];
-}
-
-// RealMovementOps::findActualLocationForType, movementPolicies.h:69-122.
-// f0, f1, f2: the types resolved by first match (home, school, work except in
-// the plan helpers, movementPolicies.h:1073-1080, :1144, :1209-1214).
-// [b, e): the agent's entries in the per-agent location list.
-__device__ uint32_t find_location_range(const KArgs& k, uint32_t b, uint32_t e, uint32_t lt, int retry,
-                                        psim_stream* rng, uint32_t f0, uint32_t f1, uint32_t f2) {
-    if (lt == f0 || lt == f1 || lt == f2) {
-        for (uint32_t j = b; j < e; ++j) {
-            const uint2 en = poss_entry(k, j);
-            if (lt == en.y) return en.x;
-        }
-        return NONE;
-    }
-    uint32_t counter = 0, pos = 0, first = NONE;
-    for (uint32_t j = b; j < e; ++j) {
-        const uint2 en = poss_entry(k, j);
-        if (lt == en.y) {
-            if (counter == 0) {
-                pos = j;
-                first = en.x;
-            }
-            counter++;
-        }
-    }
-    if (counter == 1) return first;
-    if (counter > 1) {
-        uint32_t counter2 = counter, rand_idx = counter2;
-        // the reference loops until the pick is open or its one retry is
-        // spent: a second pass always ends (retry is 0 by then)
-        for (int pass = 0; pass < 2; ++pass) {
-            while (rand_idx == counter2) rand_idx = psim_below(rng, counter);
-            counter2 = 0;
-            for (uint32_t j = pos; j < e; ++j) {
-                const uint2 en = poss_entry(k, j);
-                if (lt == en.y) {
-                    if (counter2 == rand_idx) {
-                        if (retry && loc_open(k, en.x) == 0) {
-                            retry = 0;
-                            break;
-                        }
-                        return en.x;
-                    }
-                    counter2++;
-                }
-            }
-        }
-    }
-    return NONE;
-}
-
-// The same for agent i by its list's layout; lb: the list's first entry.
-__device__ __forceinline__ uint32_t find_location_at(const KArgs& k, uint32_t i, uint32_t layout, uint32_t lb,
-                                                     uint32_t lt, int retry, psim_stream* rng, uint32_t f0,
-                                                     uint32_t f1, uint32_t f2) {
-    if (layout == 0) return find_location_range(k, lb, k.a.loc_offset[i + 1], lt, retry, rng, f0, f1, f2);
-    if (lt >= LAYOUT_TYPES) return NONE;
-    const uint32_t e = k.m.layout[layout * LAYOUT_TYPES + lt];
-    const uint32_t count = e >> 8, first = lb + (e & 0xFFu);
-    if (count == 0) return NONE;
-    uint32_t pick = 0;
-    const bool any = count > 1 && lt != f0 && lt != f1 && lt != f2;
-    if (any) pick = psim_below(rng, count);
-    uint32_t loc = k.a.poss4[first + pick] & 0x3FFFFFFu;
-    if (any && retry && loc_open(k, loc) == 0) {
-        // its one retry: another pick, open or not
-        const uint32_t before = pick;
-        while (pick == before) pick = psim_below(rng, count);
-        loc = k.a.poss4[first + pick] & 0x3FFFFFFu;
-    }
-    return loc;
-}
-
-__device__ __forceinline__ uint32_t find_location3(const KArgs& k, uint32_t i, uint32_t lt, int retry, psim_stream* rng,
-                                                   uint32_t f0, uint32_t f1, uint32_t f2) {
-    return find_location_at(k, i, k.a.layout[i], k.a.loc_offset[i], lt, retry, rng, f0, f1, f2);
-}
-
-__device__ __forceinline__ uint32_t find_location(const KArgs& k, uint32_t i, uint32_t lt, int retry, psim_stream* rng) {
-    return find_location3(k, i, lt, retry, rng, k.p.home_type, k.p.school_type, k.p.work_type);
-}
-
-// A location quarantine written by a decision at step t: merged into
-// quarantine_until by the scan of step t (build[3] = the step whose decisions
-// wrote; every writer of a step stores the same value).
-__device__ __forceinline__ void qu_write(const KArgs& k, uint32_t loc, uint32_t until, uint32_t t) {
-    if (loc < k.l.n) {
-        atomicMax(&k.l.qu_pending[loc], until);
-        k.l.build[3] = t;
-        k.l.build[4] = 1u;
-    }
-}
-
-// RealMovementOps::quarantineAgent, movementPolicies.h:176-245
-// Returns whether the agent was quarantined (its flag set).  The stream is a
-// copy: a decision that quarantines draws nothing after it.
-__device__ __forceinline__ bool quarantine_agent(const KArgs& k, uint32_t i, uint32_t t, uint32_t until,
-                                              psim_stream rng_copy) {
-    psim_stream* rng = &rng_copy;
-    const psim_params& p = k.p;
-    if (p.quarantine_policy == 0) return false;
-    if (k.a.st_diagnosed_ts[i] > 0 && !infected_of(k, i) && !p.quarantine_immune) return false;
-    if (!k.a.diagnosed[i] && k.a.st_immunization_ts[i] > 0 && !p.quarantine_immune) return false;
-    k.a.quarantined[i] = 1;
-    k.a.st_quarantined_ts[i] = t;
-    uint32_t prev_until = k.a.st_quarantined_until[i];
-    k.a.st_quarantined_until[i] = until;
-    k.a.st_days_in_quarantine[i] += (until - t) / (24u * 60u / p.time_step);
-    if (k.a.diagnosed[i]) {
-        uint32_t my_home = find_location(k, i, p.home_type, 0, rng);
-        if (p.quarantine_policy > 1) qu_write(k, my_home, until, t);
-        if (p.quarantine_policy > 2 && prev_until < t) {
-            uint32_t classroom = find_location(k, i, p.classroom_type, 0, rng);
-            uint32_t work = find_location(k, i, p.work_type, 0, rng);
-            uint32_t to_close[2] = {classroom, work};
-            for (int c = 0; c < 2; ++c) {
-                uint32_t loc = to_close[c];
-                if (loc != NONE && (loc_type(k, loc) == p.work_type || loc_type(k, loc) == p.classroom_type) &&
-                    loc_qu(k, loc) < t && loc_open(k, loc) && loc_closed_until(k, loc) < t)
-                    qu_write(k, loc, until, t);
-            }
-        }
-    }
-    return true;
-}
-
-// returns the decision word's flags of what it set
-__device__ __forceinline__ uint32_t diagnose_and_quarantine(const KArgs& k, uint32_t i, uint32_t t, uint32_t sum,
-                                                         psim_stream rng) {
-    const uint32_t dt = k.p.time_step;
-    k.a.diagnosed[i] = 1;
-    const uint32_t ts = sum == 24u * 60u / dt ? t + 1u : t;
-    k.a.st_diagnosed_ts[i] = ts;
-    return DW_DIAGNOSED | (ts > 0 ? DW_DIAG_TS : 0u) |
-           (quarantine_agent(k, i, t, t + k.p.quarantine_length * 24u * 60u / dt, rng) ? DW_QUARANTINED : 0u);
-}
-
-// S: the agent's countdown (stepsUntilMove) as the decision just set it;
-// cur: the agent's location as the decision left it
-__device__ __forceinline__ void stayed_home_check(const KArgs& k, uint32_t i, uint32_t agent_home, uint32_t cur,
-                                                  uint32_t S) {
-    if (agent_home != NONE && cur != agent_home && S > k.hour_steps) k.a.stayed_home[i] = 0;
-}
-
-// The agent's decision word (DW_*) from its fields; t = the first timestep it
-// is used at.
-__device__ __forceinline__ uint32_t decision_word(const KArgs& k, uint32_t i, uint32_t t) {
-    const uint32_t type = k.a.type[i], st = (uint8_t)k.a.state[i], age = k.a.age[i];
-    const bool quar = k.a.quarantined[i] != 0, diag = k.a.diagnosed[i] != 0, no_work = k.a.no_work[i] != 0;
-    const bool hosp = k.a.st_hospitalized_until[i] > t, diag_ts = k.a.st_diagnosed_ts[i] > 0;
-    const bool inf = k.a.infectious[i] != 0.0f;
-    return type | (uint32_t)k.m.state_wb[st] << DW_WB_SHIFT | (quar ? DW_QUARANTINED : 0u) | (hosp ? DW_HOSPITAL : 0u) |
-           (diag ? DW_DIAGNOSED : 0u) | (diag_ts ? DW_DIAG_TS : 0u) | (inf ? DW_INFECTIOUS : 0u) |
-           (no_work ? DW_NO_WORK : 0u) | (age >= k.p.school_age_restriction ? DW_TOO_OLD : 0u) |
-           (uint32_t)k.a.layout[i] << DW_LAYOUT_SHIFT;
-}
-
-// What a decision reads of its agent, loaded together before it starts: the
-// decision word, the current location, the agent's first entry in the
-// per-agent location lists, the replica.
-struct DecisionIn {
-    uint32_t w, loc, lb, rep;
-};
-__device__ __forceinline__ void decision_in(const KArgs& k, uint32_t i, DecisionIn& d) {
-    d.loc = k.a.location[i];
-    d.lb = k.a.loc_offset[i];
-    d.rep = k.r.n == 1 ? 0u : k.a.rep[i];
-}
-
-// A location's flag word (LF_*): the running day's, or from the location's
-// fields (the per-phase entry points).  A location out of range is closed and
-// of no type, as its fields read one by one would be.
-template <bool DAY>
-__device__ __forceinline__ uint32_t loc_flags(const KArgs& k, uint32_t loc, uint32_t t) {
-    if (loc >= k.l.n) return LF_TYPE;
-    if (DAY) return k.l.lflags[loc];
-    return k.l.type[loc] | (k.l.open[loc] ? LF_OPEN : 0u) | (k.l.closed_until[loc] > t ? LF_CLOSED : 0u) |
-           (k.l.quarantine_until[loc] > t ? LF_QUARANTINE : 0u);
-}
-// closed by its open flag or its closing time
-__device__ __forceinline__ bool closed_at(const KArgs& k, uint32_t loc, uint32_t f, uint32_t t) {
-    return !(f & LF_OPEN) || ((f & LF_CLOSED) && k.l.closed_until[loc] > t);
-}
-__device__ __forceinline__ bool quarantine_type(const KArgs& k, uint32_t ty) {
-    return ty == k.p.home_type || ty == k.p.school_type || ty == k.p.classroom_type || ty == k.p.work_type;
-}
-
-// The full per-agent decision of doMovement once the countdown reached zero
-// (movementPolicies.h:333-1040).  The curfew and countdown prologue is in
-// move_agent.  S receives the agent's new countdown (stepsUntilMove after
-// the step); the caller turns it into the absolute timestamp of the next
-// decision, cur the agent's location after it (d.loc before).  Returns the
-// agent's decision word after it.
-//
-// The decisions are bound by the chain of dependent loads (word, location
-// list, window, chosen location's flags) and by instructions, not by bytes:
-// the countdowns of every event at every step come from a table computed on
-// the host (no divisions here), a location's flags are one word, the home is
-// looked up once, and an entry of a location list is found by the list's
-// layout.  22 us of decisions a step at 2M agents, against 25 without
-// those; the rare quarantine out of line (its arguments through memory) took
-// 26, and the location list in registers 23.6.
-template <bool DAY>
-__device__ __forceinline__ uint32_t move_decide(const KArgs& k, uint32_t i, uint32_t t, uint32_t step, uint32_t day,
-                                                uint32_t sum, psim_stream* rng, uint32_t& S, const DecisionIn& d,
-                                                uint32_t& cur) {
-    const psim_params& p = k.p;
-    const bool qrule = p.quarantine_policy > 1;
-    const uint32_t f_now = qrule ? loc_flags<DAY>(k, d.loc, t) : 0u;
-    // the quarantine end of a location whose quarantine sends home, else 0
-    auto quarantine_end = [&](uint32_t loc, uint32_t f) {
-        return (f & LF_QUARANTINE) && quarantine_type(k, f & LF_TYPE) ? k.l.quarantine_until[loc] : 0u;
-    };
-    auto fl = [&](uint32_t lt, int retry) {
-        return find_location_at(k, i, d.w >> DW_LAYOUT_SHIFT, d.lb, lt, retry, rng, p.home_type, p.school_type,
-                                p.work_type);
-    };
-    uint32_t w = d.w;
-    if ((w & DW_QUARANTINED) && k.a.st_quarantined_until[i] <= t) {
-        w &= ~DW_QUARANTINED;
-        k.a.quarantined[i] = 0;
-    }
-    // quarantine_agent and the word's flag
-    auto quarantine = [&](uint32_t until) {
-        if (quarantine_agent(k, i, t, until, *rng)) w |= DW_QUARANTINED;
-    };
-
-    cur = d.loc;
-    const uint32_t wb = (w >> DW_WB_SHIFT) & 7u;
-    if (wb == WB_D) {
-        S = NONE;
-        cur = k.r.cemetery[d.rep];
-        k.a.location[i] = cur;
-        return w;
-    }
-    // the first match, no draw (find_location_range): the same at every use
-    const uint32_t agent_home = fl(p.home_type, 0);
-
-    // in hospital: for another disease, or severe
-    uint32_t h_until = 0;
-    if ((w & DW_HOSPITAL) && wb != WB_S) {
-        h_until = k.a.st_hospitalized_until[i];
-        if (k.a.st_hospitalized_ts[i] > t || h_until <= t) h_until = 0;
-    }
-    if (wb == WB_S || h_until) {
-        S = h_until ? min(h_until - t - 1u, sum) : sum;
-        cur = fl(p.hospital_type, 0);
-        k.a.location[i] = cur;
-        if ((w & (DW_DIAGNOSED | DW_INFECTIOUS)) == DW_INFECTIOUS) w |= diagnose_and_quarantine(k, i, t, sum, *rng);
-        return w;
-    }
-    // sent home: by the quarantine of the current location, by the agent's own
-    const uint32_t qu_now = quarantine_end(d.loc, f_now);
-    if (t < qu_now) {
-        if (!(w & DW_QUARANTINED)) quarantine(qu_now);
-        if (w & DW_QUARANTINED) {
-            S = min(qu_now - t - 1u, sum);
-            if (agent_home != cur) k.a.location[i] = agent_home;
-            cur = agent_home;
-            return w;
-        }
-    }
-    if (p.quarantine_policy > 0 && (w & (DW_DIAGNOSED | DW_DIAG_TS | DW_QUARANTINED))) {
-        const uint32_t ql = p.quarantine_length * 24u * 60u / p.time_step;
-        if ((w & (DW_DIAGNOSED | DW_QUARANTINED)) || t - k.a.st_diagnosed_ts[i] < ql) {
-            if (!(w & DW_QUARANTINED)) quarantine(t + ql);
-            if (w & DW_QUARANTINED) {
-                cur = agent_home;
-                k.a.location[i] = cur;
-                S = sum;
-                return w;
-            }
-        }
-    }
-
-    // schedule window (AgentTypeList::getOffsetIndex, agentType.cpp:13-15;
-    // the window of the slot at this step, movementPolicies.h:585-603, from
-    // the table the host computed)
-    const uint32_t agent_type = w & DW_TYPE;
-    const uint4* wp = reinterpret_cast<const uint4*>(k.m.window + ((size_t)(7u * wb + day + agent_type * 28u) * k.spd + step));
-    const uint4 win = wp[0];
-    const uint4 first = wp[1];  // DecChoice
-    uint32_t new_type = NONE;
-    // the chosen location and its flag word
-    uint32_t spec_loc = NONE, spec_f = 0u;
-    if (win.x) {  // Case 2 and 4: an event is active
-        uint32_t num_pot = win.x, picked = 0;
-        uint32_t s_steps = first.y, s_draw = first.z;
-        new_type = first.x;
-        if (num_pot != 1) {
-            // U > chance of the first event, in integers: U = K 2^-53 and
-            // chance 2^53 (exact in float), so K > floor(chance 2^53); the
-            // few that go on compare in double as the reference does
-            const uint64_t K = psim_u53(rng);
-            const float c0 = __uint_as_float(first.w);
-            if (c0 < 0.0f || (c0 < 1.0f && K > __float2ull_rd(c0 * 9007199254740992.0f))) {
-                const double rnd = (double)K * (1.0 / 9007199254740992.0);
-                double thr = c0;
-                uint32_t idx = 0;
-                while (rnd > thr && idx < num_pot) {
-                    idx++;
-                    thr += k.m.ev_chance[win.y + idx];
-                }
-                if (idx == num_pot) idx--;
-                picked = idx;
-                const uint4 c = reinterpret_cast<const uint4*>(k.m.choice)[win.z + idx];
-                new_type = c.x;
-                s_steps = c.y;
-                s_draw = c.z;
-            }
-        }
-        if ((w & DW_NO_WORK) && new_type == p.work_type) {
-            new_type = p.home_type;
-            num_pot = 1;
-            if (!(w & DW_QUARANTINED)) k.a.st_days_in_quarantine[i]++;
-        }
-        uint32_t new_loc = new_type == p.home_type ? agent_home : fl(new_type, num_pot == 1);
-        const bool too_old = (w & DW_TOO_OLD) && (new_type == p.school_type || new_type == p.classroom_type);
-        const bool barred = p.lockdown_nonvacc && k.a.st_immunization_ts[i] == 0;
-        spec_loc = new_loc;
-        spec_f = loc_flags<DAY>(k, new_loc, t);
-        if (too_old || barred || (new_type != p.work_type && closed_at(k, new_loc, spec_f, t))) {
-            if (num_pot > 1) {
-                double rnd = psim_u01(rng) * 1.0;
-                double pc = k.m.ev_chance[win.y + picked];
-                double thr = (picked == 0) ? 0.0 : k.m.ev_chance[win.y] / (1.0 - pc);
-                uint32_t idx = 0;
-                while (rnd > thr && idx < num_pot) {
-                    idx++;
-                    thr += (picked == idx) ? 0.0 : k.m.ev_chance[win.y + idx] / (1.0 - pc);
-                }
-                if (idx == num_pot) idx--;
-                const uint4 c = reinterpret_cast<const uint4*>(k.m.choice)[win.z + idx];
-                new_type = c.x;
-                s_steps = c.y;
-                s_draw = c.z;
-                new_loc = new_type == p.home_type ? agent_home : fl(new_type, 0);
-                if (too_old || barred ||
-                    (new_type != p.work_type && closed_at(k, new_loc, loc_flags<DAY>(k, new_loc, t), t)))
-                    new_loc = agent_home;
-            } else {
-                new_loc = agent_home;
-            }
-        } else if (new_type == p.school_type) {
-            uint32_t my_class = fl(p.classroom_type, 0);
-            if (my_class != NONE && loc_closed_until(k, my_class) > t) new_loc = agent_home;
-        }
-        cur = new_loc;
-        S = s_steps + psim_below(rng, s_draw);
-        if (agent_type + 1 == 7 && p.enable_curfew && (p.curfew_begin <= step || p.curfew_end > step)) {
-            bool work_closed = new_type == p.work_type && (loc_open(k, new_loc) == 0 || loc_closed_until(k, new_loc) > t);
-            if (work_closed || (new_type != p.work_type && new_type != p.home_type)) cur = agent_home;
-        }
-    } else if (win.w) {  // Case 3: the next event lies ahead
-        S = first.y + psim_below(rng, first.z);
-        if (S >= k.hour_steps) {
-            new_type = p.home_type;
-            cur = agent_home;
-        } else if (S >= k.half_hour_steps) {
-            new_type = p.public_type;
-            cur = new_type == p.home_type ? agent_home : fl(new_type, 0);
-        }
-    } else {  // Case 1: no event for the rest of the day
-        new_type = p.home_type;
-        cur = agent_home;
-        S = sum;
-    }
-    k.a.location[i] = cur;
-    if (qrule) {
-        const uint32_t f = cur == spec_loc ? spec_f : cur == d.loc ? f_now : loc_flags<DAY>(k, cur, t);
-        const uint32_t qu = quarantine_end(cur, f);
-        if (t < qu) {
-            if (!(w & DW_QUARANTINED)) quarantine(qu);
-            if (w & DW_QUARANTINED) {
-                S = min(qu - t - 1u, sum);
-                if (agent_home != cur) k.a.location[i] = agent_home;
-                cur = agent_home;
-                return w;
-            }
-        }
-    }
-    if ((w & (DW_DIAGNOSED | DW_INFECTIOUS)) == DW_INFECTIOUS &&
-        (new_type == p.hospital_type || (new_type == p.doctor_type && psim_u01(rng) * 1.0 < 0.7)))
-        w |= diagnose_and_quarantine(k, i, t, sum, *rng);
-    stayed_home_check(k, i, agent_home, cur, S);
-    S = S - 1u;
-    return w;
-}
-
-// curfew prologue of doMovement (movementPolicies.h:267-326); returns true if
-// the agent's step is finished (S, the countdown, then holds `sum`).
-__device__ bool curfew_prologue(const KArgs& k, uint32_t i, uint32_t t, uint32_t sum, psim_stream* rng, uint32_t& S) {
-    const psim_params& p = k.p;
-    uint32_t wb = wb_of(k, i);
-    bool dead_or_hosp = (wb == WB_D || wb == WB_S);
-    bool hosp_noncovid = (k.a.st_hospitalized_ts[i] <= t && k.a.st_hospitalized_until[i] > t);
-    if (dead_or_hosp || hosp_noncovid) return false;
-    if (k.a.type[i] + 1u == 7u) {
-        uint32_t workplace = find_location(k, i, p.work_type, 0, rng);
-        if (k.a.location[i] != workplace || workplace == NONE || loc_open(k, workplace) == 0) {
-            k.a.location[i] = find_location(k, i, p.home_type, 0, rng);
-            if (workplace == NONE || loc_open(k, workplace) == 0) {
-                S = sum;
-                return true;
-            }
-        }
-        return false;
-    }
-    S = sum;
-    k.a.location[i] = find_location(k, i, p.home_type, 0, rng);
-    return true;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
-// ---------------------------------------------------------------------------
-// Per-agent pieces of a step.
-
-struct StepClock {
-    uint32_t t, step, day, sum;
-    bool curfew_now;
-};
-
-__device__ __forceinline__ StepClock step_clock(const KArgs& k, uint32_t step) {
-    StepClock c;
-    c.t = k.clock->t0 + step;
-    c.step = step;
-    c.day = k.clock->day_of_week;
-    c.sum = k.spd - step;  // the steps left of the day
-    c.curfew_now = k.p.enable_curfew && k.p.curfew_begin == step;
-    return c;
-}
-
-// The countdown of the reference (stepsUntilMove: decremented every step,
-// a decision when it reaches zero) is kept as the absolute timestamp of the
-// agent's next decision, move_at = t + 1 + stepsUntilMove after step t (u32
-// arithmetic: the dead agents' NONE countdown wraps like the reference's).
-// Before step t the countdown is move_at - t; only a decision or the curfew
-// prologue writes move_at, so the steps in between touch nothing.  The
-// library converts to and from countdowns at upload and download (time base
-// t_next, psim_api.cu).
-//
-// Steps of the running day at which some agent decides: one bit per step in
-// move_mask, set by whoever writes such a move_at (through a block-shared
-// copy, one global atomic per word and block).  The day graph's kernels read
-// it to skip the steps nobody decides at.
-__device__ __forceinline__ void mask_clear_shared(uint32_t* s_mm) {
-    for (uint32_t w = threadIdx.x; w < MOVE_MASK_WORDS; w += blockDim.x) s_mm[w] = 0u;
-    __syncthreads();
-}
-__device__ __forceinline__ void mask_note(const KArgs& k, uint32_t* s_mm, uint32_t m) {
-    const uint32_t s = m - k.clock->t0;
-    if (s < k.spd) {
-        // most deciders of a step land on a few steps: read before the
-        // atomic, whose lanes on one word would queue
-        const uint32_t bit = 1u << (s & 31u);
-        if (!(s_mm[s >> 5] & bit)) atomicOr(&s_mm[s >> 5], bit);
-    }
-}
-__device__ __forceinline__ void mask_flush(const KArgs& k, uint32_t* s_mm) {
-    __syncthreads();
-    for (uint32_t w = threadIdx.x; w < MOVE_MASK_WORDS; w += blockDim.x)
-        if (s_mm[w]) atomicOr(&k.a.move_mask[w], s_mm[w]);
-}
-
-// doMovement for agent i at step c.t; s = its countdown before the step
-// (move_at - c.t).  Writes move_at when the agent decides or the curfew
-// prologue resets its countdown.  d: the decision's inputs.  Returns the
-// agent's location after the step; w receives its decision word after it.
-template <bool DAY>
-__device__ __forceinline__ uint32_t move_agent(const KArgs& k, uint32_t i, const StepClock& c, uint32_t s,
-                                               uint32_t* s_mm, DecisionIn d, uint32_t* w) {
-    psim_stream rng;
-    psim_stream_init(&rng, k.r.seed[d.rep], i - k.r.agent_off[d.rep], c.t, PSIM_PHASE_MOVE);
-    bool done = false;
-    uint32_t S = s;
-    if (c.curfew_now) {
-        done = curfew_prologue(k, i, c.t, c.sum, &rng, S);
-        d.loc = k.a.location[i];  // the prologue may have sent the agent home
-    }
-    uint32_t cur = d.loc;
-    *w = d.w;
-    if (!done) {
-        if (S > 0)
-            S = S - 1u;
-        else
-            *w = move_decide<DAY>(k, i, c.t, c.step, c.day, c.sum, &rng, S, d, cur);
-    }
-    const uint32_t m = c.t + 1u + S;
-    k.a.move_at[i] = m;
-    mask_note(k, s_mm, m);
-    return cur;
-}
-
-// Scan tiles: 256 threads x ITEMS locations (ITEMS = 2, 4 or 8, a tuning
-// choice); the masks hold one 32-bit word per warp and item.
-constexpr int SCAN_THREADS = 256;
-
-// A location that receives an infectious term sets its hazard-mask bit at
-// once, so the mask is always a superset of the locations with a nonzero sum
-// (the day kernel's rebuild lists from it and clears the bits of zero sums;
-// the per-phase scans recompute the bits of their dirty locations).
-__device__ __forceinline__ void mark_hazardous(const KArgs& k, uint32_t loc) {
-    atomicOr(&k.l.hmask[loc >> 5], 1u << (loc & 31u));
-}
-
-// The full pass of a day's first step (k_movement, after a reset of the
-// sums): an agent whose location changed from loc0 to loc moves one count
-// (two fire-and-forget reductions), and every infectious agent adds its term
-// at its (new) location.  Returns whether the agent took a new location (its
-// kernel then publishes the timestamp of the new locations, publish_moved).
-__device__ __forceinline__ bool count_agent(const KArgs& k, bool act, uint32_t loc0, uint32_t loc, float inf,
-                                            uint32_t variant) {
-    const uint32_t L = k.l.n;
-    if (act && loc >= L) {
-        raise_error(k, ERR_LOCATION);
-        loc = NONE;
-    }
-    const bool mv = act && loc != loc0;
-    if (mv) {
-        if (loc0 < L) atomicSub(&k.l.counts[loc0], 1u);
-        if (loc != NONE) atomicAdd(&k.l.counts[loc], 1u);
-    }
-    if (act && loc != NONE && inf > 0.0f) {
-        const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
-        atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
-        mark_hazardous(k, loc);
-    }
-    return mv;
-}
-
-// Within a day the per-location sums persist: an agent changes them only
-// when it moves or its infectiousness changes (a draw that infects).  The
-// first step of a day (k_movement after a reset of the sums) adds every
-// agent's term afresh.
-// The agent went from (loc0, inf0, var0) to (loc, inf, var) in a day
-// kernel's decision: its count moves, its fixed-point term leaves (loc0,
-// var0) and joins (loc, var).  The day kernel computes every ratio from the
-// sums, so it keeps no dirty marks (the day graph marks every location dirty
-// at its start: a scan after it recomputes every ratio).  Returns whether the
-// agent took a new location.
-__device__ __forceinline__ bool count_agent_delta(const KArgs& k, bool act, uint32_t loc0, uint32_t loc, float inf0,
-                                                  uint32_t var0, float inf, uint32_t var) {
-    const uint32_t L = k.l.n;
-    if (act && loc >= L) {
-        raise_error(k, ERR_LOCATION);
-        loc = NONE;
-    }
-    const bool mv = act && loc != loc0;
-    if (mv) {
-        if (loc0 < L) atomicSub(&k.l.counts[loc0], 1u);
-        if (loc != NONE) atomicAdd(&k.l.counts[loc], 1u);
-    }
-    if (act) {
-        const long long q0 = (loc0 < L && inf0 > 0.0f) ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
-        const long long q1 = (loc != NONE && inf > 0.0f) ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
-        if (mv || q0 != q1 || var0 != var) {
-            if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
-            if (q1) {
-                atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
-                mark_hazardous(k, loc);
-            }
-        }
-    }
-    return mv;
-}
-
-// The full histogram of the current positions (after a reset of counts and sums).
-__device__ __forceinline__ void count_full(const KArgs& k, bool act, uint32_t loc, float inf, uint32_t variant) {
-    const uint32_t L = k.l.n;
-    if (!act) return;
-    if (loc >= L) {
-        raise_error(k, ERR_LOCATION);
-        return;
-    }
-    atomicAdd(&k.l.counts[loc], 1u);
-    if (inf > 0.0f) {
-        const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
-        atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
-        mark_hazardous(k, loc);
-    }
-}
-
-// CSR slot of an agent: a warp-aggregated returning atomic on the location's
-// cursor, which the scan set to the location's first slot.  Warp-collective.
-__device__ __forceinline__ uint32_t take_slot(const KArgs& k, bool ok, uint32_t loc) {
-    if (!k.tune.agg_slot) return ok ? atomicAdd(&k.l.cursor[loc], 1u) : NONE;
-    const unsigned valid = __ballot_sync(0xffffffffu, ok);
-    uint32_t pos = NONE;
-    if (ok) {
-        const unsigned peers = __match_any_sync(valid, loc);
-        const int leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(&k.l.cursor[loc], (uint32_t)__popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        pos = base + (uint32_t)__popc(peers & lanemask_lt());
-    }
-    return pos;
-}
-
-__device__ __forceinline__ void store_slot(const KArgs& k, uint32_t pos, uint32_t i) {
-    if (pos < k.a.n)
-        k.l.csr_agents[pos] = i;
-    else
-        raise_error(k, ERR_LOCATION);
-}
-
-// Infection draws of agent i at location loc with hazard h0 of variant 0
-// (LocationsList::infectAgents, locationList.h:233-310; DynamicPPState::gotInfected,
-// dynamicPPState.cpp:235-244).  Returns the sum of min(1, p) over the draws.
-// d p / d theta of one draw (p = r * s * sigma_band, r = 1 - exp(-x),
-// x = k * S/n * w * season * dt), weighted by the replica's dL/dE, added to the
-// block's FP64 accumulators
-// x: the location's hazard argument k*S/n*w*season*dt for variant v; times:
-// how many timesteps made this draw with the same p
-__device__ __noinline__ void adjoint_terms(const KArgs& k, uint32_t i, uint32_t loc, uint32_t v, uint32_t rep, float r,
-                                           float su, float s_eff, double* s_grad, float x_f, uint32_t times) {
-    const double g = k.adj.weight[rep] * (double)times;
-    if (g == 0.0) return;
-    const double x = (double)x_f;
-    const double dpdx = (double)s_eff * (1.0 - (double)r);
-    const double kf = (double)k.r.k_f[rep];
-    if (kf != 0.0) atomicAdd(&s_grad[GRAD_K], g * dpdx * x / kf);
-    const int slot = k.adj.type_slot[k.l.type[loc]];
-    const double w = (double)k.l.infectiousness[loc];
-    if (slot >= 0 && w != 0.0) atomicAdd(&s_grad[GRAD_W + slot], g * dpdx * x / w);
-    atomicAdd(&s_grad[GRAD_SIGMA + k.a.band[i]], g * (double)r * (double)su);
-}
-
-__device__ __forceinline__ double draw_agent(const KArgs& k, uint32_t i, uint32_t loc, uint32_t t, float h0,
-                                             double* s_grad) {
-    const uint32_t N = k.a.n, L = k.l.n, V = k.m.n_variants;
-    // the agent's fields load together (variant 0's susceptibility: a draw
-    // that infects rewrites the later variants' before they are read)
-    const uint32_t rep = k.a.rep[i];
-    const float sigma = k.p.sigma_band[k.a.band[i]];
-    const float su0 = k.a.susceptible[i];
-    const unsigned long long seed = k.r.seed[rep];
-    const uint32_t li = i - k.r.agent_off[rep];
-    double term_sum = 0.0;
-    for (uint32_t v = 0; v < V; ++v) {
-        const float h = v == 0 ? h0 : k.l.hazard[(size_t)v * L + loc];
-        if (!(h > 0.0f)) continue;
-        if (!k.r.variant_active[rep * V + v]) continue;
-        const float su = v == 0 ? su0 : k.a.susceptible[(size_t)v * N + i];
-        const float s_eff = su * sigma;
-        if (!(s_eff > 0.0f)) continue;
-        const float pf = h * s_eff;
-        term_sum += pf < 1.0f ? (double)pf : 1.0;
-        if (k.adj.on && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, su, s_eff, s_grad, k.l.hazard_x[(size_t)v * L + loc], 1u);
-        const double U = psim_u01_once(seed, li, t, PSIM_PHASE_INFECT + v);
-        if (U < (double)pf) {
-            k.a.state[i] = (int8_t)k.m.first_infected;
-            k.a.variant[i] = (uint8_t)v;
-            k.a.days[i] = -2;
-            update_meta(k, i);
-            k.a.st_infected_ts[i] = t;
-            k.a.st_infected_count[i] = k.a.st_infected_count[i] + 1;
-            k.a.st_infected_loc[i] = loc;
-            k.a.st_worst_state[i] = (int8_t)k.m.first_infected;
-            k.a.st_worst_ts[i] = t;
-            k.a.st_variant_mask[i] |= 1u << v;
-        }
-    }
-    return term_sum;
-}
-
-__device__ __forceinline__ void grad_begin(const KArgs& k, double* s_grad) {
-    if (!k.adj.on) return;
-    if (threadIdx.x < GRAD_N) s_grad[threadIdx.x] = 0.0;
-    __syncthreads();
-}
-
-// one global atomic per block and parameter
-__device__ __forceinline__ void grad_end(const KArgs& k, double* s_grad) {
-    if (!k.adj.on) return;
-    __syncthreads();
-    if (threadIdx.x < GRAD_N && s_grad[threadIdx.x] != 0.0) atomicAdd(&k.adj.grad[threadIdx.x], s_grad[threadIdx.x]);
-}
-
-// expected-infection accumulation: one atomic per replica present in the warp
-__device__ __forceinline__ void add_expected(const KArgs& k, bool act, uint32_t i, double term) {
-    const unsigned am = __ballot_sync(0xffffffffu, act && term != 0.0);
-    if (!(act && term != 0.0)) return;
-    const uint32_t rep = k.a.rep[i];
-    const unsigned peers = __match_any_sync(am, rep);
-    const int leader = __ffs(peers) - 1;
-    unsigned rest = peers;
-    double tot = 0.0;
-    while (rest) {
-        const int src = __ffs(rest) - 1;
-        tot += __shfl_sync(peers, term, src);
-        rest &= rest - 1;
-    }
-    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&k.r.expected[rep], tot);
-}
-
-// Timeline stamps of the profiled day graph (KArgs::prof): one atomic per
-// block, from thread 0, on the global nanosecond timer.
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// the block's entry (no wait for the other threads)
-__device__ __forceinline__ void prof_enter(const KArgs& k, uint32_t slot) {
-    if (k.prof && threadIdx.x == 0) atomicMax(&k.prof[slot], ~global_ns());
-}
-// the block's threads are past this point (every thread calls it)
-__device__ __forceinline__ void prof_mark(const KArgs& k, uint32_t slot) {
-    if (!k.prof) return;
-    __syncthreads();
-    if (threadIdx.x == 0) atomicMax(&k.prof[slot], global_ns());
-}
-
-// Where a warp's lanes put the entries they flagged (bits of `flags`, one
-// per agent of the lane) in a block's list: the first one's place (one
-// shared-memory atomic per warp).
-__device__ __forceinline__ uint32_t list_place(uint32_t flags, uint32_t* s_cnt) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t mine = __popc(flags);
-    uint32_t inc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    uint32_t base = 0;
-    if (lane == 31 && inc) base = atomicAdd(s_cnt, inc);
-    return __shfl_sync(0xffffffffu, base, 31) + inc - mine;
-}
 
 // Movement of every agent + histogram + fixed-point infectiousness sums (the
 // day's first step, after a reset of the sums).  Records the steps of the day
 // at which agents decide next.  The day kernel follows: the locations' flag
 // words of the day are there, the agents' decision words are written.
+template <int POL>
 __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
     __shared__ uint32_t s_mm[MOVE_MASK_WORDS];
     prof_enter(k, PROF_N);
@@ -815,10 +50,10 @@ __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
             loc0 = loc = k.a.location[i];
             inf = k.a.infectious[i];
             uint32_t w = decision_word(k, i, c.t);
-            if (c.curfew_now || s == 0) {
+            if ((POL == 2 && c.curfew_now) || s == 0) {
                 decision_in(k, i, d);
                 d.w = w;
-                loc = move_agent<true>(k, i, c, s, s_mm, d, &w);
+                loc = move_agent<true, POL>(k, i, c, s, s_mm, d, &w);
             } else {
                 mask_note(k, s_mm, m0);  // an agent counting down decides later today
             }
@@ -892,7 +127,7 @@ __global__ void __launch_bounds__(PHASE_THREADS) k_phase_movement(KArgs k, uint3
             decision_in(k, i, d);
             uint32_t w = d.w = decision_word(k, i, c.t);
             const float f = k.a.infectious[i];
-            const uint32_t loc = move_agent<false>(k, i, c, k.a.move_at[i] - c.t, s_mm, d, &w);
+            const uint32_t loc = move_agent<false, 2>(k, i, c, k.a.move_at[i] - c.t, s_mm, d, &w);
             moved |= count_agent(k, true, d.loc, loc, f, f > 0.0f ? k.a.variant[i] : 0u);
         }
         __syncthreads();
@@ -1456,833 +691,6 @@ __global__ void __launch_bounds__(PHASE_THREADS, 4) k_phase_draw(KArgs k, uint32
         __syncthreads();
     }
     grad_end(k, s_grad);
-}
-
-// ---------------------------------------------------------------------------
-// The day graph's day kernel: one launch for all timesteps of a day, a
-// persistent grid (every block resident, a cooperative launch) whose phases
-// are separated by grid barriers only where one phase needs another's results.
-// Most timesteps of a day move nobody (at 2M agents 22 of 144 have deciders),
-// so the day is cut into segments: the timesteps from one whose agents took
-// new locations to the next that somebody decides at.  Per segment:
-//   list      one pass over the block's agents: when agents took new locations
-//             (or a rebuild is pending) those at a location with a nonzero sum
-//             enter the block's agent list (their id, location and
-//             susceptibility x age-band factor of every variant); those that
-//             decide at the segment's end enter the block's work list.  The
-//             location quarantine writes of the decisions before are merged
-//             here too.
-//   draw      every listed entry, one per thread, for all the timesteps of the
-//             segment at once: nobody moves, so a location's infection ratio
-//             stays what it is until somebody there is infected.  An entry
-//             that would be infected commits nothing: it flags its location |
-//             if any was flagged, their entries gathered by location |
-//             the flagged locations (a few) replayed exactly, a warp each,
-//             timestep by timestep with the ratio of the location's sum as the
-//             timestep started (LocationsList::infectAgents,
-//             locationList.h:233-310)
-//   decide  | doMovement of the queued agents and the histogram and sum deltas
-//             of their moves |
-// (| a grid barrier).  A block lists, draws and decides its own agents, so
-// nothing but the flagged locations and the moves passes between blocks.
-// What it replaces drew every timestep in a launch of its own (2.9-5.8 us and
-// a launch gap of 0.9-1.3 us each at 10k-2M agents, ~100 timesteps of a day).
-
-constexpr uint32_t DAY_THREADS = 512;  // two blocks per SM at 64 registers
-
-// Grid barrier of the day kernel: every block adds one to a count that only
-// grows (zeroed when the day graph starts) and waits until it reaches the
-// barrier's target.  On GB300 1.4 us with 304 blocks of 512 threads, against
-// 2.5 us for a returning arrival, a reset and a generation word with 608
-// blocks of 256 (arrivals on one address are serialized, so fewer blocks and
-// no returned value).  Every wait is bounded: on expiry the block records
-// ERR_BARRIER and returns false, the others follow (they look at the error
-// flags while they wait), and every later barrier and day kernel returns at
-// once, so a failure ends in an error report, never a hang.  The block's
-// writes reach the other blocks through the arrival (release: the block's
-// threads' writes are ordered before it by the __syncthreads before) and the
-// count's read (acquire).
-constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_add_release_gpu(uint32_t* p, uint32_t x) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
-}
-
-// Block-shared scratch of the day kernel.
-struct DayShared {
-    double grad[GRAD_N];
-    float h[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // per warp: a replayed location's ratios
-    float x[DAY_THREADS / 32][PSIM_MAX_STRAINS + 1];  // and their arguments
-    uint32_t mm[MOVE_MASK_WORDS];
-    uint32_t red[32];
-    uint32_t target;  // the barrier count the next barrier waits for
-    uint32_t cnt;     // agents in the block's work list
-    uint32_t listed;  // entries of the block's agent list
-    bool ok;
-};
-
-__device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t target = sh.target;
-        bool ok = true;
-        red_add_release_gpu(&k.l.bar[0], 1u);
-        uint32_t spins = 0;
-        while ((int32_t)(ld_acquire_gpu(&k.l.bar[0]) - target) < 0) {
-            if ((++spins & 1023u) == 0u) {
-                if (spins >= BARRIER_SPIN_LIMIT) raise_error(k, ERR_BARRIER);
-                if (ld_acquire_gpu(k.err) & ERR_BARRIER) {
-                    ok = false;
-                    break;
-                }
-            }
-            __nanosleep(20);
-        }
-        sh.target = target + gridDim.x;
-        sh.ok = ok;
-    }
-    __syncthreads();
-    return sh.ok;
-}
-
-// the location quarantine writes of the last decisions into quarantine_until
-// (grid-stride)
-__device__ __forceinline__ void merge_quarantine(const KArgs& k) {
-    const uint32_t L = k.l.n;
-    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < L; l += gridDim.x * blockDim.x) {
-        const uint32_t qq = k.l.qu_pending[l];
-        if (qq) {
-            if (qq > k.l.quarantine_until[l]) k.l.quarantine_until[l] = qq;
-            k.l.lflags[l] |= (uint16_t)LF_QUARANTINE;
-            k.l.qu_pending[l] = 0u;
-        }
-    }
-}
-
-// The day kernel is compiled for VC variants (0: any number) and with or
-// without the expected infections and the adjoint (SUMS): what a simulation
-// without them does not need costs its decisions registers (one kernel for
-// all spilled 224 bytes a thread and decided 7% slower).
-template <int VC>
-__device__ __forceinline__ uint32_t nvar(const KArgs& k) {
-    return VC ? (uint32_t)VC : k.m.n_variants;
-}
-
-template <int VC, bool SUMS>
-__device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
-    bool nz = k.l.sfix[l] != 0ull;
-    for (uint32_t v = 1; v < nvar<VC>(k) && !nz; ++v) nz = k.l.sfix[(size_t)v * k.l.n + l] != 0ull;
-    return nz;
-}
-
-// The block's lists of its own agents (four consecutive agents per thread,
-// one 16-byte load of a field, two quads in flight; the blocks' quads are
-// dealt in turn).  list: the agent list afresh.  Only the agents at locations
-// with a nonzero sum are listed, because the draws of every step until the
-// next listing need no other location: until then no other location gains a
-// nonzero sum (nobody moves, since a move makes the next segment list again,
-// and a draw infects only agents at a location with a nonzero sum).  The
-// hazard mask is a superset of those locations (every kernel that adds an
-// infectious term sets the bit at once); an agent that finds a zero sum behind
-// its location's bit clears it.  Agents of one location lie in many blocks'
-// lists: the replay gathers those it needs, so no location needs a segment of
-// its own (reserving segments first, a pass over the mask, a barrier and a
-// returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
-// 20M).  queue: the work list of those that decide at s1.
-template <int VC, bool SUMS>
-__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, uint32_t s1, uint32_t cap,
-                                            DayShared& sh) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (list) sh.listed = 0u;
-        if (queue) sh.cnt = 0u;
-    }
-    __syncthreads();
-    const bool everybody = k.p.enable_curfew && k.p.curfew_begin == s1;
-    const uint32_t t1 = k.clock->t0 + s1;
-    const uint32_t quads = (N + 3u) >> 2;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const size_t seg = (size_t)blockIdx.x * cap;
-    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // block-uniform trips
-        uint32_t loc[8], m[8];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t q = q0 + (uint32_t)h * stride + threadIdx.x;
-            const uint32_t i0 = q * 4u;
-            const bool whole = q < quads && i0 + 3u < N;
-            if (list && whole) {
-                const uint4 v = *reinterpret_cast<const uint4*>(k.a.location + i0);
-                loc[4 * h + 0] = v.x;
-                loc[4 * h + 1] = v.y;
-                loc[4 * h + 2] = v.z;
-                loc[4 * h + 3] = v.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    loc[4 * h + u] = list && q < quads && i0 + u < N ? k.a.location[i0 + u] : NONE;
-            }
-            if (queue && whole) {
-                const uint4 v = *reinterpret_cast<const uint4*>(k.a.move_at + i0);
-                m[4 * h + 0] = v.x;
-                m[4 * h + 1] = v.y;
-                m[4 * h + 2] = v.z;
-                m[4 * h + 3] = v.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    m[4 * h + u] = queue && q < quads && i0 + u < N ? k.a.move_at[i0 + u] : t1 + 1u;
-            }
-        }
-        const auto agent_of = [&](int u) {
-            return (q0 + (uint32_t)(u >> 2) * stride + threadIdx.x) * 4u + (uint32_t)(u & 3);
-        };
-        if (list) {
-            uint32_t lw[8], flags = 0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if ((lw[u] >> (loc[u] & 31u)) & 1u) {
-                    if (nonzero_sum<VC, SUMS>(k, loc[u]))
-                        flags |= 1u << u;
-                    else
-                        atomicAnd(&k.l.hmask[loc[u] >> 5], ~(1u << (loc[u] & 31u)));
-                }
-            if (__any_sync(0xffffffffu, flags != 0u)) {
-                uint32_t at = list_place(flags, &sh.listed);
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if ((flags >> u) & 1u) {
-                        const uint32_t i = agent_of(u);
-                        const size_t pos = seg + at++;
-                        k.l.list_agent[pos] = i;
-                        k.l.list_loc[pos] = loc[u];
-                        const float sigma = k.p.sigma_band[k.a.band[i]];
-                        for (uint32_t v = 0; v < V; ++v)
-                            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
-                    }
-            }
-        }
-        if (queue) {
-            uint32_t flags = 0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (agent_of(u) < N && (everybody || m[u] == t1)) flags |= 1u << u;
-            if (__any_sync(0xffffffffu, flags != 0u)) {
-                uint32_t at = list_place(flags, &sh.cnt);
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if ((flags >> u) & 1u) k.a.worklist[seg + at++] = agent_of(u);
-            }
-        }
-    }
-    __syncthreads();
-    if (list && threadIdx.x == 0) k.l.list_count[blockIdx.x] = sh.listed;  // for a later launch
-}
-
-// the locations with a nonzero sum and the agents listed (profiled graph only)
-template <int VC, bool SUMS>
-__device__ void count_listed(const KArgs& k, const DayShared& sh) {
-    uint32_t locs = 0;
-    for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < k.l.n; l += gridDim.x * blockDim.x)
-        locs += nonzero_sum<VC, SUMS>(k, l) ? 1u : 0u;
-    locs = __reduce_add_sync(__activemask(), locs);
-    if ((threadIdx.x & 31) == 0 && locs) atomicAdd(&k.prof[PROF_LISTED_LOCATIONS], (unsigned long long)locs);
-    if (threadIdx.x == 0 && sh.listed) atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)sh.listed);
-}
-
-// expected-infection accumulation of the draws: one atomic per replica
-// present in the warp (warp-collective; rep given, not looked up)
-__device__ __forceinline__ void add_expected_rep(const KArgs& k, bool act, uint32_t rep, double term) {
-    const unsigned am = __ballot_sync(0xffffffffu, act && term != 0.0);
-    if (!(act && term != 0.0)) return;
-    const unsigned peers = __match_any_sync(am, rep);
-    const int leader = __ffs(peers) - 1;
-    unsigned rest = peers;
-    double tot = 0.0;
-    while (rest) {
-        const int src = __ffs(rest) - 1;
-        tot += __shfl_sync(peers, term, src);
-        rest &= rest - 1;
-    }
-    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&k.r.expected[rep], tot);
-}
-
-// DynamicPPState::gotInfected (dynamicPPState.cpp:235-244) and the agent's
-// statistics (locationList.h:283-304); inf: its new infectiousness
-// (update_meta).  What it reads it reads first, in one round trip.
-template <int VC, bool SUMS>
-__device__ __forceinline__ void infect_agent(const KArgs& k, uint32_t i, uint32_t v, uint32_t loc, uint32_t t,
-                                             float inf) {
-    const uint32_t N = k.a.n, st = k.m.first_infected;
-    const uint8_t count = k.a.st_infected_count[i];
-    const uint32_t mask = k.a.st_variant_mask[i];
-    const uint32_t w = k.a.dinfo[i] & ~(7u << DW_WB_SHIFT | DW_INFECTIOUS);
-    const uint32_t wb = k.m.state_wb[st];
-    const float su = k.m.state_susceptible[st] ? 1.0f : 0.0f;
-    k.a.state[i] = (int8_t)st;
-    k.a.variant[i] = (uint8_t)v;
-    k.a.days[i] = -2;
-    k.a.infectious[i] = inf;
-    for (uint32_t q = 0; q < nvar<VC>(k); ++q) k.a.susceptible[(size_t)q * N + i] = su;
-    k.a.st_infected_ts[i] = t;
-    k.a.st_infected_count[i] = (uint8_t)(count + 1);
-    k.a.st_infected_loc[i] = loc;
-    k.a.st_worst_state[i] = (int8_t)st;
-    k.a.st_worst_ts[i] = t;
-    k.a.st_variant_mask[i] = mask | 1u << v;
-    k.a.dinfo[i] = w | wb << DW_WB_SHIFT | (inf != 0.0f ? DW_INFECTIOUS : 0u);
-}
-
-// U < p for the 53-bit uniform U = K * 2^-53 of the words (a, b)
-// (psim_u01_from) and a float probability p > 0, in integers: p * 2^53 is
-// exact in float (a power-of-two scaling of a normal or subnormal p), and
-// K < p * 2^53 holds exactly when K < ceil(p * 2^53).  u01_limit is that
-// bound (above every K for p >= 1).
-__device__ __forceinline__ unsigned long long u01_limit(float p) {
-    return p >= 1.0f ? ~0ull : __float2ull_ru(p * 9007199254740992.0f);
-}
-__device__ __forceinline__ bool u01_below(uint32_t a, uint32_t b, unsigned long long limit) {
-    return (((unsigned long long)(a >> 5) << 26) | (unsigned long long)(b >> 6)) < limit;
-}
-// the first two words of the stream (seed, agent, t, infection + v), as
-// psim_u01_once draws them
-__device__ __forceinline__ psim_ctr4 infect_words(unsigned long long seed, uint32_t li, uint32_t t, uint32_t v) {
-    psim_ctr4 c;
-    c.v[0] = li;
-    c.v[1] = t;
-    c.v[2] = PSIM_PHASE_INFECT + v;
-    c.v[3] = 0u;
-    return psim_philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-}
-
-// Infection ratio of variant v at location loc (count cnt, weight wl,
-// replica coefficient kf) from the location's fixed-point sum: the formula
-// the scans evaluate (psim_hazard_x), so every entry of a location computes
-// the same value.  x receives its argument.
-__device__ __forceinline__ float entry_hazard(const KArgs& k, uint32_t loc, uint32_t v, uint32_t cnt, float wl,
-                                              float kf, float season, uint32_t dt, float* x) {
-    const long long fix = (long long)k.l.sfix[(size_t)v * k.l.n + loc];
-    *x = 0.0f;
-    return fix != 0 ? psim_hazard_x(fix, cnt, kf, wl, season, dt, x) : 0.0f;
-}
-
-// A replica's infection coefficient, seed and first agent.
-struct RepConst {
-    float kf;
-    uint32_t off;
-    unsigned long long seed;
-};
-__device__ __forceinline__ RepConst rep_const(const KArgs& k, uint32_t rep) {
-    RepConst c;
-    c.kf = k.r.k_f[rep];
-    c.off = k.r.agent_off[rep];
-    c.seed = k.r.seed[rep];
-    return c;
-}
-
-// The timesteps of one segment's draws: its first one (timestamp t), how many
-// there are, the day's season, the replay stamp of its flagged locations.
-struct DrawRun {
-    uint32_t t, n, epoch;
-    float season;
-};
-
-// The draws of every entry of the block's agent list for all the timesteps
-// of the segment, one entry per thread.  Each entry evaluates its location's
-// ratio from the location's sum, count and weight (the same inputs give the
-// same value at every entry) and compares the agent's Philox draw of every
-// timestep with it.  Nothing is committed here: an entry that would be
-// infected flags its location (a stamp per location keeps it in the list
-// once; the first to flag it reserves room for the location's agents), and
-// phase_replay repeats that location's draws with the ratio changing as its
-// agents are infected.  At a location without such an entry the ratio
-// cannot change, so the draws compared with it were the right ones.
-template <int VC, bool SUMS>
-__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, uint32_t* n_entries,
-                           uint32_t* n_hazard) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
-    const bool one_rep = k.r.n == 1;
-    const RepConst rc0 = rep_const(k, 0);
-    uint32_t entries = 0, hazard = 0;
-    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
-        const size_t pos = seg + j;
-        const uint32_t loc = k.l.list_loc[pos];
-        const uint32_t i = k.l.list_agent[pos];
-        const float su0 = k.l.list_su[pos];
-        if (loc >= L || i >= N) {
-            raise_error(k, ERR_AGENT_LIST);
-            continue;
-        }
-        const uint32_t cnt = k.l.counts[loc];
-        const float wl = k.l.infectiousness[loc];
-        const uint32_t rep = one_rep ? 0u : k.l.rep[loc];
-        const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
-        bool any_h = false, hit = false;
-        for (uint32_t v = 0; v < V && !hit; ++v) {
-            float x;
-            const float h = entry_hazard(k, loc, v, cnt, wl, rc.kf, dr.season, dt, &x);
-            if (!(h > 0.0f)) continue;
-            any_h = true;
-            if (!k.r.variant_active[rep * V + v]) continue;
-            const float s_eff = v == 0 ? su0 : k.l.list_su[v * k.l.list_cap + pos];
-            if (!(s_eff > 0.0f)) continue;
-            const unsigned long long limit = u01_limit(h * s_eff);
-            const uint32_t li = i - rc.off;
-#pragma unroll 2
-            for (uint32_t q = 0; q < dr.n; ++q) {
-                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + q, v);
-                hit |= u01_below(o.v[0], o.v[1], limit);
-            }
-        }
-        if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
-            const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
-            const uint32_t room = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
-            k.l.replay_cursor[loc] = room;
-            if (at < L)
-                k.l.replay_list[at] = make_uint4(loc, room, cnt, rep);
-            else
-                raise_error(k, ERR_AGENT_LIST);
-        }
-        entries += dr.n;
-        hazard += any_h ? dr.n : 0u;
-    }
-    *n_entries += entries;
-    *n_hazard += hazard;
-}
-
-// The entries of the flagged locations, gathered by location.
-__device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed) {
-    const uint32_t L = k.l.n, N = k.a.n;
-    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
-        const uint32_t loc = k.l.list_loc[seg + j];
-        if (loc >= L || k.l.replay_stamp[loc] != dr.epoch) continue;
-        const uint32_t i = k.l.list_agent[seg + j];
-        const uint32_t p = atomicAdd(&k.l.replay_cursor[loc], 1u);
-        if (p < N)
-            k.l.replay_slot[p] = make_uint2((uint32_t)(seg + j), i);
-        else
-            raise_error(k, ERR_AGENT_LIST);
-    }
-}
-
-// The expected infections (and the adjoint's terms) of the segment's draws at
-// the locations that are not replayed: every timestep's are the same.
-template <int VC, bool SUMS>
-__device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
-    for (uint32_t base = 0; base < listed; base += blockDim.x) {  // block-uniform trips
-        const uint32_t j = base + threadIdx.x;
-        const size_t pos = seg + j;
-        const uint32_t loc = j < listed ? k.l.list_loc[pos] : NONE;
-        const uint32_t i = loc < L ? k.l.list_agent[pos] : NONE;
-        const bool act = loc < L && i < N && k.l.replay_stamp[loc] != dr.epoch;
-        uint32_t rep = 0;
-        double term = 0.0;
-        if (act) {
-            const uint32_t cnt = k.l.counts[loc];
-            const float wl = k.l.infectiousness[loc];
-            rep = k.l.rep[loc];
-            const float kf = k.r.k_f[rep];
-            for (uint32_t v = 0; v < V; ++v) {
-                float x;
-                const float h = entry_hazard(k, loc, v, cnt, wl, kf, dr.season, dt, &x);
-                if (!(h > 0.0f) || !k.r.variant_active[rep * V + v]) continue;
-                const float s_eff = k.l.list_su[v * k.l.list_cap + pos];
-                if (!(s_eff > 0.0f)) continue;
-                const float pf = h * s_eff;
-                term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
-                if ((SUMS && k.adj.on) && pf < 1.0f)
-                    adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x, dr.n);
-            }
-        }
-        if ((SUMS && k.track_expected)) add_expected_rep(k, act, rep, term);
-    }
-}
-
-// The sum change of an agent at location loc infected there.
-template <int VC, bool SUMS>
-__device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t loc, float inf0, uint32_t var0,
-                                                     float inf, uint32_t var) {
-    const uint32_t L = k.l.n;
-    const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
-    const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
-    if (q0 == q1 && var0 == var) return;
-    if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc], (unsigned long long)(-q0));
-    if (q1) {
-        atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
-        mark_hazardous(k, loc);
-    }
-}
-
-// One entry's draws of timestep t with its location's ratios s_h (arguments
-// s_x): the agent i of list entry pos.  An agent that is infected updates its
-// entry's susceptibility products (read by no other entry) and its location's sums,
-// which the ratios of the next timestep are computed from.  Adds the sum of
-// min(1, p) over its draws to *term when expected infections are tracked;
-// returns whether the agent was infected.
-template <int VC, bool SUMS>
-__device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t i, uint32_t loc, uint32_t rep,
-                                           const RepConst& rc, uint32_t t, const float* s_h, const float* s_x,
-                                           double* s_grad, double* term) {
-    const uint32_t N = k.a.n, V = nvar<VC>(k);
-    bool infected = false;
-    float inf0 = 0.0f, inf = 0.0f, sigma = 0.0f;
-    uint32_t var0 = 0, var = 0;
-    for (uint32_t v = 0; v < V; ++v) {
-        const float h = s_h[v];
-        if (!(h > 0.0f)) continue;
-        if (!k.r.variant_active[rep * V + v]) continue;
-        // after an infection the later variants read the agent's new
-        // susceptibility (what the entry then gets)
-        const float s_eff = infected ? k.a.susceptible[(size_t)v * N + i] * sigma : k.l.list_su[v * k.l.list_cap + pos];
-        if (!(s_eff > 0.0f)) continue;
-        const float pf = h * s_eff;
-        if ((SUMS && k.track_expected)) *term += pf < 1.0f ? (double)pf : 1.0;
-        if ((SUMS && k.adj.on) && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1u);
-        const psim_ctr4 o = infect_words(rc.seed, i - rc.off, t, v);
-        if (u01_below(o.v[0], o.v[1], u01_limit(pf))) {
-            if (!infected) {
-                inf0 = k.a.infectious[i];
-                var0 = inf0 > 0.0f ? k.a.variant[i] : 0u;
-                sigma = k.p.sigma_band[k.a.band[i]];
-                infected = true;
-            }
-            inf = k.m.state_infectious[k.m.first_infected] * k.m.variant_multiplier[v];
-            var = v;
-            infect_agent<VC, SUMS>(k, i, v, loc, t, inf);
-        }
-    }
-    if (infected) {
-        const float su = (k.m.state_susceptible[k.m.first_infected] ? 1.0f : 0.0f) * sigma;
-        for (uint32_t v = 0; v < V; ++v) k.l.list_su[v * k.l.list_cap + pos] = su;
-        add_infection_change<VC, SUMS>(k, loc, inf0, var0, inf, inf > 0.0f ? var : 0u);
-    }
-    return infected;
-}
-
-// The ratios of a replayed location (and their arguments) from its sums, in
-// the warp's shared memory.  Past L1: the sums change in L2 (reductions).
-template <int VC, bool SUMS>
-__device__ __forceinline__ void replay_ratios(const KArgs& k, const DrawRun& dr, const uint4& r, float wl, float kf,
-                                              float* s_h, float* s_x) {
-    const uint32_t lane = threadIdx.x & 31u;
-    __syncwarp();
-    if (lane < nvar<VC>(k)) {
-        const long long fix = (long long)__ldcg(&k.l.sfix[(size_t)lane * k.l.n + r.x]);
-        float x = 0.0f;
-        s_h[lane] = fix != 0 ? psim_hazard_x(fix, r.z, kf, wl, dr.season, k.p.time_step, &x) : 0.0f;
-        s_x[lane] = x;
-    }
-    __syncwarp();
-}
-
-// A replayed location of up to 64 agents and VM variants at most (almost all
-// of them): two entries per lane in registers, with the draws' bounds.  A
-// timestep without an infection is a Philox block per entry and variant and a
-// vote; one with an infection goes through draw_entry for the agents it hit
-// and computes the bounds again.  Expected infections and adjoint terms are
-// added for all timesteps since the bounds last changed.
-template <int VC, bool SUMS, int VM>
-__device__ __forceinline__ void replay_registers(const KArgs& k, const DrawRun& dr, const uint4& r, float wl,
-                                                 const RepConst& rc, float* s_h, float* s_x, double* s_grad,
-                                                 double* term) {
-    constexpr int Q = 2;
-    const uint32_t N = k.a.n, lane = threadIdx.x & 31u;
-    const bool sums = (SUMS && k.track_expected) || (SUMS && k.adj.on);
-    uint32_t pos[Q], id[Q];
-    float su[Q][VM];
-    unsigned long long limit[Q][VM];
-#pragma unroll
-    for (int e = 0; e < Q; ++e) {
-        const uint32_t p = lane + 32u * (uint32_t)e;
-        const uint2 s = p < r.z ? k.l.replay_slot[r.y + p] : make_uint2(0u, NONE);
-        pos[e] = s.x;
-        id[e] = s.y;
-    }
-    uint32_t active = 0;
-#pragma unroll
-    for (int v = 0; v < VM; ++v)
-        if ((uint32_t)v < nvar<VC>(k) && k.r.variant_active[r.w * nvar<VC>(k) + v]) active |= 1u << v;
-    const auto bounds = [&]() {
-        replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, s_h, s_x);
-#pragma unroll
-        for (int e = 0; e < Q; ++e)
-#pragma unroll
-            for (int v = 0; v < VM; ++v) {
-                const bool on = id[e] < N && ((active >> v) & 1u);
-                su[e][v] = on ? k.l.list_su[v * k.l.list_cap + pos[e]] : 0.0f;
-                const float p = on ? s_h[v] * su[e][v] : 0.0f;
-                limit[e][v] = p > 0.0f ? u01_limit(p) : 0ull;
-            }
-    };
-    // (one copy each of what is rare)
-    const auto add = [&](uint32_t hit, uint32_t times) {
-#pragma unroll 1
-        for (int e = 0; e < Q; ++e) {
-            const uint32_t i = e ? id[1] : id[0], n = times - ((hit >> e) & 1u);
-#pragma unroll
-            for (int v = 0; v < VM; ++v) {
-                const float s = e ? su[1][v] : su[0][v], h = s_h[v], pf = h * s;
-                if (!((active >> v) & 1u) || !(pf > 0.0f) || !n) continue;
-                if ((SUMS && k.track_expected)) *term += (double)n * (pf < 1.0f ? (double)pf : 1.0);
-                if ((SUMS && k.adj.on) && pf < 1.0f)
-                    adjoint_terms(k, i, r.x, v, r.w, h, k.a.susceptible[(size_t)v * N + i], s, s_grad, s_x[v], n);
-            }
-        }
-    };
-    bounds();
-    uint32_t since = 0;  // timesteps since the bounds changed
-    for (uint32_t q = 0; q < dr.n; ++q) {
-        uint32_t hit = 0;
-#pragma unroll
-        for (int e = 0; e < Q; ++e)
-#pragma unroll
-            for (int v = 0; v < VM; ++v)
-                if (limit[e][v]) {
-                    const psim_ctr4 o = infect_words(rc.seed, id[e] - rc.off, dr.t + q, v);
-                    hit |= u01_below(o.v[0], o.v[1], limit[e][v]) ? 1u << e : 0u;
-                }
-        if (!__any_sync(0xffffffffu, hit)) {
-            ++since;
-            continue;
-        }
-        if (sums) add(hit, since + 1u);  // (draw_entry adds this timestep's of those it hit)
-#pragma unroll 1
-        for (int e = 0; e < Q; ++e)
-            if ((hit >> e) & 1u)
-                draw_entry<VC, SUMS>(k, e ? pos[1] : pos[0], e ? id[1] : id[0], r.x, r.w, rc, dr.t + q, s_h, s_x, s_grad, term);
-        since = 0;
-        if (q + 1u == dr.n) break;
-        __threadfence();  // the reductions before the sums are read again
-        bounds();
-    }
-    if (sums && since) add(0u, since);
-}
-
-// The flagged locations' draws, a warp per location, timestep after timestep:
-// in registers where they fit, else over the entries 32 at a time with the
-// ratios computed again after a timestep that infected somebody (all its
-// draws first: a timestep's ratios come from the sums as it started).
-template <int VC, bool SUMS>
-__device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_replay, DayShared& sh) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a block's warps take locations far apart in the list: few locations
-    // spread over all SMs
-    for (uint32_t f = (uint32_t)warp * gridDim.x + blockIdx.x; f < n_replay; f += gridDim.x * (blockDim.x >> 5)) {
-        const uint4 r = k.l.replay_list[f];  // location, first entry, agents, replica
-        if (r.x >= L || r.y > N || r.z > N - r.y) {
-            if (lane == 0) raise_error(k, ERR_AGENT_LIST);
-            continue;
-        }
-        const float wl = k.l.infectiousness[r.x];
-        const RepConst rc = rep_const(k, r.w);
-        double term = 0.0;
-        if (VC != 2 && V == 1 && r.z <= 64u) {
-            replay_registers<VC, SUMS, 1>(k, dr, r, wl, rc, sh.h[warp], sh.x[warp], sh.grad, &term);
-        } else if (VC != 1 && V == 2 && r.z <= 64u) {
-            replay_registers<VC, SUMS, 2>(k, dr, r, wl, rc, sh.h[warp], sh.x[warp], sh.grad, &term);
-        } else {
-            bool stale = true;  // the ratios: at the start and after an infection
-            for (uint32_t q = 0; q < dr.n; ++q) {
-                if (stale) replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, sh.h[warp], sh.x[warp]);
-                bool infected = false;
-                for (uint32_t p = (uint32_t)lane; p < r.z; p += 32u) {
-                    const uint2 s = k.l.replay_slot[r.y + p];
-                    if (s.y >= N) {
-                        raise_error(k, ERR_AGENT_LIST);
-                        break;
-                    }
-                    infected |= draw_entry<VC, SUMS>(k, s.x, s.y, r.x, r.w, rc, dr.t + q, sh.h[warp], sh.x[warp], sh.grad, &term);
-                }
-                stale = __any_sync(0xffffffffu, infected);
-                if (stale) __threadfence();  // the reductions before the sums are read again
-            }
-        }
-        if ((SUMS && k.track_expected)) add_expected_rep(k, true, r.w, term);
-    }
-}
-
-// doMovement of the agents the block queued for s1 (its own segment, whose
-// count the queue left in shared memory: every block starts its decisions at
-// the same barrier, so handing segments out by ticket balanced nothing), then
-// the histogram and sum deltas of the agents that took a new location.
-template <int VC, bool SUMS>
-__device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t* s_mm, const uint32_t* s_cnt) {
-    const StepClock c = step_clock(k, s1);
-    bool moved = false;
-    {
-        uint32_t n = *s_cnt;
-        if (n > cap) {
-            if (threadIdx.x == 0) raise_error(k, ERR_AGENT_LIST);
-            n = 0;
-        }
-        const uint32_t* seg = k.a.worklist + (size_t)blockIdx.x * cap;
-        // the next trip's inputs are loaded before this trip's decision, its
-        // agent a trip earlier still (22.0 -> 21.1 us a step at 2M agents,
-        // 201 -> 190 at 20M)
-        const uint32_t tid = threadIdx.x, T = blockDim.x;
-        DecisionIn nd;
-        auto inputs = [&](uint32_t i, DecisionIn& d) {
-            if (i >= k.a.n) return;
-            decision_in(k, i, d);
-            d.w = k.a.dinfo[i];
-        };
-        uint32_t ni = tid < n ? seg[tid] : NONE;
-        inputs(ni, nd);
-        uint32_t n2 = tid + T < n ? seg[tid + T] : NONE;
-        for (uint32_t j = tid; j < n; j += T) {
-            const uint32_t i = ni;
-            const DecisionIn d = nd;
-            ni = n2;
-            inputs(ni, nd);
-            n2 = j + 2u * T < n ? seg[j + 2u * T] : NONE;
-            if (i >= k.a.n) {
-                raise_error(k, ERR_AGENT_LIST);
-                continue;
-            }
-            // (queued for its timestamp, unless everybody is at the curfew)
-            const uint32_t s = c.curfew_now ? k.a.move_at[i] - c.t : 0u;
-            uint32_t w, var = 0;
-            float inf = 0.0f;
-            const uint32_t loc = move_agent<true>(k, i, c, s, s_mm, d, &w);
-            if (w != d.w) k.a.dinfo[i] = w;
-            if (w & DW_INFECTIOUS) {
-                inf = k.a.infectious[i];
-                var = VC == 1 ? 0u : k.a.variant[i];
-            }
-            moved |= count_agent_delta(k, true, d.loc, loc, inf, var, inf, var);
-        }
-    }
-    publish_moved(k, moved, c.t);
-}
-
-// One segment of the day (see the section comment), starting at timestep
-// `step`; *next receives the timestep the next one starts at (step_end after
-// the last).  False when a grid barrier expired (the kernel then ends).  cap =
-// the work-list segment size of a block.
-template <int VC, bool SUMS>
-__device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint32_t step_end, uint32_t phases,
-                                            uint32_t cap, DayShared& sh, uint32_t* next) {
-    const uint32_t tl = PROF_T + PROF_TW * step;  // the segment's timeline slots (profiled graph)
-    prof_enter(k, tl);
-    const uint32_t t = k.clock->t0 + step;
-    const uint32_t moved = k.l.build[0], force = k.l.build[1], q_step = k.l.build[3];
-    DrawRun dr;
-    dr.t = t;
-    dr.epoch = k.l.build[6] + 1u;  // (0 is the stamp of a location never flagged)
-    dr.season = k.clock->season;
-    // the segment's end: the first later timestep that somebody decides at
-    // (everyone at the curfew)
-    uint32_t e = step + 1;
-    bool decides = false;
-    while (e < k.spd) {
-        uint32_t w = k.a.move_mask[e >> 5] >> (e & 31u);
-        if (k.p.enable_curfew && k.p.curfew_begin >= e && k.p.curfew_begin >> 5 == e >> 5)
-            w |= 1u << (k.p.curfew_begin - e);
-        if (w) {
-            e += (uint32_t)(__ffs(w) - 1);
-            decides = e < k.spd;
-            break;
-        }
-        e = (e & ~31u) + 32u;
-    }
-    if (!decides) e = k.spd;
-    // (a caller's shorter range ends the draws, not the decisions after them)
-    dr.n = min(e, step_end) - step;
-    decides = decides && e <= step_end && (phases & PH_DECIDE);
-    *next = min(e, step_end);
-    const bool list = (phases & PH_REBUILD) && csr_decide_from(k, t, moved, force);
-    // the location quarantine writes of the decisions for t
-    const bool merge = (phases & PH_REBUILD) && k.p.quarantine_policy > 1 && q_step == t;
-    if (merge) merge_quarantine(k);
-    const size_t seg = (size_t)blockIdx.x * cap;
-    if (list || decides) {
-        phase_lists<VC, SUMS>(k, list, decides, e, cap, sh);
-        if (decides) mask_clear_shared(sh.mm);
-        if (k.prof) {
-            if (list) count_listed<VC, SUMS>(k, sh);
-            if (threadIdx.x == 0) {
-                if (list && blockIdx.x == 0) atomicAdd(&k.prof[PROF_REBUILDS], 1ull);
-                if (decides && sh.cnt) atomicAdd(&k.prof[PROF_MOVERS], (unsigned long long)sh.cnt);
-                if (decides && blockIdx.x == 0) atomicAdd(&k.prof[PROF_QUEUE_STEPS], 1ull);
-            }
-        }
-        prof_mark(k, tl + (list ? 1 : 2));
-    }
-    const bool draws = (phases & PH_DRAW) != 0;
-    if (draws) {
-        uint32_t entries = 0, hazard = 0;
-        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, &entries, &hazard);
-        if (k.prof) {
-            __syncwarp();
-            entries = __reduce_add_sync(0xffffffffu, entries);
-            hazard = __reduce_add_sync(0xffffffffu, hazard);
-            if ((threadIdx.x & 31) == 0 && (entries | hazard)) {
-                atomicAdd(&k.prof[PROF_DRAW_ENTRIES], (unsigned long long)entries);
-                atomicAdd(&k.prof[PROF_DRAW_HAZARD], (unsigned long long)hazard);
-            }
-        }
-    }
-    prof_mark(k, tl + 3);
-    // every draw before any replay, every draw and merge before any decision
-    if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
-    if (draws) {
-        const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
-        const bool expected = (SUMS && k.track_expected) || (SUMS && k.adj.on);
-        if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
-        if (n_replay || expected) {
-            grad_begin(k, sh.grad);
-            if (n_replay) {
-                phase_gather(k, dr, seg, sh.listed);
-                if (!grid_barrier(k, sh)) return false;
-                phase_replay<VC, SUMS>(k, dr, n_replay, sh);
-            }
-            if (expected) phase_expected<VC, SUMS>(k, dr, seg, sh.listed, sh.grad);
-            grad_end(k, sh.grad);
-            if (decides || n_replay) {
-                // every replay before any decision and before the list is emptied
-                if (!grid_barrier(k, sh)) return false;
-                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
-            }
-        }
-    }
-    prof_mark(k, tl + 4);
-    if (decides) {
-        phase_decide<VC, SUMS>(k, e, cap, sh.mm, &sh.cnt);
-        mask_flush(k, sh.mm);
-    }
-    prof_mark(k, tl + 5);
-    return true;
-}
-
-// The day kernel: timesteps step0 .. step_end - 1.
-template <int VC, bool SUMS>
-__global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0, uint32_t step_end, uint32_t phases,
-                                                        uint32_t cap) {
-    __shared__ DayShared sh;
-    if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
-    if (threadIdx.x == 0) {
-        sh.target = gridDim.x;
-        sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
-        sh.cnt = 0u;
-    }
-    __syncthreads();
-    uint32_t step = step0;
-    for (;;) {
-        uint32_t next = step_end;
-        if (!day_segment<VC, SUMS>(k, step, step_end, phases, cap, sh, &next)) return;
-        if (next >= step_end) return;
-        step = next;
-        if (!grid_barrier(k, sh)) return;
-    }
 }
 
 // Canonical CSR order (ascending agent id inside a location, the output of
@@ -3013,10 +1421,14 @@ static unsigned agent_grid(const KArgs& k, unsigned wave) {
     return std::min(g, grid_for(k.a.n, 1 << 20));
 }
 
+// the policies of a context's decisions (move_decide's POL)
+static int policies(const KArgs& k) { return k.p.enable_curfew ? 2 : k.p.quarantine_policy > 0 ? 1 : 0; }
 void launch_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
-    static unsigned g = 0;
-    if (!g) g = wave_grid(k_movement, 1u << 30);
-    k_movement<<<agent_grid(k, g), 256, 0, s>>>(k, step);
+    static void (*const kernels[3])(KArgs, uint32_t) = {k_movement<0>, k_movement<1>, k_movement<2>};
+    static unsigned g[3] = {0, 0, 0};
+    const int q = policies(k);
+    if (!g[q]) g[q] = wave_grid(kernels[q], 1u << 30);
+    kernels[q]<<<agent_grid(k, g[q]), 256, 0, s>>>(k, step);
 }
 static unsigned quad_grid(uint32_t n, unsigned wave) { return std::min(wave, grid_for((n + 3u) / 4u, 1 << 20)); }
 void launch_phase_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
@@ -3031,20 +1443,23 @@ void launch_day_begin(const KArgs& k, cudaStream_t s) { k_day_begin<<<grid_for(k
 // blocks of 256 threads) capped at the kernel's occupancy, and no more blocks
 // than the population gives work to.  Each block's segment of the lists holds
 // the agents its pass visits.
-typedef void (*DayKernel)(KArgs, uint32_t, uint32_t, uint32_t, uint32_t);
 // the instance for a context, and its resident blocks per SM
 static DayKernel day_kernel(const KArgs& k, unsigned* per_sm) {
-    static const DayKernel kernels[4] = {k_day<1, false>, k_day<2, false>, k_day<1, true>, k_day<0, true>};
-    static int occ[4] = {0, 0, 0, 0};
+    static int occ[DAY_KERNELS] = {};
     const bool sums = k.track_expected || k.adj.on;
-    const int q = k.m.n_variants == 1 ? (sums ? 2 : 0) : k.m.n_variants == 2 && !sums ? 1 : 3;
+    const int pol = policies(k);
+    const int q = k.m.n_variants == 1 && !sums               ? DAY_ONE_PLAIN + pol
+                  : k.m.n_variants == 1 && sums && pol == 0  ? DAY_ONE_SUMS
+                  : k.m.n_variants == 2 && !sums && pol <= 1 ? DAY_TWO
+                                                             : DAY_ANY;
+    DayKernel f = q <= DAY_ONE_QUARANTINE ? day_kernel_a(q) : q <= DAY_ONE_SUMS ? day_kernel_b(q) : day_kernel_c(q);
     if (!occ[q]) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernels[q], DAY_THREADS, 0) != cudaSuccess || n < 1) n = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, DAY_THREADS, 0) != cudaSuccess || n < 1) n = 1;
         occ[q] = n;
     }
     *per_sm = (unsigned)occ[q];
-    return kernels[q];
+    return f;
 }
 static void day_geometry(const KArgs& k, unsigned occ, unsigned* grid, uint32_t* cap) {
     const unsigned bps = k.tune.blocks_per_sm

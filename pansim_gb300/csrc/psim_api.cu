@@ -169,23 +169,24 @@ double seasonality(const psim_params& p, uint32_t t, uint32_t spd) {
     return calc;
 }
 
+// the host's clock for the day containing t
+void host_clock(psim_ctx* c, uint32_t t) {
+    const uint32_t t0 = t - t % c->spd;
+    c->h_clock.t0 = t0;
+    c->h_clock.day_of_week = c->params.holiday_mode ? 6u : (c->params.start_day + t0 / c->spd) % 7u;
+    c->h_clock.season = (float)seasonality(c->params, t0, c->spd);
+}
+
 // set the device clock for the day containing t
-// sync = false: the copy is left in the stream; the caller synchronises
-// before the next set_clock (the copy reads the pinned clock when it runs)
-int set_clock(psim_ctx* c, uint32_t t, bool sync = true) {
-    uint32_t t0 = t - t % c->spd;
-    DevClock nc = c->h_clock;
-    nc.t0 = t0;
-    nc.day_of_week = c->params.holiday_mode ? 6u : (c->params.start_day + t0 / c->spd) % 7u;
-    nc.season = (float)seasonality(c->params, t0, c->spd);
-    if (c->clock_valid && nc.t0 == c->h_clock.t0 && nc.day_of_week == c->h_clock.day_of_week &&
-        nc.season == c->h_clock.season)
-        return 0;
-    c->h_clock = nc;
+int set_clock(psim_ctx* c, uint32_t t) {
+    const DevClock old = c->h_clock;
+    host_clock(c, t);
+    const DevClock& nc = c->h_clock;
+    if (c->clock_valid && nc.t0 == old.t0 && nc.day_of_week == old.day_of_week && nc.season == old.season) return 0;
     *c->h_clock_pin = nc;
     // only the first three fields; the scan bookkeeping stays on the device
     CK(cudaMemcpyAsync(c->k.clock, c->h_clock_pin, 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
-    if (sync) CK(cudaStreamSynchronize(c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     c->clock_valid = true;
     return 0;
 }
@@ -332,10 +333,34 @@ int do_step(psim_ctx* c, uint32_t step) {
     return launch_check(c);
 }
 
-int capture_day_graph(psim_ctx* c) {
-    if (c->day_graph) {
-        cudaGraphExecDestroy(c->day_graph);
-        c->day_graph = nullptr;
+// The kernels of a day's midnight phases in stream order; t = its timestamp
+// or CLOCK_T (captured: the device clock's).  The statistics go to the pinned
+// buffers.  Returns the number of kernels.
+uint64_t enqueue_midnight(psim_ctx* c, uint32_t t) {
+    uint64_t kernels = 0;
+    if (t > 0 && c->params.testing_enabled) {
+        launch_test(c->k, t, c->stream);
+        kernels += 2;
+    }
+    if (t > 0) {
+        launch_progress(c->k, t, c->stream);
+        kernels += 1;
+    }
+    launch_stats(c->k, t, c->stream);
+    cudaMemcpyAsync(c->h_stats, c->k.stats, sizeof(DevStatsAcc) * c->R, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemcpyAsync(c->h_expected, c->k.r.expected, sizeof(double) * c->R, cudaMemcpyDeviceToHost, c->stream);
+    cudaMemsetAsync(c->k.r.expected, 0, sizeof(double) * c->R, c->stream);
+    launch_plan(c->k, t, c->stream);
+    return kernels + 2 + 5 + (c->params.quarantine_policy > 3 && c->k.l.n_schools ? 1 : 0);
+}
+
+// One graph launch per day: the day's first movement and all its timesteps,
+// and with `midnight` the clock and the midnight phases before them (at 10k
+// agents issuing those one by one took as long as a fifth of the day).
+int capture_graph(psim_ctx* c, psim_ctx::DayGraph* out, bool midnight) {
+    if (out->exec) {
+        cudaGraphExecDestroy(out->exec);
+        out->exec = nullptr;
     }
     cudaGraph_t g = nullptr;
     // profiled: the day kernel's counters and timeline stamps (KArgs::prof)
@@ -343,23 +368,29 @@ int capture_day_graph(psim_ctx* c) {
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     // (the capture stays open until EndCapture: errors are checked after it)
     cudaError_t me = cudaSuccess;
-    if (c->profile) me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
+    uint64_t kernels = 3;  // the day's beginning, its first movement, the day kernel
+    if (midnight) {
+        me = cudaMemcpyAsync(c->k.clock, c->h_clock_pin, 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
+        kernels += enqueue_midnight(c, CLOCK_T);
+        if (me == cudaSuccess) me = cudaEventRecordWithFlags(c->ev0, c->stream, cudaEventRecordExternal);
+    }
+    if (me == cudaSuccess && c->profile)
+        me = cudaMemsetAsync(c->d_prof, 0, sizeof(unsigned long long) * PROF_WORDS, c->stream);
     launch_day_begin(c->k, c->stream);
     launch_movement(c->k, 0, c->stream);
-    // one launch of the day kernel for all timesteps; the profiled graph is
-    // the same launch with the kernel's timeline stamps
     launch_day(c->k, 0, c->spd, PH_ALL, c->stream);
+    if (midnight && me == cudaSuccess) me = cudaEventRecordWithFlags(c->ev1, c->stream, cudaEventRecordExternal);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e == cudaSuccess && me != cudaSuccess) {
         cudaGraphDestroy(g);
         e = me;
     }
     if (e != cudaSuccess) return fail(c, PSIM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&c->day_graph, g, 0);
+    e = cudaGraphInstantiate(&out->exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(c, PSIM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    c->graph_kernels = 3;  // the day's beginning, movement(0), the day kernel
-    c->graph_dirty = false;
+    out->kernels = kernels;
+    out->stale = false;
     c->prof_valid = false;
     return 0;
 }
@@ -820,7 +851,8 @@ int psim_destroy(psim_ctx* c) {
     other_disease_free(c);
     for (auto& kv : c->checkpoints)
         if (kv.second) cudaFree(kv.second);
-    if (c->day_graph) cudaGraphExecDestroy(c->day_graph);
+    if (c->steps_graph.exec) cudaGraphExecDestroy(c->steps_graph.exec);
+    if (c->day_graph.exec) cudaGraphExecDestroy(c->day_graph.exec);
     for (void* p : c->allocs) cudaFree(p);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -916,7 +948,7 @@ int psim_set_params(psim_ctx* c, const psim_params* p) {
     if (p->time_step != c->params.time_step) return fail(c, PSIM_ERR_ARG, "time_step cannot change");
     c->params = *p;
     c->k.p = *p;
-    c->graph_dirty = true;
+    c->graphs_stale();
     c->clock_valid = false;
     if (c->uploaded && p->home_type != c->home_type_done) {
         launch_homes(c->k, c->stream);
@@ -942,7 +974,7 @@ int psim_set_tuning(psim_ctx* c, const psim_tuning* t) {
     c->k.tune.scan_items = t->scan_items ? t->scan_items : 8u;
     if (t->scan_mode > 3) return fail(c, PSIM_ERR_ARG, "scan_mode must be 0, 1, 2 or 3");
     c->k.tune.scan_mode = t->scan_mode;
-    c->graph_dirty = true;
+    c->graphs_stale();
     return 0;
 }
 
@@ -993,7 +1025,7 @@ int psim_set_adjoint(psim_ctx* c, int on, const double* weights) {
     const uint32_t o = on ? 1u : 0u;
     if (o != c->k.adj.on) {
         c->k.adj.on = o;
-        c->graph_dirty = true;
+        c->graphs_stale();
     }
     return 0;
 }
@@ -1074,7 +1106,7 @@ int psim_checkpoint_bytes(psim_ctx* c, uint64_t* out) {
 int psim_set_tracking(psim_ctx* c, int expected) {
     if (!c) return PSIM_ERR_ARG;
     c->k.track_expected = expected ? 1u : 0u;
-    c->graph_dirty = true;
+    c->graphs_stale();
     return 0;
 }
 
@@ -1226,15 +1258,13 @@ int psim_run_steps(psim_ctx* c, uint32_t day) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     int rc = set_clock(c, day * c->spd);
     if (rc) return rc;
-    if (c->graph_dirty || !c->day_graph) {
-        if ((rc = capture_day_graph(c))) return rc;
-    }
+    if (c->steps_graph.stale && (rc = capture_graph(c, &c->steps_graph, false))) return rc;
     CK(cudaEventRecord(c->ev0, c->stream));
-    CK(cudaGraphLaunch(c->day_graph, c->stream));
+    CK(cudaGraphLaunch(c->steps_graph.exec, c->stream));
     CK(cudaEventRecord(c->ev1, c->stream));
     CK(cudaEventSynchronize(c->ev1));
     CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
-    c->launches += c->graph_kernels;
+    c->launches += c->steps_graph.kernels;
     c->prof_valid = c->profile;
     c->csr_fresh = false;
     c->list_sparse = true;
@@ -1254,37 +1284,17 @@ int psim_run_day(psim_ctx* c, uint32_t day, psim_day_stats* out) {
         if (rc) return rc;
         return psim_run_steps(c, day);
     }
-    // The midnight phases, the clock and the day graph in stream order with
-    // one synchronisation at the end: the statistics and the error flags come
-    // back through pinned buffers.
+    // The clock, the midnight phases and the day's steps in one graph launch;
+    // the statistics and the error word come back through pinned buffers.
     int rc = 0;
-    if (c->graph_dirty || !c->day_graph) {
-        if ((rc = capture_day_graph(c))) return rc;
-    }
-    if (t > 0 && c->params.testing_enabled) {
-        launch_test(c->k, t, c->stream);
-        c->launches += 2;
-    }
-    if (t > 0) {
-        launch_progress(c->k, t, c->stream);
-        c->launches += 1;
-    }
-    launch_stats(c->k, t, c->stream);
-    c->launches += 2;
-    CK(cudaMemcpyAsync(c->h_stats, c->k.stats, sizeof(DevStatsAcc) * c->R, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(c->h_expected, c->k.r.expected, sizeof(double) * c->R, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemsetAsync(c->k.r.expected, 0, sizeof(double) * c->R, c->stream));
-    launch_plan(c->k, t, c->stream);
-    c->launches += 5 + (c->params.quarantine_policy > 3 && c->k.l.n_schools ? 1 : 0);
-    c->t_next = t;
-    if ((rc = launch_check(c))) return rc;
-    if ((rc = set_clock(c, t, false))) return rc;
-    CK(cudaEventRecord(c->ev0, c->stream));
-    CK(cudaGraphLaunch(c->day_graph, c->stream));
-    CK(cudaEventRecord(c->ev1, c->stream));
+    if (c->day_graph.stale && (rc = capture_graph(c, &c->day_graph, true))) return rc;
+    host_clock(c, t);
+    *c->h_clock_pin = c->h_clock;
+    c->clock_valid = true;
+    CK(cudaGraphLaunch(c->day_graph.exec, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     CK(cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
-    c->launches += c->graph_kernels;
+    c->launches += c->day_graph.kernels;
     c->prof_valid = c->profile;
     c->csr_fresh = false;
     c->list_sparse = true;
@@ -1346,7 +1356,7 @@ int psim_set_profiling(psim_ctx* c, int on) {
     if (!c) return PSIM_ERR_ARG;
     if ((on != 0) != c->profile) {
         c->profile = on != 0;
-        c->graph_dirty = true;
+        c->graphs_stale();
     }
     c->prof_valid = false;
     return 0;

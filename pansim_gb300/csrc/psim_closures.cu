@@ -175,7 +175,7 @@ int upload_events(psim_ctx* c) {
     dm.n_events = (uint32_t)ne;
     CK(cudaStreamSynchronize(c->stream));
     if ((rc = upload_window_table(c))) return rc;
-    c->graph_dirty = true;
+    c->graphs_stale();
     return 0;
 }
 
@@ -261,7 +261,7 @@ void unset_stay_home(psim_ctx* c, double p, uint32_t home) {
 
 int push_params(psim_ctx* c) {
     c->k.p = c->params;
-    c->graph_dirty = true;
+    c->graphs_stale();
     c->clock_valid = false;
     return 0;
 }

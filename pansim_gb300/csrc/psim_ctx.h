@@ -53,10 +53,15 @@ struct psim_ctx {
     // host copies of the per-day clock
     DevClock h_clock{};
     bool clock_valid = false;
-    // graph of the steps of one day
-    cudaGraphExec_t day_graph = nullptr;
-    bool graph_dirty = true;
-    uint64_t graph_kernels = 0;
+    // graph of the steps of one day (psim_run_steps), and of a whole day with
+    // its midnight phases (psim_run_day without host logic between them)
+    struct DayGraph {
+        cudaGraphExec_t exec = nullptr;
+        bool stale = true;
+        uint64_t kernels = 0;
+    };
+    DayGraph steps_graph, day_graph;
+    void graphs_stale() { steps_graph.stale = day_graph.stale = true; }
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
     uint64_t launches = 0;

@@ -224,6 +224,8 @@ struct DevLocs {
                                   // [6] the stamp of the last segment of draws (counts segments
                                   //     over the context's lifetime, so a replayed day never meets
                                   //     its own stamps)
+                                  // [7] nonzero: the plan flagged a home with a child to stay
+                                  //     with
 };
 
 // Incremental CSR: at most steps of a day no agent moves, and then the
@@ -334,7 +336,13 @@ enum {
     SC_INFV = 40           // ever infected per variant, 7 slots (ends at 47)
 };
 
+// Midnight timestamp of the phases captured in the whole-day graph: the
+// device clock's (kernels: midnight_of).
+constexpr uint32_t CLOCK_T = NONE;
+
 #if defined(__CUDACC__)
+__device__ __forceinline__ uint32_t midnight_of(const KArgs& k, uint32_t t) { return t == CLOCK_T ? k.clock->t0 : t; }
+
 // The first scan kernel of the step at timestamp t decides whether the CSR is
 // rebuilt (agents took new locations for t, or a rebuild is pending) and
 // records the decision in build[2]; its block 0 turns BUILD_PENDING into t,

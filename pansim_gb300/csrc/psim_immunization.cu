@@ -33,9 +33,10 @@ constexpr uint32_t WB_W = 0;
 __device__ __forceinline__ bool has_entry(const KArgs& k, uint32_t i, uint32_t poss_type_a, uint32_t poss_type_b,
                                           uint32_t loc_type_a, uint32_t loc_type_b, bool essential) {
     for (uint32_t q = k.a.loc_offset[i]; q < k.a.loc_offset[i + 1]; ++q) {
-        const uint32_t pt = k.a.poss_type[q];
+        const uint32_t v = k.a.poss4 ? k.a.poss4[q] : 0u;
+        const uint32_t pt = k.a.poss4 ? v >> 26 : k.a.poss_type[q];
         if (pt != poss_type_a && pt != poss_type_b) continue;
-        const uint32_t loc = k.a.poss_loc[q];
+        const uint32_t loc = k.a.poss4 ? v & 0x3FFFFFFu : k.a.poss_loc[q];
         if (essential) {
             if (k.l.essential[loc] == 1) return true;
         } else {
@@ -73,13 +74,28 @@ __device__ __forceinline__ uint32_t local_id(const KArgs& k, uint32_t i, uint32_
     return i - k.r.agent_off[*rep];
 }
 
-__global__ void k_imm_categories(KArgs k, uint32_t g, uint32_t order_value, float level) {
+// The category passes in their order (order value, then category index).
+struct CategoryPasses {
+    uint32_t n;
+    uint8_t category[PSIM_IMM_CATEGORIES], order[PSIM_IMM_CATEGORIES];
+    float level[PSIM_IMM_CATEGORIES];
+};
+// All of them in one pass over the agents: an agent without a round draws in
+// the first category it belongs to, which decides its round (a kernel per
+// category read the agents and their location lists six times over: 1.3 ms at
+// 20M agents).
+__global__ void __launch_bounds__(256) k_imm_categories(KArgs k, CategoryPasses passes) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
-        if (k.a.imm_round[i] != 0 || !in_category(k, i, g)) continue;
-        uint32_t rep;
-        const uint32_t li = local_id(k, i, &rep);
-        const double U = psim_u01_once(k.r.seed[rep], li, 0, PSIM_PHASE_IMM_CATEGORY + g);
-        k.a.imm_round[i] = U < (double)level ? (uint8_t)order_value : (uint8_t)255;
+        if (k.a.imm_round[i] != 0) continue;
+        for (uint32_t q = 0; q < passes.n; ++q) {
+            const uint32_t g = passes.category[q];
+            if (!in_category(k, i, g)) continue;
+            uint32_t rep;
+            const uint32_t li = local_id(k, i, &rep);
+            const double U = psim_u01_once(k.r.seed[rep], li, 0, PSIM_PHASE_IMM_CATEGORY + g);
+            k.a.imm_round[i] = U < (double)passes.level[q] ? passes.order[q] : (uint8_t)255;
+            if (k.a.imm_round[i] != 0) break;
+        }
     }
 }
 
@@ -346,13 +362,16 @@ int psim_immunization_init(psim_ctx* c, const psim_immunization* imm) {
     // categories: for each order value 1..10, every category carrying it in
     // index order; an agent still without a round draws once
     const unsigned grid = grid_n(c->N);
+    CategoryPasses passes{};
     for (int v = 1; v <= PSIM_IMM_CATEGORIES; ++v)
         for (uint32_t g = 0; g < PSIM_IMM_CATEGORIES; ++g)
             if (imm->order[g] == v) {
-                k_imm_categories<<<grid, 256, 0, c->stream>>>(c->k, g, (uint32_t)(uint8_t)imm->order[g],
-                                                              imm->group_level[g]);
-                c->launches += 1;
+                passes.category[passes.n] = (uint8_t)g;
+                passes.order[passes.n] = (uint8_t)v;
+                passes.level[passes.n++] = imm->group_level[g];
             }
+    k_imm_categories<<<grid, 256, 0, c->stream>>>(c->k, passes);
+    c->launches += 1;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
     return 0;

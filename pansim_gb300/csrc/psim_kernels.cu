@@ -769,6 +769,10 @@ __device__ uint32_t select_next(const ProgTables& T, size_t ti, float scaling, p
 }
 
 __global__ void __launch_bounds__(256) k_progress(KArgs k, uint32_t t, int staged) {
+    // (the whole-day graph: no progression and no tests at the first midnight)
+    const bool day = t == CLOCK_T;
+    t = midnight_of(k, t);
+    if (day && t == 0) return;
     extern __shared__ uint32_t smem[];
     const uint32_t nt = k.m.n_prog * k.m.n_states;
     ProgTables T;
@@ -856,6 +860,10 @@ __device__ __forceinline__ bool quarantine_window_ok(uint32_t qu, uint32_t t, ui
 
 // flagLocations, testingPolicies.h:64-148
 __global__ void __launch_bounds__(256) k_test_flag(KArgs k, uint32_t t) {
+    // (the whole-day graph: no progression and no tests at the first midnight)
+    const bool day = t == CLOCK_T;
+    t = midnight_of(k, t);
+    if (day && t == 0) return;
     const psim_params& p = k.p;
     const uint32_t day_steps = 24u * 60u / p.time_step;
     const uint32_t ql_steps = p.quarantine_length * 24u * 60u / p.time_step;
@@ -881,38 +889,58 @@ __global__ void __launch_bounds__(256) k_test_flag(KArgs k, uint32_t t) {
     }
 }
 
-// doTesting, testingPolicies.h:162-281
+// doTesting, testingPolicies.h:162-281.  The probability of a test is a sum of
+// terms that an agent has or has not (seven of them), so a block computes the
+// 128 sums once, in the reference's order in double, as bounds of the 53-bit
+// draw (TEST_ALWAYS above 1: no draw); an agent compares integers.  Summed and
+// compared per agent in double the kernel was bound by the FP64 pipe (950 us
+// at 20M agents).
+constexpr unsigned long long TEST_ALWAYS = ~0ull;
 __global__ void __launch_bounds__(256) k_test(KArgs k, uint32_t t) {
+    // (the whole-day graph: no progression and no tests at the first midnight)
+    const bool day = t == CLOCK_T;
+    t = midnight_of(k, t);
+    if (day && t == 0) return;
+    __shared__ unsigned long long s_limit[128];
     const psim_params& p = k.p;
     const uint32_t day_steps = 24u * 60u / p.time_step;
     const uint32_t delay_steps = p.testing_delay * 24u * 60u / p.time_step;
+    if (threadIdx.x < 128u) {
+        const uint32_t c = threadIdx.x;
+        double prob = p.t_random;
+        prob = prob + (double)(c & 1u) * p.t_home;
+        prob = prob + (double)((c >> 1) & 1u) * p.t_work;
+        prob = prob + (double)((c >> 2) & 1u) * p.t_school;
+        prob = prob + ((double)((c >> 3) & 1u) * 3.0) * p.t_school;
+        if (c & 16u) prob = prob + p.t_hospital;
+        if (c & 32u) prob = prob + p.t_nursery;
+        if (c & 64u) prob = prob + p.t_hospital;
+        s_limit[c] = prob > 1.0 ? TEST_ALWAYS : prob > 0.0 ? __double2ull_ru(prob * 9007199254740992.0) : 0ull;
+    }
+    __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
-        if (t > delay_steps && k.a.last_test[i] != NONE && k.a.last_test[i] > t - delay_steps) continue;
-        if (wb_of(k, i) == WB_D || k.a.diagnosed[i]) continue;
-        const uint32_t rep = k.a.rep[i];
+        const uint32_t last = k.a.last_test[i];
+        const bool diagnosed = k.a.diagnosed[i] != 0;
+        if (t > delay_steps && last != NONE && last > t - delay_steps) continue;
+        if (wb_of(k, i) == WB_D || diagnosed) continue;
+        const uint32_t rep = k.r.n == 1 ? 0u : k.a.rep[i];
         psim_stream rng;
         psim_stream_init(&rng, k.r.seed[rep], i - k.r.agent_off[rep], t, PSIM_PHASE_TEST);
-        uint32_t home = k.a.home[i];
-        int home_flag = (home != NONE && home < k.l.n) ? k.l.flags[home] : 0;
-        uint32_t work = find_location(k, i, p.work_type, 0, &rng);
-        int work_flag = (work != NONE && work < k.l.n) ? k.l.flags[work] : 0;
-        uint32_t school = find_location(k, i, p.school_type, 0, &rng);
-        int school_flag = 0, class_flag = 0;
+        const uint32_t home = k.a.home[i];
+        uint32_t c = home != NONE && home < k.l.n && k.l.flags[home] ? 1u : 0u;
+        const uint32_t work = find_location(k, i, p.work_type, 0, &rng);
+        const uint32_t work_type = loc_type(k, work);
+        if (work != NONE && work < k.l.n && k.l.flags[work]) c |= 2u;
+        const uint32_t school = find_location(k, i, p.school_type, 0, &rng);
         if (school != NONE && school < k.l.n) {
-            school_flag = k.l.flags[school];
-            uint32_t classroom = find_location(k, i, p.classroom_type, 0, &rng);
-            if (classroom != NONE) class_flag = 1;
+            if (k.l.flags[school]) c |= 4u;
+            if (find_location(k, i, p.classroom_type, 0, &rng) != NONE) c |= 8u;
         }
-        double prob = p.t_random;
-        prob = prob + (double)home_flag * p.t_home;
-        prob = prob + (double)work_flag * p.t_work;
-        prob = prob + (double)school_flag * p.t_school;
-        prob = prob + ((double)class_flag * 3.0) * p.t_school;
-        if (work != NONE && (loc_type(k, work) == p.doctor_type || loc_type(k, work) == p.hospital_type))
-            prob = prob + p.t_hospital;
-        if (work != NONE && loc_type(k, work) == p.nursery_type) prob = prob + p.t_nursery;
-        if (k.a.st_hospitalized_ts[i] <= t && k.a.st_hospitalized_until[i] > t) prob = prob + p.t_hospital;
-        if (prob > 1.0 || psim_u01(&rng) * 1.0 < prob) {
+        if (work != NONE && (work_type == p.doctor_type || work_type == p.hospital_type)) c |= 16u;
+        if (work != NONE && work_type == p.nursery_type) c |= 32u;
+        if (k.a.st_hospitalized_until[i] > t && k.a.st_hospitalized_ts[i] <= t) c |= 64u;
+        const unsigned long long limit = s_limit[c];
+        if (limit == TEST_ALWAYS || psim_u53(&rng) < limit) {
             k.a.last_test[i] = t;
             if (infected_of(k, i)) {
                 const uint8_t st = (uint8_t)k.a.state[i];
@@ -1007,6 +1035,7 @@ __device__ __forceinline__ void stats_flush_warp(const KArgs& k, uint32_t rep, u
 // (at least the context's); the per-lane sums take registers.
 template <int VM>
 __global__ void __launch_bounds__(256, VM > 2 ? 4 : 5) k_stats(KArgs k, uint32_t t, int with_tests) {
+    t = midnight_of(k, t);
     static_assert(SC_P2 < 17 && SC_HIST == 17 && SC_VAR == 33 && SC_INFV == 40 && PSIM_MAX_STRAINS <= 7,
                   "the flag words hold fields 0-31 and 32-46");
     __shared__ unsigned s_c[STAT_FIELDS];
@@ -1125,6 +1154,7 @@ __global__ void k_variant_active(KArgs k) {
 // planLocations, movementPolicies.h:1428-1622
 // checkSchoolQuarantine, :1285-1310 (quarantinePolicy > 3)
 __global__ void k_plan_schools(KArgs k, uint32_t t) {
+    t = midnight_of(k, t);
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < k.l.n_schools; s += gridDim.x * blockDim.x) {
         const uint32_t school = k.l.schools[s];
         if (k.l.quarantine_until[school] > t) continue;
@@ -1147,6 +1177,7 @@ __global__ void k_plan_schools(KArgs k, uint32_t t) {
 
 // resets + checkSchoolWorkQuarantine (:1188-1240)
 __global__ void __launch_bounds__(256) k_plan_agents(KArgs k, uint32_t t) {
+    t = midnight_of(k, t);
     const psim_params& p = k.p;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
         k.a.move_at[i] = t + p.curfew_end;  // stepsUntilMove = curfewEnd before step t
@@ -1180,7 +1211,9 @@ __global__ void __launch_bounds__(256) k_plan_agents(KArgs k, uint32_t t) {
 
 // clear quarantine flags, close quarantined schools/classrooms (:1571-1583)
 __global__ void __launch_bounds__(256) k_plan_locations(KArgs k, uint32_t t) {
+    t = midnight_of(k, t);
     const psim_params& p = k.p;
+    if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[7] = 0u;
     for (uint32_t l = blockIdx.x * blockDim.x + threadIdx.x; l < k.l.n; l += gridDim.x * blockDim.x) {
         k.l.no_work_loc[l] = 0u;
         if (p.quarantine_policy > 2) {
@@ -1198,6 +1231,7 @@ __global__ void __launch_bounds__(256) k_plan_locations(KArgs k, uint32_t t) {
 
 // checkUnderageAtHome, :1056-1094 (flag = 0xFFFFFFFF)
 __global__ void __launch_bounds__(256) k_plan_underage(KArgs k, uint32_t t) {
+    t = midnight_of(k, t);
     const psim_params& p = k.p;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
         if (k.a.age[i] > 14) continue;
@@ -1215,13 +1249,17 @@ __global__ void __launch_bounds__(256) k_plan_underage(KArgs k, uint32_t t) {
             flag = too_old || (school != NONE && (loc_open(k, school) == 0 || loc_closed_until(k, school) > t)) ||
                    (classroom != NONE && (loc_open(k, classroom) == 0 || loc_closed_until(k, classroom) > t));
         }
-        if (flag && home < k.l.n) k.l.no_work_loc[home] = NONE;
+        if (flag && home < k.l.n) {
+            k.l.no_work_loc[home] = NONE;
+            k.l.build[7] = 1u;
+        }
     }
 }
 
 // setNoWorkToday, :1137-1158: the lowest-id eligible adult of a flagged home
 // (the home is a first match: the agent's stream is not drawn from)
 __global__ void __launch_bounds__(256) k_plan_nowork_min(KArgs k, uint32_t t) {
+    if (!k.l.build[7]) return;  // no home is flagged
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
         const uint8_t age = k.a.age[i];
         if (!(age > 26 && age < 65)) continue;
@@ -1232,6 +1270,7 @@ __global__ void __launch_bounds__(256) k_plan_nowork_min(KArgs k, uint32_t t) {
 }
 
 __global__ void __launch_bounds__(256) k_plan_nowork_set(KArgs k, uint32_t t) {
+    if (!k.l.build[7]) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
         const uint8_t age = k.a.age[i];
         if (!(age > 26 && age < 65)) continue;

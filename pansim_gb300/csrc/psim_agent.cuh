@@ -657,9 +657,9 @@ __device__ __forceinline__ void store_slot(const KArgs& k, uint32_t pos, uint32_
 // x = k * S/n * w * season * dt), weighted by the replica's dL/dE, added to the
 // block's FP64 accumulators
 // x: the location's hazard argument k*S/n*w*season*dt for variant v; times:
-// how many timesteps made this draw with the same p
+// how many timesteps made this draw with the same p (negative: taken back)
 static __device__ __noinline__ void adjoint_terms(const KArgs& k, uint32_t i, uint32_t loc, uint32_t v, uint32_t rep, float r,
-                                           float su, float s_eff, double* s_grad, float x_f, uint32_t times) {
+                                           float su, float s_eff, double* s_grad, float x_f, int times) {
     const double g = k.adj.weight[rep] * (double)times;
     if (g == 0.0) return;
     const double x = (double)x_f;
@@ -693,7 +693,7 @@ __device__ __forceinline__ double draw_agent(const KArgs& k, uint32_t i, uint32_
         const float pf = h * s_eff;
         term_sum += pf < 1.0f ? (double)pf : 1.0;
         if (k.adj.on && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, su, s_eff, s_grad, k.l.hazard_x[(size_t)v * L + loc], 1u);
+            adjoint_terms(k, i, loc, v, rep, h, su, s_eff, s_grad, k.l.hazard_x[(size_t)v * L + loc], 1);
         const double U = psim_u01_once(seed, li, t, PSIM_PHASE_INFECT + v);
         if (U < (double)pf) {
             k.a.state[i] = (int8_t)k.m.first_infected;

@@ -242,21 +242,35 @@ __device__ void count_listed(const KArgs& k, const DayShared& sh) {
     if (threadIdx.x == 0 && sh.listed) atomicAdd(&k.prof[PROF_LISTED_AGENTS], (unsigned long long)sh.listed);
 }
 
-// expected-infection accumulation of the draws: one atomic per replica
-// present in the warp (warp-collective; rep given, not looked up)
-__device__ __forceinline__ void add_expected_rep(const KArgs& k, bool act, uint32_t rep, double term) {
-    const unsigned am = __ballot_sync(0xffffffffu, act && term != 0.0);
-    if (!(act && term != 0.0)) return;
-    const unsigned peers = __match_any_sync(am, rep);
-    const int leader = __ffs(peers) - 1;
-    unsigned rest = peers;
-    double tot = 0.0;
-    while (rest) {
-        const int src = __ffs(rest) - 1;
-        tot += __shfl_sync(peers, term, src);
-        rest &= rest - 1;
+// dst[key] += v over the warp's active lanes (a warp-collective): one sum of
+// the lanes and one atomic per key present.  Lane by lane on a few addresses
+// the FP64 atomics of shared memory (a compare-and-swap loop each) took longer
+// than the draws.
+__device__ __forceinline__ void add_by_key(double* dst, bool act, uint32_t key, double v) {
+    unsigned todo = __ballot_sync(0xffffffffu, act && v != 0.0);
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        const uint32_t one = __shfl_sync(0xffffffffu, key, src);  // (by every lane, active or not)
+        const bool mine = act && key == one;
+        double x = mine ? v : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((int)(threadIdx.x & 31u) == src) atomicAdd(&dst[key], x);
+        todo &= ~__ballot_sync(0xffffffffu, mine);
     }
-    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&k.r.expected[rep], tot);
+}
+
+// The adjoint's terms of draws at locations of replica rep (see adjoint_terms):
+// a = the sum over a lane's draws of dp/dx x, b = of r su, for agents of `band`
+// at location loc.
+__device__ __forceinline__ void add_gradient(const KArgs& k, double* s_grad, bool act, uint32_t rep, uint32_t loc,
+                                             uint32_t band, double a, double b) {
+    const double g = act ? k.adj.weight[rep] : 0.0;
+    const double kf = act ? (double)k.r.k_f[rep] : 0.0, w = act ? (double)k.l.infectiousness[loc] : 0.0;
+    const int slot = act ? k.adj.type_slot[k.l.type[loc]] : -1;
+    add_by_key(s_grad, kf != 0.0, GRAD_K, kf != 0.0 ? g * a / kf : 0.0);
+    add_by_key(s_grad + GRAD_W, slot >= 0 && w != 0.0, (uint32_t)slot, slot >= 0 && w != 0.0 ? g * a / w : 0.0);
+    add_by_key(s_grad + GRAD_SIGMA, act, band, g * b);
 }
 
 // DynamicPPState::gotInfected (dynamicPPState.cpp:235-244) and the agent's
@@ -349,54 +363,77 @@ struct DrawRun {
 // phase_replay repeats that location's draws with the ratio changing as its
 // agents are infected.  At a location without such an entry the ratio
 // cannot change, so the draws compared with it were the right ones.
+//
+// SUMS: the expected infections and the adjoint's terms of all entries are
+// added here as if nobody were infected; phase_replay takes those of its
+// locations back and adds the right ones.
 template <int VC, bool SUMS>
-__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, uint32_t* n_entries,
-                           uint32_t* n_hazard) {
+__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad,
+                           uint32_t* n_entries, uint32_t* n_hazard) {
     const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
     const bool one_rep = k.r.n == 1;
     const RepConst rc0 = rep_const(k, 0);
     uint32_t entries = 0, hazard = 0;
-    for (uint32_t j = threadIdx.x; j < listed; j += blockDim.x) {
+    for (uint32_t j0 = 0; j0 < listed; j0 += blockDim.x) {  // block-uniform trips
+        const uint32_t j = j0 + threadIdx.x;
         const size_t pos = seg + j;
-        const uint32_t loc = k.l.list_loc[pos];
-        const uint32_t i = k.l.list_agent[pos];
-        const float su0 = k.l.list_su[pos];
-        if (loc >= L || i >= N) {
+        bool act = j < listed;
+        if (!SUMS && !act) break;
+        const uint32_t loc = act ? k.l.list_loc[pos] : NONE;
+        const uint32_t i = act ? k.l.list_agent[pos] : NONE;
+        const float su0 = act ? k.l.list_su[pos] : 0.0f;
+        if (act && (loc >= L || i >= N)) {
             raise_error(k, ERR_AGENT_LIST);
-            continue;
+            act = false;
         }
-        const uint32_t cnt = k.l.counts[loc];
-        const float wl = k.l.infectiousness[loc];
-        const uint32_t rep = one_rep ? 0u : k.l.rep[loc];
-        const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
-        bool any_h = false, hit = false;
-        for (uint32_t v = 0; v < V && !hit; ++v) {
-            float x;
-            const float h = entry_hazard(k, loc, v, cnt, wl, rc.kf, dr.season, dt, &x);
-            if (!(h > 0.0f)) continue;
-            any_h = true;
-            if (!k.r.variant_active[rep * V + v]) continue;
-            const float s_eff = v == 0 ? su0 : k.l.list_su[v * k.l.list_cap + pos];
-            if (!(s_eff > 0.0f)) continue;
-            const unsigned long long limit = u01_limit(h * s_eff);
-            const uint32_t li = i - rc.off;
+        uint32_t rep = 0;
+        double term = 0.0, ga = 0.0, gb = 0.0;
+        if (act) {
+            const uint32_t cnt = k.l.counts[loc];
+            const float wl = k.l.infectiousness[loc];
+            rep = one_rep ? 0u : k.l.rep[loc];
+            const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
+            bool any_h = false, hit = false;
+            for (uint32_t v = 0; v < V && (SUMS || !hit); ++v) {
+                float x;
+                const float h = entry_hazard(k, loc, v, cnt, wl, rc.kf, dr.season, dt, &x);
+                if (!(h > 0.0f)) continue;
+                any_h = true;
+                if (!k.r.variant_active[rep * V + v]) continue;
+                const float s_eff = v == 0 ? su0 : k.l.list_su[v * k.l.list_cap + pos];
+                if (!(s_eff > 0.0f)) continue;
+                const float pf = h * s_eff;
+                const unsigned long long limit = u01_limit(pf);
+                const uint32_t li = i - rc.off;
 #pragma unroll 1
-            for (uint32_t q = 0; q < dr.n; ++q) {
-                const psim_ctr4 o = infect_words(rc.seed, li, dr.t + q, v);
-                hit |= u01_below(o.v[0], o.v[1], limit);
+                for (uint32_t q = 0; q < dr.n; ++q) {
+                    const psim_ctr4 o = infect_words(rc.seed, li, dr.t + q, v);
+                    hit |= u01_below(o.v[0], o.v[1], limit);
+                }
+                if (SUMS) {
+                    if (k.track_expected) term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
+                    if (k.adj.on && pf < 1.0f) {
+                        ga += (double)dr.n * ((double)s_eff * (1.0 - (double)h) * (double)x);
+                        gb += (double)dr.n * ((double)h * (double)k.a.susceptible[(size_t)v * N + i]);
+                    }
+                }
             }
+            if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
+                const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
+                const uint32_t room = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
+                k.l.replay_cursor[loc] = room;
+                if (at < L)
+                    k.l.replay_list[at] = make_uint4(loc, room, cnt, rep);
+                else
+                    raise_error(k, ERR_AGENT_LIST);
+            }
+            entries += dr.n;
+            hazard += any_h ? dr.n : 0u;
         }
-        if (hit && atomicExch(&k.l.replay_stamp[loc], dr.epoch) != dr.epoch) {
-            const uint32_t at = atomicAdd(&k.l.bar[BAR_REPLAY], 1u);
-            const uint32_t room = atomicAdd(&k.l.bar[BAR_REPLAY_SLOTS], cnt);
-            k.l.replay_cursor[loc] = room;
-            if (at < L)
-                k.l.replay_list[at] = make_uint4(loc, room, cnt, rep);
-            else
-                raise_error(k, ERR_AGENT_LIST);
+        if (SUMS) {
+            if (k.track_expected) add_by_key(k.r.expected, act, rep, term);
+            if (k.adj.on) add_gradient(k, s_grad, act, rep, act ? loc : 0u, act ? k.a.band[i] : 0u, ga, gb);
         }
-        entries += dr.n;
-        hazard += any_h ? dr.n : 0u;
     }
     *n_entries += entries;
     *n_hazard += hazard;
@@ -414,40 +451,6 @@ __device__ __forceinline__ void phase_gather(const KArgs& k, const DrawRun& dr, 
             k.l.replay_slot[p] = make_uint2((uint32_t)(seg + j), i);
         else
             raise_error(k, ERR_AGENT_LIST);
-    }
-}
-
-// The expected infections (and the adjoint's terms) of the segment's draws at
-// the locations that are not replayed: every timestep's are the same.
-template <int VC, bool SUMS>
-__device__ void phase_expected(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
-    for (uint32_t base = 0; base < listed; base += blockDim.x) {  // block-uniform trips
-        const uint32_t j = base + threadIdx.x;
-        const size_t pos = seg + j;
-        const uint32_t loc = j < listed ? k.l.list_loc[pos] : NONE;
-        const uint32_t i = loc < L ? k.l.list_agent[pos] : NONE;
-        const bool act = loc < L && i < N && k.l.replay_stamp[loc] != dr.epoch;
-        uint32_t rep = 0;
-        double term = 0.0;
-        if (act) {
-            const uint32_t cnt = k.l.counts[loc];
-            const float wl = k.l.infectiousness[loc];
-            rep = k.l.rep[loc];
-            const float kf = k.r.k_f[rep];
-            for (uint32_t v = 0; v < V; ++v) {
-                float x;
-                const float h = entry_hazard(k, loc, v, cnt, wl, kf, dr.season, dt, &x);
-                if (!(h > 0.0f) || !k.r.variant_active[rep * V + v]) continue;
-                const float s_eff = k.l.list_su[v * k.l.list_cap + pos];
-                if (!(s_eff > 0.0f)) continue;
-                const float pf = h * s_eff;
-                term += (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
-                if ((SUMS && k.adj.on) && pf < 1.0f)
-                    adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, x, dr.n);
-            }
-        }
-        if ((SUMS && k.track_expected)) add_expected_rep(k, act, rep, term);
     }
 }
 
@@ -491,7 +494,7 @@ __device__ __forceinline__ bool draw_entry(const KArgs& k, size_t pos, uint32_t 
         const float pf = h * s_eff;
         if ((SUMS && k.track_expected)) *term += pf < 1.0f ? (double)pf : 1.0;
         if ((SUMS && k.adj.on) && pf < 1.0f)
-            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1u);
+            adjoint_terms(k, i, loc, v, rep, h, k.a.susceptible[(size_t)v * N + i], s_eff, s_grad, s_x[v], 1);
         const psim_ctr4 o = infect_words(rc.seed, i - rc.off, t, v);
         if (u01_below(o.v[0], o.v[1], u01_limit(pf))) {
             if (!infected) {
@@ -575,26 +578,34 @@ __device__ __forceinline__ void replay_registers(const KArgs& k, const DrawRun& 
             }
         }
     };
+    double ga = 0.0, gb[Q] = {0.0, 0.0};
     // the terms of `times` timesteps, of which the last infected the entries of
     // hit0, hit1 (an agent infected by a variant is not susceptible to the
     // later ones); one copy of what is rare
-    const auto add = [&](uint32_t times, uint32_t hit0, uint32_t hit1) {
+    const auto add = [&](int times, uint32_t hit0, uint32_t hit1) {
 #pragma unroll 1
         for (int e = 0; e < Q; ++e) {
             const uint32_t i = e ? id[1] : id[0], by = e ? hit1 : hit0;
 #pragma unroll
             for (int v = 0; v < VM; ++v) {
                 const float s = e ? su[1][v] : su[0][v], pf = h[v] * s;
-                const uint32_t n = times - (by && (uint32_t)v >= by ? 1u : 0u);
+                const int n = times - (by && (uint32_t)v >= by ? 1 : 0);
                 if (!(pf > 0.0f) || !n) continue;
                 if (k.track_expected) *term += (double)n * (pf < 1.0f ? (double)pf : 1.0);
-                if (k.adj.on && pf < 1.0f)
-                    adjoint_terms(k, i, r.x, v, r.w, h[v], k.a.susceptible[(size_t)v * N + i], s, s_grad, x[v], n);
+                if (k.adj.on && pf < 1.0f) {
+                    ga += (double)n * ((double)s * (1.0 - (double)h[v]) * (double)x[v]);
+                    const double b = (double)n * ((double)h[v] * (double)k.a.susceptible[(size_t)v * N + i]);
+                    if (e)
+                        gb[1] += b;
+                    else
+                        gb[0] += b;
+                }
             }
         }
     };
     bounds();
-    uint32_t since = 0;  // timesteps since the bounds changed
+    if (sums) add(-(int)dr.n, 0u, 0u);  // what phase_draw added
+    int since = 0;  // timesteps since the bounds changed
     for (uint32_t q = 0; q < dr.n; ++q) {
         uint32_t hit[Q];  // 1 + the variant that infects the entry, in the reference's order
 #pragma unroll
@@ -646,6 +657,10 @@ __device__ __forceinline__ void replay_registers(const KArgs& k, const DrawRun& 
         bounds();
     }
     if (sums && since) add(since, 0u, 0u);
+    if (SUMS && k.adj.on)
+#pragma unroll
+        for (int e = 0; e < Q; ++e)
+            add_gradient(k, s_grad, id[e] < N, r.w, r.x, id[e] < N ? k.a.band[id[e]] : 0u, e ? 0.0 : ga, gb[e]);
     if (changed) {
 #pragma unroll
         for (int v = 0; v < VM; ++v)
@@ -682,6 +697,24 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
             replay_registers<VC, SUMS, 2>(k, dr, r, wl, rc, sh.grad, &term);
         } else {
             bool stale = true;  // the ratios: at the start and after an infection
+            if (SUMS && (k.track_expected || k.adj.on)) {
+                // what phase_draw added
+                replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, sh.h[warp], sh.x[warp]);
+                for (uint32_t p = (uint32_t)lane; p < r.z; p += 32u) {
+                    const uint2 s = k.l.replay_slot[r.y + p];
+                    for (uint32_t v = 0; v < V && s.y < N; ++v) {
+                        const float h = sh.h[warp][v];
+                        if (!(h > 0.0f) || !k.r.variant_active[r.w * V + v]) continue;
+                        const float s_eff = k.l.list_su[v * k.l.list_cap + s.x], pf = h * s_eff;
+                        if (!(s_eff > 0.0f)) continue;
+                        if (k.track_expected) term -= (double)dr.n * (pf < 1.0f ? (double)pf : 1.0);
+                        if (k.adj.on && pf < 1.0f)
+                            adjoint_terms(k, s.y, r.x, v, r.w, h, k.a.susceptible[(size_t)v * N + s.y], s_eff, sh.grad,
+                                          sh.x[warp][v], -(int)dr.n);
+                    }
+                }
+                stale = false;
+            }
             for (uint32_t q = 0; q < dr.n; ++q) {
                 if (stale) replay_ratios<VC, SUMS>(k, dr, r, wl, rc.kf, sh.h[warp], sh.x[warp]);
                 bool infected = false;
@@ -697,7 +730,7 @@ __device__ void phase_replay(const KArgs& k, const DrawRun& dr, uint32_t n_repla
                 if (stale) __threadfence();  // the reductions before the sums are read again
             }
         }
-        if ((SUMS && k.track_expected)) add_expected_rep(k, true, r.w, term);
+        if ((SUMS && k.track_expected)) add_by_key(k.r.expected, true, r.w, term);
     }
 }
 
@@ -811,7 +844,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     const bool draws = (phases & PH_DRAW) != 0;
     if (draws) {
         uint32_t entries = 0, hazard = 0;
-        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, &entries, &hazard);
+        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, sh.grad, &entries, &hazard);
         if (k.prof) {
             __syncwarp();
             entries = __reduce_add_sync(0xffffffffu, entries);
@@ -827,22 +860,14 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
     if (draws) {
         const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
-        const bool expected = (SUMS && k.track_expected) || (SUMS && k.adj.on);
         if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
-        if (n_replay || expected) {
-            grad_begin(k, sh.grad);
-            if (n_replay) {
-                phase_gather(k, dr, seg, sh.listed);
-                if (!grid_barrier(k, sh)) return false;
-                phase_replay<VC, SUMS>(k, dr, n_replay, sh);
-            }
-            if (expected) phase_expected<VC, SUMS>(k, dr, seg, sh.listed, sh.grad);
-            grad_end(k, sh.grad);
-            if (decides || n_replay) {
-                // every replay before any decision and before the list is emptied
-                if (!grid_barrier(k, sh)) return false;
-                if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
-            }
+        if (n_replay) {
+            phase_gather(k, dr, seg, sh.listed);
+            if (!grid_barrier(k, sh)) return false;
+            phase_replay<VC, SUMS>(k, dr, n_replay, sh);
+            // every replay before any decision and before the list is emptied
+            if (!grid_barrier(k, sh)) return false;
+            if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
         }
     }
     prof_mark(k, tl + 4);
@@ -865,15 +890,17 @@ __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0,
         sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
         sh.cnt = 0u;
     }
+    if (SUMS) grad_begin(k, sh.grad);
     __syncthreads();
     uint32_t step = step0;
     for (;;) {
         uint32_t next = step_end;
         if (!day_segment<VC, SUMS, POL>(k, step, step_end, phases, cap, sh, &next)) return;
-        if (next >= step_end) return;
+        if (next >= step_end) break;
         step = next;
         if (!grid_barrier(k, sh)) return;
     }
+    if (SUMS) grad_end(k, sh.grad);
 }
 
 }  // namespace psim

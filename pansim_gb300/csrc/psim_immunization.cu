@@ -30,37 +30,41 @@ namespace {
 
 constexpr uint32_t WB_W = 0;
 
-__device__ __forceinline__ bool has_entry(const KArgs& k, uint32_t i, uint32_t poss_type_a, uint32_t poss_type_b,
-                                          uint32_t loc_type_a, uint32_t loc_type_b, bool essential) {
+// What the categories ask of an agent's location list (the reference's type
+// ids), in one walk over it: bit 0 it works at a hospital or doctor (12, 14),
+// 1 it works or lives in a nursery home (22), 2 at an essential location, 3
+// at a school (3).
+__device__ __forceinline__ uint32_t list_bits(const KArgs& k, uint32_t i) {
+    uint32_t bits = 0;
     for (uint32_t q = k.a.loc_offset[i]; q < k.a.loc_offset[i + 1]; ++q) {
         const uint32_t v = k.a.poss4 ? k.a.poss4[q] : 0u;
         const uint32_t pt = k.a.poss4 ? v >> 26 : k.a.poss_type[q];
-        if (pt != poss_type_a && pt != poss_type_b) continue;
+        if (pt != 4u && pt != 2u) continue;
         const uint32_t loc = k.a.poss4 ? v & 0x3FFFFFFu : k.a.poss_loc[q];
-        if (essential) {
-            if (k.l.essential[loc] == 1) return true;
-        } else {
-            const uint32_t lt = k.l.type[loc];
-            if (lt == loc_type_a || lt == loc_type_b) return true;
+        const uint32_t lt = k.l.type[loc];
+        if (lt == 22u) bits |= 2u;
+        if (pt == 4u) {
+            if (lt == 12u || lt == 14u) bits |= 1u;
+            if (lt == 3u) bits |= 8u;
+            if (k.l.essential[loc] == 1) bits |= 4u;
         }
     }
-    return false;
+    return bits;
 }
 
 // the ten categories of initCategories (immunization.h:277-375)
-__device__ bool in_category(const KArgs& k, uint32_t i, uint32_t g) {
-    const uint32_t age = k.a.age[i], pre = k.a.precond[i];
+__device__ __forceinline__ bool in_category(uint32_t g, uint32_t age, uint32_t pre, uint32_t bits) {
     switch (g) {
-        case 0: return has_entry(k, i, 4, 4, 12, 14, false);   // health workers
-        case 1: return has_entry(k, i, 4, 2, 22, 22, false);   // nursery home workers and residents
-        case 2: return pre > 0 && age >= 60;                   // 60+ with an underlying condition
-        case 3: return age >= 60;                              // 60+
-        case 4: return pre > 0 && age >= 18 && age < 60;       // 18-59 with an underlying condition
-        case 5: return has_entry(k, i, 4, 4, 0, 0, true);      // essential workers
-        case 6: return has_entry(k, i, 4, 4, 3, 3, false);     // school workers
-        case 7: return age > 17 && age < 60;                   // 18-59
-        case 8: return age >= 12 && age < 18;                  // 12-17
-        default: return age >= 5 && age < 12;                  // 5-11
+        case 0: return bits & 1u;                 // health workers
+        case 1: return bits & 2u;                 // nursery home workers and residents
+        case 2: return pre > 0 && age >= 60;      // 60+ with an underlying condition
+        case 3: return age >= 60;                 // 60+
+        case 4: return pre > 0 && age >= 18 && age < 60;  // 18-59 with an underlying condition
+        case 5: return bits & 4u;                 // essential workers
+        case 6: return bits & 8u;                 // school workers
+        case 7: return age > 17 && age < 60;      // 18-59
+        case 8: return age >= 12 && age < 18;     // 12-17
+        default: return age >= 5 && age < 12;     // 5-11
     }
 }
 
@@ -87,9 +91,10 @@ struct CategoryPasses {
 __global__ void __launch_bounds__(256) k_imm_categories(KArgs k, CategoryPasses passes) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k.a.n; i += gridDim.x * blockDim.x) {
         if (k.a.imm_round[i] != 0) continue;
+        const uint32_t age = k.a.age[i], pre = k.a.precond[i], bits = list_bits(k, i);
         for (uint32_t q = 0; q < passes.n; ++q) {
             const uint32_t g = passes.category[q];
-            if (!in_category(k, i, g)) continue;
+            if (!in_category(g, age, pre, bits)) continue;
             uint32_t rep;
             const uint32_t li = local_id(k, i, &rep);
             const double U = psim_u01_once(k.r.seed[rep], li, 0, PSIM_PHASE_IMM_CATEGORY + g);

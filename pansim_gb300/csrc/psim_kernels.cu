@@ -1186,19 +1186,30 @@ __global__ void __launch_bounds__(256) k_plan_agents(KArgs k, uint32_t t) {
         if (p.quarantine_policy > 2) {
             if (k.a.quarantined[i]) continue;
             if (k.a.st_diagnosed_ts[i] > 0 && !infected_of(k, i)) continue;
-            const uint32_t rep = k.a.rep[i];
-            psim_stream rng;
-            psim_stream_init(&rng, k.r.seed[rep], i - k.r.agent_off[rep], t, PSIM_PHASE_PLAN_SWQ);
-            const uint32_t work = find_location3(k, i, p.work_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
-            const uint32_t school = find_location3(k, i, p.school_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
-            const uint32_t classroom = find_location3(k, i, p.classroom_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
-            uint32_t until = 0;
-            if (school != NONE && loc_qu(k, school) > t)
-                until = loc_qu(k, school);
-            else if (classroom != NONE && loc_qu(k, classroom) > t)
-                until = loc_qu(k, classroom);
-            else if (work != NONE && loc_qu(k, work) > t)
-                until = loc_qu(k, work);
+            // the agent's work, school and classroom: by its list's layout
+            // where no draw decides (their entries and then their quarantine
+            // ends load together), else one after another
+            uint32_t work, school, classroom;
+            const uint32_t layout = k.a.layout[i], lb = k.a.loc_offset[i];
+            const uint16_t* row = k.m.layout + layout * LAYOUT_TYPES;
+            const bool rows = layout && p.work_type < LAYOUT_TYPES && p.school_type < LAYOUT_TYPES &&
+                              p.classroom_type < LAYOUT_TYPES;
+            const uint32_t ew = rows ? row[p.work_type] : 0u, es = rows ? row[p.school_type] : 0u,
+                           ec = rows ? row[p.classroom_type] : 0u;
+            if (rows && ew < 0x200u) {
+                work = ew ? k.a.poss4[lb + (ew & 0xFFu)] & 0x3FFFFFFu : NONE;
+                school = es ? k.a.poss4[lb + (es & 0xFFu)] & 0x3FFFFFFu : NONE;
+                classroom = ec ? k.a.poss4[lb + (ec & 0xFFu)] & 0x3FFFFFFu : NONE;
+            } else {
+                const uint32_t rep = k.a.rep[i];
+                psim_stream rng;
+                psim_stream_init(&rng, k.r.seed[rep], i - k.r.agent_off[rep], t, PSIM_PHASE_PLAN_SWQ);
+                work = find_location3(k, i, p.work_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
+                school = find_location3(k, i, p.school_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
+                classroom = find_location3(k, i, p.classroom_type, 0, &rng, p.home_type, p.school_type, p.classroom_type);
+            }
+            const uint32_t qs = loc_qu(k, school), qc = loc_qu(k, classroom), qw = loc_qu(k, work);
+            const uint32_t until = qs > t ? qs : qc > t ? qc : qw > t ? qw : 0u;
             if (until > 0) {
                 k.a.quarantined[i] = 1;
                 k.a.st_quarantined_ts[i] = t;
@@ -1316,7 +1327,9 @@ __global__ void k_layouts(KArgs k, uint32_t* owner) {
             }
             for (uint32_t probe = 0; runs && probe < 16u && !layout; ++probe) {
                 const uint32_t row = 1u + (hash + probe) % (LAYOUTS - 1u);
-                const uint32_t prev = atomicCAS(&owner[row], 0u, i + 1u);
+                // (looked at before the exchange: millions of agents share a row)
+                uint32_t prev = *(volatile uint32_t*)&owner[row];
+                if (!prev) prev = atomicCAS(&owner[row], 0u, i + 1u);
                 bool same = prev == 0u;
                 if (!same) {
                     const uint32_t ob = k.a.loc_offset[prev - 1u];

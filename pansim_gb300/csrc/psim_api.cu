@@ -304,10 +304,12 @@ int initial_regroup(psim_ctx* c) {
     CK(cudaMemsetAsync(c->k.l.counts, 0, sizeof(uint32_t) * c->L, c->stream));
     if ((rc0 = reset_sums(c))) return rc0;
     launch_count(c->k, c->stream);
-    launch_scan(c->k, 0, 1, 0, c->stream);
+    launch_scan(c->k, 0, 1, 0, false, c->stream);
     launch_scatter(c->k, 0, false, c->stream);
     c->list_sparse = false;
     c->csr_full = true;
+    c->sums_zero = true;
+    c->moved = false;
     // the variant gating of the first steps (the statistics come at midnight)
     launch_variant_flags(c->k, c->stream);
     c->launches += 3 + (uint64_t)scan_kernels(c->k);
@@ -322,14 +324,20 @@ int do_step(psim_ctx* c, uint32_t step) {
         int rc = force_rebuild(c);
         if (rc) return rc;
     }
+    if (!c->sums_zero) {
+        int rc = reset_sums(c);
+        if (rc) return rc;
+    }
     launch_phase_movement(c->k, step, c->stream);
     const bool merge = c->params.quarantine_policy > 1;
-    launch_scan(c->k, step, 1, merge, c->stream);
+    launch_scan(c->k, step, 1, merge, false, c->stream);
     launch_scatter(c->k, step, merge, c->stream);
+    c->sums_zero = true;
     launch_phase_draw(c->k, step, c->stream);
-    c->launches += 4 + (uint64_t)scan_kernels(c->k);
+    c->launches += 3 + (uint64_t)scan_kernels(c->k);
     c->list_sparse = false;
     c->csr_full = true;
+    c->moved = false;
     return launch_check(c);
 }
 
@@ -819,6 +827,7 @@ int psim_create(int device, const psim_model* m, const psim_agents* a, const psi
         c->h_expected = (double*)(p + b_stats);
         c->h_clock_pin = (DevClock*)(p + b_stats + b_exp);
         c->k.err_host = (uint32_t*)(p + b_stats + b_exp + sizeof(DevClock) + 32);
+        c->k.moved_host = c->k.err_host + 1;
     }
     // healthcare workers per replica (Simulation::flagHealthcareWorkers, simulation.h:670-693)
     c->hcw_count.assign(R, 0u);
@@ -1073,6 +1082,7 @@ int psim_checkpoint_restore(psim_ctx* c, uint32_t slot) {
     CK(cudaMemsetAsync(c->k.l.smask, 0xFF, sizeof(uint32_t) * (((size_t)c->L + 2047) / 2048 * 64 + 64), c->stream));
     c->csr_full = false;
     c->list_sparse = true;
+    c->sums_zero = false;
     CK(cudaStreamSynchronize(c->stream));
     c->csr_fresh = false;
     return 0;
@@ -1114,19 +1124,25 @@ int psim_movement(psim_ctx* c, uint32_t t) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     int rc = set_clock(c, t);
     if (rc) return rc;
+    if (!c->sums_zero && (rc = reset_sums(c))) return rc;
+    *(volatile uint32_t*)c->k.moved_host = 0u;
     launch_phase_movement(c->k, t % c->spd, c->stream);
-    c->launches += 2;
+    c->launches += 1;
     c->csr_fresh = true;
+    c->sums_zero = false;
     c->t_next = t + 1;
     rc = launch_check(c);
     if (rc) return rc;
-    return check_device_err(c);
+    rc = check_device_err(c);
+    if (*(volatile uint32_t*)c->k.moved_host) c->moved = true;
+    return rc;
 }
 
 int psim_regroup(psim_ctx* c) {
     if (!c || !c->uploaded) return PSIM_ERR_STATE;
     // the list of the last regroup serves when nobody has moved since
     int rc0 = 0;
+    const bool keep = c->csr_full && c->csr_fresh && !c->moved;
     if (!(c->csr_full && c->csr_fresh) && (rc0 = force_rebuild(c))) return rc0;
     if (!c->csr_fresh) {
         CK(cudaMemsetAsync(c->k.l.counts, 0, sizeof(uint32_t) * c->L, c->stream));
@@ -1138,12 +1154,15 @@ int psim_regroup(psim_ctx* c) {
     const uint32_t since = c->t_next - 1u - c->h_clock.t0;
     const uint32_t step = c->csr_fresh && since < c->spd ? since : 0u;
     const bool merge = c->params.quarantine_policy > 1;
-    launch_scan(c->k, step, 1, merge, c->stream);
-    launch_scatter(c->k, step, merge, c->stream);
-    c->launches += 1 + (uint64_t)scan_kernels(c->k);
+    launch_scan(c->k, step, 1, merge, keep, c->stream);
+    // (nobody moved: there is nothing to scatter)
+    if (!keep) launch_scatter(c->k, step, merge, c->stream);
+    c->launches += (keep ? 0 : 1) + (uint64_t)scan_kernels(c->k);
     c->csr_fresh = false;
     c->list_sparse = false;
     c->csr_full = true;
+    c->moved = false;
+    c->sums_zero = true;
     int rc = launch_check(c);
     if (rc) return rc;
     return check_device_err(c);
@@ -1269,6 +1288,7 @@ int psim_run_steps(psim_ctx* c, uint32_t day) {
     c->csr_fresh = false;
     c->list_sparse = true;
     c->csr_full = false;
+    c->sums_zero = false;
     c->t_next = (day + 1) * c->spd;
     return check_device_err(c);
 }
@@ -1299,6 +1319,7 @@ int psim_run_day(psim_ctx* c, uint32_t day, psim_day_stats* out) {
     c->csr_fresh = false;
     c->list_sparse = true;
     c->csr_full = false;
+    c->sums_zero = false;
     c->t_next = (day + 1) * c->spd;
     if (*(volatile uint32_t*)c->k.err_host) return check_device_err(c);
     if (out) assemble_stats(c, t, out);
@@ -1314,7 +1335,7 @@ int psim_get_csr(psim_ctx* c, int canonical, uint32_t* offsets, uint32_t* agents
         // step rebuilds)
         int rc = force_rebuild(c);
         if (rc) return rc;
-        launch_scan(c->k, 0, 0, 0, c->stream);
+        launch_scan(c->k, 0, 0, 0, false, c->stream);
         launch_scatter(c->k, 0, false, c->stream);
         c->launches += 1 + (uint64_t)scan_kernels(c->k);
         c->list_sparse = false;
@@ -1498,6 +1519,7 @@ int psim_time_step_kernels(psim_ctx* c, uint32_t t, float* ms) {
     c->csr_fresh = false;
     c->list_sparse = true;
     c->csr_full = false;
+    c->sums_zero = false;
     c->t_next = t + 2;
     rc = launch_check(c);
     if (rc) return rc;

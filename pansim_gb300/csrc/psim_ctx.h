@@ -69,6 +69,8 @@ struct psim_ctx {
     bool csr_fresh = false;      // counts of the current positions are built
     bool csr_full = false;       // the agent list is that of the last regroup; movements since then
                                  // that moved somebody have marked it (build[1])
+    bool moved = false;          // a movement since the last regroup moved somebody
+    bool sums_zero = false;      // the sums were used and zeroed by a scan, nothing was added since
     bool list_sparse = false;    // the agent list holds only the locations the day kernel's
                                  // last rebuild listed (psim_get_csr builds the full one)
     // pinned host memory (one block): the statistics accumulators and the

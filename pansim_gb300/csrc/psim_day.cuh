@@ -65,6 +65,7 @@ struct DayShared {
     uint32_t mm[MOVE_MASK_WORDS];
     uint32_t red[32];
     uint32_t target;  // the barrier count the next barrier waits for
+    bool cluster;     // the grid is one cluster
     uint32_t cnt;     // agents in the block's work list
     uint32_t listed;  // entries of the block's agent list
     bool ok;
@@ -887,6 +888,7 @@ __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0,
     if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
     if (threadIdx.x == 0) {
         sh.target = gridDim.x;
+        sh.cluster = (phases & PH_CLUSTER) != 0;
         sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
         sh.cnt = 0u;
     }

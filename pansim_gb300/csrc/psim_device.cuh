@@ -318,6 +318,7 @@ struct KArgs {
     DevClock* clock;
     uint32_t* err;
     uint32_t* err_host;   // nonzero after an error (host memory, read after a wait for the stream)
+    uint32_t* moved_host; // set by a per-phase movement that moved somebody (host memory too)
     DevStatsAcc* stats;   // [R]
     uint32_t spd;         // steps per day
     uint32_t hour_steps, half_hour_steps;  // 60 and 30 minutes in steps (rounded down)
@@ -392,11 +393,13 @@ __device__ __forceinline__ void update_meta(const KArgs& k, uint32_t i) {
 void launch_day_begin(const KArgs& k, cudaStream_t s);
 // the day's first step, before the day kernel
 void launch_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
-// a step of the per-phase entry points, the sums afresh
+// a step of the per-phase entry points (the sums are zero)
 void launch_phase_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
 void launch_count(const KArgs& k, cudaStream_t s);
 // merge_quarantine: the location quarantines that decisions wrote since the last merge
-void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merge_quarantine, cudaStream_t s);
+// keep: the agent list stands, only the ratios
+void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merge_quarantine, bool keep,
+                 cudaStream_t s);
 // merged: the scan before merged the location quarantines
 void launch_scatter(const KArgs& k, uint32_t step_in_day, bool merged, cudaStream_t s);
 void launch_phase_draw(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
@@ -406,6 +409,7 @@ int scan_kernels(const KArgs& k);
 // the day kernel (psim_kernels.cu, k_day): the phases a launch runs, for the
 // timesteps step0 .. step_end - 1 of the day
 constexpr uint32_t PH_REBUILD = 1u, PH_DRAW = 2u, PH_DECIDE = 4u, PH_ALL = 7u;
+constexpr uint32_t PH_CLUSTER = 8u;  // (set by launch_day) the grid is one cluster
 typedef void (*DayKernel)(KArgs, uint32_t, uint32_t, uint32_t, uint32_t);
 constexpr uint32_t DAY_THREADS = 512;  // two blocks per SM at 64 registers
 // the day kernel's instances: one variant without sums and its policies, one

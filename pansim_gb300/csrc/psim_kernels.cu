@@ -67,7 +67,8 @@ __global__ void __launch_bounds__(256) k_movement(KArgs k, uint32_t step) {
     prof_mark(k, PROF_N + 1);
 }
 
-// The same for a step of the per-phase entry points (psim_movement): most
+// The same for a step of the per-phase entry points (psim_movement; the sums
+// are zero, the scan of the step before zeroed them): most
 // agents count down and are not infectious, so a thread reads three words of
 // four agents each (16-byte loads); the block's deciders are collected and
 // decide together, full warps of them.
@@ -136,22 +137,7 @@ __global__ void __launch_bounds__(PHASE_THREADS) k_phase_movement(KArgs k, uint3
     if (__syncthreads_or(moved) && threadIdx.x == 0) {
         k.l.build[0] = c.t;
         k.l.build[1] = BUILD_PENDING;
-    }
-}
-
-// The sums afresh before a step of the per-phase entry points: zeroed where
-// the masks say that one may be nonzero (every kernel that adds a term marks
-// its location), and those locations dirty for the scan.
-__global__ void __launch_bounds__(256) k_reset_sums(KArgs k) {
-    const uint32_t L = k.l.n, V = k.m.n_variants;
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < (L + 31u) >> 5; w += gridDim.x * blockDim.x) {
-        const uint32_t sm = k.l.smask[w], m = sm | k.l.hmask[w];
-        if (m != sm) k.l.smask[w] = m;
-        for (uint32_t rest = m; rest; rest &= rest - 1u) {
-            const uint32_t l = w * 32u + (uint32_t)(__ffs(rest) - 1);
-            if (l < L)
-                for (uint32_t v = 0; v < V; ++v) k.l.sfix[(size_t)v * L + l] = 0ull;
-        }
+        *(volatile uint32_t*)k.moved_host = 1u;
     }
 }
 
@@ -311,6 +297,9 @@ __device__ __forceinline__ uint32_t scan_lookback(const KArgs& k, uint32_t tile,
     return prefix;
 }
 
+// with_hazard: 1 the ratios, and SCAN_KEEP where the caller knows that the
+// agent list stands.
+constexpr int SCAN_KEEP = 2;
 template <int ITEMS, bool LOOKBACK>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, int with_hazard, int merge_q) {
     constexpr int TILE = SCAN_THREADS * ITEMS;
@@ -324,7 +313,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
     // rebuild no ticket is taken and the cursors keep the ends of the step
     // before (no prefix, no cursor writes).
     const uint32_t t_step = k.clock->t0 + step;
-    const bool rebuild = LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step);
+    const bool rebuild = !(with_hazard & SCAN_KEEP) && (LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step));
     // merge_q: the location quarantines are merged if decisions wrote some
     merge_q = merge_q && k.l.build[4] != 0u;
     if (!rebuild && !with_hazard && !merge_q) return;
@@ -392,10 +381,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
     const float season = k.clock->season;
     const uint32_t V = k.m.n_variants;
     if (with_hazard) {
-        // only the locations marked dirty (their sum or, with a nonzero sum,
-        // their count changed) are read; their hazards are recomputed from
-        // the persistent sums and their hazard-mask bits (sum nonzero)
-        // rewritten.  Elsewhere hazards and mask bits stay as they are.
+        // only the locations marked dirty (a term was added, or the ratio of
+        // the scan before is not zero) are read; their hazards are computed
+        // from the sums, which are zeroed for the next movement, and their
+        // hazard-mask bits (sum nonzero) rewritten.  Those stay dirty: their
+        // ratios change with the next movement's sums.  Elsewhere hazards and
+        // mask bits stay as they are.
         uint32_t sws[ITEMS];
 #pragma unroll
         for (int q = 0; q < ITEMS; ++q) sws[q] = k.l.smask[(wbase + q * 32) >> 5];
@@ -418,6 +409,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
                     if (fix != 0) {
                         h = psim_hazard_x(fix, c[q], k_f, w_l, season, dt, &x);
                         nz = true;
+                        k.l.sfix[idx] = 0ull;
                     }
                     k.l.hazard[idx] = h;
                     if (k.adj.on) k.l.hazard_x[idx] = x;
@@ -425,10 +417,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
             }
             // one word per 32 locations (wbase is a multiple of 32)
             const unsigned nzw = __ballot_sync(0xffffffffu, nz);
-            if (lane == 0) {
-                k.l.hmask[wi] = (k.l.hmask[wi] & ~sw) | nzw;
-                k.l.smask[wi] = 0u;
-            }
+            if (lane == 0) k.l.smask[wi] = k.l.hmask[wi] = (k.l.hmask[wi] & ~sw) | nzw;
         }
     }
     if (merge_q) {
@@ -497,7 +486,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
     // without a rebuild the cursors keep the ends of the step before, and
     // the counts are read at the flagged locations only
     const uint32_t t_step = k.clock->t0 + step;
-    const bool rebuild = LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step);
+    const bool rebuild = !(with_hazard & SCAN_KEEP) && (LOOKBACK ? csr_decide(k, t_step) : csr_rebuild(k, t_step));
     merge_q = merge_q && k.l.build[4] != 0u;
     if (!rebuild && !with_hazard && !merge_q) return;
     uint32_t tile = blockIdx.x;
@@ -586,6 +575,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
                     if (fix != 0) {
                         h = psim_hazard_x(fix, n_l, k_f, w_l, season, dt, &xx);
                         nzb |= 1u << ((l0 & 31u) + e);
+                        k.l.sfix[idx] = 0ull;
                     }
                     k.l.hazard[idx] = h;
                     if (k.adj.on) k.l.hazard_x[idx] = xx;
@@ -595,10 +585,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
         // the word's bits from the 32 / PER consecutive threads that share it
 #pragma unroll
         for (int o = 1; o < 32 / PER; o <<= 1) nzb |= __shfl_xor_sync(0xffffffffu, nzb, o);
-        if ((l0 & 31u) == 0u && sw) {
-            k.l.hmask[wi] = (k.l.hmask[wi] & ~sw) | nzb;
-            k.l.smask[wi] = 0u;
-        }
+        if ((l0 & 31u) == 0u && sw) k.l.smask[wi] = k.l.hmask[wi] = (k.l.hmask[wi] & ~sw) | nzb;
     }
     if (merge_q) {
 #pragma unroll
@@ -1486,7 +1473,6 @@ static unsigned quad_grid(uint32_t n, unsigned wave) { return std::min(wave, gri
 void launch_phase_movement(const KArgs& k, uint32_t step, cudaStream_t s) {
     static unsigned g = 0;
     if (!g) g = wave_grid(k_phase_movement, 1u << 30);
-    k_reset_sums<<<grid_for((k.l.n + 31u) / 32u, 8), 256, 0, s>>>(k);
     k_phase_movement<<<quad_grid(k.a.n, g), PHASE_THREADS, 0, s>>>(k, step);
 }
 void launch_day_begin(const KArgs& k, cudaStream_t s) { k_day_begin<<<grid_for(k.l.n, 8), 256, 0, s>>>(k); }
@@ -1513,31 +1499,68 @@ static DayKernel day_kernel(const KArgs& k, unsigned* per_sm) {
     *per_sm = (unsigned)occ[q];
     return f;
 }
-static void day_geometry(const KArgs& k, unsigned occ, unsigned* grid, uint32_t* cap) {
+// blocks: the grid, or 0 for as many as fit
+static void day_geometry(const KArgs& k, unsigned occ, unsigned blocks, unsigned* grid, uint32_t* cap) {
     const unsigned bps = k.tune.blocks_per_sm
                              ? std::min<unsigned>((k.tune.blocks_per_sm * 256u + DAY_THREADS - 1) / DAY_THREADS, occ)
                              : occ;
     const size_t want = ((size_t)k.a.n + DAY_THREADS - 1) / DAY_THREADS;
     unsigned g = (unsigned)std::min<size_t>((size_t)sm_count() * bps, std::max<size_t>(want, 1));
     g = std::min(g, (unsigned)(WORK_MAX_THREADS / DAY_THREADS));
+    if (blocks) g = blocks;
     *grid = g;
     // the queue's quads: ceil(quads / (g * threads)) per thread, 4 agents each
     const size_t quads = ((size_t)k.a.n + 3) / 4, threads = (size_t)g * DAY_THREADS;
     *cap = (uint32_t)(((quads + threads - 1) / threads) * DAY_THREADS * 4);
+}
+// Up to CLUSTER_AGENTS agents one cluster of at most 16 blocks runs the day: a
+// barrier of the cluster takes 0.24 us where one of the grid takes 1.15 (at 20
+// blocks), and a day of 10k agents has some eighty.  Above, more blocks than a
+// cluster holds are worth more than the faster barrier.
+constexpr uint32_t CLUSTER_BLOCKS = 16, CLUSTER_AGENTS = 16384;
+static bool cluster_fits(DayKernel kernel, unsigned blocks) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(DAY_THREADS);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return n > 0;
 }
 void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s) {
     unsigned g;
     uint32_t cap;
     unsigned occ;
     const DayKernel kernel = day_kernel(k, &occ);
-    day_geometry(k, occ, &g, &cap);
+    const unsigned few = std::min(CLUSTER_BLOCKS, (k.a.n + DAY_THREADS - 1) / DAY_THREADS);
+    const bool cluster = k.a.n <= CLUSTER_AGENTS && cluster_fits(kernel, few);
+    day_geometry(k, occ, cluster ? few : 0u, &g, &cap);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g);
     cfg.blockDim = dim3(DAY_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
+    if (cluster) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = g;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        phases |= PH_CLUSTER;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, k, step0, step_end, phases, cap);
@@ -1557,7 +1580,7 @@ static void launch_scan_items(const KArgs& k, uint32_t step, int with_hazard, in
         if (k.tune.scan_mode == 3) {
             k_scan_v<Q, true><<<tiles, SCAN_THREADS, 0, s>>>(k, step, with_hazard, merge_q);
         } else {
-            k_tile_sums_v<Q><<<tiles, SCAN_THREADS, 0, s>>>(k, step);
+            if (!(with_hazard & SCAN_KEEP)) k_tile_sums_v<Q><<<tiles, SCAN_THREADS, 0, s>>>(k, step);
             k_scan_v<Q, false><<<tiles, SCAN_THREADS, 0, s>>>(k, step, with_hazard, merge_q);
         }
         return;
@@ -1565,13 +1588,14 @@ static void launch_scan_items(const KArgs& k, uint32_t step, int with_hazard, in
     if (k.tune.scan_mode == 0 || k.tune.scan_mode == 3) {
         k_scan<ITEMS, true><<<tiles, SCAN_THREADS, 0, s>>>(k, step, with_hazard, merge_q);
     } else {
-        k_tile_sums<ITEMS><<<tiles, SCAN_THREADS, 0, s>>>(k, step);
+        if (!(with_hazard & SCAN_KEEP)) k_tile_sums<ITEMS><<<tiles, SCAN_THREADS, 0, s>>>(k, step);
         k_scan<ITEMS, false><<<tiles, SCAN_THREADS, 0, s>>>(k, step, with_hazard, merge_q);
     }
 }
 // step: the step in the day whose CSR the scan prepares (rebuilt only when
 // agents took new locations for it, see csr_decide)
-void launch_scan(const KArgs& k, uint32_t step, int with_hazard, int merge_q, cudaStream_t s) {
+void launch_scan(const KArgs& k, uint32_t step, int with_hazard, int merge_q, bool keep, cudaStream_t s) {
+    if (keep) with_hazard |= SCAN_KEEP;
     if (k.tune.scan_items == 2)
         launch_scan_items<2>(k, step, with_hazard, merge_q, s);
     else if (k.tune.scan_items == 4)

@@ -14,8 +14,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libpansim_gb300.so")
-SOURCES = ["psim_kernels.cu", "psim_day_a.cu", "psim_day_b.cu", "psim_day_c.cu", "psim_api.cu", "psim_closures.cu",
-           "psim_immunization.cu", "psim_other_disease.cu", "psim_noalloc.cu"]
+SOURCES = ["psim_kernels.cu", "psim_day_a.cu", "psim_day_b.cu", "psim_day_c.cu", "psim_day_d.cu", "psim_api.cu",
+           "psim_closures.cu", "psim_immunization.cu", "psim_other_disease.cu", "psim_noalloc.cu"]
 # every header of csrc/: a change to any of them rebuilds every object
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".h", ".cuh")))
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

@@ -47,6 +47,8 @@ namespace psim {
 // writes reach the other blocks through the arrival (release: the block's
 // threads' writes are ordered before it by the __syncthreads before) and the
 // count's read (acquire).
+//
+// CLUSTER: the grid is one cluster (launch_day) and its hardware barrier does.
 constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
     uint32_t v;
@@ -65,13 +67,17 @@ struct DayShared {
     uint32_t mm[MOVE_MASK_WORDS];
     uint32_t red[32];
     uint32_t target;  // the barrier count the next barrier waits for
-    bool cluster;     // the grid is one cluster
     uint32_t cnt;     // agents in the block's work list
     uint32_t listed;  // entries of the block's agent list
     bool ok;
 };
 
+template <bool CLUSTER>
 __device__ __forceinline__ bool grid_barrier(const KArgs& k, DayShared& sh) {
+    if (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         const uint32_t target = sh.target;
@@ -793,7 +799,7 @@ __device__ void phase_decide(const KArgs& k, uint32_t s1, uint32_t cap, uint32_t
 // `step`; *next receives the timestep the next one starts at (step_end after
 // the last).  False when a grid barrier expired (the kernel then ends).  cap =
 // the work-list segment size of a block.
-template <int VC, bool SUMS, int POL>
+template <int VC, bool SUMS, int POL, bool CLUSTER>
 __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint32_t step_end, uint32_t phases,
                                             uint32_t cap, DayShared& sh, uint32_t* next) {
     const uint32_t tl = PROF_T + PROF_TW * step;  // the segment's timeline slots (profiled graph)
@@ -858,16 +864,16 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     }
     prof_mark(k, tl + 3);
     // every draw before any replay, every draw and merge before any decision
-    if ((draws || (merge && decides)) && !grid_barrier(k, sh)) return false;
+    if ((draws || (merge && decides)) && !grid_barrier<CLUSTER>(k, sh)) return false;
     if (draws) {
         const uint32_t n_replay = min(k.l.bar[BAR_REPLAY], k.l.n);
         if (blockIdx.x == 0 && threadIdx.x == 0) k.l.build[6] = dr.epoch;
         if (n_replay) {
             phase_gather(k, dr, seg, sh.listed);
-            if (!grid_barrier(k, sh)) return false;
+            if (!grid_barrier<CLUSTER>(k, sh)) return false;
             phase_replay<VC, SUMS>(k, dr, n_replay, sh);
             // every replay before any decision and before the list is emptied
-            if (!grid_barrier(k, sh)) return false;
+            if (!grid_barrier<CLUSTER>(k, sh)) return false;
             if (blockIdx.x == 0 && threadIdx.x == 0) k.l.bar[BAR_REPLAY] = k.l.bar[BAR_REPLAY_SLOTS] = 0u;
         }
     }
@@ -881,14 +887,13 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
 }
 
 // The day kernel: timesteps step0 .. step_end - 1.
-template <int VC, bool SUMS, int POL>
+template <int VC, bool SUMS, int POL, bool CLUSTER = false>
 __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0, uint32_t step_end, uint32_t phases,
                                                         uint32_t cap) {
     __shared__ DayShared sh;
     if (*((volatile uint32_t*)k.err) & ERR_BARRIER) return;  // an earlier barrier expired
     if (threadIdx.x == 0) {
         sh.target = gridDim.x;
-        sh.cluster = (phases & PH_CLUSTER) != 0;
         sh.listed = min(k.l.list_count[blockIdx.x], cap);  // an earlier launch's list, if this one draws from it
         sh.cnt = 0u;
     }
@@ -897,10 +902,10 @@ __global__ void __launch_bounds__(DAY_THREADS, 2) k_day(KArgs k, uint32_t step0,
     uint32_t step = step0;
     for (;;) {
         uint32_t next = step_end;
-        if (!day_segment<VC, SUMS, POL>(k, step, step_end, phases, cap, sh, &next)) return;
+        if (!day_segment<VC, SUMS, POL, CLUSTER>(k, step, step_end, phases, cap, sh, &next)) return;
         if (next >= step_end) break;
         step = next;
-        if (!grid_barrier(k, sh)) return;
+        if (!grid_barrier<CLUSTER>(k, sh)) return;
     }
     if (SUMS) grad_end(k, sh.grad);
 }

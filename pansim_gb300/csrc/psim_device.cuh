@@ -409,7 +409,6 @@ int scan_kernels(const KArgs& k);
 // the day kernel (psim_kernels.cu, k_day): the phases a launch runs, for the
 // timesteps step0 .. step_end - 1 of the day
 constexpr uint32_t PH_REBUILD = 1u, PH_DRAW = 2u, PH_DECIDE = 4u, PH_ALL = 7u;
-constexpr uint32_t PH_CLUSTER = 8u;  // (set by launch_day) the grid is one cluster
 typedef void (*DayKernel)(KArgs, uint32_t, uint32_t, uint32_t, uint32_t);
 constexpr uint32_t DAY_THREADS = 512;  // two blocks per SM at 64 registers
 // the day kernel's instances: one variant without sums and its policies, one
@@ -421,11 +420,14 @@ enum {
     DAY_ONE_SUMS,
     DAY_TWO,
     DAY_ANY,
+    DAY_ONE_PLAIN_CLUSTER,  // a small population's, as one cluster of blocks
+    DAY_ONE_QUARANTINE_CLUSTER,
     DAY_KERNELS
 };
 DayKernel day_kernel_a(int instance);
 DayKernel day_kernel_b(int instance);
 DayKernel day_kernel_c(int instance);
+DayKernel day_kernel_d(int instance);
 void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s);
 void launch_time_shift(uint32_t* a, uint32_t n, uint32_t delta, cudaStream_t s);
 // words of the barrier array: the barrier's arrivals, the count of the replay

@@ -1481,25 +1481,32 @@ void launch_day_begin(const KArgs& k, cudaStream_t s) { k_day_begin<<<grid_for(k
 // blocks of 256 threads) capped at the kernel's occupancy, and no more blocks
 // than the population gives work to.  Each block's segment of the lists holds
 // the agents its pass visits.
-// the instance for a context, and its resident blocks per SM
-static DayKernel day_kernel(const KArgs& k, unsigned* per_sm) {
-    static int occ[DAY_KERNELS] = {};
+static DayKernel day_function(int q) {
+    return q <= DAY_ONE_QUARANTINE ? day_kernel_a(q)
+           : q <= DAY_ONE_SUMS     ? day_kernel_b(q)
+           : q <= DAY_ANY          ? day_kernel_c(q)
+                                   : day_kernel_d(q);
+}
+// the instance for a context
+static int day_instance(const KArgs& k) {
     const bool sums = k.track_expected || k.adj.on;
     const int pol = policies(k);
-    const int q = k.m.n_variants == 1 && !sums               ? DAY_ONE_PLAIN + pol
-                  : k.m.n_variants == 1 && sums && pol == 0  ? DAY_ONE_SUMS
-                  : k.m.n_variants == 2 && !sums && pol <= 1 ? DAY_TWO
-                                                             : DAY_ANY;
-    DayKernel f = q <= DAY_ONE_QUARANTINE ? day_kernel_a(q) : q <= DAY_ONE_SUMS ? day_kernel_b(q) : day_kernel_c(q);
+    return k.m.n_variants == 1 && !sums               ? DAY_ONE_PLAIN + pol
+           : k.m.n_variants == 1 && sums && pol == 0  ? DAY_ONE_SUMS
+           : k.m.n_variants == 2 && !sums && pol <= 1 ? DAY_TWO
+                                                      : DAY_ANY;
+}
+// its resident blocks per SM
+static unsigned day_blocks_per_sm(int q) {
+    static int occ[DAY_KERNELS] = {};
     if (!occ[q]) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, DAY_THREADS, 0) != cudaSuccess || n < 1) n = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, day_function(q), DAY_THREADS, 0) != cudaSuccess || n < 1)
+            n = 1;
         occ[q] = n;
     }
-    *per_sm = (unsigned)occ[q];
-    return f;
+    return (unsigned)occ[q];
 }
-// blocks: the grid, or 0 for as many as fit
 static void day_geometry(const KArgs& k, unsigned occ, unsigned blocks, unsigned* grid, uint32_t* cap) {
     const unsigned bps = k.tune.blocks_per_sm
                              ? std::min<unsigned>((k.tune.blocks_per_sm * 256u + DAY_THREADS - 1) / DAY_THREADS, occ)
@@ -1513,11 +1520,13 @@ static void day_geometry(const KArgs& k, unsigned occ, unsigned blocks, unsigned
     const size_t quads = ((size_t)k.a.n + 3) / 4, threads = (size_t)g * DAY_THREADS;
     *cap = (uint32_t)(((quads + threads - 1) / threads) * DAY_THREADS * 4);
 }
-// Up to CLUSTER_AGENTS agents one cluster of at most 16 blocks runs the day: a
-// barrier of the cluster takes 0.24 us where one of the grid takes 1.15 (at 20
-// blocks), and a day of 10k agents has some eighty.  Above, more blocks than a
-// cluster holds are worth more than the faster barrier.
-constexpr uint32_t CLUSTER_BLOCKS = 16, CLUSTER_AGENTS = 16384;
+// Up to CLUSTER_AGENTS agents one cluster of at most 16 blocks runs the day
+// (one variant, no curfew, no sums): its barrier waits for the blocks' writes
+// alone, 0.288 against 0.317 ms a day at 10k agents and 0.317 against 0.341 at
+// 32k; at 48k the blocks that a cluster cannot hold are worth more (0.379
+// against 0.360).
+constexpr unsigned CLUSTER_BLOCKS = 16;
+constexpr uint32_t CLUSTER_AGENTS = 32768;
 static bool cluster_fits(DayKernel kernel, unsigned blocks) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -1542,21 +1551,27 @@ static bool cluster_fits(DayKernel kernel, unsigned blocks) {
 void launch_day(const KArgs& k, uint32_t step0, uint32_t step_end, uint32_t phases, cudaStream_t s) {
     unsigned g;
     uint32_t cap;
-    unsigned occ;
-    const DayKernel kernel = day_kernel(k, &occ);
-    const unsigned few = std::min(CLUSTER_BLOCKS, (k.a.n + DAY_THREADS - 1) / DAY_THREADS);
-    const bool cluster = k.a.n <= CLUSTER_AGENTS && cluster_fits(kernel, few);
-    day_geometry(k, occ, cluster ? few : 0u, &g, &cap);
+    int q = day_instance(k);
+    unsigned blocks = 0;
+    if (k.a.n <= CLUSTER_AGENTS && q <= DAY_ONE_QUARANTINE) {
+        const int qc = q == DAY_ONE_PLAIN ? DAY_ONE_PLAIN_CLUSTER : DAY_ONE_QUARANTINE_CLUSTER;
+        blocks = std::min(CLUSTER_BLOCKS, (k.a.n + DAY_THREADS - 1) / DAY_THREADS);
+        if (cluster_fits(day_function(qc), blocks))
+            q = qc;
+        else
+            blocks = 0;
+    }
+    const DayKernel kernel = day_function(q);
+    day_geometry(k, blocks ? 0u : day_blocks_per_sm(q), blocks, &g, &cap);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g);
     cfg.blockDim = dim3(DAY_THREADS);
     cfg.stream = s;
     cudaLaunchAttribute at;
-    if (cluster) {
+    if (blocks) {
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = g;
         at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        phases |= PH_CLUSTER;
     } else {
         at.id = cudaLaunchAttributeCooperative;
         at.val.cooperative = 1;

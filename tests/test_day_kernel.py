@@ -4,7 +4,9 @@ A segment draws all its timesteps at once and replays the locations where
 somebody is infected: populations where a location holds one agent, a warp and
 a few warps of agents, few and most of them infected within a day, one and
 several variants; curfews that begin at the edges of the words of the
-decision mask.
+decision mask; populations at the edges of a cluster of blocks; location lists
+whose sequence of types has a layout row and lists that have none.  The day in
+one launch against the phases called one by one.
 """
 import numpy as np
 import pytest
@@ -42,3 +44,122 @@ def test_curfew_at_the_edges_of_the_decision_mask(gpu_lib, begin):
     s = small_snapshot(n=2000, locs=500, initial_infected_frac=0.05)
     s.params.update(enable_curfew=1, curfew_begin=begin, curfew_end=30)
     _equal_days(s)
+
+
+@pytest.mark.parametrize("variants", [1, 2])
+@pytest.mark.parametrize("n", [64, 65, 130])
+def test_replays_at_the_edge_of_the_registers(gpu_lib, n, variants):
+    s = small_snapshot(n=n, locs=4, k=5e-3, initial_infected_frac=0.1, n_variants=variants)
+    ill = np.nonzero(s.agents["st_infected_count"])[0]
+    s.agents["variant"][ill] = np.arange(len(ill)) % variants
+    _equal_days(s)
+
+
+@pytest.mark.parametrize("policy", [0, 3])
+@pytest.mark.parametrize("n", [31, 513, 8192, 32768, 32769])
+def test_populations_at_the_edge_of_a_cluster(gpu_lib, n, policy):
+    s = small_snapshot(n=n, locs=max(4, n // 4), k=1e-3, initial_infected_frac=0.05)
+    s.params.update(quarantine_policy=policy, testing_enabled=1)
+    _equal_days(s)
+
+
+def _with_lists(s, rng, form):
+    """Location lists in other forms: entries of a type in two runs, longer
+    than a layout row holds, or in an order of their own."""
+    a = s.agents
+    off, loc, typ, n = a["loc_offset"], a["poss_loc"], a["poss_type"], s.n_agents
+    shops = np.nonzero(s.locs["type"] == s.params["public_type"])[0]
+    new_loc, new_typ, new_off = [], [], [0]
+    for i in range(n):
+        l, t = list(loc[off[i]:off[i + 1]]), list(typ[off[i]:off[i + 1]])
+        f = ("plain", "two_runs", "long", "own_order")[i % 4] if form == "mixed" else form
+        if f == "two_runs":
+            l, t = [l[-1]] + l, [t[-1]] + t
+        elif f == "long":
+            more = rng.integers(0, len(shops), 100 + i % 60)
+            l, t = l + list(shops[more]), t + [s.params["public_type"]] * len(more)
+        elif f == "own_order":
+            o = rng.permutation(len(l))
+            l, t = [l[j] for j in o], [t[j] for j in o]
+        new_loc += l
+        new_typ += t
+        new_off.append(len(new_loc))
+    a["poss_loc"] = np.array(new_loc, loc.dtype)
+    a["poss_type"] = np.array(new_typ, typ.dtype)
+    a["loc_offset"] = np.array(new_off, off.dtype)
+    return s
+
+
+@pytest.mark.parametrize("form", ["two_runs", "long", "own_order", "mixed"])
+@pytest.mark.parametrize("wide", [False, True])
+def test_location_lists_with_and_without_a_layout_row(gpu_lib, form, wide):
+    s = _with_lists(small_snapshot(n=2500, locs=600, initial_infected_frac=0.05), np.random.default_rng(5), form)
+    if wide:  # 8-byte entries
+        shop = int(s.params["public_type"])
+        for arr in (s.locs["type"], s.agents["poss_type"], s.model["ev_loc_type"]):
+            arr[arr == shop] = 100
+        s.params["public_type"] = 100
+    s.params.update(quarantine_policy=2, testing_enabled=1)
+    _equal_days(s)
+
+
+def test_phases_from_a_restored_step(gpu_lib):
+    """Phases called one by one, 30 steps of them taken back (the steps after
+    the restore include some in which nobody moves), the agent list and the
+    hazards read on the way."""
+    from pansim_gb300.native import GpuSim
+    s_cpu = small_snapshot(n=6000, locs=1500, initial_infected_frac=0.03)
+    s_gpu = s_cpu.copy()
+    o, g = ob.Oracle(s_cpu), GpuSim(s_gpu)
+    assert stats_rows(o.midnight(0)) == stats_rows(g.midnight(0))
+    for t in range(50):
+        o.movement(t), o.regroup(), o.infect(t)
+        g.movement(t), g.regroup(), g.infect(t)
+    g.checkpoint_save(1)
+    for t in range(50, 80):
+        g.movement(t), g.regroup(), g.infect(t)
+    g.checkpoint_restore(1)
+    for t in range(50, 144):
+        o.movement(t), o.regroup()
+        out = o.infect(t)
+        g.movement(t), g.regroup(), g.infect(t)
+        if t in (50, 51, 77, 143):
+            assert np.array_equal(g.hazard(), out["hazard"]), t
+            for x, y in zip(o.csr(), g.csr(canonical=True)):
+                assert np.array_equal(x, y), t
+    g.download()
+    assert diff_state(s_cpu, s_gpu) == []
+
+
+@pytest.mark.parametrize("variants", [1, 2])
+@pytest.mark.parametrize("policy", [0, 3])
+def test_sums_of_a_day_equal_the_phases_sums(gpu_lib, variants, policy):
+    """Expected infections and gradient of a day in one launch against a day
+    of the phases one by one: the same float64 terms in another order, under
+    1e6 of them, so 1e6 * 2^-53 of the sum of their absolute values apart at
+    most; the gradient's terms have the sign of what they are derivatives of
+    but for truncation at 1, so 1e-9 of the value bounds it."""
+    from pansim_gb300.native import GpuSim
+    s = small_snapshot(n=4000, locs=900, k=1e-3, initial_infected_frac=0.05, n_variants=variants)
+    ill = np.nonzero(s.agents["st_infected_count"])[0]
+    s.agents["variant"][ill] = np.arange(len(ill)) % variants
+    s.params.update(quarantine_policy=policy, testing_enabled=1)
+    rows, grads, ends = [], [], []
+    for whole in (True, False):
+        e = s.copy()
+        g = GpuSim(e)
+        g.set_tracking(True)
+        g.set_adjoint(True, np.ones(1))
+        if whole:
+            g.run_day(0)
+        else:
+            g.midnight(0)
+            for t in range(144):
+                g.movement(t), g.regroup(), g.infect(t)
+        grads.append(g.gradient())
+        rows.append(g.midnight(144)[0].expected_new_infections)
+        g.download()
+        ends.append(e)
+    assert diff_state(*ends) == []
+    assert rows[0] == pytest.approx(rows[1], rel=1e-9)
+    assert np.allclose(grads[0], grads[1], rtol=1e-9, atol=1e-12 * np.abs(grads[1]).max())

@@ -304,11 +304,12 @@ int initial_regroup(psim_ctx* c) {
     CK(cudaMemsetAsync(c->k.l.counts, 0, sizeof(uint32_t) * c->L, c->stream));
     if ((rc0 = reset_sums(c))) return rc0;
     launch_count(c->k, c->stream);
-    launch_scan(c->k, 0, 1, 0, false, c->stream);
+    // (the caller's first regroup takes its ratios from these sums)
+    launch_scan(c->k, 0, SCAN_RATIOS | SCAN_SUMS, 0, false, c->stream);
     launch_scatter(c->k, 0, false, c->stream);
     c->list_sparse = false;
     c->csr_full = true;
-    c->sums_zero = true;
+    c->sums_zero = false;
     c->moved = false;
     // the variant gating of the first steps (the statistics come at midnight)
     launch_variant_flags(c->k, c->stream);
@@ -330,7 +331,7 @@ int do_step(psim_ctx* c, uint32_t step) {
     }
     launch_phase_movement(c->k, step, c->stream);
     const bool merge = c->params.quarantine_policy > 1;
-    launch_scan(c->k, step, 1, merge, false, c->stream);
+    launch_scan(c->k, step, SCAN_RATIOS, merge, false, c->stream);
     launch_scatter(c->k, step, merge, c->stream);
     c->sums_zero = true;
     launch_phase_draw(c->k, step, c->stream);
@@ -1154,7 +1155,7 @@ int psim_regroup(psim_ctx* c) {
     const uint32_t since = c->t_next - 1u - c->h_clock.t0;
     const uint32_t step = c->csr_fresh && since < c->spd ? since : 0u;
     const bool merge = c->params.quarantine_policy > 1;
-    launch_scan(c->k, step, 1, merge, keep, c->stream);
+    launch_scan(c->k, step, SCAN_RATIOS, merge, keep, c->stream);
     // (nobody moved: there is nothing to scatter)
     if (!keep) launch_scatter(c->k, step, merge, c->stream);
     c->launches += (keep ? 0 : 1) + (uint64_t)scan_kernels(c->k);

@@ -396,6 +396,8 @@ void launch_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
 // a step of the per-phase entry points (the sums are zero)
 void launch_phase_movement(const KArgs& k, uint32_t step_in_day, cudaStream_t s);
 void launch_count(const KArgs& k, cudaStream_t s);
+// with_hazard: 0 or SCAN_RATIOS, with SCAN_SUMS where another scan will use the sums again
+constexpr int SCAN_RATIOS = 1, SCAN_KEEP = 2, SCAN_SUMS = 4;
 // merge_quarantine: the location quarantines that decisions wrote since the last merge
 // keep: the agent list stands, only the ratios
 void launch_scan(const KArgs& k, uint32_t step_in_day, int with_hazard, int merge_quarantine, bool keep,

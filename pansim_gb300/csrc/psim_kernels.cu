@@ -297,9 +297,8 @@ __device__ __forceinline__ uint32_t scan_lookback(const KArgs& k, uint32_t tile,
     return prefix;
 }
 
-// with_hazard: 1 the ratios, and SCAN_KEEP where the caller knows that the
-// agent list stands.
-constexpr int SCAN_KEEP = 2;
+// with_hazard: SCAN_RATIOS, and SCAN_KEEP where the caller knows that the
+// agent list stands, SCAN_SUMS where another scan will use the sums again.
 template <int ITEMS, bool LOOKBACK>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, int with_hazard, int merge_q) {
     constexpr int TILE = SCAN_THREADS * ITEMS;
@@ -409,7 +408,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(KArgs k, uint32_t step, i
                     if (fix != 0) {
                         h = psim_hazard_x(fix, c[q], k_f, w_l, season, dt, &x);
                         nz = true;
-                        k.l.sfix[idx] = 0ull;
+                        if (!(with_hazard & SCAN_SUMS)) k.l.sfix[idx] = 0ull;
                     }
                     k.l.hazard[idx] = h;
                     if (k.adj.on) k.l.hazard_x[idx] = x;
@@ -575,7 +574,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_v(KArgs k, uint32_t step,
                     if (fix != 0) {
                         h = psim_hazard_x(fix, n_l, k_f, w_l, season, dt, &xx);
                         nzb |= 1u << ((l0 & 31u) + e);
-                        k.l.sfix[idx] = 0ull;
+                        if (!(with_hazard & SCAN_SUMS)) k.l.sfix[idx] = 0ull;
                     }
                     k.l.hazard[idx] = h;
                     if (k.adj.on) k.l.hazard_x[idx] = xx;

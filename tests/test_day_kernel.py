@@ -163,3 +163,30 @@ def test_sums_of_a_day_equal_the_phases_sums(gpu_lib, variants, policy):
     assert diff_state(*ends) == []
     assert rows[0] == pytest.approx(rows[1], rel=1e-9)
     assert np.allclose(grads[0], grads[1], rtol=1e-9, atol=1e-12 * np.abs(grads[1]).max())
+
+
+@pytest.mark.parametrize("scan_mode", [0, 1, 2, 3])
+def test_regroup_of_an_uploaded_state(gpu_lib, scan_mode):
+    """The first regroup of a state, of the next one put in its place, and one
+    more of the same: agent list and ratios of the oracle, before any step."""
+    from pansim_gb300.native import GpuSim
+    s_gpu = small_snapshot(n=6000, locs=1500, initial_infected_frac=0.03)
+    g = GpuSim(s_gpu)
+    g.set_tuning(scan_mode=scan_mode)
+    rng = np.random.default_rng(3)
+    for turn in range(3):
+        if turn:
+            s_gpu.agents["location"][:] = rng.permutation(s_gpu.agents["location"])
+            g.upload()
+        s_cpu = s_gpu.copy()
+        o = ob.Oracle(s_cpu)
+        o.regroup()
+        out = o.infect(0)
+        for _ in range(2):
+            g.regroup()
+            for x, y in zip(o.csr(), g.csr(canonical=True)):
+                assert np.array_equal(x, y), turn
+            assert np.array_equal(g.hazard(), out["hazard"]), turn
+    g.infect(0)
+    g.download()
+    assert diff_state(s_cpu, s_gpu) == []

@@ -196,11 +196,18 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
         };
         if (list) {
             uint32_t lw[8], flags = 0;
+            float sus[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
 #pragma unroll
             for (int u = 0; u < 8; ++u)
                 if ((lw[u] >> (loc[u] & 31u)) & 1u) {
+                    if (VC == 1) {
+                        // in flight with the sum: 14.2 -> 13.1 us a listing at
+                        // 2M agents, 20M unchanged (122 us)
+                        const uint32_t i = agent_of(u);
+                        sus[u] = k.a.susceptible[i] * k.p.sigma_band[k.a.band[i]];
+                    }
                     if (nonzero_sum<VC, SUMS>(k, loc[u]))
                         flags |= 1u << u;
                     else
@@ -215,6 +222,10 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
                         const size_t pos = seg + at++;
                         k.l.list_agent[pos] = i;
                         k.l.list_loc[pos] = loc[u];
+                        if (VC == 1) {
+                            k.l.list_su[pos] = sus[u];
+                            continue;
+                        }
                         const float sigma = k.p.sigma_band[k.a.band[i]];
                         for (uint32_t v = 0; v < V; ++v)
                             k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;

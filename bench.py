@@ -39,39 +39,38 @@ STEP_BYTES = (32, 20)
 
 
 def kernel_bytes(N, L, V, spd, counts):
-    """Algorithmic bytes per simulated day of each phase of the step kernel,
+    """Algorithmic bytes per simulated day of each phase of the day kernel,
     from the profiled day's counters (entries E, entries at a location with a
-    nonzero ratio EH, queued agents M, queue passes Q, rebuilds R, listed
+    nonzero ratio EH, decisions M, work-list passes Q, rebuilds R, listed
     locations LL and agents LA, summed over the rebuilds and steps):
-      rebuild   per rebuild the hazard mask read twice (L / 4) and every
-                agent's location (4 N); per listed location its sums read
-                (8 V), its count read twice and its first slot written (12);
-                per listed agent its age band and susceptibilities read, its
-                slot's atomic, id, location and susceptibility products
-                written (17 + 8 V)
-      draw      per entry its slot's location, agent and susceptibility
-                products (8 + 4 V) and its location's count, weight, replica
-                and sums (10 + 8 V)
-      decide    per queue pass the decision timestamps (4 N); per decision
-                76: its work-list entry written and read (8), the agent's
-                location, decision timestamp, state, type, age, flags and
-                timestamps (38), its location-list entries (12), the new
-                location's flags (5), the location and timestamp written (8),
-                the histogram deltas (8)
+      rebuild   per rebuild every agent's location (4 N) and the hazard mask
+                (L / 8); per listed agent its location's sums and its
+                susceptibilities read (12 V), its age band (1), its id and
+                location written (8) and its products (4 V)
+      draw      per listed agent its entry (8 + 4 V); per listed location its
+                count, weight, replica and sums (10 + 8 V)
+      decide    per work-list pass the decision timestamps (4 N); per decision
+                52: its work-list entry written and read (8), the agent's
+                location and decision word (8), its layout and list offset
+                (6), its location-list entries (12), the new location's flag
+                word (2), the location and timestamp written (8), the
+                histogram deltas (8)
     """
     E, EH, M, Q, R, LL, LA = (float(x) for x in counts)
-    return {"rebuild": R * (L / 4.0 + 4.0 * N) + (12 + 8 * V) * LL + (17 + 8 * V) * LA,
-            "draw": (18 + 12 * V) * E,
-            "decide": 4.0 * N * Q + 76.0 * M}
+    return {"rebuild": R * (L / 8.0 + 4.0 * N) + (9 + 16 * V) * LA,
+            "draw": (8 + 4 * V) * LA + (10 + 8 * V) * LL,
+            "decide": 4.0 * N * Q + 52.0 * M}
 
 
-KERNEL_LABELS = {"rebuild": "k_step rebuild phase", "draw": "k_step draw phase", "decide": "k_step queue + decide phase"}
+KERNEL_LABELS = {"rebuild": "k_day lists of the agents at infectious locations", "draw": "k_day draws",
+                 "decide": "k_day work list + decisions"}
 
 
 def step_kinds(tl):
-    """The profiled day's steps by kind (tl: per step the kernel span, the
-    rebuild's listing and slots, the draws, the queue, the decisions, the
-    time since the previous kernel, us): count and mean span, gap and phase
+    """The profiled day's steps by kind (tl: per step its span, 0, its
+    rebuild's lists, the draws (a segment's, divided among its steps), the
+    queue, the decisions, the time since the step before, us): count and mean
+    span, gap and phase
     times of the draw-only steps, the steps with a rebuild and no decisions,
     with decisions and no rebuild, with both."""
     reb, dec = tl[:, 1:3].sum(axis=1) > 0, tl[:, 5] > 0
@@ -610,16 +609,16 @@ def main():
         for name in KERNEL_LABELS:
             kern[name]["share_of_steps"] = kern[name]["ms_per_day"] / tot_k
         steps_by_kind = step_kinds(tl_sum / n_prof)
-        # The step kernel (one launch per timestep, its phases fused with
-        # grid barriers) is the kernel of the day graph: its algorithmic
-        # bytes per launch are the phases' bytes of a day over the day's
-        # timesteps, its launch time the timed days' graph time (less the
-        # day's first movement pass) over their timesteps.
-        step_alg = sum(kb.values()) / spd
-        step_ms = (graph_ms / args.steps - float(kms_day[0])) / spd
-        ach = step_alg / (step_ms * 1e-3) / 1e9
+        # The day kernel (one launch per day, its phases separated by grid
+        # barriers) runs all timesteps of the day graph: its algorithmic bytes
+        # per launch are the phases' bytes of a day, its launch time the timed
+        # days' graph time less the day's first movement pass.
+        day_alg = sum(kb.values())
+        day_ms = graph_ms / args.steps - float(kms_day[0])
+        step_ms = day_ms / spd
+        ach = day_alg / (day_ms * 1e-3) / 1e9
         tr = committed_traffic()
-        traffic = tr.get("k_step") if tr else None
+        traffic = tr.get("k_day") if tr else None
         # the step-rate figure: the reference's per-step bytes over our
         # average timestep time
         step_bytes = STEP_BYTES[0] * N + STEP_BYTES[1] * L
@@ -631,12 +630,11 @@ def main():
             "ms_per_step": t_max / args.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic",
             "config": workload_config(snap, ws),
-            "roofline": {"bound": "hbm", "kernel": "k_step (one launch per timestep: rebuild, draw, decide phases)",
+            "roofline": {"bound": "hbm", "kernel": "k_day (one launch per day: lists, draws, decisions of its timesteps)",
                          "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": traffic,
-                         "peak_kind": peak_kind, "alg_bytes_per_launch": step_alg, "launch_ms": step_ms,
-                         "launch_ms_source": "day-graph CUDA events over the timed days, less the first movement "
-                                             "pass, over their timesteps",
-                         "dominant": "k_step", "dominant_phase": max(KERNEL_LABELS, key=lambda n: kern[n]["ms_per_day"]),
+                         "peak_kind": peak_kind, "alg_bytes_per_launch": day_alg, "launch_ms": day_ms,
+                         "launch_ms_source": "the day graph's timed days, less the first movement pass",
+                         "dominant": "k_day", "dominant_phase": max(KERNEL_LABELS, key=lambda n: kern[n]["ms_per_day"]),
                          "per_phase": kern, "day_counts": counts_d, "steps_by_kind": steps_by_kind,
                          "step_rate": {"reference_bytes_per_timestep": step_bytes, "timestep_ms": step_ms,
                                        "gbs": step_bytes / (step_ms * 1e-3) / 1e9,

@@ -124,8 +124,8 @@ struct DevAgents {
     float* scaling_v;             // [V*N] symptom scaling of the states up to 6, per variant
     uint8_t* hcw;                 // healthcare worker flag
     uint32_t* rank;               // scratch of the canonical CSR ordering
-    uint32_t* worklist;           // agents that decide at the next step (k_queue), one segment
-                                  // per queue block
+    uint32_t* worklist;           // agents that decide at the end of the running segment, a stretch
+                                  // per block of the day kernel
     uint32_t* home;               // [N] the agent's home: the first home-type entry of its location
                                   // list (findActualLocationForType's first match, no draw),
                                   // computed when the context is made or the home type changes

@@ -140,14 +140,18 @@ __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
 // nonzero sum (nobody moves, since a move makes the next segment list again,
 // and a draw infects only agents at a location with a nonzero sum).  The
 // hazard mask is a superset of those locations (every kernel that adds an
-// infectious term sets the bit at once); an agent that finds a zero sum behind
-// its location's bit clears it.  Agents of one location lie in many blocks'
+// infectious term sets the bit at once); an entry whose location's sum turns
+// out to be zero clears its bit.  The pass itself only places the agents: what
+// the draws need of them (sum, susceptibility, age band) loads with one thread
+// per entry, by the segment's draws, or here where a launch draws nothing.
+// Loaded in the pass, by the few lanes that met a listed agent, trip after
+// trip, a listing took 13.1 us at 2M agents (now 10.6) and 122 at 20M (now 99).  Agents of one location lie in many blocks'
 // lists: the replay gathers those it needs, so no location needs a segment of
 // its own (reserving segments first, a pass over the mask, a barrier and a
 // returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
 // 20M).  queue: the work list of those that decide at s1.
 template <int VC, bool SUMS, int POL>
-__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, uint32_t s1, uint32_t cap,
+__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, bool prepare, uint32_t s1, uint32_t cap,
                                             DayShared& sh) {
     const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
     __syncthreads();
@@ -196,39 +200,17 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
         };
         if (list) {
             uint32_t lw[8], flags = 0;
-            float sus[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if ((lw[u] >> (loc[u] & 31u)) & 1u) {
-                    if (VC == 1) {
-                        // in flight with the sum: 14.2 -> 13.1 us a listing at
-                        // 2M agents, 20M unchanged (122 us)
-                        const uint32_t i = agent_of(u);
-                        sus[u] = k.a.susceptible[i] * k.p.sigma_band[k.a.band[i]];
-                    }
-                    if (nonzero_sum<VC, SUMS>(k, loc[u]))
-                        flags |= 1u << u;
-                    else
-                        atomicAnd(&k.l.hmask[loc[u] >> 5], ~(1u << (loc[u] & 31u)));
-                }
+            for (int u = 0; u < 8; ++u) flags |= (lw[u] >> (loc[u] & 31u) & 1u) << u;
             if (__any_sync(0xffffffffu, flags != 0u)) {
                 uint32_t at = list_place(flags, &sh.listed);
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
                     if ((flags >> u) & 1u) {
-                        const uint32_t i = agent_of(u);
-                        const size_t pos = seg + at++;
-                        k.l.list_agent[pos] = i;
-                        k.l.list_loc[pos] = loc[u];
-                        if (VC == 1) {
-                            k.l.list_su[pos] = sus[u];
-                            continue;
-                        }
-                        const float sigma = k.p.sigma_band[k.a.band[i]];
-                        for (uint32_t v = 0; v < V; ++v)
-                            k.l.list_su[v * k.l.list_cap + pos] = k.a.susceptible[(size_t)v * N + i] * sigma;
+                        k.l.list_agent[seg + at] = agent_of(u);
+                        k.l.list_loc[seg + at++] = loc[u];
                     }
             }
         }
@@ -246,7 +228,17 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
         }
     }
     __syncthreads();
-    if (list && threadIdx.x == 0) k.l.list_count[blockIdx.x] = sh.listed;  // for a later launch
+    if (!list) return;
+    const uint32_t listed = sh.listed;
+    if (threadIdx.x == 0) k.l.list_count[blockIdx.x] = listed;  // for a later launch
+    // (for a launch of the draws that follows)
+    for (uint32_t j = threadIdx.x; prepare && j < listed; j += blockDim.x) {
+        const uint32_t i = k.l.list_agent[seg + j], l = k.l.list_loc[seg + j];
+        const float sigma = k.p.sigma_band[k.a.band[i]];
+        for (uint32_t v = 0; v < V; ++v)
+            k.l.list_su[v * k.l.list_cap + seg + j] = k.a.susceptible[(size_t)v * N + i] * sigma;
+        if (!nonzero_sum<VC, SUMS>(k, l)) atomicAnd(&k.l.hmask[l >> 5], ~(1u << (l & 31u)));
+    }
 }
 
 // the locations with a nonzero sum and the agents listed (profiled graph only)
@@ -386,7 +378,7 @@ struct DrawRun {
 // added here as if nobody were infected; phase_replay takes those of its
 // locations back and adds the right ones.
 template <int VC, bool SUMS>
-__device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32_t listed, double* s_grad,
+__device__ void phase_draw(const KArgs& k, const DrawRun& dr, bool fresh, size_t seg, uint32_t listed, double* s_grad,
                            uint32_t* n_entries, uint32_t* n_hazard) {
     const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k), dt = k.p.time_step;
     const bool one_rep = k.r.n == 1;
@@ -399,7 +391,7 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32
         if (!SUMS && !act) break;
         const uint32_t loc = act ? k.l.list_loc[pos] : NONE;
         const uint32_t i = act ? k.l.list_agent[pos] : NONE;
-        const float su0 = act ? k.l.list_su[pos] : 0.0f;
+        float su0 = act && !fresh ? k.l.list_su[pos] : 0.0f;
         if (act && (loc >= L || i >= N)) {
             raise_error(k, ERR_AGENT_LIST);
             act = false;
@@ -411,6 +403,15 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, size_t seg, uint32
             const float wl = k.l.infectiousness[loc];
             rep = one_rep ? 0u : k.l.rep[loc];
             const RepConst rc = one_rep ? rc0 : rep_const(k, rep);
+            if (fresh) {  // listed for this segment: its products, its location's bit
+                const float sigma = k.p.sigma_band[k.a.band[i]];
+                for (uint32_t v = 0; v < V; ++v) {
+                    const float s = k.a.susceptible[(size_t)v * N + i] * sigma;
+                    k.l.list_su[v * k.l.list_cap + pos] = s;
+                    if (v == 0) su0 = s;
+                }
+                if (!nonzero_sum<VC, SUMS>(k, loc)) atomicAnd(&k.l.hmask[loc >> 5], ~(1u << (loc & 31u)));
+            }
             bool any_h = false, hit = false;
             for (uint32_t v = 0; v < V && (SUMS || !hit); ++v) {
                 float x;
@@ -847,7 +848,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     if (merge) merge_quarantine(k);
     const size_t seg = (size_t)blockIdx.x * cap;
     if (list || decides) {
-        phase_lists<VC, SUMS, POL>(k, list, decides, e, cap, sh);
+        phase_lists<VC, SUMS, POL>(k, list, decides, !(phases & PH_DRAW), e, cap, sh);
         if (decides) mask_clear_shared(sh.mm);
         if (k.prof) {
             if (list) count_listed<VC, SUMS>(k, sh);
@@ -862,7 +863,7 @@ __device__ __forceinline__ bool day_segment(const KArgs& k, uint32_t step, uint3
     const bool draws = (phases & PH_DRAW) != 0;
     if (draws) {
         uint32_t entries = 0, hazard = 0;
-        phase_draw<VC, SUMS>(k, dr, seg, sh.listed, sh.grad, &entries, &hazard);
+        phase_draw<VC, SUMS>(k, dr, list, seg, sh.listed, sh.grad, &entries, &hazard);
         if (k.prof) {
             __syncwarp();
             entries = __reduce_add_sync(0xffffffffu, entries);

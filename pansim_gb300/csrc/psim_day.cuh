@@ -132,43 +132,17 @@ __device__ __forceinline__ bool nonzero_sum(const KArgs& k, uint32_t l) {
     return nz;
 }
 
-// The block's lists of its own agents (four consecutive agents per thread,
-// one 16-byte load of a field, two quads in flight; the blocks' quads are
-// dealt in turn).  list: the agent list afresh.  Only the agents at locations
-// with a nonzero sum are listed, because the draws of every step until the
-// next listing need no other location: until then no other location gains a
-// nonzero sum (nobody moves, since a move makes the next segment list again,
-// and a draw infects only agents at a location with a nonzero sum).  The
-// hazard mask is a superset of those locations (every kernel that adds an
-// infectious term sets the bit at once); an entry whose location's sum turns
-// out to be zero clears its bit.  The pass itself only places the agents: what
-// the draws need of them (sum, susceptibility, age band) loads with one thread
-// per entry, by the segment's draws, or here where a launch draws nothing.
-// Loaded in the pass, by the few lanes that met a listed agent, trip after
-// trip, a listing took 13.1 us at 2M agents (now 10.6) and 122 at 20M (now 99).  Agents of one location lie in many blocks'
-// lists: the replay gathers those it needs, so no location needs a segment of
-// its own (reserving segments first, a pass over the mask, a barrier and a
-// returning atomic per agent took 9.8 + 10.7 us at 2M agents and 20 + 70 us at
-// 20M).  queue: the work list of those that decide at s1.
-template <int VC, bool SUMS, int POL>
-__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, bool prepare, uint32_t s1, uint32_t cap,
-                                            DayShared& sh) {
-    const uint32_t L = k.l.n, N = k.a.n, V = nvar<VC>(k);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (list) sh.listed = 0u;
-        if (queue) sh.cnt = 0u;
-    }
-    __syncthreads();
-    const bool everybody = POL == 2 && k.p.enable_curfew && k.p.curfew_begin == s1;
-    const uint32_t t1 = k.clock->t0 + s1;
+// The pass over the agents, QF quads of a thread in flight.
+template <int QF>
+__device__ __forceinline__ void list_pass(const KArgs& k, bool list, bool queue, bool everybody, uint32_t t1,
+                                          size_t seg, DayShared& sh) {
+    const uint32_t L = k.l.n, N = k.a.n;
     const uint32_t quads = (N + 3u) >> 2;
     const uint32_t stride = gridDim.x * blockDim.x;
-    const size_t seg = (size_t)blockIdx.x * cap;
-    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += 2u * stride) {  // block-uniform trips
-        uint32_t loc[8], m[8];
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < quads; q0 += (uint32_t)QF * stride) {  // block-uniform trips
+        uint32_t loc[4 * QF], m[4 * QF];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < QF; ++h) {
             const uint32_t q = q0 + (uint32_t)h * stride + threadIdx.x;
             const uint32_t i0 = q * 4u;
             const bool whole = q < quads && i0 + 3u < N;
@@ -199,15 +173,15 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
             return (q0 + (uint32_t)(u >> 2) * stride + threadIdx.x) * 4u + (uint32_t)(u & 3);
         };
         if (list) {
-            uint32_t lw[8], flags = 0;
+            uint32_t lw[4 * QF], flags = 0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
+            for (int u = 0; u < 4 * QF; ++u) lw[u] = loc[u] < L ? k.l.hmask[loc[u] >> 5] : 0u;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) flags |= (lw[u] >> (loc[u] & 31u) & 1u) << u;
+            for (int u = 0; u < 4 * QF; ++u) flags |= (lw[u] >> (loc[u] & 31u) & 1u) << u;
             if (__any_sync(0xffffffffu, flags != 0u)) {
                 uint32_t at = list_place(flags, &sh.listed);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
+                for (int u = 0; u < 4 * QF; ++u)
                     if ((flags >> u) & 1u) {
                         k.l.list_agent[seg + at] = agent_of(u);
                         k.l.list_loc[seg + at++] = loc[u];
@@ -217,16 +191,56 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
         if (queue) {
             uint32_t flags = 0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < 4 * QF; ++u)
                 if (agent_of(u) < N && (everybody || m[u] == t1)) flags |= 1u << u;
             if (__any_sync(0xffffffffu, flags != 0u)) {
                 uint32_t at = list_place(flags, &sh.cnt);
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
+                for (int u = 0; u < 4 * QF; ++u)
                     if ((flags >> u) & 1u) k.a.worklist[seg + at++] = agent_of(u);
             }
         }
     }
+}
+
+// The block's lists of its own agents (four consecutive agents per thread, one
+// 16-byte load of a field; the blocks' quads are dealt in turn).  list: the
+// agent list afresh.  Only the agents at locations with a nonzero sum are
+// listed, because the draws of every step until the next listing need no other
+// location: until then no other location gains a nonzero sum (nobody moves,
+// since a move makes the next segment list again, and a draw infects only
+// agents at a location with a nonzero sum).  The
+// hazard mask is a superset of those locations (every kernel that adds an
+// infectious term sets the bit at once); an entry whose location's sum turns
+// out to be zero clears its bit.  The pass itself only places the agents: what
+// the draws need of them (sum, susceptibility, age band) loads with one thread
+// per entry, by the segment's draws, or here where a launch draws nothing.
+// Loaded in the pass, by the few lanes that met a listed agent, trip after
+// trip, a listing took 13.1 us at 2M agents (now 10.6) and 122 at 20M (now 99).
+// Agents of one location lie in many blocks' lists: the replay gathers those
+// it needs, so no location needs a segment of its own (reserving segments
+// first, a pass over the mask, a barrier and a returning atomic per agent took
+// 9.8 + 10.7 us at 2M agents and 20 + 70 us at 20M).  queue: the work list of
+// those that decide at s1.
+template <int VC, bool SUMS, int POL>
+__device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queue, bool prepare, uint32_t s1, uint32_t cap,
+                                            DayShared& sh) {
+    const uint32_t N = k.a.n, V = nvar<VC>(k);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (list) sh.listed = 0u;
+        if (queue) sh.cnt = 0u;
+    }
+    __syncthreads();
+    const bool everybody = POL == 2 && k.p.enable_curfew && k.p.curfew_begin == s1;
+    const uint32_t t1 = k.clock->t0 + s1;
+    const size_t seg = (size_t)blockIdx.x * cap;
+    // one trip of one quad where the grid's threads have no more: 1.2% of a
+    // day at 10k to 320k agents; two in flight above: 1.5% at 7M and 20M
+    if (((N + 3u) >> 2) <= gridDim.x * blockDim.x)
+        list_pass<1>(k, list, queue, everybody, t1, seg, sh);
+    else
+        list_pass<2>(k, list, queue, everybody, t1, seg, sh);
     __syncthreads();
     if (!list) return;
     const uint32_t listed = sh.listed;

@@ -11,6 +11,24 @@ __device__ __forceinline__ void raise_error(const KArgs& k, uint32_t bits) {
     atomicOr(k.err, bits);
     *(volatile uint32_t*)k.err_host = 1u;
 }
+
+// Atomics nobody reads the result of.  As instructions: the compiler puts code
+// of its own around the atomic functions, which the hot ones (two counts and
+// up to two sums of every move) pay for on every decision: 0.43 -> 0.37 ms of
+// decisions a day at 2M agents, 4.16 -> 3.69 at 20M.
+__device__ __forceinline__ void red_add(uint32_t* p, uint32_t x) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long x) {
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(x) : "memory");
+}
+__device__ __forceinline__ void red_or(uint32_t* p, uint32_t x) {
+    asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+__device__ __forceinline__ void red_and(uint32_t* p, uint32_t x) {
+    asm volatile("red.relaxed.gpu.global.and.b32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
+}
+
 __device__ __forceinline__ uint32_t wb_of(const KArgs& k, uint32_t i) {
     return k.m.state_wb[(uint8_t)k.a.state[i]];
 }
@@ -544,7 +562,7 @@ constexpr int SCAN_THREADS = 256;
 // (the day kernel's rebuild lists from it and clears the bits of zero sums;
 // the per-phase scans recompute the bits of their dirty locations).
 __device__ __forceinline__ void mark_hazardous(const KArgs& k, uint32_t loc) {
-    atomicOr(&k.l.hmask[loc >> 5], 1u << (loc & 31u));
+    red_or(&k.l.hmask[loc >> 5], 1u << (loc & 31u));
 }
 
 // The full pass of a day's first step (k_movement, after a reset of the
@@ -561,13 +579,13 @@ __device__ __forceinline__ bool count_agent(const KArgs& k, bool act, uint32_t l
     }
     const bool mv = act && loc != loc0;
     if (mv) {
-        if (loc0 < L) atomicSub(&k.l.counts[loc0], 1u);
-        if (loc != NONE) atomicAdd(&k.l.counts[loc], 1u);
+        if (loc0 < L) red_add(&k.l.counts[loc0], 0u - 1u);
+        if (loc != NONE) red_add(&k.l.counts[loc], 1u);
     }
     if (act && loc != NONE && inf > 0.0f) {
         const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
-        atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
+        red_add(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
+        red_or(&k.l.smask[loc >> 5], 1u << (loc & 31u));
         mark_hazardous(k, loc);
     }
     return mv;
@@ -592,16 +610,16 @@ __device__ __forceinline__ bool count_agent_delta(const KArgs& k, bool act, uint
     }
     const bool mv = act && loc != loc0;
     if (mv) {
-        if (loc0 < L) atomicSub(&k.l.counts[loc0], 1u);
-        if (loc != NONE) atomicAdd(&k.l.counts[loc], 1u);
+        if (loc0 < L) red_add(&k.l.counts[loc0], 0u - 1u);
+        if (loc != NONE) red_add(&k.l.counts[loc], 1u);
     }
     if (act) {
         const long long q0 = (loc0 < L && inf0 > 0.0f) ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
         const long long q1 = (loc != NONE && inf > 0.0f) ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
         if (mv || q0 != q1 || var0 != var) {
-            if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
+            if (q0) red_add(&k.l.sfix[(size_t)var0 * L + loc0], (unsigned long long)(-q0));
             if (q1) {
-                atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
+                red_add(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
                 mark_hazardous(k, loc);
             }
         }
@@ -617,11 +635,11 @@ __device__ __forceinline__ void count_full(const KArgs& k, bool act, uint32_t lo
         raise_error(k, ERR_LOCATION);
         return;
     }
-    atomicAdd(&k.l.counts[loc], 1u);
+    red_add(&k.l.counts[loc], 1u);
     if (inf > 0.0f) {
         const long long q = __float2ll_rn(inf * PSIM_FIX_SCALE_F);
-        atomicAdd(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
-        atomicOr(&k.l.smask[loc >> 5], 1u << (loc & 31u));
+        red_add(&k.l.sfix[(size_t)variant * L + loc], (unsigned long long)q);
+        red_or(&k.l.smask[loc >> 5], 1u << (loc & 31u));
         mark_hazardous(k, loc);
     }
 }

@@ -251,7 +251,7 @@ __device__ __forceinline__ void phase_lists(const KArgs& k, bool list, bool queu
         const float sigma = k.p.sigma_band[k.a.band[i]];
         for (uint32_t v = 0; v < V; ++v)
             k.l.list_su[v * k.l.list_cap + seg + j] = k.a.susceptible[(size_t)v * N + i] * sigma;
-        if (!nonzero_sum<VC, SUMS>(k, l)) atomicAnd(&k.l.hmask[l >> 5], ~(1u << (l & 31u)));
+        if (!nonzero_sum<VC, SUMS>(k, l)) red_and(&k.l.hmask[l >> 5], ~(1u << (l & 31u)));
     }
 }
 
@@ -424,7 +424,7 @@ __device__ void phase_draw(const KArgs& k, const DrawRun& dr, bool fresh, size_t
                     k.l.list_su[v * k.l.list_cap + pos] = s;
                     if (v == 0) su0 = s;
                 }
-                if (!nonzero_sum<VC, SUMS>(k, loc)) atomicAnd(&k.l.hmask[loc >> 5], ~(1u << (loc & 31u)));
+                if (!nonzero_sum<VC, SUMS>(k, loc)) red_and(&k.l.hmask[loc >> 5], ~(1u << (loc & 31u)));
             }
             bool any_h = false, hit = false;
             for (uint32_t v = 0; v < V && (SUMS || !hit); ++v) {
@@ -495,9 +495,9 @@ __device__ __forceinline__ void add_infection_change(const KArgs& k, uint32_t lo
     const long long q0 = inf0 > 0.0f ? __float2ll_rn(inf0 * PSIM_FIX_SCALE_F) : 0ll;
     const long long q1 = inf > 0.0f ? __float2ll_rn(inf * PSIM_FIX_SCALE_F) : 0ll;
     if (q0 == q1 && var0 == var) return;
-    if (q0) atomicAdd(&k.l.sfix[(size_t)var0 * L + loc], (unsigned long long)(-q0));
+    if (q0) red_add(&k.l.sfix[(size_t)var0 * L + loc], (unsigned long long)(-q0));
     if (q1) {
-        atomicAdd(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
+        red_add(&k.l.sfix[(size_t)var * L + loc], (unsigned long long)q1);
         mark_hazardous(k, loc);
     }
 }

@@ -12,10 +12,10 @@ __device__ __forceinline__ void raise_error(const KArgs& k, uint32_t bits) {
     *(volatile uint32_t*)k.err_host = 1u;
 }
 
-// Atomics nobody reads the result of.  As instructions: the compiler puts code
-// of its own around the atomic functions, which the hot ones (two counts and
-// up to two sums of every move) pay for on every decision: 0.43 -> 0.37 ms of
-// decisions a day at 2M agents, 4.16 -> 3.69 at 20M.
+// Atomics nobody reads the result of, as the instructions.  With the atomic
+// functions the decisions ran as many instructions but waited longer for
+// memory (12.9 against 10.8 warps stalled on it per issue): 0.43 against 0.37
+// ms of decisions a day at 2M agents and 4.16 against 3.69 at 20M.
 __device__ __forceinline__ void red_add(uint32_t* p, uint32_t x) {
     asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(x) : "memory");
 }

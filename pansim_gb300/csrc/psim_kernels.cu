@@ -1521,9 +1521,9 @@ static void day_geometry(const KArgs& k, unsigned occ, unsigned blocks, unsigned
 }
 // Up to CLUSTER_AGENTS agents one cluster of at most 16 blocks runs the day
 // (one variant, no curfew, no sums): its barrier waits for the blocks' writes
-// alone, 0.288 against 0.317 ms a day at 10k agents and 0.317 against 0.341 at
-// 32k; at 48k the blocks that a cluster cannot hold are worth more (0.379
-// against 0.360).
+// alone, 0.249 against 0.274 ms a day at 10k agents and 0.275 against 0.311 at
+// 32k; at 48k the blocks that a cluster cannot hold are worth more (0.333
+// against 0.311).
 constexpr unsigned CLUSTER_BLOCKS = 16;
 constexpr uint32_t CLUSTER_AGENTS = 32768;
 static bool cluster_fits(DayKernel kernel, unsigned blocks) {

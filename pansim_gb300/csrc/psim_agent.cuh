@@ -251,7 +251,7 @@ __device__ __forceinline__ bool quarantine_type(const KArgs& k, uint32_t ty) {
 // the countdowns of every event at every step come from a table computed on
 // the host (no divisions here), a location's flags are one word, the home is
 // looked up once, and an entry of a location list is found by the list's
-// layout.  22 us of decisions a step at 2M agents, against 25 without
+// layout.  22 us of decisions a step at 2M agents (17 now), against 25 without
 // those; the rare quarantine out of line (its arguments through memory) took
 // 26, and the location list in registers 23.6.
 //

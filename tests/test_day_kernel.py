@@ -190,3 +190,9 @@ def test_regroup_of_an_uploaded_state(gpu_lib, scan_mode):
     g.infect(0)
     g.download()
     assert diff_state(s_cpu, s_gpu) == []
+
+
+@pytest.mark.parametrize("n", [622592, 622595])
+def test_listing_at_the_edge_of_one_quad_per_thread(gpu_lib, n):
+    """304 blocks of 512 threads with four agents each, and three agents more."""
+    _equal_days(small_snapshot(n=n, locs=n // 5, initial_infected_frac=0.005), days=1)
